@@ -1,34 +1,24 @@
 // xw_anneal.cu -- the population annealing kernel for weighing matrices.
 //
-// One warp owns one replica at a time.  The replica's int8 W (column-major),
-// int32 Gram, row residuals, minority lists and row support masks live in the
-// warp's shared-memory slot; lane o owns "other" rows o, o+32, ... of every
-// O(n) delta, so a candidate's exact change to W W^T and to the score is one
-// pass over shared memory plus one redux.sync.  The whole iteration is
-// warp-synchronous: no __syncthreads, no block-wide reductions.
+// One warp (or a half-warp) owns one replica at a time, its state in the
+// warp's shared-memory slot; the whole iteration is warp-synchronous: no
+// __syncthreads, no block-wide reductions.  Orders up to 128 run on packed
+// rows (xw_packed.cuh); orders 129 to 256 keep G as int16 with one row per
+// lane and pass (run_replica_wide below).
 //
 // Per iteration (the semantics of the reference kernel anneal_kernel,
 // src/xweigh_cuda.cu:988-1130, with cuRAND replaced by counter-based Philox):
 //   A  every lane computes one Philox block of this iteration's draws
 //      (move-level block + the common blocks of the first candidates) into
 //      shared memory;
-//   C  8 lanes per candidate run the hot-row tournament (xweigh_cuda.cu:291-300)
-//      and a segmented max picks the first best sample;
-//   D  lane c proposes candidate c (propose_move, xweigh_cuda.cu:423-447);
-//   E  the warp evaluates the candidates in order and keeps the first best
-//      (device_better_evaluation, xweigh_cuda.cu:227-244);
+//   C  hot-row tournaments (xweigh_cuda.cu:291-300), 8 samples per candidate;
+//   D  proposals (propose_move, xweigh_cuda.cu:423-447);
+//   E  candidate evaluation, the first best kept (device_better_evaluation,
+//      xweigh_cuda.cu:227-244);
 //   F  Metropolis on the replica's objective with the integer draw and the
 //      deterministic acceptance exponential;
-//   G  the warp commits the move (commit_*, xweigh_cuda.cu:607-877);
+//   G  the commit (commit_*, xweigh_cuda.cu:607-877);
 //   H  best tracking, cooling and reheat (xweigh_cuda.cu:1087-1129).
-//
-// Every move kind changes at most two rows of W, and each changed Gram row
-// is old + a*W[:,x] + b*W[:,y] for two columns x, y; evaluation and commit
-// run that one form (plus the row1-row2 pair term of a double flip over two
-// rows), so the hot loop has one code path instead of one per move kind.
-// Instruction-cache misses, not arithmetic, bound this kernel when the
-// per-kind paths are specialised and inlined; the proposal helpers are kept
-// out of line for the same reason.
 //
 // Work distribution is persistent: each warp takes replica ids from a
 // global counter until the launch's item list is exhausted, so replicas of
@@ -41,24 +31,11 @@
 
 #include "xw_device.cuh"
 #include "xw_kernels.h"
+#include "xw_packed.cuh"
 
 namespace xw {
 
 namespace {
-
-constexpr unsigned FULL = 0xffffffffu;
-
-// Lane groups.  A replica is owned by a group of GW lanes: the whole warp
-// (GW = 32), or one half of it (GW = 16, orders up to 16: two replicas per
-// warp, each half with its own shared-memory slot and its own work items).
-// Warp collectives name only the group's lanes; the two halves' replicas
-// are independent and the hardware runs them side by side wherever their
-// control flow agrees.
-template <int GW>
-__device__ __forceinline__ unsigned group_mask() {
-    if constexpr (GW == 32) return FULL;
-    else return 0xffffu << (threadIdx.x & 16);
-}
 
 // Move statistics in the replica header (accepted moves, the rows they
 // changed, two-row candidate evaluations); a build with XW_MOVE_STATS=0
@@ -67,9 +44,6 @@ __device__ __forceinline__ unsigned group_mask() {
 #define XW_MOVE_STATS 1
 #endif
 constexpr bool kMoveStats = XW_MOVE_STATS != 0;
-
-// Metropolis thresholds kept per replica for objective increases 1..kThrTable.
-constexpr uint32_t kThrTable = 64;
 
 // Replica-constant fields the proposal code reads, kept in the warp's slot.
 struct View {
@@ -109,8 +83,6 @@ __host__ __device__ inline SlotLayout slot_layout(int n, int m, bool wide) {
     return L;
 }
 
-__device__ __forceinline__ int iabs(int v) { return v < 0 ? -v : v; }
-
 // First set bit at or after `start`, cyclically, of a 128-bit row mask.
 __device__ __forceinline__ int cyclic_first(uint64_t lo, uint64_t hi, int start) {
     const uint64_t a_lo = start < 64 ? (lo & (~0ull << start)) : 0ull;
@@ -145,13 +117,6 @@ template <int MW>
 __device__ __forceinline__ void row_mask(const uint64_t* mask, int row, uint64_t (&m)[MW]) {
 #pragma unroll
     for (int k = 0; k < MW; ++k) m[k] = mask[MW * row + k];
-}
-
-// Draw words outside the cached blocks (rare: attempts past the first,
-// tournaments past 8 samples, candidates past the cached ones).
-__device__ __noinline__ uint32_t slow_word(uint32_t slot, uint64_t it, uint32_t stream, uint32_t k0, uint32_t k1,
-                                           int j) {
-    return pick(draw_block(slot, it, stream, k0, k1), j);
 }
 
 __device__ __forceinline__ uint32_t word(const View* v, uint64_t it, int c, int b, int j) {
@@ -452,7 +417,7 @@ __device__ __forceinline__ Deltas eval_lane(const Update& u, const int8_t* W, co
 // commit_sign_flip / commit_support_switch / commit_double_sign_flip
 // (xweigh_cuda.cu:607-877) and the within-row swap, in the two-row form.
 template <int OPL, int MW, typename GT, bool GEN, int GW = 32>
-__device__ void commit(uint32_t d0, uint32_t d1, const Update& u, int ds, int8_t* W, GT* G, int32_t* res,
+__device__ void commit_wide(uint32_t d0, uint32_t d1, const Update& u, int ds, int8_t* W, GT* G, int32_t* res,
                        uint8_t* mino, uint64_t* mask, int n, int ld, int m, int sparse, int lane) {
     const unsigned gm = group_mask<GW>();
     int s1 = 0;
@@ -525,35 +490,6 @@ __device__ void commit(uint32_t d0, uint32_t d1, const Update& u, int ds, int8_t
     __syncwarp(gm);
 }
 
-// tab[d-1] = ceil(exp(-d/T) * 2^32), computed with the same division and
-// exponential as metropolis_accept, so that for a 32-bit draw u
-//   u * 2^-32 < exp(-d/T)  <=>  u < tab[d-1]
-// exactly (both sides scaled by 2^32 without rounding; u is an integer).
-// Rebuilt whenever the replica's temperature changes.
-template <int GW = 32>
-__device__ __noinline__ void build_thresholds(uint64_t* tab, double T, int lane) {
-    const double t = T > 1.0e-12 ? T : 1.0e-12;
-    for (uint32_t d = lane + 1; d <= kThrTable; d += GW) {
-        const double e = acceptance_exp(__ddiv_rn(-(double)d, t));
-        tab[d - 1] = (uint64_t)ceil(__dmul_rn(e, 0x1p32));
-    }
-    __syncwarp(group_mask<GW>());
-}
-
-template <int GW = 32>
-__device__ __forceinline__ void copy16(void* dst, const void* src, uint32_t bytes, int lane) {
-    const uint32_t chunks = xw_pad16(bytes) / 16u;
-    uint4* d = reinterpret_cast<uint4*>(dst);
-    const uint4* s = reinterpret_cast<const uint4*>(src);
-    for (uint32_t i = lane; i < chunks; i += GW) d[i] = s[i];
-}
-
-__device__ __forceinline__ uint64_t globaltimer() {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
 // Phase C: the hot-row tournaments of candidates 0..3 (hot_row,
 // xweigh_cuda.cu:291-300), 8 lanes (samples) per candidate with a segmented
 // maximum: one pass of a warp, two of a half-warp.  Returns the row of the
@@ -604,447 +540,6 @@ __device__ __forceinline__ int coop_hot_row(const uint32_t* sDw, const int32_t* 
     }
 }
 
-// A loaded replica: its shared-memory structures, the job's constants the
-// iteration reads, and the scalar state the loop carries.
-template <int OPL, int GW>
-struct Replica {
-    static constexpr int MW = OPL > 4 ? 4 : 2;
-    using GT = typename std::conditional<(OPL > 4), int16_t, int32_t>::type;
-    uint8_t* rec;
-    RepHeader* H;
-    XwJob* J;
-    int8_t* sW;
-    GT* sG;
-    int32_t* sRes;
-    uint8_t* sMino;
-    uint64_t* sMask;
-    uint64_t* sThr;
-    int n, w, m, sparse, ld, obj_kind;
-    uint32_t nn, status0;
-    // scalar state
-    uint64_t it, iters, moves, cand_evals;
-    uint32_t accepted, accepted_rows, two_row_evals;
-    int score, conflicts, best_s, best_c, msi, cool;
-    int64_t obj_total;
-    double T, reheat_T;
-    // the copy that writes the record (a cluster's other CTAs keep an
-    // identical copy in their own shared memory and write nothing)
-    bool owner;
-};
-
-// Loads replica `rid` into the slot: W and the minority lists, the masks,
-// Gram and residuals rebuilt from W and checked against the header.  False
-// when the replica does not run (job done or solved, budget spent, or a
-// failed self-check, which flags the header).  The group's lanes call it.
-// `owner` false: a copy that writes nothing to the record; it also skips
-// the exits on the job's done and solved flags, which other kernels may set
-// while it loads (its owner decides whether the replica runs).
-template <int OPL, bool GEN, int GW>
-__device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, uint8_t* slot, int lane,
-                                             uint64_t chunk_iters, Replica<OPL, GW>& R, bool owner = true) {
-    constexpr int MW = Replica<OPL, GW>::MW;
-    using GT = typename Replica<OPL, GW>::GT;
-    const unsigned gm = group_mask<GW>();
-    uint8_t* rec = a.arena + a.rec_off[rid];
-    RepHeader* H = reinterpret_cast<RepHeader*>(rec);
-    const uint32_t jid = H->job;
-    XwJob* J = a.jobs + jid;
-    R.owner = owner;
-    if (owner && *(volatile int32_t*)&J->done) return false;
-    if (owner && a.stop_on_solve == 1 && *(volatile int32_t*)&J->solved) return false;
-
-    // eight rows per lane: int16 Gram and 256-bit row masks (slot_layout)
-    const int n = J->n, w = J->w, m = J->m, sparse = J->sparse;
-    const SlotLayout L = slot_layout(n, m, OPL > 4);
-    const int ld = L.ld;
-    int8_t* sW = reinterpret_cast<int8_t*>(slot);
-    GT* sG = reinterpret_cast<GT*>(slot + L.off_g);
-    int32_t* sRes = reinterpret_cast<int32_t*>(slot + L.off_res);
-    uint8_t* sMino = slot + L.off_mino;
-    uint64_t* sMask = reinterpret_cast<uint64_t*>(slot + L.off_mask);
-
-    uint64_t it = H->it;
-    uint64_t iters = chunk_iters;
-    if (J->budget_iters) {
-        if (it >= J->budget_iters) return false;
-        if (iters > J->budget_iters - it) iters = J->budget_iters - it;
-    }
-
-    // ---- load W and the minority lists; rebuild masks, Gram, residuals ----
-    const uint32_t nn = (uint32_t)(n * n);
-    copy16<GW>(sW, rec + J->off_w, nn, lane);
-    const uint32_t status0 = H->status;
-    if (m > 0 && (status0 & XW_STATUS_INIT)) copy16<GW>(sMino, rec + J->off_mino, (uint32_t)(n * m), lane);
-    __syncwarp(gm);
-    int bad_rows = 0;
-#pragma unroll
-    for (int k = 0; k < OPL; ++k) {
-        const int o = lane + GW * k;
-        if (o < n) {
-            int pos = 0, weight = 0;
-#pragma unroll
-            for (int q = 0; q < MW; ++q) {
-                uint64_t word = 0;
-#pragma unroll 1
-                for (int c = 64 * q; c < n && c < 64 * q + 64; ++c) {
-                    const bool nz = sW[c * n + o] != 0;
-                    if (nz) word |= 1ull << (c & 63);
-                    if (m > 0 && !(status0 & XW_STATUS_INIT) && nz == (sparse != 0)) {
-                        if (pos < m) sMino[o * m + pos] = (uint8_t)c;
-                        ++pos;
-                    }
-                }
-                sMask[MW * o + q] = word;
-                weight += __popcll(word);
-            }
-            if (weight != w) bad_rows = 1;
-            if (m > 0 && !(status0 & XW_STATUS_INIT) && pos != m) bad_rows = 1;
-        }
-    }
-    if (__any_sync(gm, bad_rows)) {
-        if (lane == 0) H->err |= XW_ERR_MINORITY;
-        return false;
-    }
-    __syncwarp(gm);
-    int p_score = 0, p_conf = 0, p_par = 0;
-    long long p_sq = 0;
-#pragma unroll
-    for (int k = 0; k < OPL; ++k) {
-        const int o = lane + GW * k;
-        if (o < n) {
-            int r_sum = 0;
-#pragma unroll 1
-            for (int r = 0; r < n; ++r) {
-                int dot = 0;
-#pragma unroll 1
-                for (int c = 0; c < n; ++c) dot += sW[c * n + r] * sW[c * n + o];
-                sG[r * ld + o] = (GT)dot;
-                if (r != o) {
-                    const int ad = iabs(dot);
-                    r_sum += ad;
-                    p_conf += dot != 0;
-                    p_sq += (long long)(dot * dot);
-                    p_par += ad & 1;
-                }
-            }
-            sRes[o] = r_sum;
-            p_score += r_sum;
-        }
-    }
-    const int score0 = __reduce_add_sync(gm, p_score) / 2;
-    const int conf0 = __reduce_add_sync(gm, p_conf) / 2;
-#pragma unroll
-    for (int off = GW / 2; off > 0; off >>= 1) p_sq += __shfl_xor_sync(gm, p_sq, off, GW);
-    const long long sq0 = p_sq / 2;
-    const int par0 = __reduce_add_sync(gm, p_par) / 2;
-    __syncwarp(gm);
-
-    const int obj_kind = GEN ? H->obj_kind : 0;
-    if (!GEN && (H->obj_kind != 0 || J->move_set != 0)) {
-        // the lean kernel was launched for a replica that needs the general one
-        if (lane == 0) H->err |= XW_ERR_KERNEL;
-        return false;
-    }
-    const int64_t obj0 = obj_kind == 1 ? sq0 : obj_kind == 2 ? par0 : score0;
-    R.T = H->temperature;
-    R.reheat_T = H->reheat_temperature;
-    if (status0 & XW_STATUS_INIT) {
-        if (H->score != score0 || H->conflicts != conf0 || H->obj_total != obj0) {
-            if (lane == 0) H->err |= XW_ERR_SCORE;
-            return false;
-        }
-        R.best_s = H->best_score;
-        R.best_c = H->best_conflicts;
-        R.msi = H->msi;
-        R.cool = H->cool_ctr;
-        R.moves = H->moves;
-        R.cand_evals = H->cand_evals;
-        R.accepted = H->accepted;
-        R.accepted_rows = H->accepted_rows;
-        R.two_row_evals = H->two_row_evals;
-    } else {
-        R.best_s = score0;
-        R.best_c = conf0;
-        R.msi = 0;
-        R.cool = 0;
-        R.moves = 0;
-        R.cand_evals = 0;
-        R.accepted = 0;
-        R.accepted_rows = 0;
-        R.two_row_evals = 0;
-        if (owner) copy16<GW>(rec + J->off_best, sW, nn, lane);
-    }
-    R.score = score0;
-    R.conflicts = conf0;
-    R.obj_total = obj0;
-    R.rec = rec;
-    R.H = H;
-    R.J = J;
-    R.sW = sW;
-    R.sG = sG;
-    R.sRes = sRes;
-    R.sMino = sMino;
-    R.sMask = sMask;
-    R.sThr = reinterpret_cast<uint64_t*>(slot + L.off_thr);
-    R.n = n;
-    R.w = w;
-    R.m = m;
-    R.sparse = sparse;
-    R.ld = ld;
-    R.obj_kind = obj_kind;
-    R.nn = nn;
-    R.status0 = status0;
-    R.it = it;
-    R.iters = iters;
-    return true;
-}
-
-// Writes the replica's W, minority lists and scalar state back to its record.
-template <int OPL, int GW>
-__device__ __forceinline__ void store_replica(const Replica<OPL, GW>& R, int lane) {
-    const unsigned gm = group_mask<GW>();
-    __syncwarp(gm);
-    copy16<GW>(R.rec + R.J->off_w, R.sW, R.nn, lane);
-    if (R.m > 0) copy16<GW>(R.rec + R.J->off_mino, R.sMino, (uint32_t)(R.n * R.m), lane);
-    if (lane == 0) {
-        RepHeader* H = R.H;
-        H->it = R.it;
-        H->moves = R.moves;
-        H->cand_evals = R.cand_evals;
-        H->accepted = R.accepted;
-        H->accepted_rows = R.accepted_rows;
-        H->two_row_evals = R.two_row_evals;
-        H->score = R.score;
-        H->conflicts = R.conflicts;
-        H->best_score = R.best_s;
-        H->best_conflicts = R.best_c;
-        H->obj_total = R.obj_total;
-        H->temperature = R.T;
-        H->msi = R.msi;
-        H->cool_ctr = R.cool;
-        H->status = R.status0 | XW_STATUS_INIT | (R.best_s == 0 ? XW_STATUS_SOLVED : 0u);
-    }
-    __syncwarp(gm);
-}
-
-// The proposing side of an iteration: the job constants the draws and
-// proposals read, this group's draw buffer and View, and the lane's
-// cached-block slots and register context.
-template <int GW>
-struct Proposer {
-    uint4* sDraw;
-    const uint32_t* sDw;
-    View* sView;
-    Reg rg;
-    uint32_t my_slot, my_slot2;
-    uint32_t k0, k1, stream;
-    uint64_t thr_greedy;
-    int cs, ts, bpc;
-    bool coop;
-};
-
-// Sets up the proposer of a loaded replica with the draw buffer and View at
-// `draws` and `view` (the group's own).  The group's lanes call it.
-template <int OPL, int GW>
-__device__ __forceinline__ void setup_proposer(const Replica<OPL, GW>& R, uint4* draws, View* view, int lane,
-                                               Proposer<GW>& P) {
-    const XwJob* J = R.J;
-    const int n = R.n;
-    P.sDraw = draws;
-    P.sDw = reinterpret_cast<const uint32_t*>(draws);
-    P.sView = view;
-    P.cs = J->candidate_samples;
-    P.ts = J->target_samples;
-    P.k0 = J->key0;
-    P.k1 = J->key1;
-    P.stream = R.H->stream;
-    P.thr_greedy = J->thr_greedy;
-    P.bpc = 4 + (P.ts <= 4 ? 1 : 2);          // cached blocks per candidate
-    P.coop = P.ts <= 8;                       // cooperative hot-row tournament
-    if (lane == 0) {
-        View v;
-        v.W = R.sW; v.mino = R.sMino; v.res = R.sRes; v.mask = R.sMask; v.dw = P.sDw;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int lo = 64 * q;
-            v.valid[q] = n >= lo + 64 ? ~0ull : n <= lo ? 0ull : ((1ull << (n - lo)) - 1ull);
-        }
-        v.thr_target = J->thr_target; v.thr_dbl = J->thr_double; v.thr_sign = J->thr_sign;
-        v.thr_swsign = J->thr_swsign;
-        v.n = n; v.w = R.w; v.m = R.m; v.sparse = R.sparse; v.ts = P.ts; v.bpc = P.bpc; v.cc = 31 / P.bpc;
-        v.move_set = J->move_set;
-        v.stream = P.stream; v.k0 = P.k0; v.k1 = P.k1; v.pad = 0;
-        *view = v;
-    }
-    __syncwarp(group_mask<GW>());
-
-    // lane -> cached Philox blocks of an iteration (block 0 is the
-    // move-level block, 1 + c*bpc + b block b of candidate c); a half-warp
-    // group computes two blocks per lane
-    const int bpc = P.bpc;
-    P.my_slot = 0;
-    P.my_slot2 = 0;
-    if (lane > 0) {
-        const int q = lane - 1, c = q / bpc, b = q - c * bpc;
-        P.my_slot = cand_slot(c, b);
-    }
-    if constexpr (GW == 16) {
-        const int q = lane + 15, c = q / bpc, b = q - c * bpc;
-        P.my_slot2 = cand_slot(c, b);
-    }
-    // register context of candidate `lane` for the inlined proposal path
-    Reg& rg = P.rg;
-    rg.W = R.sW; rg.mino = R.sMino; rg.mask = R.sMask;
-    rg.cw = P.sDw + (1 + lane * bpc) * 4;
-    rg.cached = lane < 31 / bpc;
-    rg.thr_target = J->thr_target; rg.thr_dbl = J->thr_double; rg.thr_sign = J->thr_sign;
-    rg.thr_swsign = J->thr_swsign;
-    rg.n = n; rg.w = R.w; rg.m = R.m; rg.sparse = R.sparse; rg.move_set = J->move_set;
-    rg.stream = P.stream; rg.k0 = P.k0; rg.k1 = P.k1;
-}
-
-// The move an iteration puts to the Metropolis test: the first best of its
-// candidates (b0 = 0: none was valid), its deltas, the iteration's
-// acceptance draw and the number of candidates evaluated.
-struct Choice {
-    uint32_t b0, b1;
-    int bds, bdc, bprim;
-    uint32_t u;
-    uint32_t evals, evals2;   // candidates evaluated; those changing two rows
-};
-
-// Phases A-E of iteration `it` against the replica's current state: draws,
-// hot-row tournaments, proposals, and the evaluation of the candidates in
-// order.  Reads the state and writes only the group's draw buffer.
-template <int OPL, bool GEN, int GW>
-__device__ __forceinline__ Choice choose_move(const Replica<OPL, GW>& R, Proposer<GW>& P, uint64_t it, int lane) {
-    constexpr int MW = Replica<OPL, GW>::MW;
-    using GT = typename Replica<OPL, GW>::GT;
-    const unsigned gm = group_mask<GW>();
-    const int n = R.n, ts = P.ts, bpc = P.bpc;
-    const uint32_t k0 = P.k0, k1 = P.k1, stream = P.stream;
-    const uint32_t* sDw = P.sDw;
-    const int32_t* sRes = R.sRes;
-    // A: draws
-    P.sDraw[lane] = draw_block(P.my_slot, it, stream, k0, k1);
-    if constexpr (GW == 16) P.sDraw[lane + 16] = draw_block(P.my_slot2, it, stream, k0, k1);
-    __syncwarp(gm);
-    const uint4 mblk = P.sDraw[0];
-    const int count = (uint64_t)mblk.x < P.thr_greedy ? P.cs : 1;
-
-    // C: cooperative hot-row tournaments
-    const int coop_row = coop_hot_row<GW>(sDw, sRes, bpc, count, ts, P.coop, n, it, stream, k0, k1, lane);
-
-    // D: proposals, lane c proposes candidate c
-    uint2 desc = make_uint2(0u, 0u);
-    P.rg.it = it;
-    if (lane < count) desc = d_propose<MW, GEN>(P.rg, P.sView, lane, P.coop && lane < 4, coop_row);
-    __syncwarp(gm);
-
-    // E: evaluate in candidate order, keep the first best
-    Choice ch;
-    ch.b0 = 0; ch.b1 = 0; ch.bds = 0; ch.bdc = 0; ch.bprim = 0;
-    ch.u = mblk.y;
-    ch.evals = 0;
-    ch.evals2 = 0;
-#pragma unroll 1
-    for (int c = 0; c < count; ++c) {
-        const uint32_t e0 = __shfl_sync(gm, desc.x, c, GW);
-        const uint32_t e1 = __shfl_sync(gm, desc.y, c, GW);
-        if (!(e0 & 1u)) continue;
-        const Update u = decode(e0, e1, R.sW, n);
-        const Deltas d = eval_lane<OPL, GT, GEN, GW>(u, R.sW, R.sG, n, R.ld, lane);
-        const int packed = __reduce_add_sync(gm, d.ds * 4096 + d.dc);
-        const int dc = ((packed + 2048) & 4095) - 2048;
-        const int ds = (packed - dc) >> 12;
-        int prim = ds;
-        if (GEN) {
-            if (R.obj_kind == 1) prim = __reduce_add_sync(gm, d.dsq);
-            else if (R.obj_kind == 2) prim = __reduce_add_sync(gm, d.dpar);
-        }
-        ++ch.evals;
-        if constexpr (kMoveStats) ch.evals2 += u.R2 >= 0;
-        bool better = ch.b0 == 0;
-        if (!better) {
-            if (prim != ch.bprim) better = prim < ch.bprim;
-            else if (ds != ch.bds) better = ds < ch.bds;
-            else better = dc < ch.bdc;
-        }
-        if (better) {
-            ch.b0 = e0; ch.b1 = e1; ch.bds = ds; ch.bdc = dc; ch.bprim = prim;
-        }
-    }
-    return ch;
-}
-
-// Phases F-H of an iteration whose choice is valid: Metropolis on the
-// replica's objective, the commit of an accepted move, best tracking
-// (the best W copied to the record on improvement, the job's solve flag),
-// cooling and reheat.  Returns whether the move was accepted.  The group's
-// lanes call it.
-template <int OPL, bool GEN, int GW>
-__device__ __forceinline__ bool apply_move(Replica<OPL, GW>& R, const Choice& ch, int tempering, int mpc, int stuck,
-                                           double t_min, double cooling, double reheat, int lane) {
-    constexpr int MW = Replica<OPL, GW>::MW;
-    using GT = typename Replica<OPL, GW>::GT;
-    ++R.moves;
-    // F: Metropolis
-    bool accept = ch.bprim <= 0;
-    if (!accept)
-        accept = ch.bprim <= (int64_t)kThrTable ? (uint64_t)ch.u < R.sThr[ch.bprim - 1]
-                                                : metropolis_accept(ch.bprim, R.T, ch.u);
-
-    // G: commit
-    if (accept) {
-        const Update u = decode(ch.b0, ch.b1, R.sW, R.n);
-        commit<OPL, MW, GT, GEN, GW>(ch.b0, ch.b1, u, ch.bds, R.sW, R.sG, R.sRes, R.sMino, R.sMask, R.n, R.ld,
-                                     R.m, R.sparse, lane);
-        R.score += ch.bds;
-        R.conflicts += ch.bdc;
-        R.obj_total += ch.bprim;
-        if constexpr (kMoveStats) {
-            ++R.accepted;
-            R.accepted_rows += u.R2 >= 0 ? 2u : 1u;
-        }
-    }
-
-    // H: best tracking, cooling, reheat
-    if (R.score < R.best_s || (R.score == R.best_s && R.conflicts < R.best_c)) {
-        R.best_s = R.score;
-        R.best_c = R.conflicts;
-        R.msi = 0;
-        if (R.owner) copy16<GW>(R.rec + R.J->off_best, R.sW, R.nn, lane);
-        if (R.best_s == 0 && lane == 0 && R.owner) {
-            RepHeader* H = R.H;
-            XwJob* J = R.J;
-            H->solve_it = R.it;
-            H->solve_ns = globaltimer();
-            if (atomicCAS(&J->solved, 0, 1) == 0) {
-                J->solved_replica = (int32_t)H->stream;
-                J->solved_it = R.it;
-                J->solve_ns = H->solve_ns;
-            }
-        }
-    } else {
-        ++R.msi;
-    }
-    if (!tempering) {
-        const double T0 = R.T;
-        if (++R.cool >= mpc) {
-            R.cool = 0;
-            R.T = __dmul_rn(R.T, cooling);
-            if (R.T < t_min) R.T = t_min;
-        }
-        if (R.msi >= stuck) {
-            R.msi = 0;
-            R.T = __dmul_rn(R.reheat_T, reheat);
-            if (R.T < t_min) R.T = t_min;
-        }
-        if (R.T != T0) build_thresholds<GW>(R.sThr, R.T, lane);
-    }
-    return accept;
-}
-
 // The one-warp (or half-warp) replica loop.  Its phases A-H are those of
 // choose_move and apply_move above, written out in one body: as separate
 // functions, even inlined, they hold more values live across the loop and
@@ -1055,7 +550,7 @@ __device__ __forceinline__ bool apply_move(Replica<OPL, GW>& R, const Choice& ch
 // the order is NFIX as well.  A replica of another shape is flagged
 // (XW_ERR_KERNEL) and not annealed.
 template <int OPL, bool GEN, int GW = 32, bool ONEZ = false, int NFIX = 0>
-__device__ void run_replica(const AnnealArgs& a, uint32_t rid, uint8_t* slot, int lane, uint64_t chunk_iters) {
+__device__ void run_replica_wide(const AnnealArgs& a, uint32_t rid, uint8_t* slot, int lane, uint64_t chunk_iters) {
     const unsigned gm = group_mask<GW>();
     uint8_t* rec = a.arena + a.rec_off[rid];
     RepHeader* H = reinterpret_cast<RepHeader*>(rec);
@@ -1322,7 +817,7 @@ __device__ void run_replica(const AnnealArgs& a, uint32_t rid, uint8_t* slot, in
         // G: commit
         if (accept) {
             const Update u = decode(b0, b1, sW, n);
-            commit<OPL, MW, GT, GEN, GW>(b0, b1, u, bds, sW, sG, sRes, sMino, sMask, n, ld, m, sparse, lane);
+            commit_wide<OPL, MW, GT, GEN, GW>(b0, b1, u, bds, sW, sG, sRes, sMino, sMask, n, ld, m, sparse, lane);
             score += bds;
             conflicts += bdc;
             obj_total += bprim;
@@ -1392,6 +887,43 @@ __device__ void run_replica(const AnnealArgs& a, uint32_t rid, uint8_t* slot, in
 }
 
 // ---------------------------------------------------------------------------
+// The one-warp (or half-warp) replica loop.
+template <int WPL, bool GEN, int GW, bool ONEZ>
+__device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane,
+                                            uint64_t iters) {
+    const unsigned gm = group_mask<GW>();
+    Env E;
+    State S;
+    if (!load_replica<WPL, GEN, GW, ONEZ>(a, rid, slot, slot + Slot<WPL>::draws, lane, iters, E, S, true)) return;
+    const int tempering = S.J->tempering, mpc = S.J->moves_per_cool, stuck = S.J->stuck_threshold;
+    uint64_t left = iters, evals = 0, calls = 0;
+    uint32_t evals2 = 0;
+    bool stop = false;
+    // 32-bit counts within a block of iterations (a multiple of 64)
+    while (left > 0 && !stop) {
+        const uint32_t block = left < (1u << 24) ? (uint32_t)left : 1u << 24;
+        uint32_t cand_l = 0, two_l = 0, k = 0;
+#pragma unroll 1
+        for (; k < block; ++k) {
+            // 1: every replica of the job stops soon after any solve;
+            // 2: a replica stops at its own solve only, so that each replica's
+            //    trajectory is independent of how the launches are scheduled
+            if (a.stop_on_solve) {
+                stop = S.best_s == 0 || (a.stop_on_solve == 1 && (k & 63) == 63 && *(volatile int32_t*)&S.J->solved);
+                if (stop) break;
+            }
+            Pick P = choose<WPL, GEN, GW, ONEZ>(E, S.it, lane, cand_l, two_l);
+            apply<WPL, GEN, GW, ONEZ>(E, S, P, accepts<WPL>(E, P), tempering, mpc, stuck, lane);
+            ++S.it;
+        }
+        left -= k;
+        calls += k;
+        evals += __reduce_add_sync(gm, E.l == 0 ? cand_l : 0u);
+        evals2 += __reduce_add_sync(gm, E.l == 0 ? two_l : 0u);
+    }
+    store_replica<WPL, GW>(E, S, calls, evals, evals2, lane);
+}
+
 // Latency mode: one replica per CTA of K warps, speculating K iterations at
 // a time.  Warp k computes iteration it + k (phases A-E) against the
 // replica's current state, each with its own draw buffer: the draws of an
@@ -1406,44 +938,38 @@ __device__ void run_replica(const AnnealArgs& a, uint32_t rid, uint8_t* slot, in
 // the time of one iteration, so a lone search runs that much faster.
 
 // Per-warp results and the round's control word, after the slot's own
-// (warp 0's) structures and the other warps' draw buffers and Views.
+// (warp 0's) structures and the other warps' draw buffers.
 struct SpecOut {
-    Choice ch;
+    Move mv;
+    int32_t ds, dc, prim;
+    uint32_t u;
+    uint32_t evals, evals2;   // candidates evaluated; those changing two rows
     int32_t acc;        // the Metropolis outcome at the round's starting temperature
-    int32_t pad;
 };
 struct SpecCtl {
     uint64_t it;        // first iteration of the round
     int32_t count;      // iterations of the round (0: the replica stops)
     int32_t pad;
-    double T;           // the temperature at the round's start
 };
 
 // Per round buffer (two, used in turn): the outcomes of all the round's
 // warps (K per CTA, CL CTAs), and the job's solved flag as the cluster's
 // owner read it.
 struct SpecLayout {
-    SlotLayout L;
-    uint32_t off_extra, per_warp, off_out, out_stride, off_flag, off_ctl, bytes;
+    uint32_t off_extra, off_out, out_stride, off_flag, off_ctl, bytes;
 };
 
 // the latency-mode regions after a slot of `slot_bytes` (the one-warp
-// layout of the replica, or the largest of a launch's replicas), for K
-// warps per CTA and CL CTAs per replica
-__host__ __device__ inline void spec_regions(uint32_t slot_bytes, int K, int CL, SpecLayout& S) {
-    S.per_warp = 32u * 16u + xw_pad16((uint32_t)sizeof(View));
+// layout of the largest of a launch's replicas), for K warps per CTA and
+// CL CTAs per replica
+__host__ __device__ inline SpecLayout spec_layout(uint32_t slot_bytes, int K, int CL) {
+    SpecLayout S;
     S.off_extra = xw_pad16(slot_bytes);
-    S.off_out = S.off_extra + (uint32_t)(K - 1) * S.per_warp;
+    S.off_out = S.off_extra + (uint32_t)(K - 1) * 512u;
     S.out_stride = xw_pad16((uint32_t)(K * CL) * (uint32_t)sizeof(SpecOut));
     S.off_flag = S.off_out + 2u * S.out_stride;
     S.off_ctl = xw_pad16(S.off_flag + 2u * 4u);
     S.bytes = S.off_ctl + (uint32_t)sizeof(SpecCtl);
-}
-
-__host__ __device__ inline SpecLayout spec_layout(int n, int m, int K, int CL) {
-    SpecLayout S;
-    S.L = slot_layout(n, m, false);
-    spec_regions(S.L.bytes, K, CL, S);
     return S;
 }
 
@@ -1457,39 +983,35 @@ __host__ __device__ inline SpecLayout spec_layout(int n, int m, int K, int CL) {
 // CTAs' identical state or read by rank 0 alone and exchanged (whether
 // the replica runs at all, and the job's solved flag each round), so the
 // CTAs take the same branches and meet at every barrier.
-template <bool GEN, int CL>
-__device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slot, int warp, int K, int lane) {
+template <int WPL, bool GEN, int CL>
+__device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, int K, int lane) {
     namespace cg = cooperative_groups;
     const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
     const bool owner = rank == 0;
-    SpecCtl* ctl = nullptr;
-    Replica<1, 32> R;
+    const XwJob* J = a.jobs + reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid])->job;
+    const SpecLayout L = spec_layout(packed_slot_bytes(J->n, J->m, WPL), K, CL);
+    SpecCtl* ctl = reinterpret_cast<SpecCtl*>(xw_smem + L.off_ctl);
+    Env E;
+    State S;
     bool ok = false;
+    uint64_t iters = a.iters;
     // warp 0 loads the replica; the round size goes to the others through
     // shared memory
-    if (warp == 0) ok = load_replica<1, GEN, 32>(a, rid, slot, lane, a.iters, R, owner);
-    // every warp reads the order to find the layout
-    const XwJob* J = a.jobs + reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid])->job;
-    const SpecLayout S = spec_layout(J->n, J->m, K, CL);
-    ctl = reinterpret_cast<SpecCtl*>(slot + S.off_ctl);
+    if (warp == 0) ok = load_replica<WPL, GEN, 32, false>(a, rid, 0u, Slot<WPL>::draws, lane, iters, E, S, owner);
     const int tempering = J->tempering;
     const int mpc = J->moves_per_cool, stuck = J->stuck_threshold;
-    const double t_min = J->t_min, cooling = J->cooling, reheat = J->reheat;
     const int KT = K * CL;
-    uint64_t done = 0;
-    if (warp == 0) {
-        if (ok) build_thresholds<32>(R.sThr, R.T, lane);
-        if (lane == 0 && owner) {
-            SpecCtl c;
-            c.it = ok ? R.it : 0;
-            c.T = ok ? R.T : 0.0;
-            c.pad = 0;
-            const bool stop = !ok || R.iters == 0 || (a.stop_on_solve && R.best_s == 0);
-            c.count = stop ? 0 : (int32_t)(R.iters < (uint64_t)KT ? R.iters : (uint64_t)KT);
-            *ctl = c;
-            if constexpr (CL > 1) {
-                for (int q = 1; q < CL; ++q) *cg::this_cluster().map_shared_rank(ctl, q) = c;
-            }
+    uint64_t done = 0, evals = 0, calls = 0;
+    uint32_t evals2 = 0;
+    if (warp == 0 && lane == 0 && owner) {
+        SpecCtl c;
+        c.it = ok ? S.it : 0;
+        c.pad = 0;
+        const bool stop = !ok || iters == 0 || (a.stop_on_solve && S.best_s == 0);
+        c.count = stop ? 0 : (int32_t)(iters < (uint64_t)KT ? iters : (uint64_t)KT);
+        *ctl = c;
+        if constexpr (CL > 1) {
+            for (int q = 1; q < CL; ++q) *cg::this_cluster().map_shared_rank(ctl, q) = c;
         }
     }
     if constexpr (CL > 1) cg::this_cluster().sync();
@@ -1497,57 +1019,44 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slo
     if (ctl->count == 0) {
         // nothing to run: the loaded replica's record still gets its
         // rebuilt state, as the one-warp kernel writes it
-        if (warp == 0 && ok && owner) store_replica<1, 32>(R, lane);
+        if (warp == 0 && ok && owner) store_replica<WPL, 32>(E, S, 0, 0, 0, lane);
         return;
     }
     // every warp: the replica's structures (read-only until warp 0 commits)
-    // and its own proposer
+    // and its own draw buffer
     if (warp != 0) {
-        const SlotLayout& L = S.L;
-        R.J = const_cast<XwJob*>(J);
-        R.rec = a.arena + a.rec_off[rid];
-        R.H = reinterpret_cast<RepHeader*>(R.rec);
-        R.n = J->n; R.w = J->w; R.m = J->m; R.sparse = J->sparse; R.ld = L.ld;
-        R.obj_kind = GEN ? R.H->obj_kind : 0;
-        R.owner = owner;
-        R.sW = reinterpret_cast<int8_t*>(slot);
-        R.sG = reinterpret_cast<int32_t*>(slot + L.off_g);
-        R.sRes = reinterpret_cast<int32_t*>(slot + L.off_res);
-        R.sMino = slot + L.off_mino;
-        R.sMask = reinterpret_cast<uint64_t*>(slot + L.off_mask);
-        R.sThr = reinterpret_cast<uint64_t*>(slot + L.off_thr);
+        const RepHeader* H = reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid]);
+        make_env<WPL, 32, false>(E, J, H, 0u, L.off_extra + (uint32_t)(warp - 1) * 512u, lane, GEN ? H->obj_kind : 0);
     }
-    uint8_t* mine = warp == 0 ? slot + S.L.off_draws : slot + S.off_extra + (uint32_t)(warp - 1) * S.per_warp;
-    View* view = warp == 0 ? reinterpret_cast<View*>(slot + S.L.off_view)
-                           : reinterpret_cast<View*>(mine + 32u * 16u);
-    Proposer<32> P;
-    setup_proposer<1, 32>(R, reinterpret_cast<uint4*>(mine), view, lane, P);
 
     const int g = rank * K + warp;   // this warp's iteration within the round
 #pragma unroll 1
     for (int round = 0;; ++round) {
         const int buf = round & 1;
-        SpecOut* outs = reinterpret_cast<SpecOut*>(slot + S.off_out + (uint32_t)buf * S.out_stride);
-        int32_t* flag = reinterpret_cast<int32_t*>(slot + S.off_flag) + buf;
+        SpecOut* outs = reinterpret_cast<SpecOut*>(xw_smem + L.off_out + (uint32_t)buf * L.out_stride);
+        int32_t* flag = reinterpret_cast<int32_t*>(xw_smem + L.off_flag) + buf;
         const uint64_t it0 = ctl->it;
         const int cnt = ctl->count;
         if (g < cnt) {
-            const Choice ch = choose_move<1, GEN, 32>(R, P, it0 + (uint64_t)g, lane);
+            uint32_t cand_l = 0, two_l = 0;
+            const Pick P = choose<WPL, GEN, 32, false>(E, it0 + (uint64_t)g, lane, cand_l, two_l);
+            SpecOut o;
+            o.mv.rc = __shfl_sync(FULL, P.mv.rc, P.src);
+            o.mv.cf = __shfl_sync(FULL, P.mv.cf, P.src);
+            o.mv.ax = __shfl_sync(FULL, P.mv.ax, P.src);
+            o.ds = P.ds;
+            o.dc = P.dc;
+            o.prim = P.prim;
+            o.u = P.u;
+            // both counts in one sum (at most 32 candidates)
+            const uint32_t ev = __reduce_add_sync(FULL, E.l == 0 ? cand_l + (two_l << 16) : 0u);
+            o.evals = ev & 0xffffu;
+            o.evals2 = ev >> 16;
             // the Metropolis test at the round's starting temperature: the
             // one warp 0 would make if no cooling or reheat step falls
             // between the round's start and this iteration
-            bool acc = false;
-            if (ch.b0) {
-                acc = ch.bprim <= 0;
-                if (!acc)
-                    acc = ch.bprim <= (int64_t)kThrTable ? (uint64_t)ch.u < R.sThr[ch.bprim - 1]
-                                                         : metropolis_accept(ch.bprim, ctl->T, ch.u);
-            }
+            o.acc = accepts<WPL>(E, P) ? 1 : 0;
             if (lane == 0) {
-                SpecOut o;
-                o.ch = ch;
-                o.acc = acc ? 1 : 0;
-                o.pad = 0;
                 outs[g] = o;
                 if constexpr (CL > 1) {
                     for (int q = 0; q < CL; ++q)
@@ -1557,7 +1066,7 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slo
         }
         if constexpr (CL > 1) {
             if (owner && warp == 0 && lane == 0) {
-                const int32_t sv = a.stop_on_solve == 1 ? *(volatile int32_t*)&R.J->solved : 0;
+                const int32_t sv = a.stop_on_solve == 1 ? *(volatile int32_t*)&S.J->solved : 0;
                 for (int q = 0; q < CL; ++q) *cg::this_cluster().map_shared_rank(flag, q) = sv;
             }
             cg::this_cluster().sync();
@@ -1569,37 +1078,34 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slo
             // the rejected calls before it change only counters (moves, msi,
             // cool) unless one of them reaches a cooling or reheat step, so
             // when none can, they are counted in bulk and only the accepted
-            // move goes through apply_move.  Otherwise the ordered walk.
+            // move goes through apply.  Otherwise the ordered walk.
             // The job's solved flag: read here on one CTA, as the owner read
             // it this round on a cluster.
             auto solved = [&]() -> bool {
                 if constexpr (CL > 1) return *flag != 0;
-                else return *(volatile int32_t*)&R.J->solved != 0;
+                else return *(volatile int32_t*)&S.J->solved != 0;
+            };
+            auto outcome = [&](int q) -> Pick {
+                const SpecOut& o = outs[q];
+                Pick P;
+                P.mv = o.mv;
+                P.src = lane;   // every lane holds the move
+                P.ds = o.ds;
+                P.dc = o.dc;
+                P.prim = o.prim;
+                P.u = o.u;
+                return P;
             };
             // lane l holds the outcomes of iterations l and 32 + l (up to 64
             // iterations a round, on a cluster of four)
-            Choice cl0 = {}, cl1 = {};
-            int al0 = 0, al1 = 0;
-            if (lane < cnt) {
-                cl0 = outs[lane].ch;
-                al0 = outs[lane].acc;
-            }
-            if (32 + lane < cnt) {
-                cl1 = outs[32 + lane].ch;
-                al1 = outs[32 + lane].acc;
-            }
-            const uint64_t have_m = (uint64_t)__ballot_sync(FULL, cl0.b0 != 0) |
-                                    ((uint64_t)__ballot_sync(FULL, cl1.b0 != 0) << 32);
-            const uint64_t acc_m = (uint64_t)__ballot_sync(FULL, cl0.b0 != 0 && al0 != 0) |
-                                   ((uint64_t)__ballot_sync(FULL, cl1.b0 != 0 && al1 != 0) << 32);
-            // calls (iterations with a candidate) that leave the temperature
-            // unchanged: fewer than `room`
-            const int room = tempering ? 0x7fffffff : min(mpc - R.cool, stuck - R.msi);
+            const bool l0 = lane < cnt, l1 = 32 + lane < cnt;
+            const uint64_t acc_m = (uint64_t)__ballot_sync(FULL, l0 && outs[l0 ? lane : 0].acc != 0) |
+                                   ((uint64_t)__ballot_sync(FULL, l1 && outs[l1 ? 32 + lane : 0].acc != 0) << 32);
+            // calls that leave the temperature unchanged: fewer than `room`
+            const int room = tempering ? 0x7fffffff : min(mpc - S.cool, stuck - S.msi);
             const int ja = acc_m ? __ffsll((long long)acc_m) - 1 : -1;
             const int jend = ja >= 0 ? ja + 1 : cnt;
-            const uint64_t span = jend >= 64 ? ~0ull : ((1ull << jend) - 1ull);
-            const int calls = __popcll(have_m & span);
-            const int rejects = ja >= 0 ? calls - 1 : calls;
+            const int rejects = ja >= 0 ? jend - 1 : jend;
             bool fast = rejects < room;
             // a check of the job's solved flag (every 64th iteration) that
             // falls in the span and finds it set: take the span in order
@@ -1607,19 +1113,19 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slo
             int j = 0;
             bool stop = false;
             if (fast) {
-                const bool in0 = (span >> lane) & 1ull, in1 = (span >> (32 + lane)) & 1ull;
-                R.cand_evals += __reduce_add_sync(FULL, (in0 ? cl0.evals : 0u) + (in1 ? cl1.evals : 0u));
-                R.two_row_evals += __reduce_add_sync(FULL, (in0 ? cl0.evals2 : 0u) + (in1 ? cl1.evals2 : 0u));
-                R.moves += (uint64_t)rejects;
-                R.msi += rejects;
-                if (!tempering) R.cool += rejects;
+                const bool in0 = lane < jend, in1 = 32 + lane < jend;
+                const uint32_t ev = __reduce_add_sync(FULL, (in0 ? outs[lane].evals + (outs[lane].evals2 << 16) : 0u) +
+                                                                (in1 ? outs[32 + lane].evals + (outs[32 + lane].evals2 << 16) : 0u));
+                evals += ev & 0xffffu;
+                evals2 += ev >> 16;
+                calls += (uint64_t)jend;
+                S.msi += rejects;
+                if (!tempering) S.cool += rejects;
+                S.it += (uint64_t)rejects;
                 if (ja >= 0) {
-                    R.it += (uint64_t)ja;
-                    const Choice ch = outs[ja].ch;
-                    apply_move<1, GEN, 32>(R, ch, tempering, mpc, stuck, t_min, cooling, reheat, lane);
-                    ++R.it;
-                } else {
-                    R.it += (uint64_t)cnt;
+                    Pick P = outcome(ja);
+                    apply<WPL, GEN, 32, false>(E, S, P, true, tempering, mpc, stuck, lane);
+                    ++S.it;
                 }
                 j = jend;
             } else {
@@ -1629,16 +1135,13 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slo
                         stop = true;
                         break;
                     }
-                    const Choice ch = outs[j].ch;
-                    R.cand_evals += ch.evals;
-                    R.two_row_evals += ch.evals2;
-                    if (!ch.b0) {
-                        ++R.it;
-                        continue;
-                    }
-                    const bool accept =
-                        apply_move<1, GEN, 32>(R, ch, tempering, mpc, stuck, t_min, cooling, reheat, lane);
-                    ++R.it;
+                    evals += outs[j].evals;
+                    evals2 += outs[j].evals2;
+                    ++calls;
+                    Pick P = outcome(j);
+                    const bool accept = accepts<WPL>(E, P);
+                    apply<WPL, GEN, 32, false>(E, S, P, accept, tempering, mpc, stuck, lane);
+                    ++S.it;
                     if (accept) {
                         ++j;
                         break;
@@ -1646,93 +1149,89 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, uint8_t* slo
                 }
             }
             done += (uint64_t)j;
-            if (a.stop_on_solve && R.best_s == 0) stop = true;
+            if (a.stop_on_solve && S.best_s == 0) stop = true;
             if (lane == 0) {
-                ctl->it = R.it;
-                ctl->T = R.T;
-                const uint64_t left = R.iters - done;
+                ctl->it = S.it;
+                const uint64_t left = iters - done;
                 ctl->count = stop || left == 0 ? 0 : (int32_t)(left < (uint64_t)KT ? left : (uint64_t)KT);
             }
         }
         __syncthreads();
         if (ctl->count == 0) break;
     }
-    if (warp == 0 && owner) store_replica<1, 32>(R, lane);
+    if (warp == 0 && owner) store_replica<WPL, 32>(E, S, calls, evals, evals2, lane);
     // the other CTAs' copies stay in their shared memory until every CTA
     // of the cluster has made its last remote write into this one
     if constexpr (CL > 1) cg::this_cluster().sync();
 }
 
 // Register budget per thread; it sets how many replica warps an SM holds.
-// An SM's registers are split between its four schedulers (16384 each), so
-// 128 registers per thread give 4 warps per scheduler and 96 give 5.  The
-// lean one-row-per-lane kernel gains from the fifth warp (W(26,25) with
-// 4096 replicas: 0.82 -> 0.87 G moves/s); the general and the wider kernels
-// lose more to the spills of a 96-register budget than they gain (measured
-// 6-18% slower), and keep 128.
+// An SM's registers are split between its four schedulers (16384 each): 64
+// registers per thread give 8 warps per scheduler, 80 give 6, 128 give 4.
+// Orders above 32 are held back by shared memory before registers.
 #ifndef XW_ANNEAL_MAXNREG
 #define XW_ANNEAL_MAXNREG 128
 #endif
 #ifndef XW_ANNEAL_MAXNREG_LEAN1
-#define XW_ANNEAL_MAXNREG_LEAN1 96
+#define XW_ANNEAL_MAXNREG_LEAN1 64
+#endif
+#ifndef XW_ANNEAL_MAXNREG_GEN1
+#define XW_ANNEAL_MAXNREG_GEN1 80
 #endif
 #ifndef XW_ANNEAL_MAXNREG_PAIR
-#define XW_ANNEAL_MAXNREG_PAIR 96
+#define XW_ANNEAL_MAXNREG_PAIR 80
 #endif
 constexpr int anneal_maxnreg(int opl, bool general, int gw) {
     return gw == 16 ? XW_ANNEAL_MAXNREG_PAIR
-                    : opl == 1 && !general ? XW_ANNEAL_MAXNREG_LEAN1 : XW_ANNEAL_MAXNREG;
+                    : opl == 1 ? (general ? XW_ANNEAL_MAXNREG_GEN1 : XW_ANNEAL_MAXNREG_LEAN1) : XW_ANNEAL_MAXNREG;
 }
 // Each lane group (the warp, or each half of it) takes work items from the
 // launch's counter on its own: a replica (all of its launch iterations) or
 // one chunk of them.
-template <int OPL, bool GEN, int GW, bool ONEZ = false, int NFIX = 0>
+template <int OPL, bool GEN, int GW, bool ONEZ = false>
 __global__ void __maxnreg__(anneal_maxnreg(OPL, GEN, GW)) anneal_kernel(AnnealArgs a) {
-    extern __shared__ __align__(16) uint8_t smem[];
     const int lane = threadIdx.x & (GW - 1);
     const int group = threadIdx.x / GW;
     const unsigned gm = group_mask<GW>();
-    uint8_t* slot = smem + (size_t)group * a.slot_bytes;
+    const uint32_t slot = (uint32_t)group * a.slot_bytes;
     const uint64_t total = (uint64_t)a.n_items * a.chunks;
     for (;;) {
         uint32_t item = 0;
         if (lane == 0) item = atomicAdd(a.counter, 1u);
         item = __shfl_sync(gm, item, 0, GW);
         if (item >= total) break;
-        if (a.chunks == 1) {
-            run_replica<OPL, GEN, GW, ONEZ, NFIX>(a, a.items[item], slot, lane, a.iters);
-            continue;
-        }
-        const uint32_t c = item / a.n_items;
+        // chunk c of the replica's launch iterations (one chunk: all of them)
+        const uint32_t c = a.chunks == 1 ? 0u : item / a.n_items;
         const uint32_t rid = a.items[item - c * a.n_items];
         const uint64_t lo = a.iters * c / a.chunks, hi = a.iters * (c + 1) / a.chunks;
         RepHeader* H = reinterpret_cast<RepHeader*>(a.arena + a.rec_off[rid]);
-        const bool ok = chunk_begin(a.chunk_done + rid, c, a.chunk_wait_ns, &H->err, lane, gm);
-        if (ok) run_replica<OPL, GEN, GW, ONEZ, NFIX>(a, rid, slot, lane, hi - lo);
-        chunk_end(a.chunk_done + rid, c, ok, lane, gm);
+        const bool chunked = a.chunks > 1;
+        const bool ok = !chunked || chunk_begin(a.chunk_done + rid, c, a.chunk_wait_ns, &H->err, lane, gm);
+        if (ok) {
+            if constexpr (OPL == 8) run_replica_wide<8, GEN>(a, rid, xw_smem + slot, lane, hi - lo);
+            else run_replica<OPL, GEN, GW, ONEZ>(a, rid, slot, lane, hi - lo);
+        }
+        if (chunked) chunk_end(a.chunk_done + rid, c, ok, lane, gm);
     }
 }
 
-// Latency mode: each CTA of K warps owns one replica at a time (orders up
-// to 32), taken from the launch's counter.
 // The latency mode: one CTA (CL = 1, a persistent loop over the launch's
 // replicas) or one cluster of CL CTAs (one replica per cluster) per replica.
 template <bool GEN, int CL>
 __global__ void __launch_bounds__(512, 1) anneal_spec_kernel(AnnealArgs a, int K) {
-    extern __shared__ __align__(16) uint8_t smem[];
     __shared__ uint32_t s_item;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     if constexpr (CL > 1) {
         const uint32_t item = blockIdx.x / CL;
-        if (item < a.n_items) run_replica_spec<GEN, CL>(a, a.items[item], smem, warp, K, lane);
+        if (item < a.n_items) run_replica_spec<1, GEN, CL>(a, a.items[item], warp, K, lane);
     } else {
         for (;;) {
             if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1u);
             __syncthreads();
             const uint32_t item = s_item;
             if (item >= a.n_items) break;
-            run_replica_spec<GEN, 1>(a, a.items[item], smem, warp, K, lane);
+            run_replica_spec<1, GEN, 1>(a, a.items[item], warp, K, lane);
             __syncthreads();
         }
     }
@@ -1865,40 +1364,18 @@ __global__ void stamp_kernel(uint64_t* t) { *t = globaltimer(); }
 
 }  // namespace
 
-uint32_t anneal_slot_bytes(int n, int m, int opl) { return slot_layout(n, m, opl > 4).bytes; }
-
-int anneal_opl(int n) { return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 4 : 8; }
-
-template <int N>
-const void* one_zero_order_fn() {
-    return reinterpret_cast<const void*>(&anneal_kernel<1, false, 32, true, N>);
+uint32_t anneal_slot_bytes(int n, int m, int opl) {
+    return opl > 4 ? slot_layout(n, m, true).bytes : packed_slot_bytes(n, m, opl);
 }
 
-// the one-zero kernel compiled for one order: the even orders 6..26 (W(n, n-1)
-// does not exist for odd n), nullptr for the others.  28, 30 and 32 compile
-// with 380 bytes of spills a thread (40 for the kernel of any order) and are
-// left to that kernel.
-const void* one_zero_fixed_fn(int n) {
-    switch (n) {
-    case 6: return one_zero_order_fn<6>();
-    case 8: return one_zero_order_fn<8>();
-    case 10: return one_zero_order_fn<10>();
-    case 12: return one_zero_order_fn<12>();
-    case 14: return one_zero_order_fn<14>();
-    case 16: return one_zero_order_fn<16>();
-    case 18: return one_zero_order_fn<18>();
-    case 20: return one_zero_order_fn<20>();
-    case 22: return one_zero_order_fn<22>();
-    case 24: return one_zero_order_fn<24>();
-    case 26: return one_zero_order_fn<26>();
-    default: return nullptr;
-    }
-}
+// rows per lane; W(128,128) has off-diagonal Gram entries of +-128, which a
+// signed byte does not hold, and takes the 16-bit kernel of the orders above
+int anneal_opl(int n, int w) { return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 && w < 128 ? 4 : 8; }
 
-const void* anneal_kernel_fn(int opl, bool general, int rpw, bool one_zero, int fixed_order) {
-    if (one_zero && opl == 1 && !general && rpw == 1) {
-        if (const void* f = fixed_order > 0 ? one_zero_fixed_fn(fixed_order) : nullptr) return f;
-        return reinterpret_cast<const void*>(&anneal_kernel<1, false, 32, true>);
+const void* anneal_kernel_fn(int opl, bool general, int rpw, bool one_zero) {
+    if (one_zero && opl == 1 && rpw == 1) {
+        return general ? reinterpret_cast<const void*>(&anneal_kernel<1, true, 32, true>)
+                       : reinterpret_cast<const void*>(&anneal_kernel<1, false, 32, true>);
     }
     if (rpw == 2) {
         return general ? reinterpret_cast<const void*>(&anneal_kernel<1, true, 16>)
@@ -1922,16 +1399,14 @@ cudaError_t launch_anneal(const AnnealArgs& args, int opl, bool general, int war
     const size_t smem = (size_t)warps_per_block * rpw * args.slot_bytes;
     const dim3 grid(blocks), block(32 * warps_per_block);
     void* kargs[] = {const_cast<AnnealArgs*>(&args)};
-    return cudaLaunchKernel(anneal_kernel_fn(opl, general, rpw, args.one_zero != 0, args.fixed_order), grid, block,
+    return cudaLaunchKernel(anneal_kernel_fn(opl, general, rpw, args.one_zero != 0), grid, block,
                             kargs, smem, stream);
 }
 
 // wpr warps per replica on `ctas` CTAs (1, 2 or 4; a cluster above 1) of
 // wpr / ctas warps each
 uint32_t anneal_spec_cta_bytes(uint32_t slot_bytes, int wpr, int ctas) {
-    SpecLayout S;
-    spec_regions(slot_bytes, wpr / ctas, ctas, S);
-    return S.bytes;
+    return spec_layout(slot_bytes, wpr / ctas, ctas).bytes;
 }
 
 const void* anneal_spec_kernel_fn(bool general, int ctas) {

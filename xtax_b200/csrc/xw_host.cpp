@@ -477,7 +477,7 @@ void Batch::derive_layout() {
     uint32_t pair_count = 0, one_row_count = 0;
     for (uint32_t i = n_large; i < total_replicas; ++i) {
         const XwJob& J = jobs[job_of[items[i]]];
-        const int kind = tune_kind(J.n, J.candidate_samples);
+        const int kind = tune_kind(J.n, J.w, J.candidate_samples);
         pair_count += kind == kTunePairKind;
         one_row_count += kind == 1;
     }
@@ -486,16 +486,16 @@ void Batch::derive_layout() {
     classes.clear();
     for (uint32_t i = n_large; i < total_replicas; ++i) {
         const XwJob& J = jobs[job_of[items[i]]];
-        int kind = tune_kind(J.n, J.candidate_samples);
+        int kind = tune_kind(J.n, J.w, J.candidate_samples);
         if (kind == kTunePairKind && !split_pair_class) {
             int rpw = params.replicas_per_warp;
             if (rpw == 0) rpw = tuned_shape(kTunePairKind, anneal_slot_bytes(J.n, J.m, 1), params.device).rpw;
-            if (rpw == 1 || (merge_pairs && params.replicas_per_warp != 2)) kind = anneal_opl(J.n);
+            if (rpw == 1 || (merge_pairs && params.replicas_per_warp != 2)) kind = anneal_opl(J.n, J.w);
         }
         if (classes.empty() || classes.back().kind != kind) {
             LaunchClass c;
             c.kind = kind;
-            c.opl = anneal_opl(J.n);
+            c.opl = anneal_opl(J.n, J.w);
             c.min_n = c.max_n = J.n;
             c.item_begin = i;
             classes.push_back(c);
@@ -855,7 +855,7 @@ bool Batch::configure_class(size_t k, int wpb, int rpw) {
     if (rpw == 2 && c.kind != kTunePairKind) return false;
     c.wpr = 1;
     c.ctas = 1;
-    const void* fn = anneal_kernel_fn(c.opl, c.general, rpw, c.one_zero, c.min_n == c.max_n ? c.min_n : 0);
+    const void* fn = anneal_kernel_fn(c.opl, c.general, rpw, c.one_zero);
     raise_smem_limit(fn, params.device);
     const size_t smem = (size_t)wpb * rpw * c.slot_bytes;
     int per_sm = 0;
@@ -978,7 +978,6 @@ void Batch::enqueue_rounds(uint64_t iters, bool timed) {
             ca.slot_bytes = c.slot_bytes;
             ca.counter = counters + l;
             ca.one_zero = c.one_zero ? 1 : 0;
-            ca.fixed_order = c.one_zero && c.min_n == c.max_n ? c.min_n : 0;
             ca.chunks = ca.iters >= c.chunks ? c.chunks : 1;
             if (ca.chunks > 1) ca.chunk_done = static_cast<uint32_t*>(d_chunk_done);
             cudaStream_t st = on(l);
@@ -1937,13 +1936,13 @@ int32_t xw_run(int32_t n, int32_t w, const xw_params* pin, const int8_t* start, 
         const int m = std::min(w, n - w);
         const bool large = n >= large_min_order();
         const int form = large && anneal_large_planes_fit(n, m) ? large_form_wanted() : 0;
-        const uint32_t slot = large ? anneal_large_slot_bytes(n, m, form) : anneal_slot_bytes(n, m, anneal_opl(n));
+        const uint32_t slot = large ? anneal_large_slot_bytes(n, m, form) : anneal_slot_bytes(n, m, anneal_opl(n, w));
         if (replicas == 0) {
             // one resident wave: warp slots per SM times SMs
             const int wpb = large ? 4 : p.warps_per_block > 0 ? p.warps_per_block : 4;
             int per_sm = 0;
             const void* fn = large ? anneal_large_kernel_fn(needs_general_kernel(p), form)
-                                   : anneal_kernel_fn(anneal_opl(n), needs_general_kernel(p));
+                                   : anneal_kernel_fn(anneal_opl(n, w), needs_general_kernel(p));
             raise_smem_limit(fn, p.device);
             cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * wpb, (size_t)wpb * slot);
             replicas = std::max(1, per_sm * wpb * out->device.multiprocessors);

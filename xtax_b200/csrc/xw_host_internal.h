@@ -83,7 +83,7 @@ DeviceVerifier& shared_verifier(int device, std::mutex*& mu);
 // class of the order (1, 2, 4, 8), or kTunePairKind for orders up to 16
 // (with at most 16 candidates per move), which may run two replicas per warp.
 constexpr int kTunePairKind = 16;
-int tune_kind(int n, int candidate_samples);
+int tune_kind(int n, int w, int candidate_samples);
 struct TunedShape {
     int wpb;   // warps per CTA
     int rpw;   // replicas per warp

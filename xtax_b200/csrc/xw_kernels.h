@@ -21,7 +21,7 @@ struct AnnealArgs {
     uint64_t iters;            // iterations per replica this launch
     int32_t stop_on_solve;
     // 1: every replica of the launch has one zero per row (w = n - 1); the
-    // lean one-row, one-replica-per-warp kernel then runs its instantiation
+    // one-row, one-replica-per-warp kernels then run their instantiation
     // with the minority size and side as constants (other kernels ignore it)
     int32_t one_zero;
     uint8_t* gram = nullptr;            // large-order kernel: Gram and mask arena
@@ -34,17 +34,14 @@ struct AnnealArgs {
     uint32_t* chunk_done = nullptr;
     // device-time limit of a chunk's wait for its predecessor, 0 = 30 s
     uint64_t chunk_wait_ns = 0;
-    // with one_zero: the launch's single order, whose instantiation (the even
-    // orders 6..26) then runs with the order as a constant; 0 = any order
-    int32_t fixed_order = 0;
-    int32_t fixed_pad = 0;
 };
 
 // shared-memory bytes one warp needs for a replica of order n, minority m,
 // in a launch of the `opl` rows-per-lane kernel
 uint32_t anneal_slot_bytes(int n, int m, int opl);
-// lanes' rows per lane: 1 for n <= 32, 2 for n <= 64, 4 for n <= 128, 8 for n <= 256
-int anneal_opl(int n);
+// lanes' rows per lane: 1 for n <= 32, 2 for n <= 64, 4 for n <= 128, 8 for
+// n <= 256 (and W(128,128), whose Gram entries need 16 bits)
+int anneal_opl(int n, int w);
 // `general`: some replica of the launch uses the squared or parity objective
 // or the within-row swap move set; otherwise the lean kernel (L1 score,
 // the reference's moves) runs, which drops that work from the hot loop.
@@ -52,9 +49,8 @@ int anneal_opl(int n);
 // of a warp owns a replica and a shared-memory slot of args.slot_bytes, so
 // a CTA holds warps_per_block * rpw slots).
 // `one_zero`: the instantiation for launches whose replicas all have one zero
-// per row (AnnealArgs::one_zero); it applies to opl 1, lean, rpw 1 only;
-// `fixed_order` > 0: all of them have that order (AnnealArgs::fixed_order).
-const void* anneal_kernel_fn(int opl, bool general, int rpw = 1, bool one_zero = false, int fixed_order = 0);
+// per row (AnnealArgs::one_zero); it applies to opl 1, rpw 1 only.
+const void* anneal_kernel_fn(int opl, bool general, int rpw = 1, bool one_zero = false);
 cudaError_t launch_anneal(const AnnealArgs& args, int opl, bool general, int warps_per_block, int blocks,
                           cudaStream_t stream, int rpw = 1);
 // Latency mode (orders up to 32): one replica per CTA of K warps (2..16),

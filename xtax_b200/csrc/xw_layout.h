@@ -94,4 +94,10 @@ static_assert(sizeof(RepHeader) == 128, "replica header is 128 bytes");
 #define XW_HD
 #endif
 
-static inline XW_HD uint32_t xw_pad16(uint32_t v) { return (v + 15u) & ~15u; }
+#ifdef __cplusplus
+#define XW_CONSTEXPR constexpr
+#else
+#define XW_CONSTEXPR
+#endif
+
+static inline XW_HD XW_CONSTEXPR uint32_t xw_pad16(uint32_t v) { return (v + 15u) & ~15u; }

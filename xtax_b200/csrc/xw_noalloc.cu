@@ -190,7 +190,7 @@ extern "C" int32_t xw_anneal_noalloc(int32_t n, int32_t w, const xw_params* p, i
     if (dev < 0 || dev >= kMaxDevices) return nfail(XW_ERR_INVALID, "xw_anneal_noalloc: device ordinal too large");
 
     const bool job_general = needs_general_kernel(*p);
-    const int opl = anneal_opl(n);
+    const int opl = anneal_opl(n, w);
     const uint32_t slot = anneal_slot_bytes(n, m, opl);
     const int wpb = p->warps_per_block > 0 ? p->warps_per_block : 4;
     const void* fn = anneal_kernel_fn(opl, job_general);

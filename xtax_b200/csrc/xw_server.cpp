@@ -55,9 +55,10 @@ namespace {
 constexpr int kClasses = 5;
 constexpr size_t kBestStride = (size_t)XW_MAX_N * XW_MAX_N;
 
-int class_of(int n, int candidate_samples) {
+int class_of(int n, int w, int candidate_samples) {
     if (n <= 16 && candidate_samples <= 16) return 0;
-    return n <= 32 ? 1 : n <= 64 ? 2 : n <= 128 ? 3 : 4;
+    const int opl = anneal_opl(n, w);
+    return opl == 1 ? 1 : opl == 2 ? 2 : opl == 4 ? 3 : 4;
 }
 int opl_of_class(int c) { return c == 0 ? 1 : 1 << (c - 1); }
 int kind_of_class(int c) { return c == 0 ? kTunePairKind : opl_of_class(c); }
@@ -205,7 +206,7 @@ struct Server {
     void place(const ReqPtr& q);
     void select_round();
     void rebuild_items();
-    int blocks_for(int cls, bool general, uint32_t slot_bytes, int wpb, int rpw, size_t items);
+    int blocks_for(int cls, bool general, bool one_zero, uint32_t slot_bytes, int wpb, int rpw, size_t items);
     void round(bool& any_tempering);
     void retire(const ReqPtr& q, const JobOut& o, double t_host, uint64_t stamp, int state, const VerifyStats& vs);
     DeviceVerifier verifier;   // retiring requests' W, checked on the tensor cores
@@ -413,7 +414,7 @@ void Server::rebuild_items() {
     }
     for (int s : order) {
         const ReqPtr& q = slot_req[s];
-        const int c = class_of(q->spec.n, q->job.candidate_samples);
+        const int c = class_of(q->spec.n, q->spec.w, q->job.candidate_samples);
         for (int r = 0; r < q->spec.replicas; ++r) items_host[c].push_back((uint32_t)(q->rep_begin + r));
         class_slot[c] = std::max(class_slot[c], anneal_slot_bytes(q->spec.n, q->job.m, opl_of_class(c)));
         class_general[c] = class_general[c] || q->job.general != 0;
@@ -427,13 +428,14 @@ void Server::rebuild_items() {
     items_dirty = false;
 }
 
-int Server::blocks_for(int cls, bool general, uint32_t slot_bytes, int wpb, int rpw, size_t items) {
-    const auto key = std::make_pair(((cls * 64 + wpb) * 2 + (general ? 1 : 0)) * 4 + rpw, slot_bytes);
+int Server::blocks_for(int cls, bool general, bool one_zero, uint32_t slot_bytes, int wpb, int rpw, size_t items) {
+    const auto key =
+        std::make_pair((((cls * 64 + wpb) * 2 + (general ? 1 : 0)) * 2 + (one_zero ? 1 : 0)) * 4 + rpw, slot_bytes);
     auto it = per_sm_cache.find(key);
     int per_sm = 0;
     if (it == per_sm_cache.end()) {
         check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                       &per_sm, anneal_kernel_fn(opl_of_class(cls), general, rpw), 32 * wpb,
+                       &per_sm, anneal_kernel_fn(opl_of_class(cls), general, rpw, one_zero), 32 * wpb,
                        (size_t)wpb * rpw * slot_bytes),
                    "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
         per_sm_cache[key] = per_sm;
@@ -469,7 +471,8 @@ void Server::round(bool& any_tempering) {
         const int wpb = std::max(1, std::min({16, t.wpb, fit}));
         cls_wpb[c] = wpb;
         cls_rpw[c] = t.rpw;
-        cls_blocks[c] = blocks_for(c, class_general[c], class_slot[c], wpb, t.rpw, items_host[c].size());
+        cls_blocks[c] = blocks_for(c, class_general[c], class_one_zero[c] && t.rpw == 1, class_slot[c], wpb, t.rpw,
+                                   items_host[c].size());
         cls_chunks[c] = choose_chunks((uint32_t)items_host[c].size(), (uint32_t)(cls_blocks[c] * wpb * t.rpw));
         if (cls_chunks[c] > (uint32_t)cfg.quantum_iters) cls_chunks[c] = 1;
         any_chunked = any_chunked || cls_chunks[c] > 1;
@@ -777,7 +780,7 @@ void Server::start() {
         for (bool general : {false, true})
             for (int rpw = 1; rpw <= (c == 0 ? 2 : 1); ++rpw)
                 raise_smem_limit(anneal_kernel_fn(opl_of_class(c), general, rpw), cfg.device);
-    raise_smem_limit(anneal_kernel_fn(1, false, 1, true), cfg.device);
+    for (bool general : {false, true}) raise_smem_limit(anneal_kernel_fn(1, general, 1, true), cfg.device);
     if (cfg.max_active_replicas <= 0) {
         // eight waves of the resident warps at the order-32 slot: enough work
         // per round to keep every SM busy through the round's tails (the C5

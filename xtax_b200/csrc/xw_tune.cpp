@@ -90,9 +90,9 @@ int env_int(const char* name, int lo, int hi) {
 
 }  // namespace
 
-int tune_kind(int n, int candidate_samples) {
+int tune_kind(int n, int w, int candidate_samples) {
     if (n <= 16 && candidate_samples <= 16) return kTunePairKind;
-    return anneal_opl(n);
+    return anneal_opl(n, w);
 }
 
 TunedShape tuned_shape(int kind, uint32_t slot_bytes, int device) {
