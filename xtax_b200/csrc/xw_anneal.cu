@@ -29,6 +29,7 @@
 
 #include <cooperative_groups.h>
 
+#define XW_EDGE_INLINE
 #include "xw_device.cuh"
 #include "xw_kernels.h"
 #include "xw_packed.cuh"
@@ -888,40 +889,111 @@ __device__ void run_replica_wide(const AnnealArgs& a, uint32_t rid, uint8_t* slo
 
 // ---------------------------------------------------------------------------
 // The one-warp (or half-warp) replica loop.
+//
+// An iteration proposes one candidate or, with the job's greedy
+// probability, candidate_samples of them.  A step of this loop gives its
+// four candidate groups either the candidates of one iteration or, in a run
+// of one-candidate iterations, the next up to four iterations of the run:
+// their draws and the kind of each are known ahead (counter-based), and
+// while no move is accepted they see the same state.  The first accepted
+// one is committed; the iterations after it are proposed again.  The
+// trajectory is that of one iteration at a time.  (Acceptance is 11% on the
+// W(26,25) ladder: 0.85 steps an iteration.)
 template <int WPL, bool GEN, int GW, bool ONEZ>
 __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane,
                                             uint64_t iters) {
+    constexpr int LPC = GW / 4;
+    constexpr int kWin = GW;   // iterations whose move-level draws are computed at once
     const unsigned gm = group_mask<GW>();
+    const int wl0 = GW == 32 ? 0 : (int)(threadIdx.x & 16u);
     Env E;
-    State S;
-    if (!load_replica<WPL, GEN, GW, ONEZ>(a, rid, slot, slot + Slot<WPL>::draws, lane, iters, E, S, true)) return;
-    const int tempering = S.J->tempering, mpc = S.J->moves_per_cool, stuck = S.J->stuck_threshold;
-    uint64_t left = iters, evals = 0, calls = 0;
-    uint32_t evals2 = 0;
-    bool stop = false;
-    // 32-bit counts within a block of iterations (a multiple of 64)
-    while (left > 0 && !stop) {
-        const uint32_t block = left < (1u << 24) ? (uint32_t)left : 1u << 24;
-        uint32_t cand_l = 0, two_l = 0, k = 0;
+    if (!load_replica<WPL, GEN, GW, ONEZ>(a, rid, slot, lane, iters, E, true)) return;
+    auto job = [&]() -> XwJob* { return a.jobs + reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid])->job; };
+    // stop rules: 1, every replica of the job stops soon after any solve;
+    // 2, a replica stops at its own solve only, so that each replica's
+    // trajectory is independent of how the launches are scheduled
+    auto stops = [&](const Con* con, int k) -> bool {
+        if (k >= con->k_end) return true;
+        if (a.stop_on_solve && con->best.z == 0) return true;
+        return a.stop_on_solve == 1 && (k & 63) == 63 && *(volatile int32_t*)&job()->solved;
+    };
+    // the next k at which something besides moves happens
+    auto event = [&](const Con* con, int k) -> int {
+        int e = max(next_event<WPL>(job(), con), k + 1);
+        if (a.stop_on_solve == 1) e = min(e, (k | 63) == k ? k + 64 : k | 63);
+        return e;
+    };
+    int k = 0;                       // calls made
+    uint32_t multis = 0, two_l = 0;  // iterations of several candidates; two-row candidates of this lane's group
+    uint32_t wmask = 0;              // bit j: iteration j of the window has several candidates
+    int wpos = kWin;
+    int k_evt = event(con_of<WPL>(slot), 0);
+    bool live = !stops(con_of<WPL>(slot), 0);
 #pragma unroll 1
-        for (; k < block; ++k) {
-            // 1: every replica of the job stops soon after any solve;
-            // 2: a replica stops at its own solve only, so that each replica's
-            //    trajectory is independent of how the launches are scheduled
-            if (a.stop_on_solve) {
-                stop = S.best_s == 0 || (a.stop_on_solve == 1 && (k & 63) == 63 && *(volatile int32_t*)&S.J->solved);
-                if (stop) break;
-            }
-            Pick P = choose<WPL, GEN, GW, ONEZ>(E, S.it, lane, cand_l, two_l);
-            apply<WPL, GEN, GW, ONEZ>(E, S, P, accepts<WPL>(E, P), tempering, mpc, stuck, lane);
-            ++S.it;
+    while (live) {
+        // values derived from these are computed where they are used: held
+        // across the loop they cost more in spilled registers
+        asm volatile("" : "+r"(E.slot), "+r"(lane));
+        const Con* con = con_of<WPL>(E.slot);
+        const int g = lane / LPC;
+        const uint32_t win = E.slot + Slot<WPL>::win;
+        if (wpos >= kWin) {
+            const uint4 b = draw_block(0u, con->it0 + (uint64_t)(k + lane), con->stream, con->k0, con->k1);
+            wmask = __ballot_sync(gm, (uint64_t)b.x < con->thr_greedy) >> wl0;
+            *reinterpret_cast<uint32_t*>(xw_smem + win + 4u * (uint32_t)lane) = b.y;
+            wpos = 0;
+            __syncwarp(gm);
         }
-        left -= k;
-        calls += k;
-        evals += __reduce_add_sync(gm, E.l == 0 ? cand_l : 0u);
-        evals2 += __reduce_add_sync(gm, E.l == 0 ? two_l : 0u);
+        const uint32_t rem = wmask >> wpos;
+        const bool multi = rem & 1u;
+        const uint64_t it = con->it0 + (uint64_t)k;
+        bool accept;
+        int used = 1, acc, prim;
+        Move mv;
+        multis += rem & 1u;
+        if (multi && con->cs > 4) {
+            const Winner w = choose_many<WPL, GEN, GW, ONEZ>(E, it, con->cs, lane);
+            mv = w.mv;
+            acc = w.acc;
+            prim = w.prim;
+            if (lane == 0) two_l += (uint32_t)w.two;
+            accept = accepts<WPL>(E.slot, prim, lds32(win + 4u * (uint32_t)wpos));
+        } else {
+            const int run = multi ? con->cs : min(min(__ffs((int)(rem | 16u)) - 1, kWin - wpos), k_evt - k);
+            const bool act = g < run;
+            fill_draws<GW>(E, con, it, 0, multi, lane);
+            __syncwarp(gm);
+            const Cand q = candidate<WPL, GEN, GW, ONEZ>(E, it, multi ? 0 : g, multi ? g : 0, act, lane);
+            const bool ok = accepts<WPL>(E.slot, q.prim, lds32(win + 4u * (uint32_t)(wpos + (multi ? 0 : g))));
+            const uint32_t oks = __ballot_sync(gm, act && ok) >> wl0;
+            // the best candidate, or the first accepted iteration of a run
+            uint32_t A, B;
+            best_keys(GEN && E.obj_kind != 0, q, act && (multi || ok), g, !multi, gm, A, B);
+            const int src = (int)(B & 3u) * LPC;
+            accept = (oks >> src) & 1u;   // (a run without one: group 3, whose bit is clear)
+            if (!multi) used = accept ? (int)(B & 3u) + 1 : run;
+            two_l += q.R2 != q.R1 && (multi ? act : g < used) ? 1u : 0u;
+            if (accept) {
+                mv = move_of(pack_move(q), wl0 + src, gm);
+                acc = __shfl_sync(gm, q.acc, wl0 + src);
+                prim = __shfl_sync(gm, q.prim, wl0 + src);
+            }
+        }
+        k += used;
+        wpos += used;
+        // an improvement puts the reheat off (an event due now still comes)
+        if (accept && accept_move<WPL, GEN, GW, ONEZ>(a, E, mv, acc, prim, k, lane) && k < k_evt)
+            k_evt = a.stop_on_solve && con->best.z == 0 ? k : event(con, k);
+        if (k >= k_evt) {
+            temperature_step<WPL, GW>(a, E.slot, k, lane);
+            live = !stops(con, k);
+            k_evt = event(con, k);
+        }
     }
-    store_replica<WPL, GW>(E, S, calls, evals, evals2, lane);
+    const uint64_t evals =
+        (uint64_t)((uint32_t)k - multis) + (uint64_t)multis * (uint64_t)con_of<WPL>(E.slot)->cs;
+    const uint32_t evals2 = __reduce_add_sync(gm, (lane & (LPC - 1)) == 0 ? two_l : 0u);
+    store_replica<WPL, GW>(a, E, k, evals, evals2, lane);
 }
 
 // Latency mode: one replica per CTA of K warps, speculating K iterations at
@@ -941,15 +1013,14 @@ __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, u
 // (warp 0's) structures and the other warps' draw buffers.
 struct SpecOut {
     Move mv;
-    int32_t ds, dc, prim;
+    int32_t dsc, prim;        // score change + 4096 x conflict change; objective change
     uint32_t u;
     uint32_t evals, evals2;   // candidates evaluated; those changing two rows
-    int32_t acc;        // the Metropolis outcome at the round's starting temperature
+    int32_t acc;              // the Metropolis outcome at the round's starting temperature
 };
 struct SpecCtl {
-    uint64_t it;        // first iteration of the round
+    int32_t k;          // calls made before the round
     int32_t count;      // iterations of the round (0: the replica stops)
-    int32_t pad;
 };
 
 // Per round buffer (two, used in turn): the outcomes of all the round's
@@ -983,35 +1054,38 @@ __host__ __device__ inline SpecLayout spec_layout(uint32_t slot_bytes, int K, in
 // CTAs' identical state or read by rank 0 alone and exchanged (whether
 // the replica runs at all, and the job's solved flag each round), so the
 // CTAs take the same branches and meet at every barrier.
-template <int WPL, bool GEN, int CL>
+template <int WPL, bool GEN, int CL, bool ONEZ>
 __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, int K, int lane) {
     namespace cg = cooperative_groups;
     const int rank = CL > 1 ? (int)cg::this_cluster().block_rank() : 0;
     const bool owner = rank == 0;
-    const XwJob* J = a.jobs + reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid])->job;
+    const RepHeader* H = reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid]);
+    XwJob* J = a.jobs + H->job;
     const SpecLayout L = spec_layout(packed_slot_bytes(J->n, J->m, WPL), K, CL);
     SpecCtl* ctl = reinterpret_cast<SpecCtl*>(xw_smem + L.off_ctl);
+    const Con* con = con_of<WPL>(0u);
     Env E;
-    State S;
     bool ok = false;
-    uint64_t iters = a.iters;
+    const int KT = K * CL;
+    int k = 0, k_evt = 0, k_end = 0;
+    uint64_t evals = 0;
+    uint32_t evals2 = 0;
     // warp 0 loads the replica; the round size goes to the others through
     // shared memory
-    if (warp == 0) ok = load_replica<WPL, GEN, 32, false>(a, rid, 0u, Slot<WPL>::draws, lane, iters, E, S, owner);
-    const int tempering = J->tempering;
-    const int mpc = J->moves_per_cool, stuck = J->stuck_threshold;
-    const int KT = K * CL;
-    uint64_t done = 0, evals = 0, calls = 0;
-    uint32_t evals2 = 0;
-    if (warp == 0 && lane == 0 && owner) {
-        SpecCtl c;
-        c.it = ok ? S.it : 0;
-        c.pad = 0;
-        const bool stop = !ok || iters == 0 || (a.stop_on_solve && S.best_s == 0);
-        c.count = stop ? 0 : (int32_t)(iters < (uint64_t)KT ? iters : (uint64_t)KT);
-        *ctl = c;
-        if constexpr (CL > 1) {
-            for (int q = 1; q < CL; ++q) *cg::this_cluster().map_shared_rank(ctl, q) = c;
+    if (warp == 0) {
+        ok = load_replica<WPL, GEN, 32, ONEZ>(a, rid, 0u, lane, a.iters, E, owner);
+        if (ok) {
+            k_evt = max(next_event<WPL>(J, con), 1);
+            k_end = con->k_end;
+        }
+        if (lane == 0 && owner) {
+            SpecCtl c;
+            c.k = 0;
+            c.count = !ok || (a.stop_on_solve && con->best.z == 0) ? 0 : min(k_end, KT);
+            *ctl = c;
+            if constexpr (CL > 1) {
+                for (int q = 1; q < CL; ++q) *cg::this_cluster().map_shared_rank(ctl, q) = c;
+            }
         }
     }
     if constexpr (CL > 1) cg::this_cluster().sync();
@@ -1019,15 +1093,13 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
     if (ctl->count == 0) {
         // nothing to run: the loaded replica's record still gets its
         // rebuilt state, as the one-warp kernel writes it
-        if (warp == 0 && ok && owner) store_replica<WPL, 32>(E, S, 0, 0, 0, lane);
+        if (warp == 0 && ok && owner) store_replica<WPL, 32>(a, E, 0, 0, 0, lane);
         return;
     }
     // every warp: the replica's structures (read-only until warp 0 commits)
     // and its own draw buffer
-    if (warp != 0) {
-        const RepHeader* H = reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid]);
-        make_env<WPL, 32, false>(E, J, H, 0u, L.off_extra + (uint32_t)(warp - 1) * 512u, lane, GEN ? H->obj_kind : 0);
-    }
+    if (warp != 0)
+        make_env<WPL, 32, ONEZ>(E, J, 0u, L.off_extra + (uint32_t)(warp - 1) * 512u, lane, GEN ? H->obj_kind : 0);
 
     const int g = rank * K + warp;   // this warp's iteration within the round
 #pragma unroll 1
@@ -1035,27 +1107,38 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
         const int buf = round & 1;
         SpecOut* outs = reinterpret_cast<SpecOut*>(xw_smem + L.off_out + (uint32_t)buf * L.out_stride);
         int32_t* flag = reinterpret_cast<int32_t*>(xw_smem + L.off_flag) + buf;
-        const uint64_t it0 = ctl->it;
         const int cnt = ctl->count;
         if (g < cnt) {
-            uint32_t cand_l = 0, two_l = 0;
-            const Pick P = choose<WPL, GEN, 32, false>(E, it0 + (uint64_t)g, lane, cand_l, two_l);
+            const uint64_t it = con->it0 + (uint64_t)(ctl->k + g);
+            fill_draws<32, true>(E, con, it, 0, true, lane);
+            __syncwarp();
+            const uint64_t mblk = lds64(E.draws + 24u * 16u);
+            const int count = (uint64_t)(uint32_t)mblk < con->thr_greedy ? con->cs : 1;
             SpecOut o;
-            o.mv.rc = __shfl_sync(FULL, P.mv.rc, P.src);
-            o.mv.cf = __shfl_sync(FULL, P.mv.cf, P.src);
-            o.mv.ax = __shfl_sync(FULL, P.mv.ax, P.src);
-            o.ds = P.ds;
-            o.dc = P.dc;
-            o.prim = P.prim;
-            o.u = P.u;
-            // both counts in one sum (at most 32 candidates)
-            const uint32_t ev = __reduce_add_sync(FULL, E.l == 0 ? cand_l + (two_l << 16) : 0u);
-            o.evals = ev & 0xffffu;
-            o.evals2 = ev >> 16;
+            o.u = (uint32_t)(mblk >> 32);
+            o.evals = (uint32_t)count;
+            if (count > 4) {
+                const Winner w = choose_many<WPL, GEN, 32, ONEZ>(E, it, count, lane);
+                o.mv = w.mv;
+                o.dsc = w.acc;
+                o.prim = w.prim;
+                o.evals2 = (uint32_t)w.two;
+            } else {
+                const int c = lane >> 3;
+                const bool act = c < count;
+                const Cand q = candidate<WPL, GEN, 32, ONEZ>(E, it, 0, c, act, lane);
+                uint32_t A, B = 0;
+                if (count > 1) best_keys(GEN && E.obj_kind != 0, q, act, c, false, FULL, A, B);
+                const int src = (int)(B & 3u) * 8;
+                o.mv = move_of(pack_move(q), src, FULL);
+                o.dsc = __shfl_sync(FULL, q.acc, src);
+                o.prim = __shfl_sync(FULL, q.prim, src);
+                o.evals2 = (uint32_t)__popc(__ballot_sync(FULL, act && q.R2 != q.R1 && (lane & 7) == 0));
+            }
             // the Metropolis test at the round's starting temperature: the
             // one warp 0 would make if no cooling or reheat step falls
             // between the round's start and this iteration
-            o.acc = accepts<WPL>(E, P) ? 1 : 0;
+            o.acc = accepts<WPL>(0u, o.prim, o.u) ? 1 : 0;
             if (lane == 0) {
                 outs[g] = o;
                 if constexpr (CL > 1) {
@@ -1066,7 +1149,7 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
         }
         if constexpr (CL > 1) {
             if (owner && warp == 0 && lane == 0) {
-                const int32_t sv = a.stop_on_solve == 1 ? *(volatile int32_t*)&S.J->solved : 0;
+                const int32_t sv = a.stop_on_solve == 1 ? *(volatile int32_t*)&J->solved : 0;
                 for (int q = 0; q < CL; ++q) *cg::this_cluster().map_shared_rank(flag, q) = sv;
             }
             cg::this_cluster().sync();
@@ -1075,111 +1158,100 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
         }
         if (warp == 0) {
             // Iterations in order until the first accepted move.  Fast path:
-            // the rejected calls before it change only counters (moves, msi,
-            // cool) unless one of them reaches a cooling or reheat step, so
-            // when none can, they are counted in bulk and only the accepted
-            // move goes through apply.  Otherwise the ordered walk.
+            // the rejected calls before it change only counters unless one
+            // of them reaches a cooling or reheat step, so when none can,
+            // they are counted in bulk and only the accepted move is
+            // committed.  Otherwise the ordered walk.
             // The job's solved flag: read here on one CTA, as the owner read
             // it this round on a cluster.
             auto solved = [&]() -> bool {
                 if constexpr (CL > 1) return *flag != 0;
-                else return *(volatile int32_t*)&S.J->solved != 0;
+                else return *(volatile int32_t*)&J->solved != 0;
             };
-            auto outcome = [&](int q) -> Pick {
-                const SpecOut& o = outs[q];
-                Pick P;
-                P.mv = o.mv;
-                P.src = lane;   // every lane holds the move
-                P.ds = o.ds;
-                P.dc = o.dc;
-                P.prim = o.prim;
-                P.u = o.u;
-                return P;
+            // call k has been made; its temperature step
+            auto after_call = [&]() {
+                if (k >= k_evt) {
+                    temperature_step<WPL, 32>(a, 0u, k, lane);
+                    k_evt = max(next_event<WPL>(J, con), k + 1);
+                }
             };
-            // lane l holds the outcomes of iterations l and 32 + l (up to 64
-            // iterations a round, on a cluster of four)
+            auto commit_of = [&](int q) {
+                if (accept_move<WPL, GEN, 32, ONEZ>(a, E, outs[q].mv, outs[q].dsc, outs[q].prim, k, lane) && k < k_evt)
+                    k_evt = max(next_event<WPL>(J, con), k + 1);
+            };
+            // lane l looks at iterations l and 32 + l (up to 64 iterations a
+            // round, on a cluster of four)
             const bool l0 = lane < cnt, l1 = 32 + lane < cnt;
             const uint64_t acc_m = (uint64_t)__ballot_sync(FULL, l0 && outs[l0 ? lane : 0].acc != 0) |
                                    ((uint64_t)__ballot_sync(FULL, l1 && outs[l1 ? 32 + lane : 0].acc != 0) << 32);
-            // calls that leave the temperature unchanged: fewer than `room`
-            const int room = tempering ? 0x7fffffff : min(mpc - S.cool, stuck - S.msi);
             const int ja = acc_m ? __ffsll((long long)acc_m) - 1 : -1;
             const int jend = ja >= 0 ? ja + 1 : cnt;
             const int rejects = ja >= 0 ? jend - 1 : jend;
-            bool fast = rejects < room;
+            bool fast = rejects < k_evt - k;
             // a check of the job's solved flag (every 64th iteration) that
             // falls in the span and finds it set: take the span in order
-            if (fast && a.stop_on_solve == 1 && (done | 63) < done + (uint64_t)jend && solved()) fast = false;
-            int j = 0;
+            if (fast && a.stop_on_solve == 1 && (k | 63) < k + jend && solved()) fast = false;
             bool stop = false;
             if (fast) {
                 const bool in0 = lane < jend, in1 = 32 + lane < jend;
-                const uint32_t ev = __reduce_add_sync(FULL, (in0 ? outs[lane].evals + (outs[lane].evals2 << 16) : 0u) +
-                                                                (in1 ? outs[32 + lane].evals + (outs[32 + lane].evals2 << 16) : 0u));
+                const uint32_t ev = __reduce_add_sync(
+                    FULL, (in0 ? outs[lane].evals + (outs[lane].evals2 << 16) : 0u) +
+                              (in1 ? outs[32 + lane].evals + (outs[32 + lane].evals2 << 16) : 0u));
                 evals += ev & 0xffffu;
                 evals2 += ev >> 16;
-                calls += (uint64_t)jend;
-                S.msi += rejects;
-                if (!tempering) S.cool += rejects;
-                S.it += (uint64_t)rejects;
-                if (ja >= 0) {
-                    Pick P = outcome(ja);
-                    apply<WPL, GEN, 32, false>(E, S, P, true, tempering, mpc, stuck, lane);
-                    ++S.it;
-                }
-                j = jend;
+                k += jend;
+                if (ja >= 0) commit_of(ja);
+                after_call();
             } else {
 #pragma unroll 1
-                for (; j < cnt; ++j) {
-                    if (a.stop_on_solve == 1 && ((done + (uint64_t)j) & 63) == 63 && solved()) {
+                for (int j = 0; j < cnt; ++j) {
+                    if (a.stop_on_solve == 1 && (k & 63) == 63 && solved()) {
                         stop = true;
                         break;
                     }
                     evals += outs[j].evals;
                     evals2 += outs[j].evals2;
-                    ++calls;
-                    Pick P = outcome(j);
-                    const bool accept = accepts<WPL>(E, P);
-                    apply<WPL, GEN, 32, false>(E, S, P, accept, tempering, mpc, stuck, lane);
-                    ++S.it;
-                    if (accept) {
-                        ++j;
-                        break;
-                    }
+                    const bool accept = accepts<WPL>(0u, outs[j].prim, outs[j].u);
+                    ++k;
+                    if (accept) commit_of(j);
+                    after_call();
+                    if (accept) break;
                 }
             }
-            done += (uint64_t)j;
-            if (a.stop_on_solve && S.best_s == 0) stop = true;
+            if (a.stop_on_solve && con->best.z == 0) stop = true;
             if (lane == 0) {
-                ctl->it = S.it;
-                const uint64_t left = iters - done;
-                ctl->count = stop || left == 0 ? 0 : (int32_t)(left < (uint64_t)KT ? left : (uint64_t)KT);
+                ctl->k = k;
+                ctl->count = stop ? 0 : min(k_end - k, KT);
             }
         }
         __syncthreads();
         if (ctl->count == 0) break;
     }
-    if (warp == 0 && owner) store_replica<WPL, 32>(E, S, calls, evals, evals2, lane);
+    if (warp == 0 && owner) store_replica<WPL, 32>(a, E, k, evals, evals2, lane);
     // the other CTAs' copies stay in their shared memory until every CTA
     // of the cluster has made its last remote write into this one
     if constexpr (CL > 1) cg::this_cluster().sync();
 }
 
 // Register budget per thread; it sets how many replica warps an SM holds.
-// An SM's registers are split between its four schedulers (16384 each): 64
-// registers per thread give 8 warps per scheduler, 80 give 6, 128 give 4.
-// Orders above 32 are held back by shared memory before registers.
+// An SM's registers are split between its four schedulers (16384 each): 80
+// registers per thread give 6 warps per scheduler, 96 give 5, 112 and 128
+// give 4.  The one-row kernels take the smallest budget without spills:
+// measured on B200 (W(26,25) ladder, 4096 replicas, 10^4 iterations) 19.5
+// ms at 96 registers, 20.8 at 112, 21.7 at 80 (180 bytes of spills a
+// thread), 24.1 at 72; the general kernel (W(24,23), 2368 replicas, 4096
+// iterations) 9.7 ms at 112, 9.9 at 96, 10.3 at 80.
 #ifndef XW_ANNEAL_MAXNREG
 #define XW_ANNEAL_MAXNREG 128
 #endif
 #ifndef XW_ANNEAL_MAXNREG_LEAN1
-#define XW_ANNEAL_MAXNREG_LEAN1 64
+#define XW_ANNEAL_MAXNREG_LEAN1 96
 #endif
 #ifndef XW_ANNEAL_MAXNREG_GEN1
-#define XW_ANNEAL_MAXNREG_GEN1 80
+#define XW_ANNEAL_MAXNREG_GEN1 112
 #endif
 #ifndef XW_ANNEAL_MAXNREG_PAIR
-#define XW_ANNEAL_MAXNREG_PAIR 80
+#define XW_ANNEAL_MAXNREG_PAIR 96
 #endif
 constexpr int anneal_maxnreg(int opl, bool general, int gw) {
     return gw == 16 ? XW_ANNEAL_MAXNREG_PAIR
@@ -1224,14 +1296,14 @@ __global__ void __launch_bounds__(512, 1) anneal_spec_kernel(AnnealArgs a, int K
     const int warp = threadIdx.x >> 5;
     if constexpr (CL > 1) {
         const uint32_t item = blockIdx.x / CL;
-        if (item < a.n_items) run_replica_spec<1, GEN, CL>(a, a.items[item], warp, K, lane);
+        if (item < a.n_items) run_replica_spec<1, GEN, CL, false>(a, a.items[item], warp, K, lane);
     } else {
         for (;;) {
             if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1u);
             __syncthreads();
             const uint32_t item = s_item;
             if (item >= a.n_items) break;
-            run_replica_spec<1, GEN, 1>(a, a.items[item], warp, K, lane);
+            run_replica_spec<1, GEN, 1, false>(a, a.items[item], warp, K, lane);
             __syncthreads();
         }
     }

@@ -13,14 +13,18 @@ namespace xw {
 // Philox4x32-10 (Salmon, Moraes, Dror, Shaw, SC'11): ten rounds of
 // (hi0,lo0)=M0*c0, (hi1,lo1)=M1*c2, c'=(hi1^c1^k0, lo1, hi0^c3^k1, lo0),
 // with the key bumped by the Weyl constants between rounds.
+__device__ __forceinline__ uint4 philox_round(uint4 c, uint32_t k0, uint32_t k1) {
+    const uint32_t lo0 = 0xD2511F53u * c.x;
+    const uint32_t hi0 = __umulhi(0xD2511F53u, c.x);
+    const uint32_t lo1 = 0xCD9E8D57u * c.z;
+    const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z);
+    return make_uint4(hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0);
+}
+
 __device__ __forceinline__ uint4 philox4x32_10(uint4 c, uint32_t k0, uint32_t k1) {
 #pragma unroll
     for (int r = 0; r < 10; ++r) {
-        const uint32_t lo0 = 0xD2511F53u * c.x;
-        const uint32_t hi0 = __umulhi(0xD2511F53u, c.x);
-        const uint32_t lo1 = 0xCD9E8D57u * c.z;
-        const uint32_t hi1 = __umulhi(0xCD9E8D57u, c.z);
-        c = make_uint4(hi1 ^ c.y ^ k0, lo1, hi0 ^ c.w ^ k1, lo0);
+        c = philox_round(c, k0, k1);
         k0 += 0x9E3779B9u;
         k1 += 0xBB67AE85u;
     }
@@ -54,7 +58,16 @@ __device__ __forceinline__ bool lemire_ok(uint32_t v, uint32_t count, uint32_t& 
     return low >= count || low >= (0u - count) % count;
 }
 
-static __device__ __noinline__ uint32_t lemire_retry(uint32_t slot, uint64_t it, uint32_t stream,
+// Out of line, or (XW_EDGE_INLINE defined) inline: a kernel whose hot loop
+// holds a call at all keeps values across it in fewer registers, which cost
+// the packed-row kernels 4-7% in spills.
+#ifdef XW_EDGE_INLINE
+#define XW_EDGE_FN __forceinline__
+#else
+#define XW_EDGE_FN __noinline__
+#endif
+
+static __device__ XW_EDGE_FN uint32_t lemire_retry(uint32_t slot, uint64_t it, uint32_t stream,
                                               uint32_t k0, uint32_t k1, int j, uint32_t count) {
     uint32_t out = 0;
 #pragma unroll 1
@@ -69,7 +82,7 @@ static __device__ __noinline__ uint32_t lemire_retry(uint32_t slot, uint64_t it,
 // The rare branch of an index draw (low word below count): the threshold
 // test that needs an integer remainder, then retries.  Out of line so the
 // common path of every index draw is a multiply and a compare.
-static __device__ __noinline__ uint32_t lemire_edge(uint32_t v, uint32_t slot, uint64_t it, uint32_t stream,
+static __device__ XW_EDGE_FN uint32_t lemire_edge(uint32_t v, uint32_t slot, uint64_t it, uint32_t stream,
                                              uint32_t k0, uint32_t k1, int j, uint32_t count) {
     uint32_t out;
     if (lemire_ok(v, count, out)) return out;

@@ -24,13 +24,17 @@
 // candidates therefore cost one pass: 4x fewer instructions than a loop
 // over candidates with one row per lane.
 //
-// What bounds it: instruction issue of dependent integer chains.  Measured
-// on B200 against a loop over candidates with one row per lane and a 32-bit
-// Gram matrix: 593 warp instructions an iteration against 843 (W(26,25)
-// ladder, 10^4 iterations of 4096 replicas: 30.5 ms against 44.7); W(100,50),
-// 592 replicas of 1000 iterations: 5.6 ms against 13.5 (bytes let six warps
-// share an SM instead of three, and the group's lanes try the attempts of a
-// support switch eight at a time).
+// What bounds it: instruction issue of dependent integer chains (W(26,25)
+// ladder, 10^4 iterations of 4096 replicas: issue slots 71% used, ALU pipe
+// 61%, 375 warp instructions an iteration, 19.5 ms).  Measured on B200
+// against a loop over candidates with one row per lane and a 32-bit Gram
+// matrix (843 instructions, 44.7 ms): packed rows alone 30.5 ms; runs of
+// one-candidate iterations side by side and the constants and the state of
+// accepted moves in shared memory instead of registers 26.9; no calls in
+// the loop (a call keeps what lives across it in few registers: 80 bytes of
+// spills a thread) and round keys from shared memory 19.5.  W(100,50), 592
+// replicas of 1000 iterations: 13.5 -> 5.1 ms (bytes let six warps share an
+// SM instead of three; the lanes try a switch's attempts side by side).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -76,48 +80,74 @@ __host__ __device__ constexpr uint32_t packed_stride(int n, int wpl) {
     return ((((uint32_t)n + q - 1u) / q) | 1u) * q;
 }
 
-// Replica constants read by broadcast from the slot.
+// A replica's constants and the state that changes with an accepted move
+// or a temperature step, in the slot: every lane reads them by broadcast
+// when it needs them, lane 0 writes.  Kept there they cost the iteration a
+// few broadcast reads instead of the registers that set how many warps
+// share an SM.
+//
+// Calls are counted in k from the start of the launch; msi (calls since the
+// last improvement) and the cooling counter are k - mb and k - cb.
 struct Con {
+    uint4 coins;         // the four thresholds below, at most 2^32 - 1
+    uint4 keys[5];       // Philox round keys, two rounds each
+    uint32_t k0, k1, stream;
+    int32_t cs;
     uint64_t thr_target, thr_dbl, thr_sign, thr_swsign;
+    uint64_t it0;        // iteration number at k = 0
     uint64_t thr_greedy;
+    int4 best;           // score, conflicts, best score, best conflicts
+    int4 acc;            // objective total (64 bits), accepted moves, rows they changed
     double T;
+    int32_t mb, cb;
+    int32_t k_end;       // iterations of this launch
+    // the best W is the current one and its record is older: it is written
+    // when an accepted move leaves it, or at the end
+    int32_t dirty;
+    // the copy that writes the record (a cluster's other CTAs keep an
+    // identical copy in their own shared memory and write nothing)
+    int32_t owner;
+    uint32_t rid;
 };
 
 // The slot: fixed regions first, so that their offsets are constants.
 template <int WPL>
 struct Slot {
-    static constexpr uint32_t draws = 0;                      // 32 Philox blocks
+    static constexpr uint32_t draws = 0;                      // 24 Philox blocks, then the window
+    static constexpr uint32_t win = 384;                      // acceptance draws of 32 iterations
     static constexpr uint32_t thr = 512;                      // Metropolis thresholds
-    static constexpr uint32_t con = thr + 8u * kThrTable;
-    static constexpr uint32_t res = con + 64u;                // packed residuals, 4 bytes a row
+    static constexpr uint32_t con = thr + 4u * kThrTable;
+    static constexpr uint32_t res = con + 240u;               // packed residuals, 4 bytes a row
     static constexpr uint32_t mask = res + 128u * WPL;        // support masks, 4*WPL bytes a row
     static constexpr uint32_t w = mask + 128u * WPL * WPL;
 };
 
-static_assert(sizeof(Con) <= 64, "replica constants fit their region");
+static_assert(sizeof(Con) <= 240, "replica constants fit their region");
 
 __host__ __device__ constexpr uint32_t packed_slot_bytes(int n, int m, int wpl) {
-    const uint32_t fixed = 512u + 8u * kThrTable + 64u + 128u * (uint32_t)wpl + 128u * (uint32_t)(wpl * wpl);
+    const uint32_t fixed = 512u + 4u * kThrTable + 240u + 128u * (uint32_t)wpl + 128u * (uint32_t)(wpl * wpl);
     const uint32_t mat = xw_pad16((uint32_t)n * packed_stride(n, wpl));
     // the last lanes of a row may read up to one lane's width past it; the
     // minority lists' pad covers the read of an empty list
     return fixed + 2u * mat + xw_pad16((uint32_t)(n * m) + 1u);
 }
 
-// Loop-invariant context of a replica's lane group.
+// Loop-invariant context of a lane of a replica's group.
 struct Env {
     uint32_t slot;       // the replica's slot in xw_smem
     uint32_t draws;      // this group's draw buffer
+    uint32_t cw;         // the cached draw blocks of this lane's candidate
     uint32_t g, mino;    // byte offsets of G and the minority lists
     uint32_t st;         // row stride
-    int n, w, m, sparse;
-    uint32_t k0, k1, stream;
-    int cs, ts, bpc, move_set, obj_kind;
-    uint32_t my_slot, my_slot2;   // Philox counter slots of this lane's cached blocks
-    uint32_t loff;       // byte offset of the lane's rows
-    int l, grp;          // lane within its candidate, candidate within a pass
-    bool lact;           // the lane holds rows below n
+    int n, m, sparse, full;   // full: w = n
+    int ts, bpc, move_set, obj_kind;
+    uint32_t dq[2];      // draw blocks this lane computes: candidate (or iteration) << 16 | 1 + block
 };
+
+template <int WPL>
+__device__ __forceinline__ Con* con_of(uint32_t slot) {
+    return reinterpret_cast<Con*>(xw_smem + slot + Slot<WPL>::con);
+}
 
 // ---- proposals --------------------------------------------------------
 
@@ -164,8 +194,14 @@ __device__ __forceinline__ int mask_first(uint32_t slot, int row, int start, int
     }
 }
 
+// The same in a row whose only zero is column z.
+__device__ __forceinline__ int after_zero(int start, int z, int n) {
+    const int c = start + (start == z ? 1 : 0);
+    return c >= n ? 0 : c;
+}
+
 // A draw word outside the cached blocks (tournaments past 8 samples).
-__device__ __noinline__ uint32_t slow_word(uint32_t slot, uint64_t it, uint32_t stream, uint32_t k0, uint32_t k1,
+__device__ __forceinline__ uint32_t slow_word(uint32_t slot, uint64_t it, uint32_t stream, uint32_t k0, uint32_t k1,
                                            int j) {
     return pick(draw_block(slot, it, stream, k0, k1), j);
 }
@@ -173,59 +209,85 @@ __device__ __noinline__ uint32_t slow_word(uint32_t slot, uint64_t it, uint32_t 
 // Column of a sign flip in `row` from draw word `wd` (slot, word j of block
 // b), propose_sign_flip (xweigh_cuda.cu:302-325): a minority pick for a
 // sparse row, else the first nonzero at or after a random column.
-template <int WPL>
+template <int WPL, bool ONEZ>
 __device__ __forceinline__ int flip_col_exact(uint32_t slot, uint32_t mino, int n, int m, int sparse, uint32_t wd,
                                               uint32_t dslot, uint64_t it, uint32_t stream, uint32_t k0, uint32_t k1,
                                               int j, int row) {
+    if constexpr (ONEZ)
+        return after_zero((int)draw_index(wd, (uint32_t)n, dslot, it, stream, k0, k1, j), (int)lds8(mino + (uint32_t)row), n);
     if (sparse && m > 0) return (int)lds8(mino + (uint32_t)(row * m) + draw_index(wd, (uint32_t)m, dslot, it, stream, k0, k1, j));
     return mask_first<WPL>(slot, row, (int)draw_index(wd, (uint32_t)n, dslot, it, stream, k0, k1, j), n);
 }
 
+// Hot-row tournament of candidate `c` (hot_row, xweigh_cuda.cu:291-300),
+// the samples spread over the group's lanes: the first sample with the
+// largest residual.
+template <int WPL, int GW>
+__device__ __forceinline__ int tournament(uint32_t slot, uint32_t cw, int n, int ts, int c, uint64_t it, int l,
+                                          unsigned gm) {
+    constexpr int LPC = GW / 4;
+    const Con* con = con_of<WPL>(slot);
+    uint32_t key = 0;
+#pragma unroll 1
+    for (int s = l; s < ts; s += LPC) {
+        const uint32_t ds = cand_slot(c, 4 + (s >> 2));
+        const uint32_t wd = s < 8 ? lds32(cw + 64u + 4u * (uint32_t)s)
+                                  : slow_word(ds, it, con->stream, con->k0, con->k1, s & 3);
+        const uint32_t r = draw_index(wd, (uint32_t)n, ds, it, con->stream, con->k0, con->k1, s & 3);
+        key = max(key, (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - s) << 8) | r);
+    }
+#pragma unroll
+    for (int d = 1; d < LPC; d <<= 1) key = max(key, __shfl_xor_sync(gm, key, d));
+    return (int)(key & 255u);
+}
+
 // The whole proposal of candidate `c` with exact index draws and every
-// further attempt, propose_move (xweigh_cuda.cu:327-447): called by the
+// further attempt, propose_move (xweigh_cuda.cu:327-447): taken by the
 // groups whose first attempt is not legal (a second flip that repeats the
 // first, a switch whose 2x2 is not legal) or whose draws met Lemire's
 // rejection zone.  Attempts are independent given their counters, so the
-// group's lanes try LPC of them at once and the first legal one is taken;
-// in order this is one attempt after the other, each with its own Philox
-// block.  `need`: the calling lane's group wants a proposal (the other
-// lanes take part in the collectives only).  Returns
+// group's lanes try several at once and the first legal one is taken; in
+// order this is one attempt after the other, each with its own Philox
+// blocks.  `need`: this lane's group wants a proposal (the other lanes take
+// part in the collectives only); `from`: the first attempt to try (1 when
+// attempt 0 is known to fail).  Returns
 // {R1 | R2<<8 | C1<<16 | C2<<24, kind | p1<<8 | p2<<16 | s1<<24 | s2<<25}.
-template <int WPL, int GW>
-__device__ __noinline__ uint2 propose_exact(bool need, uint32_t slot, uint32_t cw, uint32_t mino, uint32_t st, int n,
-                                            int w, int m, int sparse, int hot, int c, uint64_t it, uint32_t stream,
-                                            uint32_t k0, uint32_t k1) {
+template <int WPL, int GW, bool ONEZ>
+__device__ __forceinline__ uint2 propose_exact(const Env& E, bool need, int from, int hot, int c, uint64_t it, int l) {
     constexpr int LPC = GW / 4;
     const unsigned gm = group_mask<GW>();
-    const int wl = threadIdx.x & 31, l = wl & (LPC - 1), base = wl - l;
-    const Con* con = reinterpret_cast<const Con*>(xw_smem + slot + Slot<WPL>::con);
-    const uint4 b0 = lds128(cw), b1 = lds128(cw + 16), b2 = lds128(cw + 32), b3 = lds128(cw + 48);
+    const int wl = threadIdx.x & 31, base = wl - l;
+    const uint32_t slot = E.slot, cw = E.cw, mino = E.mino, st = E.st;
+    const int n = E.n, m = ONEZ ? 1 : E.m, sparse = ONEZ ? 0 : E.sparse;
+    const Con* con = con_of<WPL>(slot);
+    const uint32_t k0 = con->k0, k1 = con->k1, stream = con->stream;
     auto ix = [&](uint32_t wd, uint32_t count, int b, int j) -> int {
         return (int)draw_index(wd, count, cand_slot(c, b), it, stream, k0, k1, j);
     };
     auto fcol = [&](uint32_t wd, int b, int j, int row) -> int {
-        return flip_col_exact<WPL>(slot, mino, n, m, sparse, wd, cand_slot(c, b), it, stream, k0, k1, j, row);
+        return flip_col_exact<WPL, ONEZ>(slot, mino, n, m, sparse, wd, cand_slot(c, b), it, stream, k0, k1, j, row);
     };
     int row = 0, r2 = 0, c1 = 0, c2 = 0, p1 = 0, p2 = 0, kind = -1;
     bool s1 = false, s2 = false, dbl = false, flip = false;
     if (need) {
+        const uint4 b0 = lds128(cw);
         row = (uint64_t)b0.x < con->thr_target ? hot : ix(b0.y, (uint32_t)n, 0, 1);
         dbl = (uint64_t)b0.z < con->thr_dbl;
-        flip = w == n || (uint64_t)b0.w < con->thr_sign;
+        flip = (!ONEZ && E.full) || (uint64_t)b0.w < con->thr_sign;
     }
     // double flip (xweigh_cuda.cu:389-421): attempt 0 from block 3, attempt
     // a > 0 from block 19 + a, 16 in all
     bool pend = need && dbl;
     if (__any_sync(gm, pend)) {
-        const int first = pend ? fcol(b2.w, 2, 3, row) : 0;
+        const int first = pend ? fcol(lds32(cw + 44u), 2, 3, row) : 0;
 #pragma unroll 1
-        for (int a0 = 0; a0 < 16; a0 += LPC) {
+        for (int a0 = from; a0 < 16; a0 += LPC) {
             const int a = a0 + l;
             int rr = 0, cc = 0;
             bool ok = false;
             if (pend && a < 16) {
                 const int b = a == 0 ? 3 : 19 + a;
-                const uint4 d = a == 0 ? b3 : draw_block(cand_slot(c, b), it, stream, k0, k1);
+                const uint4 d = a == 0 ? lds128(cw + 48) : draw_block(cand_slot(c, b), it, stream, k0, k1);
                 rr = d.x < 0x80000000u ? row : ix(d.y, (uint32_t)n, b, 1);
                 cc = fcol(d.z, b, 2, rr);
                 ok = !(rr == row && cc == first);
@@ -247,43 +309,47 @@ __device__ __noinline__ uint2 propose_exact(bool need, uint32_t slot, uint32_t c
     if (need && kind < 0 && flip) {
         kind = 0;
         r2 = row;
-        c1 = c2 = fcol(b1.x, 1, 0, row);
+        c1 = c2 = fcol(lds32(cw + 16u), 1, 0, row);
     }
     // support switch (xweigh_cuda.cu:327-387): attempt 0 in blocks 1 and 2,
-    // attempt a > 0 in blocks 36 + 2(a-1) and the next, 24 in all
+    // attempt a > 0 in blocks 36 + 2(a-1) and the next, 24 in all.  The
+    // lower half of the lanes takes an attempt each, the upper half computes
+    // the second blocks (a double flip that failed has not tried attempt 0).
     pend = need && kind < 0 && m > 0 && n > 1;
     if (__any_sync(gm, pend)) {
+        constexpr int AT = LPC / 2;
+        const bool second = l >= AT;
 #pragma unroll 1
-        for (int a0 = 0; a0 < 24; a0 += LPC) {
-            const int a = a0 + l;
-            int rr = 0, x1 = 0, x2 = 0, q = 0, qq = 0;
-            uint32_t sw1 = 0;
+        for (int a0 = __any_sync(gm, pend && dbl) ? 0 : from; a0 < 24; a0 += AT) {
+            const int a = a0 + (l & (AT - 1)), b = a == 0 ? 1 : 36 + 2 * (a - 1), o = a == 0 ? 1 : 0;
+            int rr = 0, x1 = 0;
+            uint4 d = make_uint4(0, 0, 0, 0);
             bool ok = false;
-            if (pend) {
-                const int b = a == 0 ? 1 : 36 + 2 * (a - 1), o = a == 0 ? 1 : 0;
-                const uint4 d = a == 0 ? make_uint4(b1.y, b1.z, b1.w, b2.x)
-                                       : draw_block(cand_slot(c, b), it, stream, k0, k1);
-                rr = ix(d.x, (uint32_t)(n - 1), b, o);
-                if (rr >= row) ++rr;
-                q = ix(d.y, (uint32_t)m, b, o + 1);
-                qq = ix(d.z, (uint32_t)m, b, o + 2);
-                sw1 = d.w;
-                const int q1 = (int)lds8(mino + (uint32_t)(row * m + q)), q2 = (int)lds8(mino + (uint32_t)(rr * m + qq));
-                x1 = sparse ? q1 : q2;
-                x2 = sparse ? q2 : q1;
-                // entries (row, x2) and (rr, x1) are zeros and (row, x1),
-                // (rr, x2) nonzeros: one pair by the choice of q1, q2
-                const uint32_t e1 = lds8(slot + Slot<WPL>::w + (uint32_t)q2 * st + (uint32_t)row);
-                const uint32_t e2 = lds8(slot + Slot<WPL>::w + (uint32_t)q1 * st + (uint32_t)rr);
-                ok = sparse ? e1 == 1u && e2 == 1u : e1 != 1u && e2 != 1u;
+            if (pend && a < 24) {
+                d = draw_block(cand_slot(c, b + (second ? 1 : 0)), it, stream, k0, k1);
+                if (a == 0) {
+                    const uint4 e = lds128(cw + 16), f = lds128(cw + 32);
+                    d = second ? make_uint4(f.y, 0, 0, 0) : make_uint4(e.y, e.z, e.w, f.x);
+                }
+                if (!second) {
+                    rr = ix(d.x, (uint32_t)(n - 1), b, o);
+                    if (rr >= row) ++rr;
+                    const int q = ix(d.y, (uint32_t)m, b, o + 1), qq = ix(d.z, (uint32_t)m, b, o + 2);
+                    const int q1 = (int)lds8(mino + (uint32_t)(row * m + q)), q2 = (int)lds8(mino + (uint32_t)(rr * m + qq));
+                    // entries (row, C2) and (rr, C1) are zeros, (row, C1) and
+                    // (rr, C2) nonzeros: one pair by the choice of q1, q2
+                    const uint32_t e1 = lds8(slot + Slot<WPL>::w + (uint32_t)q2 * st + (uint32_t)row);
+                    const uint32_t e2 = lds8(slot + Slot<WPL>::w + (uint32_t)q1 * st + (uint32_t)rr);
+                    ok = sparse ? e1 == 1u && e2 == 1u : e1 != 1u && e2 != 1u;
+                    x1 = (sparse ? q1 : q2) | ((sparse ? q2 : q1) << 8) | (q << 16) | (qq << 24);
+                }
             }
             const unsigned hit = (__ballot_sync(gm, ok) >> base) & ((1u << LPC) - 1u);
             const int src = hit ? base + __ffs((int)hit) - 1 : wl;
             rr = __shfl_sync(gm, rr, src);
-            x1 = __shfl_sync(gm, x1 | (x2 << 8) | (q << 16) | (qq << 24), src);
-            sw1 = __shfl_sync(gm, sw1, src);
+            x1 = __shfl_sync(gm, x1, src);
+            const uint32_t sw1 = __shfl_sync(gm, d.w, src), sw2 = __shfl_sync(gm, d.x, hit ? src + AT : wl);
             if (pend && hit) {
-                const int win = a0 + (src - base);
                 kind = 1;
                 r2 = rr;
                 c1 = x1 & 255;
@@ -291,8 +357,6 @@ __device__ __noinline__ uint2 propose_exact(bool need, uint32_t slot, uint32_t c
                 p1 = (x1 >> 16) & 255;
                 p2 = (int)((uint32_t)x1 >> 24);
                 s1 = (uint64_t)sw1 < con->thr_swsign;
-                const uint32_t sw2 =
-                    win == 0 ? b2.y : pick(draw_block(cand_slot(c, 36 + 2 * (win - 1) + 1), it, stream, k0, k1), 0);
                 s2 = (uint64_t)sw2 < con->thr_swsign;
                 pend = false;
             }
@@ -302,7 +366,7 @@ __device__ __noinline__ uint2 propose_exact(bool need, uint32_t slot, uint32_t c
     if (need && kind < 0) {
         kind = 0;
         r2 = row;
-        c1 = c2 = fcol(b2.z, 2, 2, row);
+        c1 = c2 = fcol(lds32(cw + 40u), 2, 2, row);
     }
     return make_uint2((uint32_t)row | ((uint32_t)r2 << 8) | ((uint32_t)c1 << 16) | ((uint32_t)c2 << 24),
                       (uint32_t)(kind & 3) | ((uint32_t)p1 << 8) | ((uint32_t)p2 << 16) | (s1 ? 1u << 24 : 0u) |
@@ -318,15 +382,38 @@ struct Move {
     uint32_t rc, cf, ax;
 };
 
-// The move an iteration puts to the Metropolis test: the first best of its
-// candidates, its deltas and the iteration's acceptance draw.  `mv` is the
-// move of the lane's own candidate until it is taken from lane `src`.
-struct Pick {
-    Move mv;
-    int src;
-    int ds, dc, prim;
-    uint32_t u;
+// A lane's view of its group's candidate: the move, its deltas (score
+// change + 4096 x conflict change) and its change of the objective.
+struct Cand {
+    int R1, R2, C1, C2, p1, p2, kind;
+    int a1, b1, a2, b2, pk;
+    int acc, prim;
 };
+
+__device__ __forceinline__ Move pack_move(const Cand& q) {
+    Move mv;
+    mv.rc = (uint32_t)q.R1 | ((uint32_t)q.R2 << 8) | ((uint32_t)q.C1 << 16) | ((uint32_t)q.C2 << 24);
+    mv.cf = (uint32_t)(q.a1 & 255) | ((uint32_t)(q.b1 & 255) << 8) | ((uint32_t)(q.a2 & 255) << 16) |
+            ((uint32_t)q.b2 << 24);
+    mv.ax = (uint32_t)(q.pk & 255) | ((uint32_t)q.p1 << 8) | ((uint32_t)q.p2 << 16) |
+            (q.kind == 1 ? 3u << 24 : q.kind == 3 ? 1u << 24 : 0u);
+    return mv;
+}
+
+__device__ __forceinline__ Move move_of(const Move& mv, int src, unsigned gm) {
+    Move r;
+    r.rc = __shfl_sync(gm, mv.rc, src);
+    r.cf = __shfl_sync(gm, mv.cf, src);
+    r.ax = __shfl_sync(gm, mv.ax, src);
+    return r;
+}
+
+// v << s, 0 for s >= 32 (also for a "negative" s)
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t v, uint32_t s) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(v), "r"(s));
+    return r;
+}
 
 template <int WPL>
 __device__ __forceinline__ void load_words(uint32_t a, uint32_t (&v)[WPL]) {
@@ -344,283 +431,316 @@ __device__ __forceinline__ void load_words(uint32_t a, uint32_t (&v)[WPL]) {
 // packed residual of a row: sum |G| | conflicts << 18
 constexpr int kConfShift = 18;
 
-// Iteration `it` against the replica's current state: draws, hot-row
-// tournaments, proposals, evaluation.  Reads the state and writes only the
-// group's draw buffer.  cand_l counts the candidates this lane's group
-// evaluated, two_l those that change two rows.
+// The candidate of this lane's group: hot-row tournament, proposal and
+// evaluation of candidate `c` of iteration it + d_it against the replica's
+// current state, from the draw blocks at E.cw.  Groups with act false go
+// through the same steps on whatever their blocks hold.
 template <int WPL, bool GEN, int GW, bool ONEZ>
-__device__ __forceinline__ Pick choose(const Env& E, uint64_t it, int lane, uint32_t& cand_l, uint32_t& two_l) {
+__device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, int c, bool act, int lane) {
     constexpr int LPC = GW / 4;
     const unsigned gm = group_mask<GW>();
     const int n = E.n, m = ONEZ ? 1 : E.m, sparse = ONEZ ? 0 : E.sparse;
-    const uint32_t st = E.st, slot = E.slot, wbase = E.slot + Slot<WPL>::w;
-    const Con* con = reinterpret_cast<const Con*>(xw_smem + slot + Slot<WPL>::con);
-    Pick P;
-    P.src = 0;
-    P.ds = P.dc = P.prim = 0;
-    P.mv = Move{0, 0, 0};
-    // A: draws (block 0 the move-level block, 1 + c*bpc + b block b of
-    // candidate c; a half-warp computes two blocks per lane)
-    uint4* dbuf = reinterpret_cast<uint4*>(xw_smem + E.draws);
-    dbuf[lane] = draw_block(E.my_slot, it, E.stream, E.k0, E.k1);
-    if constexpr (GW == 16) dbuf[lane + 16] = draw_block(E.my_slot2, it, E.stream, E.k0, E.k1);
-    __syncwarp(gm);
-    const uint64_t mblk = lds64(E.draws);
-    P.u = (uint32_t)(mblk >> 32);
-    const int count = (uint64_t)(uint32_t)mblk < con->thr_greedy ? E.cs : 1;
-    uint32_t bestA = 0xffffffffu, bestB = 0xffffffffu;
-    const uint32_t cw = E.draws + 16u + (uint32_t)(E.grp * E.bpc) * 16u;
+    const uint32_t st = E.st, slot = E.slot, wbase = E.slot + Slot<WPL>::w, cw = E.cw;
+    const Con* con = con_of<WPL>(slot);
+    const int l = lane & (LPC - 1);
+    Cand q;
 
-#pragma unroll 1
-    for (int c0 = 0;;) {
-        const int c = c0 + E.grp;
-        const bool act = c < count;
-        // C: hot-row tournament (hot_row, xweigh_cuda.cu:291-300): the
-        // first sample with the largest residual
-        uint32_t key = 0;
-        if (GW == 32 && E.ts <= 8) {
-            if (E.l < E.ts) {
-                const uint32_t r = draw_index(lds32(cw + 64u + 4u * (uint32_t)E.l), (uint32_t)n,
-                                              cand_slot(c, 4 + (E.l >> 2)), it, E.stream, E.k0, E.k1, E.l & 3);
-                key = (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - E.l) << 8) | r;
-            }
-        } else {
-#pragma unroll 1
-            for (int s = E.l; s < E.ts; s += LPC) {
-                const uint32_t ds = cand_slot(c, 4 + (s >> 2));
-                const uint32_t wd = s < 8 ? lds32(cw + 64u + 4u * (uint32_t)s) : slow_word(ds, it, E.stream, E.k0, E.k1, s & 3);
-                const uint32_t r = draw_index(wd, (uint32_t)n, ds, it, E.stream, E.k0, E.k1, s & 3);
-                key = max(key, (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - s) << 8) | r);
-            }
-        }
+    bool edge = false;   // a draw met Lemire's rejection test: take the exact proposal
+    auto ix = [&](uint32_t wd, uint32_t cnt) -> int {
+        const uint64_t p = (uint64_t)wd * cnt;
+        edge = edge || (uint32_t)p < cnt;
+        return (int)(p >> 32);
+    };
+    // C: hot-row tournament, one sample a lane (up to eight samples)
+    int hot;
+    if (GW == 32 && E.ts <= 8) {
+        const uint32_t r = (uint32_t)ix(lds32(cw + 64u + 4u * (uint32_t)l), (uint32_t)n);
+        uint32_t key = (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - l) << 8) | r;
+        if (l >= E.ts) key = 0;
 #pragma unroll
         for (int d = 1; d < LPC; d <<= 1) key = max(key, __shfl_xor_sync(gm, key, d));
-        const int hot = (int)(key & 255u);
-
-        // D: the first attempt of the proposal (propose_move,
-        // xweigh_cuda.cu:423-447)
-        const uint4 b0 = lds128(cw), b1 = lds128(cw + 16), b2 = lds128(cw + 32), b3 = lds128(cw + 48);
-        bool edge = false;   // a draw met Lemire's rejection test: take the exact proposal
-        auto ix = [&](uint32_t wd, uint32_t cnt) -> int {
-            const uint64_t p = (uint64_t)wd * cnt;
-            edge = edge || (uint32_t)p < cnt;
-            return (int)(p >> 32);
-        };
-        const bool targeted = (uint64_t)b0.x < con->thr_target;
-        const int rdraw = ix(b0.y, (uint32_t)n);
-        int R1 = targeted ? hot : rdraw;
-        const bool dbl = (uint64_t)b0.z < con->thr_dbl;
-        bool flip = (uint64_t)b0.w < con->thr_sign;
-        if (!ONEZ) flip = flip || E.w == n;
-        flip = flip && !dbl;
-        const bool rowswap = GEN && E.move_set == 1 && !flip && !dbl;
-        const int r2d = ix(dbl ? b3.y : b1.y, (uint32_t)(dbl ? n : n - 1));
-        int R2 = dbl ? (b3.x < 0x80000000u ? R1 : r2d) : r2d + (r2d >= R1 ? 1 : 0);
-        if (flip || rowswap) R2 = R1;
-        int C1, C2, p1 = 0, p2 = 0;
-        bool bad;
-        if constexpr (ONEZ) {
-            // the row's only zero is its minority entry
-            const int z1 = (int)lds8(E.mino + (uint32_t)R1), z2 = (int)lds8(E.mino + (uint32_t)R2);
-            int f1 = ix(dbl ? b2.w : b1.x, (uint32_t)n), f2 = ix(b3.z, (uint32_t)n);
-            f1 += f1 == z1 ? 1 : 0;
-            f2 += f2 == z2 ? 1 : 0;
-            if (f1 >= n) f1 = 0;
-            if (f2 >= n) f2 = 0;
-            const bool sw = !dbl && !flip;
-            C1 = sw ? z2 : f1;
-            C2 = sw ? z1 : dbl ? f2 : f1;
-            bad = flip ? false : (R2 == R1 || sw) && C1 == C2;
-        } else {
-            auto fcol = [&](uint32_t wd, int row) -> int {
-                const int i = ix(wd, (uint32_t)(sparse ? m : n));
-                return sparse ? (int)lds8(E.mino + (uint32_t)(row * m + i)) : mask_first<WPL>(slot, row, i, n);
-            };
-            const int f1 = fcol(dbl ? b2.w : b1.x, R1);
-            const int f2 = fcol(b3.z, R2);
-            p1 = ix(b1.z, (uint32_t)m);
-            p2 = ix(b1.w, (uint32_t)m);
-            const int q1 = (int)lds8(E.mino + (uint32_t)(R1 * m + p1)), q2 = (int)lds8(E.mino + (uint32_t)(R2 * m + p2));
-            const uint32_t e1 = lds8(wbase + (uint32_t)q2 * st + (uint32_t)R1);
-            const uint32_t e2 = lds8(wbase + (uint32_t)q1 * st + (uint32_t)R2);
-            if (dbl) {
-                C1 = f1;
-                C2 = f2;
-                bad = R2 == R1 && C1 == C2;
-            } else if (flip) {
-                C1 = C2 = f1;
-                bad = false;
-            } else {
-                C1 = sparse ? q1 : q2;
-                C2 = sparse ? q2 : q1;
-                bad = sparse ? e1 != 1u || e2 != 1u : e1 == 1u || e2 == 1u;
-            }
-        }
-        bool s1 = (uint64_t)b2.x < con->thr_swsign, s2 = (uint64_t)b2.y < con->thr_swsign;
-        int kind = dbl ? 2 : flip ? 0 : 1;
-        if (rowswap) {
-            kind = 3;
-            bad = false;
-        }
-        const bool need = act && (bad || edge);
-        if (__any_sync(gm, need)) {
-            const uint2 x = propose_exact<WPL, GW>(need, slot, cw, E.mino, st, n, E.w, m, sparse, hot, c, it, E.stream, E.k0,
-                                                   E.k1);
-            if (need) {
-                R1 = (int)(x.x & 255u);
-                if (kind != 3) {
-                    R2 = (int)((x.x >> 8) & 255u);
-                    C1 = (int)((x.x >> 16) & 255u);
-                    C2 = (int)(x.x >> 24);
-                    kind = (int)(x.y & 3u);
-                    p1 = (int)((x.y >> 8) & 255u);
-                    p2 = (int)((x.y >> 16) & 255u);
-                    s1 = (x.y >> 24) & 1u;
-                    s2 = (x.y >> 25) & 1u;
-                }
-            }
-        }
-
-        if (GEN && kind == 3) {
-            // the within-row swap: a nonzero of the row moves to one of its zeros
-            const uint32_t dsl = cand_slot(c, 1);
-            const int pos = (int)draw_index(sparse ? b1.y : b1.z, (uint32_t)m, dsl, it, E.stream, E.k0, E.k1, sparse ? 1 : 2);
-            const int start = (int)draw_index(sparse ? b1.z : b1.y, (uint32_t)n, dsl, it, E.stream, E.k0, E.k1, sparse ? 2 : 1);
-            const int q = (int)lds8(E.mino + (uint32_t)(R1 * m + pos));
-            p1 = pos;
-            R2 = R1;
-            C1 = sparse ? q : mask_first<WPL>(slot, R1, start, n);
-            C2 = sparse ? mask_first<WPL, true>(slot, R1, start, n) : q;
-            s1 = b1.w < 0x80000000u;
-        }
-
-        // E: coefficients, then the new values of the lane's rows
-        const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
-        const int e11 = (int)lds8(w1 + (uint32_t)R1) - 1, e22 = (int)lds8(w2 + (uint32_t)R2) - 1;
-        const int e21 = (int)lds8(w1 + (uint32_t)R2) - 1, e12 = (int)lds8(w2 + (uint32_t)R1) - 1;
-        const bool two = R2 != R1;
-        int a1 = kind == 1 || (GEN && kind == 3) ? -e11 : -2 * e11;
-        int b1c = 0, a2 = 0, b2c = 0, pk = 0;
-        if (kind == 1) {
-            b1c = s1 ? -e11 : e11;
-            a2 = s2 ? -e22 : e22;
-            b2c = -e22;
-        } else if (kind == 2) {
-            if (two) {
-                b2c = -2 * e22;
-                // double flip over two rows (xweigh_cuda.cu:564-583)
-                pk = a1 * e21 + b2c * e12 + (C1 == C2 ? a1 * b2c : 0);
-            } else {
-                b1c = -2 * e22;
-            }
-        } else if (GEN && kind == 3) {
-            b1c = s1 ? 1 : -1;
-        }
-        uint32_t x[WPL], y[WPL], g1[WPL], g2[WPL];
-        load_words<WPL>(w1 + E.loff, x);
-        load_words<WPL>(w2 + E.loff, y);
-        load_words<WPL>(E.g + (uint32_t)R1 * st + E.loff, g1);
-        load_words<WPL>(E.g + (uint32_t)R2 * st + E.loff, g2);
-        const uint32_t rs1 = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R1);
-        const uint32_t rs2 = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R2);
-        const uint32_t kk1 = (uint32_t)(-(a1 + b1c)) * 0x01010101u, kk2 = (uint32_t)(-(a2 + b2c)) * 0x01010101u;
-        int acc = 0, pr = 0;
-#pragma unroll
-        for (int j = 0; j < WPL; ++j) {
-            // columns R1 and R2 of the changed rows are left out (the entry
-            // of a double flip over two rows apart): their W reads as zero
-            const int widx = E.l * WPL + j;
-            const uint32_t m1 = (R1 >> 2) == widx ? 0xffu << ((R1 & 3) * 8) : 0u;
-            const uint32_t m2 = (R2 >> 2) == widx ? 0xffu << ((R2 & 3) * 8) : 0u;
-            const uint32_t mm = m1 | m2;
-            const uint32_t xx = (x[j] & ~mm) | (0x01010101u & mm), yy = (y[j] & ~mm) | (0x01010101u & mm);
-            uint32_t n1 = g1[j] + kk1 + (uint32_t)a1 * xx + (uint32_t)b1c * yy;
-            const uint32_t n2 = g2[j] + kk2 + (uint32_t)a2 * xx + (uint32_t)b2c * yy;
-            if ((R2 >> 2) == widx) n1 += (uint32_t)pk << ((R2 & 3) * 8);
-            const uint32_t v1 = __vabsdiffu4(n1, 0x80808080u), v2 = __vabsdiffu4(n2, 0x80808080u);
-            const uint32_t z1 = (v1 + 0x7f7f7f7fu) & 0x80808080u, z2 = (v2 + 0x7f7f7f7fu) & 0x80808080u;
-            uint32_t t = (uint32_t)acc;
-            t = __dp4a(v1, 0x01010101u, t);
-            t = __dp4a(v2, 0x01010101u, t);
-            t = __dp4a(z1, 0x20202020u, t);   // 128 * 32: 4096 a conflict
-            t = __dp4a(z2, 0x20202020u, t);
-            acc = (int)t;
-            if (GEN) {
-                if (E.obj_kind == 1) {
-                    const int d1 = (int)(n1 ^ 0x80808080u), d2 = (int)(n2 ^ 0x80808080u);
-                    const int o1 = (int)(g1[j] ^ 0x80808080u), o2 = (int)(g2[j] ^ 0x80808080u);
-                    pr = __dp4a(d1, d1, pr) + __dp4a(d2, d2, 0) - __dp4a(o1, o1, 0) - __dp4a(o2, o2, 0);
-                } else if (E.obj_kind == 2) {
-                    // 128 is even: the biased byte has the entry's parity
-                    pr += __popc((n1 & 0x01010101u) | ((n2 & 0x01010101u) << 1)) -
-                          __popc((g1[j] & 0x01010101u) | ((g2[j] & 0x01010101u) << 1));
-                }
-            }
-        }
-        if (!E.lact) {
-            acc = 0;
-            pr = 0;
-        }
-        if (E.l == 0) {
-            const int r1 = (int)(rs1 & ((1u << kConfShift) - 1u)) + (int)((rs1 >> kConfShift) << 12);
-            const int r2 = (int)(rs2 & ((1u << kConfShift) - 1u)) + (int)((rs2 >> kConfShift) << 12);
-            acc -= r1 + r2;
-        }
-#pragma unroll
-        for (int d = 1; d < LPC; d <<= 1) acc += __shfl_xor_sync(gm, acc, d);
-        if (GEN && E.obj_kind != 0) {
-#pragma unroll
-            for (int d = 1; d < LPC; d <<= 1) pr += __shfl_xor_sync(gm, pr, d);
-        }
-        const int dc = (acc + 2048) >> 12;
-        const int ds = acc - dc * 4096;
-        cand_l += act ? 1u : 0u;
-        two_l += act && two ? 1u : 0u;
-
-        // the first best candidate: least (objective, score, conflicts, index)
-        uint32_t ka, A, B = 0;
-        if (!GEN || E.obj_kind == 0) {
-            ka = ((uint32_t)(ds + 2048) << 14) | ((uint32_t)(dc + 256) << 5) | (uint32_t)c;
-            A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
-        } else {
-            ka = ((uint32_t)(pr + (1 << 19)) << 12) | (uint32_t)(ds + 2048);
-            A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
-            B = __reduce_min_sync(gm, act && ka == A ? ((uint32_t)(dc + 256) << 5) | (uint32_t)c : 0xffffffffu);
-        }
-        if (A < bestA || (GEN && A == bestA && B < bestB)) {
-            bestA = A;
-            bestB = B;
-            const uint32_t sup = kind == 1 ? 3u << 24 : GEN && kind == 3 ? 1u << 24 : 0u;
-            P.mv.rc = (uint32_t)R1 | ((uint32_t)R2 << 8) | ((uint32_t)C1 << 16) | ((uint32_t)C2 << 24);
-            P.mv.cf = (uint32_t)(a1 & 255) | ((uint32_t)(b1c & 255) << 8) | ((uint32_t)(a2 & 255) << 16) |
-                      ((uint32_t)b2c << 24);
-            P.mv.ax = (uint32_t)(pk & 255) | ((uint32_t)p1 << 8) | ((uint32_t)p2 << 16) | sup;
-            const uint32_t k = !GEN || E.obj_kind == 0 ? A : B;
-            // the group's first lane of the winning candidate, within the warp
-            P.src = (int)(threadIdx.x & 31u & ~(uint32_t)(GW - 1)) + (int)((k & 3u)) * LPC;
-            P.dc = (int)((k >> 5) & 511u) - 256;
-            if (!GEN || E.obj_kind == 0) {
-                P.ds = (int)(A >> 14) - 2048;
-                P.prim = P.ds;
-            } else {
-                P.ds = (int)(A & 4095u) - 2048;
-                P.prim = (int)(A >> 12) - (1 << 19);
-            }
-            if (count > 4) {
-                P.mv.rc = __shfl_sync(gm, P.mv.rc, P.src);
-                P.mv.cf = __shfl_sync(gm, P.mv.cf, P.src);
-                P.mv.ax = __shfl_sync(gm, P.mv.ax, P.src);
-            }
-        }
-        c0 += 4;
-        if (c0 >= count) break;
-        // the next four candidates' draws
-        __syncwarp(gm);
-        dbuf[lane] = draw_block(E.my_slot + 128u * (uint32_t)c0, it, E.stream, E.k0, E.k1);
-        if constexpr (GW == 16) dbuf[lane + 16] = draw_block(E.my_slot2 + 128u * (uint32_t)c0, it, E.stream, E.k0, E.k1);
-        __syncwarp(gm);
+        hot = (int)(key & 255u);
+    } else {
+        hot = tournament<WPL, GW>(slot, cw, n, E.ts, c, it + (uint64_t)d_it, l, gm);
     }
-    return P;
+
+    // D: the first attempt of the proposal (propose_move,
+    // xweigh_cuda.cu:423-447)
+    const uint4 b0 = lds128(cw), coins = con->coins;
+    const int rdraw = ix(b0.y, (uint32_t)n);
+    int R1 = b0.x < coins.x ? hot : rdraw;
+    const bool dbl = b0.z < coins.y;
+    bool flip = b0.w < coins.z;
+    if (!ONEZ) flip = flip || E.full;
+    flip = flip && !dbl;
+    const bool rowswap = GEN && E.move_set == 1 && !flip && !dbl;
+    const uint4 b1 = lds128(cw + 16), b2 = lds128(cw + 32), b3 = lds128(cw + 48);
+    const int r2d = ix(dbl ? b3.y : b1.y, (uint32_t)(dbl ? n : n - 1));
+    int R2 = dbl ? (b3.x < 0x80000000u ? R1 : r2d) : r2d + (r2d >= R1 ? 1 : 0);
+    if (flip || rowswap) R2 = R1;
+    int C1, C2, p1 = 0, p2 = 0;
+    bool bad;
+    if constexpr (ONEZ) {
+        // the row's only zero is its minority entry
+        const int z1 = (int)lds8(E.mino + (uint32_t)R1), z2 = (int)lds8(E.mino + (uint32_t)R2);
+        const int f1 = after_zero(ix(dbl ? b2.w : b1.x, (uint32_t)n), z1, n), f2 = after_zero(ix(b3.z, (uint32_t)n), z2, n);
+        const bool sw = !dbl && !flip;
+        C1 = sw ? z2 : f1;
+        C2 = sw ? z1 : dbl ? f2 : f1;
+        bad = flip ? false : (R2 == R1 || sw) && C1 == C2;
+    } else {
+        auto fcol = [&](uint32_t wd, int row) -> int {
+            const int i = ix(wd, (uint32_t)(sparse ? m : n));
+            return sparse ? (int)lds8(E.mino + (uint32_t)(row * m + i)) : mask_first<WPL>(slot, row, i, n);
+        };
+        const int f1 = fcol(dbl ? b2.w : b1.x, R1);
+        const int f2 = fcol(b3.z, R2);
+        p1 = ix(b1.z, (uint32_t)m);
+        p2 = ix(b1.w, (uint32_t)m);
+        const int q1 = (int)lds8(E.mino + (uint32_t)(R1 * m + p1)), q2 = (int)lds8(E.mino + (uint32_t)(R2 * m + p2));
+        const uint32_t e1 = lds8(wbase + (uint32_t)q2 * st + (uint32_t)R1);
+        const uint32_t e2 = lds8(wbase + (uint32_t)q1 * st + (uint32_t)R2);
+        const bool illegal = sparse ? e1 != 1u || e2 != 1u : e1 == 1u || e2 == 1u;
+        const bool sw = !dbl && !flip;
+        C1 = sw ? (sparse ? q1 : q2) : f1;
+        C2 = sw ? (sparse ? q2 : q1) : dbl ? f2 : f1;
+        bad = sw ? illegal : dbl && R2 == R1 && C1 == C2;
+    }
+    bool s1 = b2.x < coins.w, s2 = b2.y < coins.w;
+    // 2^32 - 1 may lie below a threshold of 2^32
+    edge = edge || max(max(max(b0.x, b0.z), max(b0.w, b2.x)), b2.y) == 0xffffffffu;
+    int kind = dbl ? 2 : flip ? 0 : 1;
+    if (rowswap) {
+        kind = 3;
+        bad = false;
+    }
+    if (__any_sync(gm, act && (bad || edge))) {
+        // (a tournament's edge shows in one lane of the group)
+        const bool need = (__ballot_sync(gm, act && (bad || edge)) >> ((threadIdx.x & 31u) - (uint32_t)l)) & ((1u << LPC) - 1u);
+        const bool exact = __any_sync(gm, edge);
+        if (exact) hot = tournament<WPL, GW>(slot, cw, n, E.ts, c, it + (uint64_t)d_it, l, gm);
+        const uint2 x = propose_exact<WPL, GW, ONEZ>(E, need, exact ? 0 : 1, hot, c, it + (uint64_t)d_it, l);
+        if (need) {
+            R1 = (int)(x.x & 255u);
+            if (kind != 3) {
+                R2 = (int)((x.x >> 8) & 255u);
+                C1 = (int)((x.x >> 16) & 255u);
+                C2 = (int)(x.x >> 24);
+                kind = (int)(x.y & 3u);
+                p1 = (int)((x.y >> 8) & 255u);
+                p2 = (int)((x.y >> 16) & 255u);
+                s1 = (x.y >> 24) & 1u;
+                s2 = (x.y >> 25) & 1u;
+            }
+        }
+    }
+    if (GEN && kind == 3) {
+        // the within-row swap: a nonzero of the row moves to one of its zeros
+        const uint32_t dsl = cand_slot(c, 1);
+        const int pos = (int)draw_index(sparse ? b1.y : b1.z, (uint32_t)m, dsl, it + (uint64_t)d_it, con->stream, con->k0, con->k1,
+                                        sparse ? 1 : 2);
+        const int start = (int)draw_index(sparse ? b1.z : b1.y, (uint32_t)n, dsl, it + (uint64_t)d_it, con->stream, con->k0, con->k1,
+                                          sparse ? 2 : 1);
+        const int z = (int)lds8(E.mino + (uint32_t)(R1 * m + pos));
+        p1 = pos;
+        R2 = R1;
+        if constexpr (ONEZ) {
+            C1 = after_zero(start, z, n);
+            C2 = z;
+        } else {
+            C1 = sparse ? z : mask_first<WPL>(slot, R1, start, n);
+            C2 = sparse ? mask_first<WPL, true>(slot, R1, start, n) : z;
+        }
+        s1 = b1.w < 0x80000000u;
+    }
+
+    // E: coefficients, then the new values of the lane's rows
+    const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
+    const bool lact = 4 * WPL * l < n;                           // the lane holds rows below n
+    const uint32_t loff = lact ? (uint32_t)(4 * WPL * l) : 0u;   // their byte offset
+    uint32_t x[WPL], y[WPL], g1[WPL], g2[WPL];
+    load_words<WPL>(w1 + loff, x);
+    load_words<WPL>(w2 + loff, y);
+    load_words<WPL>(E.g + (uint32_t)R1 * st + loff, g1);
+    load_words<WPL>(E.g + (uint32_t)R2 * st + loff, g2);
+    const uint32_t rs = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R1) +
+                        lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R2);
+    const int e11 = (int)lds8(w1 + (uint32_t)R1) - 1, e22 = (int)lds8(w2 + (uint32_t)R2) - 1;
+    const bool two = R2 != R1, sw = kind == 1, pair = kind == 2 && two;
+    const int m11 = sw || (GEN && kind == 3) ? -e11 : -2 * e11, m22 = sw ? -e22 : -2 * e22;
+    q.a1 = m11;
+    q.b1 = sw ? (s1 ? m11 : -m11) : kind == 2 && !two ? m22 : 0;
+    q.a2 = sw ? (s2 ? m22 : -m22) : 0;
+    q.b2 = sw || pair ? m22 : 0;
+    if (GEN && kind == 3) q.b1 = s1 ? 1 : -1;
+    {
+        // double flip over two rows (xweigh_cuda.cu:564-583): G[R1][R2]
+        const int e21 = (int)lds8(w1 + (uint32_t)R2) - 1, e12 = (int)lds8(w2 + (uint32_t)R1) - 1;
+        const int pk = m11 * e21 + m22 * (e12 + (C1 == C2 ? m11 : 0));
+        q.pk = pair ? pk : 0;
+    }
+    int acc = 0, pr = 0;
+    const uint32_t s8 = (uint32_t)(32 * WPL * l);   // bit offset of the lane's first row
+#pragma unroll
+    for (int j = 0; j < WPL; ++j) {
+        // columns R1 and R2 of the changed rows are left out (the entry of a
+        // double flip over two rows apart): their W reads as zero
+        const uint32_t h1 = 8u * (uint32_t)R1 - s8 - 32u * j, h2 = 8u * (uint32_t)R2 - s8 - 32u * j;
+        const uint32_t mm = shl_clamp(0xffu, h1) | shl_clamp(0xffu, h2);
+        const uint32_t xx = ((x[j] & ~mm) | (0x01010101u & mm)) - 0x01010101u;
+        const uint32_t yy = ((y[j] & ~mm) | (0x01010101u & mm)) - 0x01010101u;
+        const uint32_t n1 = g1[j] + (uint32_t)q.a1 * xx + (uint32_t)q.b1 * yy + shl_clamp((uint32_t)q.pk, h2);
+        const uint32_t n2 = g2[j] + (uint32_t)q.a2 * xx + (uint32_t)q.b2 * yy;
+        const uint32_t v1 = __vabsdiffu4(n1, 0x80808080u), v2 = __vabsdiffu4(n2, 0x80808080u);
+        const uint32_t z1 = (v1 + 0x7f7f7f7fu) & 0x80808080u, z2 = (v2 + 0x7f7f7f7fu) & 0x80808080u;
+        uint32_t t = (uint32_t)acc;
+        t = __dp4a(v1, 0x01010101u, t);
+        t = __dp4a(v2, 0x01010101u, t);
+        t = __dp4a(z1, 0x20202020u, t);   // 128 * 32: 4096 a conflict
+        t = __dp4a(z2, 0x20202020u, t);
+        acc = (int)t;
+        if (GEN) {
+            if (E.obj_kind == 1) {
+                const int d1 = (int)(n1 ^ 0x80808080u), d2 = (int)(n2 ^ 0x80808080u);
+                const int o1 = (int)(g1[j] ^ 0x80808080u), o2 = (int)(g2[j] ^ 0x80808080u);
+                pr = __dp4a(d1, d1, pr) + __dp4a(d2, d2, 0) - __dp4a(o1, o1, 0) - __dp4a(o2, o2, 0);
+            } else if (E.obj_kind == 2) {
+                // 128 is even: the biased byte has the entry's parity
+                pr += __popc((n1 & 0x01010101u) | ((n2 & 0x01010101u) << 1)) -
+                      __popc((g1[j] & 0x01010101u) | ((g2[j] & 0x01010101u) << 1));
+            }
+        }
+    }
+    if (!lact) {
+        acc = 0;
+        pr = 0;
+    }
+    // less the rows' old sums (their conflicts weigh 4096 here, 2^18 in rs)
+    if (l == 0) acc -= (int)rs - (int)(rs >> kConfShift) * ((1 << kConfShift) - 4096);
+#pragma unroll
+    for (int d = 1; d < LPC; d <<= 1) acc += __shfl_xor_sync(gm, acc, d);
+    if (GEN && E.obj_kind != 0) {
+#pragma unroll
+        for (int d = 1; d < LPC; d <<= 1) pr += __shfl_xor_sync(gm, pr, d);
+    } else {
+        pr = acc - ((acc + 2048) >> 12) * 4096;
+    }
+    q.R1 = R1;
+    q.R2 = R2;
+    q.C1 = C1;
+    q.C2 = C2;
+    q.p1 = p1;
+    q.p2 = p2;
+    q.kind = kind;
+    q.acc = acc;
+    q.prim = pr;
+    return q;
+}
+
+// The least (objective, score, conflicts, index) over the groups with `act`
+// (by_index: the least index), as two ordered words, B's low five bits the
+// group; all ones when there is none.
+__device__ __forceinline__ void best_keys(bool gen_obj, const Cand& q, bool act, int g, bool by_index, unsigned gm,
+                                          uint32_t& A, uint32_t& B) {
+    const int dc = (q.acc + 2048) >> 12, ds = q.acc - dc * 4096;
+    const uint32_t low = ((uint32_t)(dc + 256) << 5) | (uint32_t)g;
+    if (!gen_obj) {
+        const uint32_t ka = by_index ? (uint32_t)g : ((uint32_t)(ds + 2048) << 14) | low;
+        A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
+        B = A;
+    } else {
+        const uint32_t ka = by_index ? (uint32_t)g : ((uint32_t)(q.prim + (1 << 19)) << 12) | (uint32_t)(ds + 2048);
+        A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
+        B = __reduce_min_sync(gm, act && ka == A ? low : 0xffffffffu);
+    }
+}
+
+// draw_block with the replica's round keys from the slot: five broadcast
+// reads in place of the eighteen additions of the key schedule.
+__device__ __forceinline__ uint4 philox_keys(uint32_t slot, uint64_t it, uint32_t stream, const uint4* keys) {
+    uint4 c = make_uint4(slot, (uint32_t)it, (uint32_t)(it >> 32), stream);
+#pragma unroll
+    for (int r = 0; r < 5; ++r) {
+        const uint4 k = keys[r];
+        c = philox_round(c, k.x, k.y);
+        c = philox_round(c, k.z, k.w);
+    }
+    return c;
+}
+
+// Fills the draw buffer of a group: block b of candidate c0 + i of
+// iteration `it` (multi), or of candidate 0 of iteration it + i (a run of
+// one-candidate iterations), i = 0..3, as block i*bpc + b.  MOVE: the
+// move-level block of iteration `it` goes into block 24.
+template <int GW, bool MOVE = false>
+__device__ __forceinline__ void fill_draws(const Env& E, const Con* con, uint64_t it, int c0, bool multi, int lane) {
+    uint4* dbuf = reinterpret_cast<uint4*>(xw_smem + E.draws);
+#pragma unroll
+    for (int h = 0; h < (GW == 16 ? 2 : 1); ++h) {
+        const int qb = lane + 16 * h;
+        const uint32_t i = E.dq[h] >> 16, b1 = E.dq[h] & 255u;   // b1 = 1 + b
+        const uint32_t dslot = MOVE && qb == 24 ? 0u : b1 + (multi ? 128u * ((uint32_t)c0 + i) : 0u);
+        const uint4 d = philox_keys(dslot, it + (uint64_t)(multi ? 0u : i), con->stream, con->keys);
+        if (qb < (MOVE ? 25 : 24)) dbuf[qb] = d;
+    }
+}
+
+// The Metropolis test of a change `prim` of the objective with draw `u` at
+// the replica's temperature (xweigh_cuda.cu:1040-1060).  Thresholds beyond
+// the table are at most one above its last (the products they round lie
+// below it), so a draw above that rejects; the rest, and the draw that a
+// threshold of 2^32 would need, take the exponential.
+template <int WPL>
+__device__ __forceinline__ bool accepts_far(uint32_t slot, int prim, uint32_t u) {
+    return metropolis_accept(prim, con_of<WPL>(slot)->T, u);
+}
+
+template <int WPL>
+__device__ __forceinline__ bool accepts(uint32_t slot, int prim, uint32_t u) {
+    const int i = min(max(prim, 1), (int)kThrTable);
+    const uint32_t t = lds32(slot + Slot<WPL>::thr + 4u * (uint32_t)(i - 1));
+    const bool below = u < t || prim <= 0;
+    if (prim > 0 && ((prim > (int)kThrTable && u <= t) || u == 0xffffffffu)) return accepts_far<WPL>(slot, prim, u);
+    return below;
+}
+
+// More than four candidates: the first best of `count` candidates, four a
+// pass; the winner's move and deltas in every lane.
+struct Winner {
+    Move mv;
+    int acc, prim, two;   // two: candidates of the iteration that change two rows
+};
+
+template <int WPL, bool GEN, int GW, bool ONEZ>
+__device__ __forceinline__ Winner choose_many(const Env E, uint64_t it, int count, int lane) {
+    constexpr int LPC = GW / 4;
+    const unsigned gm = group_mask<GW>();
+    const int g = lane / LPC, wl0 = (int)(threadIdx.x & 31u) - lane;
+    uint32_t bestA = 0xffffffffu, bestB = 0xffffffffu;
+    Winner w{};
+#pragma unroll 1
+    for (int c0 = 0; c0 < count; c0 += 4) {
+        __syncwarp(gm);
+        fill_draws<GW>(E, con_of<WPL>(E.slot), it, c0, true, lane);
+        __syncwarp(gm);
+        const int c = c0 + g;
+        const bool act = c < count;
+        const Cand q = candidate<WPL, GEN, GW, ONEZ>(E, it, 0, c, act, lane);
+        w.two += __popc(__ballot_sync(gm, act && q.R2 != q.R1 && (lane & (LPC - 1)) == 0));
+        uint32_t A, B;
+        best_keys(GEN && E.obj_kind != 0, q, act, g, false, gm, A, B);
+        // a later pass wins only strictly: its candidates come after
+        const uint32_t ka = GEN && E.obj_kind != 0 ? A : A >> 5, kb = GEN && E.obj_kind != 0 ? B >> 5 : 0u;
+        if (ka < bestA || (ka == bestA && kb < bestB)) {
+            bestA = ka;
+            bestB = kb;
+            const int src = wl0 + (int)(B & 3u) * LPC;
+            w.mv = move_of(pack_move(q), src, gm);
+            w.acc = __shfl_sync(gm, q.acc, src);
+            w.prim = __shfl_sync(gm, q.prim, src);
+        }
+    }
+    return w;
 }
 
 __device__ __forceinline__ int packed_abs(int v) {
@@ -628,100 +748,136 @@ __device__ __forceinline__ int packed_abs(int v) {
     return iabs(v) + (v != 0 ? 1 << kConfShift : 0);
 }
 
-// Commits a move (commit_*, xweigh_cuda.cu:607-877): the one or two Gram
-// rows and their mirrored columns, the packed residuals, W, the support
-// masks and the minority lists.  Lane o owns rows o, o + GW, ...
-template <int WPL, bool GEN, int GW, bool ONEZ>
-__device__ __forceinline__ void commit(const Env& E, const Move& mv, int lane) {
-    constexpr int OPL = WPL;
+// Commits a move (commit_*, xweigh_cuda.cu:607-877) whose deltas are `acc`:
+// the one or two Gram rows (words, by the first group's lanes) and their
+// mirrored columns, the packed residuals, W, the support masks and the
+// minority lists.  Lane o owns rows o, o + GW, ... of the columns.
+template <int WPL, int GW, bool ONEZ>
+__device__ __forceinline__ void commit(const Env& E, const Move& mv, int acc, int lane) {
+    constexpr int LPC = GW / 4;
     const unsigned gm = group_mask<GW>();
     const int n = E.n, m = ONEZ ? 1 : E.m, sparse = ONEZ ? 0 : E.sparse;
     const uint32_t st = E.st, slot = E.slot, wbase = E.slot + Slot<WPL>::w;
     const int R1 = (int)(mv.rc & 255u), R2 = (int)((mv.rc >> 8) & 255u);
     const int C1 = (int)((mv.rc >> 16) & 255u), C2 = (int)(mv.rc >> 24);
-    const int a1 = (int)(int8_t)(mv.cf & 255u), b1 = (int)(int8_t)((mv.cf >> 8) & 255u);
-    const int a2 = (int)(int8_t)((mv.cf >> 16) & 255u), b2 = (int)(int8_t)(mv.cf >> 24);
-    const int pk = (int)(int8_t)(mv.ax & 255u);
     const bool two = R2 != R1;
     const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
-    const uint32_t g1 = E.g + (uint32_t)R1 * st, g2 = E.g + (uint32_t)R2 * st;
-    int S1 = 0, S2 = 0;
+    const uint32_t r1 = E.g + (uint32_t)R1 * st, r2 = E.g + (uint32_t)R2 * st;
+    // the new rows, as candidate() evaluated them
+    const int l = lane & (LPC - 1);
+    const bool lact = 4 * WPL * l < n;
+    const uint32_t loff = lact ? (uint32_t)(4 * WPL * l) : 0u, s8 = (uint32_t)(32 * WPL * l);
+    uint32_t x[WPL], y[WPL], g1[WPL], g2[WPL];
+    load_words<WPL>(w1 + loff, x);
+    load_words<WPL>(w2 + loff, y);
+    load_words<WPL>(r1 + loff, g1);
+    load_words<WPL>(r2 + loff, g2);
+    {
+        const int a1 = (int)(int8_t)(mv.cf & 255u), b1 = (int)(int8_t)((mv.cf >> 8) & 255u);
+        const int a2 = (int)(int8_t)((mv.cf >> 16) & 255u), b2 = (int)(int8_t)(mv.cf >> 24);
+        const int pk = (int)(int8_t)(mv.ax & 255u);
 #pragma unroll
-    for (int k = 0; k < OPL; ++k) {
+        for (int j = 0; j < WPL; ++j) {
+            const uint32_t h1 = 8u * (uint32_t)R1 - s8 - 32u * j, h2 = 8u * (uint32_t)R2 - s8 - 32u * j;
+            const uint32_t mm = shl_clamp(0xffu, h1) | shl_clamp(0xffu, h2);
+            const uint32_t xx = ((x[j] & ~mm) | (0x01010101u & mm)) - 0x01010101u;
+            const uint32_t yy = ((y[j] & ~mm) | (0x01010101u & mm)) - 0x01010101u;
+            g1[j] += (uint32_t)a1 * xx + (uint32_t)b1 * yy + shl_clamp((uint32_t)pk, h2);
+            g2[j] += (uint32_t)a2 * xx + (uint32_t)b2 * yy;
+        }
+    }
+    uint32_t old[WPL];   // old bytes of rows R1, R2 at the lane's columns
+#pragma unroll
+    for (int k = 0; k < WPL; ++k) {
         const int o = lane + GW * k;
-        if (o < n && o != R1) {
-            const int x = (int)lds8(w1 + (uint32_t)o) - 1, y = (int)lds8(w2 + (uint32_t)o) - 1;
-            const int o1 = (int)lds8(g1 + (uint32_t)o) - 128;
-            const bool pair = two && o == R2;
-            const int n1 = o1 + (pair ? pk : a1 * x + b1 * y);
-            const int d1 = packed_abs(n1) - packed_abs(o1);
-            xw_smem[g1 + (uint32_t)o] = (uint8_t)(n1 + 128);
-            xw_smem[E.g + (uint32_t)o * st + (uint32_t)R1] = (uint8_t)(n1 + 128);
-            S1 += d1;
-            int d2 = 0;
-            if (two) {
-                if (pair) {
-                    S2 += d1;
-                } else {
-                    const int o2 = (int)lds8(g2 + (uint32_t)o) - 128;
-                    const int n2 = o2 + a2 * x + b2 * y;
-                    d2 = packed_abs(n2) - packed_abs(o2);
-                    xw_smem[g2 + (uint32_t)o] = (uint8_t)(n2 + 128);
-                    xw_smem[E.g + (uint32_t)o * st + (uint32_t)R2] = (uint8_t)(n2 + 128);
-                    S2 += d2;
-                }
-            }
-            if (!pair) {
-                int* r = reinterpret_cast<int*>(xw_smem + slot + Slot<WPL>::res) + o;
-                *r += d1 + d2;
-            }
+        old[k] = 0;
+        if (o < n) old[k] = (lds8(r1 + (uint32_t)o) << 8) | (lds8(r2 + (uint32_t)o) << 24);
+    }
+    __syncwarp(gm);
+    if (lane < LPC && lact) {
+        if constexpr (WPL == 1) {
+            *reinterpret_cast<uint32_t*>(xw_smem + r1 + loff) = g1[0];
+            if (two) *reinterpret_cast<uint32_t*>(xw_smem + r2 + loff) = g2[0];
+        } else if constexpr (WPL == 2) {
+            *reinterpret_cast<uint2*>(xw_smem + r1 + loff) = make_uint2(g1[0], g1[1]);
+            if (two) *reinterpret_cast<uint2*>(xw_smem + r2 + loff) = make_uint2(g2[0], g2[1]);
+        } else {
+            *reinterpret_cast<uint4*>(xw_smem + r1 + loff) = make_uint4(g1[0], g1[1], g1[2], g1[3]);
+            if (two) *reinterpret_cast<uint4*>(xw_smem + r2 + loff) = make_uint4(g2[0], g2[1], g2[2], g2[3]);
+        }
+    }
+    __syncwarp(gm);
+    // columns R1 and R2 (entry (R2, R1) of a double flip over two rows comes
+    // from row R1) and the residuals: byte weights +1 new, -1 old
+    const int wt1 = 0x0000ff01, wt = two ? (int)0xff01ff01u : wt1;
+    int d1[WPL], d[WPL], S1 = 0;
+#pragma unroll
+    for (int k = 0; k < WPL; ++k) {
+        const int o = lane + GW * k;
+        d1[k] = d[k] = 0;
+        if (o < n) {
+            const uint32_t n1 = lds8(r1 + (uint32_t)o), n2 = lds8(r2 + (uint32_t)o);
+            const uint32_t col = E.g + (uint32_t)o * st;
+            xw_smem[col + (uint32_t)R1] = (uint8_t)n1;
+            if (o != R1) xw_smem[col + (uint32_t)R2] = (uint8_t)n2;
+            const uint32_t v = __vabsdiffu4(old[k] | n1 | (n2 << 16), 0x80808080u);
+            const uint32_t z = ((v + 0x7f7f7f7fu) & 0x80808080u) >> 7;
+            d1[k] = __dp4a((int)v, wt1, 0) + (__dp4a((int)z, wt1, 0) << kConfShift);
+            d[k] = __dp4a((int)v, wt, 0) + (__dp4a((int)z, wt, 0) << kConfShift);
+            S1 += d1[k];
         }
     }
     S1 = __reduce_add_sync(gm, S1);
-    S2 = two ? __reduce_add_sync(gm, S2) : 0;
-    __syncwarp(gm);
-    // one changed entry of W per lane 0..3; rows R1 (lane 0) and R2 (lane
-    // 1): residual, support mask and minority entry
+    const int dc = (acc + 2048) >> 12;
+    const int S = acc - dc * 4096 + dc * (1 << kConfShift);   // both rows, the pair entry once
+#pragma unroll
+    for (int k = 0; k < WPL; ++k) {
+        const int o = lane + GW * k;
+        if (o < n) {
+            int* r = reinterpret_cast<int*>(xw_smem + slot + Slot<WPL>::res) + o;
+            *r += o == R1 ? S1 : o == R2 ? S - S1 + d1[k] : d[k];
+        }
+    }
+    // one changed entry of W per lane 0..3
     if (lane < 4) {
         const int cfc = (int)(int8_t)((mv.cf >> (8 * lane)) & 255u);
         if (cfc != 0) {
             const uint32_t a = ((lane & 1) ? w2 : w1) + (uint32_t)((lane & 2) ? R2 : R1);
             xw_smem[a] = (uint8_t)(lds8(a) + (uint32_t)cfc);
         }
-        if (lane == 0 || (lane == 1 && two)) {
+        // support mask and minority entry of rows R1 (lane 0) and R2 (lane 1)
+        if (lane < 2 && ((mv.ax >> (24 + lane)) & 1u)) {
             const int R = lane ? R2 : R1;
-            int* r = reinterpret_cast<int*>(xw_smem + slot + Slot<WPL>::res) + R;
-            *r += lane ? S2 : S1;
-            if ((mv.ax >> (24 + lane)) & 1u) {
-                if constexpr (WPL == 1) {
-                    uint32_t* mk = reinterpret_cast<uint32_t*>(xw_smem + slot + Slot<WPL>::mask) + R;
-                    *mk ^= (1u << C1) ^ (1u << C2);
-                } else {
-                    uint64_t* mk = reinterpret_cast<uint64_t*>(xw_smem + slot + Slot<WPL>::mask) + (WPL / 2) * R;
-                    mk[C1 >> 6] ^= 1ull << (C1 & 63);
-                    mk[C2 >> 6] ^= 1ull << (C2 & 63);
-                }
-                // row R1 loses C1 and gains C2, row R2 the other way
-                const int lost = lane ? C2 : C1, got = lane ? C1 : C2;
-                const int p = (int)((mv.ax >> (8 + 8 * lane)) & 255u);
-                xw_smem[E.mino + (uint32_t)(R * m + p)] = (uint8_t)(sparse ? got : lost);
+            if constexpr (ONEZ) {
+            } else if constexpr (WPL == 1) {
+                uint32_t* mk = reinterpret_cast<uint32_t*>(xw_smem + slot + Slot<WPL>::mask) + R;
+                *mk ^= (1u << C1) ^ (1u << C2);
+            } else {
+                uint64_t* mk = reinterpret_cast<uint64_t*>(xw_smem + slot + Slot<WPL>::mask) + (WPL / 2) * R;
+                mk[C1 >> 6] ^= 1ull << (C1 & 63);
+                mk[C2 >> 6] ^= 1ull << (C2 & 63);
             }
+            // row R1 loses C1 and gains C2, row R2 the other way
+            const int lost = lane ? C2 : C1, got = lane ? C1 : C2;
+            const int p = (int)((mv.ax >> (8 + 8 * lane)) & 255u);
+            xw_smem[E.mino + (uint32_t)(R * m + p)] = (uint8_t)(sparse ? got : lost);
         }
     }
-    __syncwarp(gm);
 }
 
 // tab[d-1] = ceil(exp(-d/T) * 2^32), computed with the same division and
 // exponential as metropolis_accept, so that for a 32-bit draw u
 //   u * 2^-32 < exp(-d/T)  <=>  u < tab[d-1]
 // exactly (both sides scaled by 2^32 without rounding; u is an integer).
+// 2^32 itself (T above 4e9) is kept as 2^32 - 1 in a 32-bit table.
 // Rebuilt whenever the replica's temperature changes.
-template <int GW = 32>
-__device__ __noinline__ void build_thresholds(uint64_t* tab, double T, int lane) {
+template <int GW = 32, typename TAB>
+__device__ __forceinline__ void build_thresholds(TAB* tab, double T, int lane) {
     const double t = T > 1.0e-12 ? T : 1.0e-12;
     for (uint32_t d = lane + 1; d <= kThrTable; d += GW) {
         const double e = acceptance_exp(__ddiv_rn(-(double)d, t));
-        tab[d - 1] = (uint64_t)ceil(__dmul_rn(e, 0x1p32));
+        const uint64_t v = (uint64_t)ceil(__dmul_rn(e, 0x1p32));
+        tab[d - 1] = sizeof(TAB) == 4 && v > 0xffffffffull ? (TAB)0xffffffffu : (TAB)v;
     }
     __syncwarp(group_mask<GW>());
 }
@@ -748,58 +904,31 @@ __device__ __noinline__ void save_w(int8_t* dst, uint32_t wbase, uint32_t st, in
         for (int r = lane; r < n; r += GW) dst[(uint32_t)(c * n + r)] = (int8_t)((int)lds8(wbase + (uint32_t)c * st + (uint32_t)r) - 1);
 }
 
-// Scalar state of a loaded replica.
-struct State {
-    uint8_t* rec;
-    RepHeader* H;
-    XwJob* J;
-    uint64_t it;
-    int score, conflicts, best_s, best_c, msi, cool;
-    int64_t obj_total;
-    uint32_t accepted, accepted_rows;
-    // the best W is the current one and its record is older: it is written
-    // when an accepted move leaves it, or at the end
-    bool dirty;
-    // the copy that writes the record (a cluster's other CTAs keep an
-    // identical copy in their own shared memory and write nothing)
-    bool owner;
-};
-
-// Lane-invariant parts of the context, from the job and the slot.
+// The lane's context, from the job and the slot.
 template <int WPL, int GW, bool ONEZ>
-__device__ __forceinline__ void make_env(Env& E, const XwJob* J, const RepHeader* H, uint32_t slot, uint32_t draws,
-                                         int lane, int obj_kind) {
+__device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, uint32_t draws, int lane, int obj_kind) {
     constexpr int LPC = GW / 4;
     const int n = J->n;
     E.slot = slot;
     E.draws = draws;
     E.n = n;
-    E.w = ONEZ ? n - 1 : J->w;
     E.m = ONEZ ? 1 : J->m;
     E.sparse = ONEZ ? 0 : J->sparse;
+    E.full = !ONEZ && J->w == n;
     E.st = packed_stride(n, WPL);
     const uint32_t mat = xw_pad16((uint32_t)n * E.st);
     E.g = slot + Slot<WPL>::w + mat;
     E.mino = E.g + mat;
-    E.k0 = J->key0;
-    E.k1 = J->key1;
-    E.stream = H->stream;
-    E.cs = J->candidate_samples;
     E.ts = J->target_samples;
     E.bpc = 4 + (E.ts <= 4 ? 1 : 2);   // cached blocks per candidate
+    E.cw = draws + (uint32_t)((lane / LPC) * E.bpc) * 16u;
     E.move_set = J->move_set;
     E.obj_kind = obj_kind;
-    E.l = lane & (LPC - 1);
-    E.grp = lane / LPC;
-    E.lact = 4 * WPL * E.l < n;
-    E.loff = E.lact ? (uint32_t)(4 * WPL * E.l) : 0u;
-    auto slot_of = [&](int q) -> uint32_t {
-        if (q == 0) return 0u;
-        const int c = (q - 1) / E.bpc;
-        return cand_slot(c, (q - 1) - c * E.bpc);
-    };
-    E.my_slot = slot_of(lane);
-    E.my_slot2 = GW == 16 ? slot_of(lane + 16) : 0u;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const int i = (lane + 16 * h) / E.bpc;
+        E.dq[h] = ((uint32_t)i << 16) | (uint32_t)(1 + lane + 16 * h - i * E.bpc);
+    }
 }
 
 // Loads replica `rid` into the slot: W and the minority lists; the masks,
@@ -811,17 +940,13 @@ __device__ __forceinline__ void make_env(Env& E, const XwJob* J, const RepHeader
 // the exits on the job's done and solved flags, which other kernels may set
 // while it loads (its owner decides whether the replica runs).
 template <int WPL, bool GEN, int GW, bool ONEZ>
-__device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, uint32_t draws, int lane,
-                                             uint64_t& iters, Env& E, State& S, bool owner) {
+__device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane, uint64_t iters,
+                                             Env& E, bool owner) {
     constexpr int OPL = WPL;   // rows o, o + GW, ... of a lane: GW * OPL >= n
     const unsigned gm = group_mask<GW>();
     uint8_t* rec = a.arena + a.rec_off[rid];
     RepHeader* H = reinterpret_cast<RepHeader*>(rec);
     XwJob* J = a.jobs + H->job;
-    S.rec = rec;
-    S.H = H;
-    S.J = J;
-    S.owner = owner;
     if (owner && *(volatile int32_t*)&J->done) return false;
     if (owner && a.stop_on_solve == 1 && *(volatile int32_t*)&J->solved) return false;
     const int obj_kind = GEN ? H->obj_kind : 0;
@@ -830,12 +955,12 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
         if (lane == 0) H->err |= XW_ERR_KERNEL;
         return false;
     }
-    make_env<WPL, GW, ONEZ>(E, J, H, slot, draws, lane, obj_kind);
-    const int n = E.n, w = E.w, m = E.m, sparse = E.sparse;
-    S.it = H->it;
+    make_env<WPL, GW, ONEZ>(E, J, slot, slot + Slot<WPL>::draws, lane, obj_kind);
+    const int n = E.n, w = ONEZ ? n - 1 : J->w, m = E.m, sparse = E.sparse;
+    const uint64_t it = H->it;
     if (J->budget_iters) {
-        if (S.it >= J->budget_iters) return false;
-        if (iters > J->budget_iters - S.it) iters = J->budget_iters - S.it;
+        if (it >= J->budget_iters) return false;
+        if (iters > J->budget_iters - it) iters = J->budget_iters - it;
     }
     const uint32_t status0 = H->status;
     const uint32_t st = E.st, wbase = slot + Slot<WPL>::w;
@@ -851,8 +976,8 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
     const int8_t* gw = reinterpret_cast<const int8_t*>(rec + J->off_w);
 #pragma unroll
     for (int q = 0; q < WPL; ++q) {
-#pragma unroll 1
-        for (int c = 32 * q; c < n && c < 32 * q + 32; ++c) {
+#pragma unroll 4
+        for (int c = 32 * q; c < min(n, 32 * q + 32); ++c) {
 #pragma unroll
             for (int k = 0; k < OPL; ++k) {
                 const int o = lane + GW * k;
@@ -956,153 +1081,176 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
     __syncwarp(gm);
 
     const int64_t obj0 = obj_kind == 1 ? sq0 : obj_kind == 2 ? par0 : score0;
-    if (status0 & XW_STATUS_INIT) {
-        if (H->score != score0 || H->conflicts != conf0 || H->obj_total != obj0) {
-            if (lane == 0 && owner) H->err |= XW_ERR_SCORE;
-            return false;
-        }
-        S.best_s = H->best_score;
-        S.best_c = H->best_conflicts;
-        S.msi = H->msi;
-        S.cool = H->cool_ctr;
-        S.accepted = H->accepted;
-        S.accepted_rows = H->accepted_rows;
-        S.dirty = false;
-    } else {
-        S.best_s = score0;
-        S.best_c = conf0;
-        S.msi = 0;
-        S.cool = 0;
-        S.accepted = 0;
-        S.accepted_rows = 0;
-        S.dirty = true;
+    const bool init = status0 & XW_STATUS_INIT;
+    if (init && (H->score != score0 || H->conflicts != conf0 || H->obj_total != obj0)) {
+        if (lane == 0 && owner) H->err |= XW_ERR_SCORE;
+        return false;
     }
-    S.score = score0;
-    S.conflicts = conf0;
-    S.obj_total = obj0;
     if (lane == 0) {
         Con c;
         c.thr_target = J->thr_target;
         c.thr_dbl = GEN && J->move_set == 1 ? 0 : J->thr_double;
         c.thr_sign = J->thr_sign;
         c.thr_swsign = J->thr_swsign;
+        c.k0 = J->key0;
+        c.k1 = J->key1;
+        c.stream = H->stream;
+        c.cs = J->candidate_samples;
+#pragma unroll
+        for (uint32_t r = 0; r < 5; ++r)
+            c.keys[r] = make_uint4(c.k0 + 2 * r * 0x9E3779B9u, c.k1 + 2 * r * 0xBB67AE85u,
+                                   c.k0 + (2 * r + 1) * 0x9E3779B9u, c.k1 + (2 * r + 1) * 0xBB67AE85u);
+        c.it0 = it;
         c.thr_greedy = J->thr_greedy;
+        auto coin = [](uint64_t t) -> uint32_t { return t > 0xffffffffull ? 0xffffffffu : (uint32_t)t; };
+        c.coins = make_uint4(coin(c.thr_target), coin(c.thr_dbl), coin(c.thr_sign), coin(c.thr_swsign));
         c.T = H->temperature;
-        *reinterpret_cast<Con*>(xw_smem + slot + Slot<WPL>::con) = c;
+        c.best = make_int4(score0, conf0, init ? H->best_score : score0, init ? H->best_conflicts : conf0);
+        c.acc = make_int4((int)(uint32_t)obj0, (int)(obj0 >> 32), init ? (int)H->accepted : 0,
+                          init ? (int)H->accepted_rows : 0);
+        c.mb = init ? -H->msi : 0;
+        c.cb = init ? -H->cool_ctr : 0;
+        c.k_end = (int32_t)(iters < 0x7ffffffeull ? iters : 0x7ffffffeull);
+        c.dirty = init ? 0 : 1;
+        c.owner = owner ? 1 : 0;
+        c.rid = rid;
+        *con_of<WPL>(slot) = c;
     }
     __syncwarp(gm);
-    build_thresholds<GW>(reinterpret_cast<uint64_t*>(xw_smem + slot + Slot<WPL>::thr), H->temperature, lane);
+    build_thresholds<GW>(reinterpret_cast<uint32_t*>(xw_smem + slot + Slot<WPL>::thr), H->temperature, lane);
     return true;
 }
 
 // Writes the replica's W, minority lists and scalar state back to its
-// record; `calls` moves were made since it was loaded, with `evals`
-// candidates evaluated, `evals2` of them changing two rows.
+// record after `k` calls, with `evals` candidates evaluated, `evals2` of
+// them changing two rows.
 template <int WPL, int GW>
-__device__ __forceinline__ void store_replica(const Env& E, State& S, uint64_t calls, uint64_t evals, uint32_t evals2,
+__device__ __forceinline__ void store_replica(const AnnealArgs& a, const Env& E, int k, uint64_t evals, uint32_t evals2,
                                               int lane) {
     const unsigned gm = group_mask<GW>();
     __syncwarp(gm);
-    if (S.dirty) save_w<WPL, GW>(reinterpret_cast<int8_t*>(S.rec + S.J->off_best), E.slot + Slot<WPL>::w, E.st, E.n, lane);
-    save_w<WPL, GW>(reinterpret_cast<int8_t*>(S.rec + S.J->off_w), E.slot + Slot<WPL>::w, E.st, E.n, lane);
-    uint8_t* gmo = S.rec + S.J->off_mino;
+    const Con* con = con_of<WPL>(E.slot);
+    uint8_t* rec = a.arena + a.rec_off[con->rid];
+    RepHeader* H = reinterpret_cast<RepHeader*>(rec);
+    const XwJob* J = a.jobs + H->job;
+    const uint32_t wbase = E.slot + Slot<WPL>::w;
+    if (con->dirty) save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_best), wbase, E.st, E.n, lane);
+    save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_w), wbase, E.st, E.n, lane);
+    uint8_t* gmo = rec + J->off_mino;
     for (uint32_t i = lane; i < (uint32_t)(E.n * E.m); i += GW) gmo[i] = xw_smem[E.mino + i];
     if (lane == 0) {
-        RepHeader* H = S.H;
         const bool init = H->status & XW_STATUS_INIT;
-        H->it = S.it;
-        H->moves = (init ? H->moves : 0) + calls;
+        H->it = con->it0 + (uint64_t)k;
+        H->moves = (init ? H->moves : 0) + (uint64_t)k;
         H->cand_evals = (init ? H->cand_evals : 0) + evals;
-        H->accepted = S.accepted;
-        H->accepted_rows = S.accepted_rows;
+        H->accepted = (uint32_t)con->acc.z;
+        H->accepted_rows = (uint32_t)con->acc.w;
         H->two_row_evals = (init ? H->two_row_evals : 0) + evals2;
-        H->score = S.score;
-        H->conflicts = S.conflicts;
-        H->best_score = S.best_s;
-        H->best_conflicts = S.best_c;
-        H->obj_total = S.obj_total;
-        H->temperature = reinterpret_cast<const Con*>(xw_smem + E.slot + Slot<WPL>::con)->T;
-        H->msi = S.msi;
-        H->cool_ctr = S.cool;
-        H->status = H->status | XW_STATUS_INIT | (S.best_s == 0 ? XW_STATUS_SOLVED : 0u);
+        H->score = con->best.x;
+        H->conflicts = con->best.y;
+        H->best_score = con->best.z;
+        H->best_conflicts = con->best.w;
+        H->obj_total = (int64_t)(((uint64_t)(uint32_t)con->acc.y << 32) | (uint32_t)con->acc.x);
+        H->temperature = con->T;
+        H->msi = k - con->mb;
+        H->cool_ctr = J->tempering ? -con->cb : k - con->cb;   // tempering leaves it alone
+        H->status = H->status | XW_STATUS_INIT | (con->best.z == 0 ? XW_STATUS_SOLVED : 0u);
     }
     __syncwarp(gm);
 }
 
-// The Metropolis test of a chosen move at the replica's temperature (xweigh_cuda.cu:1040-1060).
-template <int WPL>
-__device__ __forceinline__ bool accepts(const Env& E, const Pick& P) {
-    if (P.prim <= 0) return true;
-    if (P.prim <= (int)kThrTable) return (uint64_t)P.u < lds64(E.slot + Slot<WPL>::thr + 8u * (uint32_t)(P.prim - 1));
-    return metropolis_accept(P.prim, reinterpret_cast<const Con*>(xw_smem + E.slot + Slot<WPL>::con)->T, P.u);
-}
-
-// One move call whose Metropolis outcome is `accept`: the commit, best
-// tracking (and the job's solve flag), cooling and reheat
-// (xweigh_cuda.cu:1087-1129).  S.it is the iteration's number.
+// Commits the accepted move `mv` of call k (iteration it0 + k - 1; k counts
+// it) with deltas `acc` and `prim`: the state, best tracking and the job's
+// solve flag.  True when the best improved.
 template <int WPL, bool GEN, int GW, bool ONEZ>
-__device__ __forceinline__ void apply(const Env& E, State& S, Pick& P, bool accept, int tempering, int mpc, int stuck,
-                                      int lane) {
+__device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, const Move& mv, int acc, int prim, int k,
+                                            int lane) {
     const unsigned gm = group_mask<GW>();
-    bool improved = false;
-    if (accept) {
-        const int ns = S.score + P.ds, nc = S.conflicts + P.dc;
-        improved = ns < S.best_s || (ns == S.best_s && nc < S.best_c);
-        if (S.dirty && !improved) {
-            if (S.owner)
-                save_w<WPL, GW>(reinterpret_cast<int8_t*>(S.rec + S.J->off_best), E.slot + Slot<WPL>::w, E.st, E.n, lane);
-            S.dirty = false;
-            __syncwarp(gm);
-        }
-        P.mv.rc = __shfl_sync(gm, P.mv.rc, P.src);
-        P.mv.cf = __shfl_sync(gm, P.mv.cf, P.src);
-        P.mv.ax = __shfl_sync(gm, P.mv.ax, P.src);
-        commit<WPL, GEN, GW, ONEZ>(E, P.mv, lane);
-        S.score = ns;
-        S.conflicts = nc;
-        S.obj_total += P.prim;
-        ++S.accepted;
-        S.accepted_rows += (P.mv.rc & 255u) != ((P.mv.rc >> 8) & 255u) ? 2u : 1u;
+    Con* con = con_of<WPL>(E.slot);
+    const int dc = (acc + 2048) >> 12;
+    int4 b = con->best, t = con->acc;
+    const bool dirty = con->dirty != 0;
+    b.x += acc - dc * 4096;
+    b.y += dc;
+    const bool improved = b.x < b.z || (b.x == b.z && b.y < b.w);
+    if (dirty && !improved && con->owner) {
+        uint8_t* rec = a.arena + a.rec_off[con->rid];
+        const XwJob* J = a.jobs + reinterpret_cast<RepHeader*>(rec)->job;
+        save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_best), E.slot + Slot<WPL>::w, E.st, E.n, lane);
+        __syncwarp(gm);
+    }
+    commit<WPL, GW, ONEZ>(E, mv, acc, lane);
+    if (lane == 0) {
+        const long long o = (long long)(((uint64_t)(uint32_t)t.y << 32) | (uint32_t)t.x) + prim;
+        t.x = (int)(uint32_t)o;
+        t.y = (int)(o >> 32);
+        t.z += 1;
+        t.w += (mv.rc & 255u) != ((mv.rc >> 8) & 255u) ? 2 : 1;
+        con->acc = t;
         if (improved) {
-            S.best_s = ns;
-            S.best_c = nc;
-            S.dirty = true;
-            if (ns == 0 && lane == 0 && S.owner) {
-                RepHeader* H = S.H;
-                XwJob* J = S.J;
-                H->solve_it = S.it;
+            b.z = b.x;
+            b.w = b.y;
+            con->mb = k;
+            if (b.x == 0 && con->owner) {
+                RepHeader* H = reinterpret_cast<RepHeader*>(a.arena + a.rec_off[con->rid]);
+                XwJob* J = a.jobs + H->job;
+                H->solve_it = con->it0 + (uint64_t)(k - 1);
                 H->solve_ns = globaltimer();
                 if (atomicCAS(&J->solved, 0, 1) == 0) {
                     J->solved_replica = (int32_t)H->stream;
-                    J->solved_it = S.it;
+                    J->solved_it = H->solve_it;
                     J->solve_ns = H->solve_ns;
                 }
             }
         }
+        con->best = b;
+        con->dirty = improved ? 1 : 0;
     }
-    S.msi = improved ? 0 : S.msi + 1;
-    if (!tempering) {
-        ++S.cool;
-        if (S.cool >= mpc || S.msi >= stuck) {
-            Con* con = reinterpret_cast<Con*>(xw_smem + E.slot + Slot<WPL>::con);
-            const double T0 = con->T, t_min = S.J->t_min;
-            double T = T0;
-            if (S.cool >= mpc) {
-                S.cool = 0;
-                T = __dmul_rn(T, S.J->cooling);
-                if (T < t_min) T = t_min;
-            }
-            if (S.msi >= stuck) {
-                S.msi = 0;
-                T = __dmul_rn(S.H->reheat_temperature, S.J->reheat);
-                if (T < t_min) T = t_min;
-            }
-            __syncwarp(gm);
-            if (lane == 0) con->T = T;
-            if (T != T0) build_thresholds<GW>(reinterpret_cast<uint64_t*>(xw_smem + E.slot + Slot<WPL>::thr), T, lane);
-            __syncwarp(gm);
-        }
+    __syncwarp(gm);
+    return improved;
+}
+
+// Calls that can be made after call k before the temperature changes or
+// the replica's calls end: the first k at which temperature_step has
+// something to do.
+template <int WPL>
+__device__ __forceinline__ int next_event(const XwJob* J, const Con* con) {
+    long long e = con->k_end;
+    if (!J->tempering) {
+        e = min(e, (long long)con->cb + J->moves_per_cool);
+        e = min(e, (long long)con->mb + J->stuck_threshold);
     }
+    return (int)e;
+}
+
+// Cooling and reheat after call k (xweigh_cuda.cu:1087-1129).
+template <int WPL, int GW>
+__device__ __forceinline__ void temperature_step(const AnnealArgs& a, uint32_t slot, int k, int lane) {
+    const unsigned gm = group_mask<GW>();
+    Con* con = con_of<WPL>(slot);
+    const RepHeader* H = reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[con->rid]);
+    const XwJob* J = a.jobs + H->job;
+    if (J->tempering) return;
+    const bool cool = (long long)k - con->cb >= J->moves_per_cool, heat = (long long)k - con->mb >= J->stuck_threshold;
+    if (!cool && !heat) return;
+    const double T0 = con->T, t_min = J->t_min;
+    double T = T0;
+    if (cool) {
+        T = __dmul_rn(T, J->cooling);
+        if (T < t_min) T = t_min;
+    }
+    if (heat) {
+        T = __dmul_rn(H->reheat_temperature, J->reheat);
+        if (T < t_min) T = t_min;
+    }
+    __syncwarp(gm);
+    if (lane == 0) {
+        if (cool) con->cb = k;
+        if (heat) con->mb = k;
+        con->T = T;
+    }
+    if (T != T0) build_thresholds<GW>(reinterpret_cast<uint32_t*>(xw_smem + slot + Slot<WPL>::thr), T, lane);
+    __syncwarp(gm);
 }
 
 }  // namespace
