@@ -106,3 +106,66 @@ def test_rescore_empty_batch_and_bad_arguments():
                               stats.ctypes.data_as(C.POINTER(C.c_int32)), None) == X.XW_OK
     assert X.lib().xw_rescore(W.ctypes.data_as(C.POINTER(C.c_int8)), 1, 257, 16,
                               stats.ctypes.data_as(C.POINTER(C.c_int32)), None) == X.XW_ERR_INVALID
+
+
+@pytest.mark.parametrize("count", [1, 5, 700])
+@pytest.mark.parametrize("n", [9, 13, 16, 17, 31, 33, 47, 63, 65, 95, 97, 100, 127, 129, 159, 161, 192, 193, 224, 255])
+def test_padded_tensor_core_rescore_matches_int64(n, count):
+    # orders off the 32-grid (padded tiles; the remainders of a 32-row block,
+    # of a 16-byte chunk and of a K-half) and orders above 128: one matrix,
+    # a part-filled tile, more tiles than CTAs; every value an integer
+    if n > 128:
+        count = min(count, 160)
+    W = random_fixed_degree(count, n, max(1, (2 * n) // 3), seed=900 + n)
+    W[0] = np.eye(n, dtype=np.int8)          # an exact W(n,1) among them
+    w = 1
+    stats, G = X.rescore(W, n, w, gram=True)
+    ref = np.matmul(W.astype(np.float64), W.astype(np.float64).transpose(0, 2, 1)).astype(np.int64)
+    assert (G == ref).all()
+    off = ref * (1 - np.eye(n, dtype=np.int64))
+    want = np.stack([np.abs(off).sum((1, 2)) // 2, (off != 0).sum((1, 2)) // 2, (off * off).sum((1, 2)) // 2,
+                     (ref == w * np.eye(n, dtype=np.int64)).all((1, 2))], 1)
+    assert (stats == want).all()
+    assert (X.rescore(W, n, w) == want).all()
+
+
+@pytest.mark.parametrize("shift", [1, 3, 8, 15])
+@pytest.mark.parametrize("n", [26, 32, 64, 100, 128, 150])
+def test_rescore_of_device_input_at_any_address(n, shift):
+    # the input starts `shift` bytes off a 16-byte boundary and ends at the
+    # end of its allocation's values
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    count, w = 9, n // 2
+    W = random_fixed_degree(count, n, w, seed=50 + n)
+    buf = torch.full((W.size + shift,), 77, dtype=torch.int8, device="cuda")
+    buf[shift:] = torch.from_numpy(W.reshape(-1)).cuda()
+    out = torch.zeros((count, 4), dtype=torch.int32, device="cuda")
+    assert X.lib().xw_rescore_device(C.c_void_p(buf.data_ptr() + shift), count, n, w, C.c_void_p(out.data_ptr()), None, 0,
+                                     C.c_void_p(torch.cuda.current_stream().cuda_stream)) == X.XW_OK
+    torch.cuda.synchronize()
+    assert X.lib().xw_rescore_status() == X.XW_OK
+    assert (out.cpu().numpy() == X.rescore(W, n, w)).all()
+    for m in range(count):
+        assert out[m].tolist() == oracle_stats(W[m], n, w)[0]
+
+
+@pytest.mark.parametrize("top", [1, 2, 5])
+@pytest.mark.parametrize("n", [32, 64, 96, 100, 128, 192])
+def test_rescore_of_entries_that_do_not_fit_a_byte(n, top):
+    # Gram entries of up to 128 and beyond: equal full rows (w = n) and
+    # entries up to `top`, in some matrices of a batch only, so that the byte
+    # form and the word form of the epilogue run side by side
+    rng = np.random.default_rng(n + top)
+    count = 40
+    W = random_fixed_degree(count, n, n // 2, seed=n)
+    for m in range(0, count, 3):
+        W[m] = rng.integers(-top, top + 1, size=(n, n))
+        W[m, 1] = W[m, n - 1] = top
+        W[m, n // 2] = -top
+    ref = np.matmul(W.astype(np.float64), W.astype(np.float64).transpose(0, 2, 1)).astype(np.int64)
+    off = ref * (1 - np.eye(n, dtype=np.int64))
+    want = np.stack([np.abs(off).sum((1, 2)) // 2, (off != 0).sum((1, 2)) // 2, (off * off).sum((1, 2)) // 2,
+                     np.zeros(count, dtype=np.int64)], 1)
+    assert want.max() < 2 ** 30   # twice the squared score is summed in 32 bits
+    assert (X.rescore(W, n, n // 2) == want).all()

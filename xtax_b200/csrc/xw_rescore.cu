@@ -22,7 +22,13 @@
 // groups of four epilogue warps drain them, each step waiting only on the
 // mbarrier of its stage or accumulator, so that loads, MMAs and epilogues of
 // successive tiles overlap.  The bound is HBM: n^2 bytes read per matrix against 2n^3
-// MACs.
+// MACs; what limits it in fact is the epilogue's integer work (n = 128, 65536
+// matrices: 0.257 ms, 4.2 TB/s).
+//
+// Other orders up to 128 (and inputs that are not 16-byte aligned, which a
+// tensor map does not take) are padded into the ring by six warps instead of
+// the TMA producer; orders 129..256 have a kernel of their own
+// (rescore_big_kernel).
 //
 // Every wait on an mbarrier has an iteration limit; on expiry the kernel
 // records an error code, waits (bounded) for its own loads still in flight,
@@ -53,7 +59,8 @@ namespace {
 // ms at n = 32 / 64 / 96 / 128 (CTAs x stages x accumulators x groups):
 //   2 x 6 x 2 x 2   0.047 / 0.121 / 0.234 / 0.278   (the default; 0.045 / 0.110 /
 //                   0.224 / 0.276 with the diagonal entry taken by a select
-//                   tree and the extra block alternating at n = 64)
+//                   tree and the extra block alternating at n = 64; 0.043 /
+//                   0.110 / 0.205 / 0.257 with entries summed four to a word)
 //   4 x 3 x 1 x 1   0.049 / 0.133 / 0.256 / 0.307
 //   1 x 8 x 4 x 4   0.070 / 0.141 / 0.311 / 0.346
 //   1 x 8 x 4 x 2   0.070 / 0.168 / 0.305 / 0.412
@@ -81,6 +88,13 @@ constexpr int kAccCols = 128;                 // columns of one accumulator (N <
 constexpr uint32_t kTmemCols = kAccs * kAccCols;
 constexpr int kGroups = XW_RESCORE_GROUPS;
 constexpr int kThreads = 64 + 128 * kGroups;
+// Orders that are not a multiple of 32 (and unaligned inputs): warps that
+// pad the matrices into the ring in place of the TMA producer
+// (8192 matrices of n = 100 / 65536 of n = 26, ms: three warps on each tile
+// 0.100 / 0.080, seven 0.074 / 0.092, six with one to three a tile 0.078 /
+// 0.057; one chunk's loads in flight instead of four 0.204 / 0.207)
+constexpr int kPackWarps = 6;   // three before the MMA warp, three after the epilogue's
+constexpr int kPackThreads = 32 * (kPackWarps + 1) + 128 * kGroups;
 constexpr int kCombineSlots = 8;
 static_assert(kAccs % kGroups == 0, "an accumulator belongs to one epilogue group");
 static_assert(kCombineSlots >= kAccs / kGroups + 1, "a combine slot outlives its tile");
@@ -90,9 +104,12 @@ constexpr long long kSpinLimit = 1ll << 22;
 
 struct RescoreParams {
     int count;          // matrices
-    int n, w;
+    int n, w;           // n: the order padded to a multiple of 32
+    int nv;             // the order
+    const int8_t* W;
     int rows_per_tile;  // matrices per tile * n
     int mpt;            // matrices per tile
+    int wpt;            // packing warps per tile
     int ntiles;
     int4* stats;        // per matrix {score, conflicts, squared, exact}
     int32_t* gram;      // nullable: per matrix n*n row-major
@@ -111,6 +128,10 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
 }
 
 // bounded wait for the phase with parity `parity` to complete
@@ -194,21 +215,67 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, int (&v)[32]) {
 // load, MMA and epilogue each wait only on the mbarrier of the stage or
 // accumulator they use, so loads run kStages tiles ahead and the MMA of the
 // next tiles overlaps the epilogue of this one.
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(bar)) : "memory");
-}
-
 __device__ __forceinline__ void rescore_fail(const RescoreParams& p, volatile int* abort_flag, int code) {
     atomicExch(p.error, code);
     *abort_flag = 1;
+}
+
+// |G|, [G != 0] and G^2 of 32 entries of a row into the thread's sums
+__device__ __forceinline__ void add_block(const int (&v)[32], int& a_abs, int& a_nz, int& a_sq) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 2) {
+        const int a0 = abs(v[j]), a1 = abs(v[j + 1]);
+        a_abs += a0 + a1;
+        a_nz += min(a0, 1) + min(a1, 1);
+        a_sq += v[j] * v[j] + v[j + 1] * v[j + 1];
+    }
+}
+
+// The same for entries of at most 127 in magnitude, four to a word of bytes:
+// 10 instructions a word against 16 (what bounds the epilogue is the integer
+// pipes: 65536 matrices of n = 96 / 128 0.227 / 0.283 ms with add_block
+// alone, 0.205 / 0.257 with this).
+__device__ __forceinline__ void add_block_bytes(const int (&v)[32], int& a_abs, int& a_nz, int& a_sq) {
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) {
+        const uint32_t lo = __byte_perm((uint32_t)v[j], (uint32_t)v[j + 1], 0x0040);
+        const uint32_t hi = __byte_perm((uint32_t)v[j + 2], (uint32_t)v[j + 3], 0x0040);
+        const uint32_t x = __byte_perm(lo, hi, 0x5410);
+        const uint32_t a = __vabsdiffu4(x ^ 0x80808080u, 0x80808080u);
+        const uint32_t z = (a + 0x7f7f7f7fu) & 0x80808080u;
+        a_abs = (int)__dp4a(a, 0x01010101u, (uint32_t)a_abs);
+        a_nz = (int)__dp4a(z, 0x01010101u, (uint32_t)a_nz);   // 128 an entry
+        a_sq = __dp4a((int)x, (int)x, a_sq);
+    }
+}
+
+// v[lane] by a five-level select tree on the lane's bits (a chain of 31
+// selects measured 4-9% slower per launch)
+__device__ __forceinline__ int pick_lane(const int (&v)[32], int lane) {
+    int u[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) u[j] = (lane & 16) ? v[j + 16] : v[j];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) u[j] = (lane & 8) ? u[j + 8] : u[j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) u[j] = (lane & 4) ? u[j + 4] : u[j];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) u[j] = (lane & 2) ? u[j + 2] : u[j];
+    return (lane & 1) ? u[1] : u[0];
 }
 
 // Per-row statistics of one tile's accumulator rows 32q..32q+31 (this
 // warp's lane quarter); see the epilogue comment below.  rot is the
 // group's count of tiles before this one.  Returns the warp's sums and
 // whether every row's diagonal entry is right.
-__device__ __forceinline__ void tile_rows(const RescoreParams& p, uint32_t tacc, int t, int rot, int q, int lane,
-                                          int4& part, int& diag_ok, int& mat) {
+//
+// |G_ij| <= sqrt(G_ii G_jj), so when every diagonal entry of the matrix is at
+// most 127 (always below w = 128 of a ternary matrix) all its entries fit a
+// byte.  A warp sees the diagonal of its own 32 rows; the warps of a matrix
+// learn of the others' through `flag` (the tile count of the last larger
+// one) and the group's barrier `bar`.  False when the wait for it ran out.
+__device__ __forceinline__ bool tile_rows(const RescoreParams& p, uint32_t tacc, int t, int rot, int q, int lane,
+                                          int4& part, int& diag_ok, int& mat, uint64_t* bar, volatile int* flag) {
     const int row0 = 32 * q;
     const int b = row0 / p.n;       // matrix of this warp within the tile
     const int i0 = row0 - b * p.n;  // first row of the warp within the matrix
@@ -218,33 +285,25 @@ __device__ __forceinline__ void tile_rows(const RescoreParams& p, uint32_t tacc,
     const int nb = p.n / 32, rb = i0 / 32;
     int s_abs = 0, s_nz = 0, s_sq = 0, dg = 0;
     int o_abs = 0, o_nz = 0, o_sq = 0;
-    auto block = [&](int c, int& a_abs, int& a_nz, int& a_sq) {
+    // nonzero entries counted 128 times by the byte form
+    int s_nzb = 0, o_nzb = 0;
+    bool wide = false;
+    auto block = [&](int c, int& a_abs, int& a_nz, int& a_nzb, int& a_sq) {
         int v[32];
         tmem_ld32(tacc + ((uint32_t)row0 << 16) + (uint32_t)(col0 + c), v);
-#pragma unroll
-        for (int j = 0; j < 32; j += 2) {
-            const int a0 = abs(v[j]), a1 = abs(v[j + 1]);
-            a_abs += a0 + a1;
-            a_nz += min(a0, 1) + min(a1, 1);
-            a_sq += v[j] * v[j] + v[j + 1] * v[j + 1];
-        }
         if (c == i0) {
-            // v[lane] by a five-level select tree on the lane's bits (a
-            // chain of 31 selects measured 4-9% slower per launch)
-            int u[16];
-#pragma unroll
-            for (int j = 0; j < 16; ++j) u[j] = (lane & 16) ? v[j + 16] : v[j];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) u[j] = (lane & 8) ? u[j + 8] : u[j];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) u[j] = (lane & 4) ? u[j + 4] : u[j];
-#pragma unroll
-            for (int j = 0; j < 2; ++j) u[j] = (lane & 2) ? u[j + 2] : u[j];
-            dg = (lane & 1) ? u[1] : u[0];
+            dg = pick_lane(v, lane);
+            wide = __any_sync(0xffffffffu, dg > 127);
         }
-        if (p.gram && mat < p.count) {
-            int32_t* dst = p.gram + (size_t)mat * p.n * p.n + (size_t)i * p.n + c;
-            if (((uintptr_t)p.gram & 15u) == 0) {   // 16-byte stores need a 16-byte aligned base
+        if (wide || p.gram) add_block(v, a_abs, a_nz, a_sq);
+        else add_block_bytes(v, a_abs, a_nzb, a_sq);
+        if (p.gram && mat < p.count && i < p.nv) {
+            int32_t* dst = p.gram + (size_t)mat * p.nv * p.nv + (size_t)i * p.nv + c;
+            if (p.nv != p.n) {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                    if (c + j < p.nv) dst[j] = v[j];
+            } else if (((uintptr_t)p.gram & 15u) == 0) {   // 16-byte stores need a 16-byte aligned base
                 int4* d4 = reinterpret_cast<int4*>(dst);
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) d4[j / 4] = make_int4(v[j], v[j + 1], v[j + 2], v[j + 3]);
@@ -264,21 +323,32 @@ __device__ __forceinline__ void tile_rows(const RescoreParams& p, uint32_t tacc,
     // alternates from tile to tile, (rb + rot) / d even, so that schedulers
     // 0 and 2 do not take the extra block on every tile (measured 5% at
     // n = 64; at n = 128 alternating measured 4% slower)
+    bool ok = true;
     if (p.gram) {
-        for (int c = 0; c < p.n; c += 32) block(c, s_abs, s_nz, s_sq);
+        for (int c = 0; c < p.n; c += 32) block(c, s_abs, s_nz, s_nzb, s_sq);
     } else {
-        block(i0, s_abs, s_nz, s_sq);
-        for (int d = 1; 2 * d <= nb; ++d) {
-            if (2 * d == nb && ((nb == 2 ? rb + rot : rb) / d & 1)) continue;
-            block(((rb + d) % nb) * 32, o_abs, o_nz, o_sq);
+        block(i0, s_abs, s_nz, s_nzb, s_sq);
+        if (nb > 1) {
+            if (lane == 0) {
+                if (wide) flag[rot & 1] = rot + 1;
+                mbar_arrive(bar);
+            }
+            ok = __all_sync(0xffffffffu, mbar_wait(bar, (uint32_t)rot & 1u));
+            wide = flag[rot & 1] == rot + 1;
+            for (int d = 1; ok && 2 * d <= nb; ++d) {
+                if (2 * d == nb && ((nb == 2 ? rb + rot : rb) / d & 1)) continue;
+                block(((rb + d) % nb) * 32, o_abs, o_nz, o_nzb, o_sq);
+            }
         }
     }
+    s_nz += s_nzb >> 7;
+    o_nz += o_nzb >> 7;
     s_abs += 2 * o_abs - abs(dg);
     s_nz += 2 * o_nz - min(abs(dg), 1);
     s_sq += 2 * o_sq - dg * dg;
     // a zero-padded matrix: its own rows carry w on the diagonal, the
     // padding rows 0 (their off-diagonal entries are 0 anyway)
-    int nv = p.n, wv = p.w;
+    int nv = p.nv, wv = p.w;
     if (p.dims && mat < p.count) {
         const int2 d = p.dims[mat];
         nv = d.x;
@@ -289,6 +359,7 @@ __device__ __forceinline__ void tile_rows(const RescoreParams& p, uint32_t tacc,
     part.y = __reduce_add_sync(0xffffffffu, s_nz);
     part.z = __reduce_add_sync(0xffffffffu, s_sq);
     diag_ok = (int)__reduce_and_sync(0xffffffffu, (unsigned)diag_ok);
+    return ok;
 }
 
 // symmetric G: the off-diagonal sums count each pair twice
@@ -296,8 +367,89 @@ __device__ __forceinline__ int4 matrix_stats(int abs_sum, int nz_sum, int sq_sum
     return make_int4(abs_sum / 2, nz_sum / 2, sq_sum / 2, (nz_sum == 0 && diag_ok) ? 1 : 0);
 }
 
-__global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const __grid_constant__ CUtensorMap tmap,
-                                                                 RescoreParams p) {
+// Rows 0..nv-1 of matrices mat0 .. mat0 + nmat - 1, columns [k0, k0 + 128),
+// into a K-major 128-byte-swizzled tile, each matrix at the next multiple
+// of 32 rows (16-byte chunk c of row r sits at chunk c ^ (r % 8)); `t` of
+// `nt` threads.  Rows and chunks past the order stay as they are (zero from
+// the start).  A row's chunk lies in five aligned words of the input,
+// shifted into place; kBatch chunks of a thread are in flight.  Words not
+// wholly inside the input (its first and last matrices) are read byte by
+// byte.
+__device__ __forceinline__ void pack_rows(const RescoreParams& p, uint8_t* tile, int mat0, int nmat, int k0, int t,
+                                          int nt) {
+    constexpr int kBatch = 4;
+    const int cols = min(128, p.nv - k0), cpr = (cols + 15) >> 4;
+    const int lp = cpr > 4 ? 3 : cpr > 2 ? 2 : cpr > 1 ? 1 : 0;   // chunks a row, a power of two of lanes
+    const int c = t & ((1 << lp) - 1);
+    if (c >= cpr) return;
+    const int rows = nmat * p.nv, step = nt >> lp;
+    const int8_t* M = p.W + (size_t)mat0 * p.nv * p.nv;
+    const int8_t* hi = p.W + (size_t)p.count * p.nv * p.nv;
+    const uint32_t low = (uint32_t)(uintptr_t)M & 3u;   // offsets below count from the aligned word of M
+    const uint32_t* Mw = reinterpret_cast<const uint32_t*>(M - low);
+    const bool inside = M - 4 >= p.W && M + rows * p.nv + 20 <= hi;
+    uint32_t keep[4];   // the chunk's bytes that belong to the row
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const int left = min(16, cols - 16 * c) - 4 * k;
+        keep[k] = left >= 4 ? 0xffffffffu : left <= 0 ? 0u : (1u << (8 * left)) - 1u;
+    }
+    int R = t >> lp, r = R, row = R;   // row of the tile's matrices, of its matrix, and of the tile
+    while (r >= p.nv) {
+        r -= p.nv;
+        row += p.n - p.nv;
+    }
+    uint32_t off = (uint32_t)(R * p.nv + k0 + 16 * c) + low;
+    while (R < rows) {
+        uint32_t x[kBatch][5], f[kBatch];
+        int dst[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            dst[k] = -1;
+            f[k] = 8u * (off & 3u);
+            if (R < rows) {
+                dst[k] = row * 128 + ((c ^ (row & 7)) << 4);
+                const uint32_t* src = Mw + (off >> 2);
+                if (inside) {
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) x[k][q] = __ldg(src + q);
+                } else {
+                    const int8_t* b = reinterpret_cast<const int8_t*>(src);
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) {
+                        x[k][q] = 0;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (b + 4 * q + e >= p.W && b + 4 * q + e < hi)
+                                x[k][q] |= (uint32_t)(uint8_t)b[4 * q + e] << (8 * e);
+                    }
+                }
+            }
+            R += step;
+            r += step;
+            row += step;
+            off += (uint32_t)(step * p.nv);
+            while (r >= p.nv) {
+                r -= p.nv;
+                row += p.n - p.nv;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k)
+            if (dst[k] >= 0)
+                *reinterpret_cast<uint4*>(tile + dst[k]) =
+                    make_uint4(__funnelshift_r(x[k][0], x[k][1], f[k]) & keep[0], __funnelshift_r(x[k][1], x[k][2], f[k]) & keep[1],
+                               __funnelshift_r(x[k][2], x[k][3], f[k]) & keep[2], __funnelshift_r(x[k][3], x[k][4], f[k]) & keep[3]);
+    }
+}
+
+// PACK: the matrices (of any order up to 128, at any address) are padded to
+// 32-row blocks of zero-filled 128-byte rows by kPackWarps warps; else a TMA
+// producer loads them.
+template <bool PACK>
+__global__ void __launch_bounds__(PACK ? kPackThreads : kThreads, kCtasPerSm)
+    rescore_tc_kernel(const __grid_constant__ CUtensorMap tmap, RescoreParams p) {
+    constexpr int kMmaWarp = PACK ? 3 : 1;
     extern __shared__ uint8_t smem_raw[];
     // tiles on a 1024-byte boundary (the 128-byte swizzle pattern repeats every 1024 bytes)
     uint8_t* tiles = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -305,6 +457,10 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
     __shared__ __align__(8) uint64_t empty_bar[kStages];
     __shared__ __align__(8) uint64_t accf_bar[kAccs];
     __shared__ __align__(8) uint64_t acce_bar[kAccs];
+    // per group: the four warps know their rows' diagonals, and the count of
+    // the last tile (of either parity) with one above 127
+    __shared__ __align__(8) uint64_t diag_bar[kGroups];
+    __shared__ volatile int diag_sh[kGroups][2];
     __shared__ uint32_t tmem_base_sh;
     __shared__ volatile int abort_sh;
     // cross-warp sums of matrices that span several lane quarters (n >= 64):
@@ -313,19 +469,24 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
     __shared__ int comb_sh[kGroups][kCombineSlots][2][5];
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (warp == 1) {
+    if (warp == kMmaWarp) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_sh)),
                      "r"(kTmemCols));
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
         for (int s = 0; s < kStages; ++s) {
-            mbar_init(&full_bar[s], 1);
+            mbar_init(&full_bar[s], PACK ? p.wpt : 1);
             mbar_init(&empty_bar[s], 1);
         }
         for (int a = 0; a < kAccs; ++a) {
             mbar_init(&accf_bar[a], 1);
             mbar_init(&acce_bar[a], 4);   // the four warps of the group that owns the accumulator
+        }
+        for (int g = 0; g < kGroups; ++g) {
+            mbar_init(&diag_bar[g], 4);
+            diag_sh[g][0] = 0;
+            diag_sh[g][1] = 0;
         }
         abort_sh = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -334,6 +495,12 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
         int* f = &comb_sh[0][0][0][0] + 5 * k;
         f[0] = f[1] = f[2] = f[4] = 0;
         f[3] = 1;
+    }
+    if constexpr (PACK) {
+        // rows and columns past the order stay zero: every tile writes the same places
+        for (int k = tid; k < kStages * kTileBytes / 16; k += blockDim.x)
+            reinterpret_cast<uint4*>(tiles)[k] = make_uint4(0, 0, 0, 0);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
@@ -347,7 +514,27 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
     const uint32_t box_bytes = 128u * (uint32_t)p.rows_per_tile;
     constexpr int S = kStages;
 
-    if (warp == 0) {
+    if (PACK && (warp < 3 || warp > kMmaWarp + 4 * kGroups)) {
+        // p.wpt warps pack a tile, the next ones the next tile
+        const int pw = warp < 3 ? warp : warp - 1 - 4 * kGroups, tiles_at_once = kPackWarps / p.wpt;
+        for (int it = pw / p.wpt; it < ntl; it += tiles_at_once) {
+            // the warp leaves the loop together
+            const int s = it % S;
+            bool ok = !abort_sh;
+            if (ok && it >= S && !mbar_wait(&empty_bar[s], (uint32_t)(it / S - 1) & 1u)) {
+                rescore_fail(p, &abort_sh, 3);
+                ok = false;
+            }
+            if (!__all_sync(0xffffffffu, ok)) break;
+            const int t = (int)blockIdx.x + it * grid;
+            pack_rows(p, tiles + s * kTileBytes, t * p.mpt, min(p.mpt, p.count - t * p.mpt), 0,
+                      32 * (pw % p.wpt) + lane, 32 * p.wpt);
+            // the writes above, by the MMA's (asynchronous) reads
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&full_bar[s]);
+        }
+    } else if (!PACK && warp == 0) {
         if (lane == 0) {
             int it = 0;
             for (; it < ntl && !abort_sh; ++it) {
@@ -365,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
             for (int k = it > S ? it - S : 0; k < it; ++k)
                 mbar_wait(&full_bar[k % S], (uint32_t)(k / S) & 1u);
         }
-    } else if (warp == 1) {
+    } else if (warp == kMmaWarp) {
         if (lane == 0) {
             const uint32_t idesc = instr_desc(p.rows_per_tile);
             // K steps of 32 columns that hold matrix entries; the box's
@@ -395,21 +582,31 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
             if (it > 0) mbar_wait(&accf_bar[(it - 1) % kAccs], (uint32_t)((it - 1) / kAccs) & 1u);
         }
     } else {
-        const int e = warp - 2, g = e >> 2, q = warp & 3;
+        const int e = warp - kMmaWarp - 1, g = e >> 2, q = warp & 3;
         const bool active = 32 * q < p.rows_per_tile;
         const int wpm = (p.n + 31) / 32;   // warps (lane quarters) per matrix
         for (int it = g; it < ntl; it += kGroups) {
-            if (abort_sh) break;
             const int a = it % kAccs;
-            if (!mbar_wait(&accf_bar[a], (uint32_t)(it / kAccs) & 1u)) {
+            bool ok = !abort_sh;
+            if (ok && !mbar_wait(&accf_bar[a], (uint32_t)(it / kAccs) & 1u)) {
                 rescore_fail(p, &abort_sh, 2);
-                break;
+                ok = false;
             }
+            if (!__all_sync(0xffffffffu, ok)) break;   // the warp leaves the loop together
             asm volatile("tcgen05.fence::after_thread_sync;");
             const int t = (int)blockIdx.x + it * grid;
             int4 part = make_int4(0, 0, 0, 0);
             int diag_ok = 1, mat = 0;
-            if (active) tile_rows(p, tmem + (uint32_t)(a * kAccCols), t, it / kGroups, q, lane, part, diag_ok, mat);
+            if (active) {
+                ok = tile_rows(p, tmem + (uint32_t)(a * kAccCols), t, it / kGroups, q, lane, part, diag_ok, mat,
+                               &diag_bar[g], diag_sh[g]);
+            } else if (lane == 0) {
+                mbar_arrive(&diag_bar[g]);
+            }
+            if (!ok) {
+                rescore_fail(p, &abort_sh, 6);
+                break;
+            }
             // the accumulator is free for the MMA of a later tile
             asm volatile("tcgen05.fence::before_thread_sync;");
             __syncwarp();
@@ -440,12 +637,133 @@ __global__ void __launch_bounds__(kThreads, kCtasPerSm) rescore_tc_kernel(const 
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
-    if (warp == 1)
+    if (warp == kMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols));
 }
 
-// SIMT path for orders that do not fill 32-row tensor-core blocks: one warp
-// per matrix, lane o accumulates column o of G.
+// Orders 129..256: one CTA per matrix at a time.  The matrix is padded into
+// two K-halves of 256 rows x 128 bytes (two matrices in turn); one thread
+// multiplies rows 0..127 by all rows (columns 0..255 of TMEM) and rows
+// 128..255 by rows 128..255 (columns 256..383): every unordered pair of
+// 32-row blocks is in one of the two.  Eight warps read the blocks on and
+// above the diagonal, two warps to a lane quarter.  The next matrix is
+// packed while the MMA of this one runs.  512 matrices of n = 256: 74 ms on
+// the SIMT kernel, which took one warp and n^3 / 32 byte loads per matrix.
+constexpr int kBigThreads = 256;
+constexpr int kBigBytes = 2 * 256 * 128;   // one matrix
+
+__global__ void __launch_bounds__(kBigThreads, 1) rescore_big_kernel(RescoreParams p) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* tiles = reinterpret_cast<uint8_t*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    __shared__ __align__(8) uint64_t acc_bar;
+    __shared__ uint32_t tmem_base_sh;
+    __shared__ int sums[4];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&tmem_base_sh)),
+                     "r"(512u));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    if (tid == 0) {
+        mbar_init(&acc_bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    for (int k = tid; k < 2 * kBigBytes / 16; k += kBigThreads) reinterpret_cast<uint4*>(tiles)[k] = make_uint4(0, 0, 0, 0);
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    const uint32_t tmem = tmem_base_sh;
+    const int ksteps = (p.nv + 31) / 32, nb = p.n / 32;
+    const uint32_t id0 = instr_desc(p.n), id1 = instr_desc(p.n - 128);
+    auto pack = [&](int mat, int buf) {
+        if (mat >= p.count) return;
+        for (int h = 0; h < 2; ++h) pack_rows(p, tiles + buf * kBigBytes + h * (kBigBytes / 2), mat, 1, 128 * h, tid, kBigThreads);
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    };
+    int it = 0;
+    pack(blockIdx.x, 0);
+    for (int mat = blockIdx.x; mat < p.count; mat += gridDim.x, ++it) {
+        const uint8_t* tile = tiles + (it & 1) * kBigBytes;
+        if (tid < 4) sums[tid] = tid == 3 ? 1 : 0;
+        // this matrix is packed; the epilogue of the one before is done
+        asm volatile("tcgen05.fence::before_thread_sync;");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        if (tid == 0) {
+            for (int k = 0; k < ksteps; ++k) {
+                const uint64_t d = smem_desc(tile + (k >> 2) * (kBigBytes / 2)) + (uint64_t)(2 * (k & 3));
+                const uint64_t e = smem_desc(tile + (k >> 2) * (kBigBytes / 2) + 128 * 128) + (uint64_t)(2 * (k & 3));
+                mma_i8(tmem, d, d, id0, k > 0);
+                mma_i8(tmem + 256u, e, e, id1, k > 0);
+            }
+            mma_commit(&acc_bar);
+        }
+        pack(mat + gridDim.x, (it + 1) & 1);
+        const bool ok = mbar_wait(&acc_bar, (uint32_t)it & 1u);
+        if (!ok) atomicExch(p.error, 5);
+        if (__syncthreads_or(!ok)) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const int q = warp & 3;
+        const int2 dim = p.dims ? p.dims[mat] : make_int2(p.nv, p.w);
+        int s_abs = 0, s_nz = 0, s_sq = 0, diag_ok = 1;
+        int turn = 0;
+        for (int rb = q; rb < nb; rb += 4) {
+            const int i = 32 * rb + lane;
+            // rows 128.. hold columns 128.. (of the symmetric matrix) only
+            for (int cb = p.gram ? (rb < 4 ? 0 : 4) : rb; cb < nb; ++cb) {
+                if ((turn++ & 1) != (warp >> 2)) continue;
+                int v[32];
+                tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(rb < 4 ? 32 * cb : 256 + 32 * (cb - 4)), v);
+                if (cb >= rb) {
+                    int a = 0, z = 0, sq = 0;
+                    add_block(v, a, z, sq);
+                    if (cb == rb) {
+                        const int dg = pick_lane(v, lane);
+                        a -= abs(dg);
+                        z -= min(abs(dg), 1);
+                        sq -= dg * dg;
+                        diag_ok &= i < dim.x ? dg == dim.y : dg == 0;
+                    }
+                    const int wt = cb == rb ? 1 : 2;
+                    s_abs += wt * a;
+                    s_nz += wt * z;
+                    s_sq += wt * sq;
+                }
+                if (p.gram && i < p.nv) {
+                    int32_t* G = p.gram + (size_t)mat * p.nv * p.nv;
+#pragma unroll
+                    for (int j = 0; j < 32; ++j) {
+                        const int c = 32 * cb + j;
+                        if (c < p.nv) {
+                            G[(size_t)i * p.nv + c] = v[j];
+                            if (rb < 4 && cb >= 4) G[(size_t)c * p.nv + i] = v[j];
+                        }
+                    }
+                }
+            }
+        }
+        s_abs = __reduce_add_sync(0xffffffffu, s_abs);
+        s_nz = __reduce_add_sync(0xffffffffu, s_nz);
+        s_sq = __reduce_add_sync(0xffffffffu, s_sq);
+        diag_ok = (int)__reduce_and_sync(0xffffffffu, (unsigned)diag_ok);
+        if (lane == 0) {
+            atomicAdd(&sums[0], s_abs);
+            atomicAdd(&sums[1], s_nz);
+            atomicAdd(&sums[2], s_sq);
+            atomicAnd(&sums[3], diag_ok);
+        }
+        __syncthreads();
+        if (tid == 0) p.stats[mat] = matrix_stats(sums[0], sums[1], sums[2], sums[3]);
+        __syncthreads();
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u));
+}
+
+// SIMT kernel: one warp per matrix, lane o accumulates column o of G.  For
+// tiny orders, and on demand for any.
 __global__ void rescore_simt_kernel(const int8_t* W, int count, int n, int w, int4* stats, int32_t* gram,
                                     const int2* dims) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
@@ -524,8 +842,17 @@ int32_t rescore_device(const int8_t* W, int64_t count, int n, int w, int32_t* st
     if (n < 1 || n > XW_MAX_ORDER_SHARED) return rfail(XW_ERR_INVALID, "rescore: order must be in [1, 256]");
     if (count == 0) return XW_OK;
     cudaError_t e;
-    // tensor cores for n in {32, 64, 96, 128}: a tile row is one 128-byte TMA row
-    const bool tc = !force_simt && n % 32 == 0 && n <= 128 && ((uintptr_t)W % 16) == 0;
+    // n in {32, 64, 96, 128} at a 16-byte aligned address is loaded by TMA
+    // (a tensor map's row pitch is a multiple of 16 bytes); other orders up
+    // to 128, and addresses, are padded by the packing warps; orders above by
+    // rescore_big_kernel.  Tiny orders stay on the SIMT kernel, whose launch
+    // is cheaper than a tile of mostly padding (us a call, SIMT / packed:
+    // n = 8, 1000 matrices 5.0 / 8.5, 20000 16.7 / 18.7; n = 12, 1000
+    // matrices 6.5 / 8.5, 4000 10.6 / 10.5; n = 16, 1000 matrices 8.5 / 8.5;
+    // n = 26, one matrix 15.4 / 6.7; n = 100, one matrix 646 / 10.6, 8192
+    // matrices 7850 / 78).
+    const bool tc = !force_simt && !(n <= 8 || (n <= 12 && count < 4000));
+    const bool pack = n % 32 != 0 || ((uintptr_t)W % 16) != 0;
     if (!tc) {
         const int blocks = (int)((count * 32 + 255) / 256);
         rescore_simt_kernel<<<blocks, 256, 0, stream>>>(W, (int)count, n, w, reinterpret_cast<int4*>(stats), gram,
@@ -533,39 +860,54 @@ int32_t rescore_device(const int8_t* W, int64_t count, int n, int w, int32_t* st
         e = cudaGetLastError();
         return e == cudaSuccess ? XW_OK : rfail(XW_ERR_CUDA, std::string("rescore launch: ") + cudaGetErrorString(e));
     }
-    EncodeTiledFn enc = encode_tiled();
-    if (!enc) return rfail(XW_ERR_CUDA, "rescore: cuTensorMapEncodeTiled is unavailable");
+    const bool big = n > 128;
+    EncodeTiledFn enc = pack || big ? nullptr : encode_tiled();
+    if (!enc && !pack && !big) return rfail(XW_ERR_CUDA, "rescore: cuTensorMapEncodeTiled is unavailable");
     RescoreParams p;
     p.count = (int)count;
-    p.n = n;
+    p.n = 32 * ((n + 31) / 32);
+    p.nv = n;
+    p.W = W;
     p.w = w;
-    p.mpt = n <= 64 ? 128 / n : 1;
-    p.rows_per_tile = p.mpt * n;
+    p.mpt = p.n <= 64 ? 128 / p.n : 1;
+    p.rows_per_tile = p.mpt * p.n;
+    // one or two packing warps a 32-row block of the tile, twice that when no
+    // CTA has a second tile to overlap
+    p.wpt = p.n == 32 ? 1 : p.n == 64 ? 2 : 3;
     p.ntiles = (int)((count + p.mpt - 1) / p.mpt);
     p.stats = reinterpret_cast<int4*>(stats);
     p.gram = gram;
     p.error = err_flag;
     p.dims = dims;
     CUtensorMap map;
-    const cuuint64_t extent[2] = {(cuuint64_t)n, (cuuint64_t)count * n};
-    const cuuint64_t strides[1] = {(cuuint64_t)n};
-    const cuuint32_t box[2] = {128u, (cuuint32_t)p.rows_per_tile};
-    const cuuint32_t estr[2] = {1u, 1u};
-    const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(W), extent, strides, box, estr,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    std::memset(&map, 0, sizeof map);
+    CUresult r = CUDA_SUCCESS;
+    if (enc) {
+        const cuuint64_t extent[2] = {(cuuint64_t)n, (cuuint64_t)count * n};
+        const cuuint64_t strides[1] = {(cuuint64_t)n};
+        const cuuint32_t box[2] = {128u, (cuuint32_t)p.rows_per_tile};
+        const cuuint32_t estr[2] = {1u, 1u};
+        r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(W), extent, strides, box, estr,
+                CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
     if (r != CUDA_SUCCESS) return rfail(XW_ERR_CUDA, "rescore: cuTensorMapEncodeTiled failed");
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    const size_t smem = (size_t)kStages * kTileBytes + 1024;
-    e = cudaFuncSetAttribute(rescore_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = (big ? 2 * (size_t)kBigBytes : (size_t)kStages * kTileBytes) + 1024;
+    const void* fn = big ? reinterpret_cast<const void*>(&rescore_big_kernel) : pack ? reinterpret_cast<const void*>(&rescore_tc_kernel<true>)
+                          : reinterpret_cast<const void*>(&rescore_tc_kernel<false>);
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return rfail(XW_ERR_CUDA, std::string("rescore attribute: ") + cudaGetErrorString(e));
     // kCtasPerSm persistent CTAs per SM; the tile loop is grid-strided, so
     // fewer resident CTAs only serialise, never skip, tiles
-    const int blocks = (int)std::min<int64_t>(p.ntiles, (int64_t)kCtasPerSm * sms);
-    rescore_tc_kernel<<<blocks, kThreads, smem, stream>>>(map, p);
-    e = cudaGetLastError();
+    const int blocks = (int)std::min<int64_t>(p.ntiles, (int64_t)(big ? 1 : kCtasPerSm) * sms);
+    if (blocks == p.ntiles) p.wpt = p.n == 64 ? 3 : 2 * p.wpt;
+    void* kargs[] = {&map, &p};
+    void* bargs[] = {&p};
+    e = cudaLaunchKernel(fn, dim3(blocks), dim3(big ? kBigThreads : pack ? kPackThreads : kThreads), big ? bargs : kargs,
+                         smem, stream);
     return e == cudaSuccess ? XW_OK : rfail(XW_ERR_CUDA, std::string("rescore launch: ") + cudaGetErrorString(e));
 }
 
