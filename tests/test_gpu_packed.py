@@ -1,0 +1,91 @@
+"""The packed-row annealing kernels at the edges of their layouts, against the
+oracle: every replica's whole state, bit for bit.
+
+Orders around each class's limits (a lane's words, a row's pad, bytes against
+halfwords of G, the permuted rows above order 248), the candidate and
+tournament counts that take several passes, coins of probability 0 and 1,
+runs of one-candidate iterations of every length, temperatures above the
+32-bit threshold table, and index draws in Lemire's rejection zone.
+"""
+import pytest
+
+import oracle_lib as O
+import xtax_b200 as X
+from test_gpu_parity import compare, oracle_job, start_of
+
+pytestmark = pytest.mark.gpu
+
+
+def replay(n, w, R, iters, seed, **kw):
+    kw.setdefault("t_init", 4.0)
+    kw.setdefault("moves_per_launch", max(1, iters // 2 - 3))
+    p = X.Params(stop_on_solve=0, warps_per_replica=kw.pop("warps_per_replica", 1), **kw)
+    batch = X.Batch([{"n": n, "w": w, "seed": seed, "replicas": R}], p)
+    temps = [batch.replica(0, r)[0].reheat_temperature for r in range(R)]
+    batch.run(iters)
+    batch.synchronize()
+    job = oracle_job(n, w, seed, p)
+    for r in range(R):
+        rep = O.Replica(job, r, start_of(n, w, seed, r, p), temps[r], r)
+        rep.run(iters, stop_on_solve=False)
+        assert rep.check() == 0
+        compare(batch, 0, r, rep)
+    batch.close()
+
+
+EDGES = [(1, 1), (2, 1), (3, 2), (5, 5), (16, 15), (17, 16), (31, 30), (32, 31), (32, 32), (33, 3), (33, 32), (48, 24),
+         (63, 62), (64, 63), (64, 64), (65, 33), (79, 78), (80, 79), (81, 4), (112, 111), (127, 126), (127, 127),
+         (128, 127), (128, 128), (129, 64), (135, 134), (136, 4), (192, 96), (241, 240), (248, 124), (249, 124),
+         (250, 125), (255, 254), (256, 256)]
+
+
+@pytest.mark.parametrize("n,w", EDGES)
+def test_orders_at_the_edges_of_the_classes(n, w):
+    replay(n, w, 3 if n < 100 else 2, 700 if n < 100 else 150, 40 + n)
+
+
+@pytest.mark.parametrize("greedy", [0.0, 0.1, 1.0])
+@pytest.mark.parametrize("n,w", [(14, 13), (26, 25), (40, 20), (100, 99)])
+def test_runs_of_one_candidate_iterations(n, w, greedy):
+    # rejections of every number before an accept: a cold replica and a warm one
+    replay(n, w, 4, 900, 7 + n, greedy_fraction=greedy, t_init=3.0, t_min=0.2, moves_per_cool=37, stuck_threshold=101)
+
+
+@pytest.mark.parametrize("cs,ts", [(1, 1), (2, 4), (4, 5), (5, 8), (32, 9), (8, 64)])
+@pytest.mark.parametrize("n,w", [(15, 8), (30, 29), (70, 69), (130, 66)])
+def test_candidate_and_tournament_counts(n, w, cs, ts):
+    replay(n, w, 2, 200 if n < 100 else 60, 3 * n + cs, candidate_samples=cs, target_samples=ts)
+
+
+@pytest.mark.parametrize("coins", [dict(target_fraction=1.0), dict(target_fraction=0.0), dict(sign_fraction=1.0),
+                                   dict(sign_fraction=0.0, double_sign_fraction=0.0), dict(double_sign_fraction=1.0),
+                                   dict(switch_sign_fraction=1.0, sign_fraction=0.0, double_sign_fraction=0.0)],
+                         ids=lambda c: "-".join(f"{k}={v}" for k, v in c.items()))
+@pytest.mark.parametrize("n,w", [(9, 8), (26, 25), (50, 25), (140, 139)])
+def test_certain_and_impossible_coins(n, w, coins):
+    replay(n, w, 3, 400 if n < 100 else 80, 90 + n, **coins)
+
+
+@pytest.mark.parametrize("n,w", [(12, 11), (64, 9), (150, 20)])
+@pytest.mark.parametrize("t", [1e-3, 1e10, 1e13])
+def test_temperatures_beyond_the_threshold_table(n, w, t):
+    replay(n, w, 2, 300 if n < 100 else 60, 11 + n, t_init=t, t_min=min(t, 0.25))
+
+
+@pytest.mark.parametrize("n,w,kw", [(8, 1, {}), (20, 19, {}), (33, 32, {}), (90, 45, {}), (150, 149, {}),
+                                    (40, 6, dict(objective=1)), (200, 199, dict(objective=2))])
+def test_within_row_swaps_of_every_class(n, w, kw):
+    replay(n, w, 3, 300 if n < 100 else 80, 5 + n, move_set=1, start_kind=1, sign_fraction=0.2, **kw)
+
+
+def test_an_index_draw_in_the_rejection_zone():
+    # W(122, 61), seed 6: iteration 186996 of replica 0 draws the second row
+    # of candidate 3's double flip from a word that Lemire's test rejects (by
+    # exhaustive search of the draws); the whole trajectory is replayed past it
+    replay(122, 61, 1, 187050, 6, greedy_fraction=1.0, double_sign_fraction=1.0, t_init=2.0, t_min=2.0,
+           moves_per_launch=100000)
+
+
+@pytest.mark.parametrize("n,w", [(13, 12), (26, 24), (32, 31)])
+def test_latency_mode_at_odd_counts(n, w):
+    replay(n, w, 2, 500, 60 + n, warps_per_replica=6, candidate_samples=6, t_init=0.7, t_min=0.1, moves_per_cool=23)

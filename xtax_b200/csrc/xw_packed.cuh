@@ -1,5 +1,5 @@
 // xw_packed.cuh -- one annealing iteration on packed rows, for orders up to
-// 128: the device code shared by the one-warp replica loop and the latency
+// 256: the device code shared by the one-warp replica loop and the latency
 // mode of xw_anneal.cu.
 //
 // W and its Gram matrix sit in the replica's shared-memory slot as biased
@@ -76,9 +76,29 @@ __device__ __forceinline__ uint64_t lds64(uint32_t a) { return *reinterpret_cast
 // 4*WPL bytes a lane reads at once, and an odd multiple, so that the
 // mirrored column of a commit, one byte in each row, spreads over the banks.
 __host__ __device__ constexpr uint32_t packed_stride(int n, int wpl) {
+    if (wpl == 8) return ((uint32_t)n + 7u) & ~7u;
     const uint32_t q = 4u * (uint32_t)wpl;
     return ((((uint32_t)n + q - 1u) / q) | 1u) * q;
 }
+
+// Orders above 128 (WPL 8): G as biased halfwords (+32768), eight to a
+// 16-byte chunk, an odd number of chunks to a row; 32 chunks (orders above
+// 248, which leave no room for a pad) have theirs permuted by the row
+// instead.
+__host__ __device__ constexpr uint32_t wide_stride(int n) {
+    const uint32_t k = ((uint32_t)n + 7u) / 8u;
+    return (k == 32u ? k : k | 1u) * 16u;
+}
+
+__device__ __forceinline__ uint32_t wide_at(uint32_t g, uint32_t gst, int row, int chunk) {
+    return g + (uint32_t)row * gst + ((uint32_t)(chunk ^ (gst == 512u ? row & 7 : 0)) << 4);
+}
+
+// Moves since the best W that are kept to be undone when it is written: a
+// chain that improves every few moves writes it only when it ends (a save at
+// each move that left the best took 3000 of 3900 instructions an iteration
+// of W(256,255) from a random start, 1000 of 1750 of W(100,50)).
+constexpr int kJournal = 32;
 
 // A replica's constants and the state that changes with an accepted move
 // or a temperature step, in the slot: every lane reads them by broadcast
@@ -101,9 +121,9 @@ struct Con {
     double T;
     int32_t mb, cb;
     int32_t k_end;       // iterations of this launch
-    // the best W is the current one and its record is older: it is written
-    // when an accepted move leaves it, or at the end
-    int32_t dirty;
+    // moves accepted since the best W, all of them in the journal: the record
+    // holds an older one.  -1: the record holds the best W.
+    int32_t jn;
     // the copy that writes the record (a cluster's other CTAs keep an
     // identical copy in their own shared memory and write nothing)
     int32_t owner;
@@ -116,20 +136,22 @@ struct Slot {
     static constexpr uint32_t draws = 0;                      // 24 Philox blocks, then the window
     static constexpr uint32_t win = 384;                      // acceptance draws of 32 iterations
     static constexpr uint32_t thr = 512;                      // Metropolis thresholds
-    static constexpr uint32_t con = thr + 4u * kThrTable;
+    static constexpr uint32_t jrn = thr + 4u * kThrTable;     // journal
+    static constexpr uint32_t con = jrn + 8u * kJournal;
     static constexpr uint32_t res = con + 240u;               // packed residuals, 4 bytes a row
     static constexpr uint32_t mask = res + 128u * WPL;        // support masks, 4*WPL bytes a row
-    static constexpr uint32_t w = mask + 128u * WPL * WPL;
+    static constexpr uint32_t w = mask + (WPL == 8 ? 0u : 128u * WPL * WPL);
 };
 
 static_assert(sizeof(Con) <= 240, "replica constants fit their region");
 
 __host__ __device__ constexpr uint32_t packed_slot_bytes(int n, int m, int wpl) {
-    const uint32_t fixed = 512u + 4u * kThrTable + 240u + 128u * (uint32_t)wpl + 128u * (uint32_t)(wpl * wpl);
+    const uint32_t fixed = 512u + 4u * kThrTable + 8u * (uint32_t)kJournal + 240u + 128u * (uint32_t)wpl +
+                           (wpl == 8 ? 0u : 128u * (uint32_t)(wpl * wpl));
     const uint32_t mat = xw_pad16((uint32_t)n * packed_stride(n, wpl));
-    // the last lanes of a row may read up to one lane's width past it; the
-    // minority lists' pad covers the read of an empty list
-    return fixed + 2u * mat + xw_pad16((uint32_t)(n * m) + 1u);
+    const uint32_t gram = wpl == 8 ? (uint32_t)n * wide_stride(n) : mat;
+    // the minority lists' pad covers the read of an empty list
+    return fixed + mat + gram + xw_pad16((uint32_t)(n * m) + 1u);
 }
 
 // Loop-invariant context of a lane of a replica's group.
@@ -138,7 +160,8 @@ struct Env {
     uint32_t draws;      // this group's draw buffer
     uint32_t cw;         // the cached draw blocks of this lane's candidate
     uint32_t g, mino;    // byte offsets of G and the minority lists
-    uint32_t st;         // row stride
+    uint32_t st;         // bytes from a column of W (and, up to order 128, a row of G) to the next
+    uint32_t gst;        // the same of G above order 128
     int n, m, sparse, full;   // full: w = n
     int ts, bpc, move_set, obj_kind;
     uint32_t dq[2];      // draw blocks this lane computes: candidate (or iteration) << 16 | 1 + block
@@ -166,7 +189,14 @@ __device__ __forceinline__ int first_from(uint64_t m, int start) {
 template <int WPL, bool COMPL = false>
 __device__ __forceinline__ int mask_first(uint32_t slot, int row, int start, int n) {
     const uint32_t a = slot + Slot<WPL>::mask + (uint32_t)row * (4u * WPL);
-    if constexpr (WPL == 1) {
+    if constexpr (WPL == 8) {
+        // no masks: the columns in turn (at most n / w of them, or n / (n - w)
+        // zeros, on average, and only the fuller kind is searched this way)
+        const uint32_t w = slot + Slot<WPL>::w + (uint32_t)row, st = packed_stride(n, 8);
+        int c = start;
+        while ((lds8(w + (uint32_t)c * st) == 1u) != COMPL) c = c + 1 == n ? 0 : c + 1;
+        return c;
+    } else if constexpr (WPL == 1) {
         uint32_t m = lds32(a);
         if (COMPL) m = ~m & (n >= 32 ? 0xffffffffu : (1u << n) - 1u);
         return first_from(m, start);
@@ -431,6 +461,64 @@ __device__ __forceinline__ void load_words(uint32_t a, uint32_t (&v)[WPL]) {
 // packed residual of a row: sum |G| | conflicts << 18
 constexpr int kConfShift = 18;
 
+// New halfwords of rows 8j .. 8j+7 of the changed Gram rows of a move above
+// order 128: g1, g2 updated in place from the move's coefficients.
+__device__ __forceinline__ void wide_rows(uint32_t w1, uint32_t w2, int R1, int R2, int j, int a1, int b1, int a2,
+                                          int b2, int pk, uint32_t (&g1)[4], uint32_t (&g2)[4]) {
+    const uint2 x8 = *reinterpret_cast<const uint2*>(xw_smem + w1 + 8u * (uint32_t)j);
+    const uint2 y8 = *reinterpret_cast<const uint2*>(xw_smem + w2 + 8u * (uint32_t)j);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const uint32_t sel = h & 1 ? 0x4342u : 0x4140u;
+        const uint32_t x = __byte_perm(h < 2 ? x8.x : x8.y, 0u, sel), y = __byte_perm(h < 2 ? y8.x : y8.y, 0u, sel);
+        // entries R1 and R2 are left out: their W reads as zero (biased 1)
+        const uint32_t h1 = 16u * (uint32_t)R1 - 128u * (uint32_t)j - 32u * h,
+                       h2 = 16u * (uint32_t)R2 - 128u * (uint32_t)j - 32u * h;
+        const uint32_t mm = shl_clamp(0xffffu, h1) | shl_clamp(0xffffu, h2);
+        const uint32_t xx = ((x & ~mm) | (0x00010001u & mm)) - 0x00010001u;
+        const uint32_t yy = ((y & ~mm) | (0x00010001u & mm)) - 0x00010001u;
+        g1[h] += (uint32_t)a1 * xx + (uint32_t)b1 * yy + shl_clamp((uint32_t)pk, h2);
+        g2[h] += (uint32_t)a2 * xx + (uint32_t)b2 * yy;
+    }
+}
+
+// |v| of both biased halfwords
+__device__ __forceinline__ uint32_t abs_halves(uint32_t v) {
+    const uint32_t t = v ^ 0x80008000u;
+    uint32_t m;   // the sign of each half
+    asm("prmt.b32 %0, %1, %1, 0xbb99;" : "=r"(m) : "r"(t));
+    return (t ^ m) + (m & 0x00010001u);
+}
+
+template <bool GEN>
+__device__ __forceinline__ void wide_chunk(const Env& E, uint32_t w1, uint32_t w2, int R1, int R2, int j,
+                                           const Cand& q, int& acc, int& pr) {
+    const uint4 o1 = lds128(wide_at(E.g, E.gst, R1, j)), o2 = lds128(wide_at(E.g, E.gst, R2, j));
+    uint32_t g1[4] = {o1.x, o1.y, o1.z, o1.w}, g2[4] = {o2.x, o2.y, o2.z, o2.w};
+    wide_rows(w1, w2, R1, R2, j, q.a1, q.b1, q.a2, q.b2, q.pk, g1, g2);
+    const uint32_t old1[4] = {o1.x, o1.y, o1.z, o1.w}, old2[4] = {o2.x, o2.y, o2.z, o2.w};
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const uint32_t v = abs_halves(g1[h]) + abs_halves(g2[h]);   // at most 512 a half
+        const uint32_t z = (((abs_halves(g1[h]) + 0x7fff7fffu) & 0x80008000u) >> 15) +
+                           (((abs_halves(g2[h]) + 0x7fff7fffu) & 0x80008000u) >> 15);
+        acc = __dp2a_lo((int)v, 0x0101, acc);
+        acc = __dp2a_lo((int)(z << 12), 0x0101, acc);               // 4096 a conflict
+        if (GEN) {
+            if (E.obj_kind == 1) {
+                auto sq = [](uint32_t a) -> int {
+                    const int lo = (int)(a & 0xffffu) - 32768, hi = (int)(a >> 16) - 32768;
+                    return lo * lo + hi * hi;
+                };
+                pr += sq(g1[h]) + sq(g2[h]) - sq(old1[h]) - sq(old2[h]);
+            } else if (E.obj_kind == 2) {
+                pr += __popc((g1[h] & 0x00010001u) | ((g2[h] & 0x00010001u) << 1)) -
+                      __popc((old1[h] & 0x00010001u) | ((old2[h] & 0x00010001u) << 1));
+            }
+        }
+    }
+}
+
 // The candidate of this lane's group: hot-row tournament, proposal and
 // evaluation of candidate `c` of iteration it + d_it against the replica's
 // current state, from the draw blocks at E.cw.  Groups with act false go
@@ -556,13 +644,16 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
 
     // E: coefficients, then the new values of the lane's rows
     const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
-    const bool lact = 4 * WPL * l < n;                           // the lane holds rows below n
+    const bool lact = WPL == 8 || 4 * WPL * l < n;               // the lane holds rows below n
     const uint32_t loff = lact ? (uint32_t)(4 * WPL * l) : 0u;   // their byte offset
-    uint32_t x[WPL], y[WPL], g1[WPL], g2[WPL];
-    load_words<WPL>(w1 + loff, x);
-    load_words<WPL>(w2 + loff, y);
-    load_words<WPL>(E.g + (uint32_t)R1 * st + loff, g1);
-    load_words<WPL>(E.g + (uint32_t)R2 * st + loff, g2);
+    constexpr int NW = WPL == 8 ? 1 : WPL;
+    uint32_t x[NW], y[NW], g1[NW], g2[NW];
+    if constexpr (WPL < 8) {
+        load_words<WPL>(w1 + loff, x);
+        load_words<WPL>(w2 + loff, y);
+        load_words<WPL>(E.g + (uint32_t)R1 * st + loff, g1);
+        load_words<WPL>(E.g + (uint32_t)R2 * st + loff, g2);
+    }
     const uint32_t rs = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R1) +
                         lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R2);
     const int e11 = (int)lds8(w1 + (uint32_t)R1) - 1, e22 = (int)lds8(w2 + (uint32_t)R2) - 1;
@@ -581,8 +672,14 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     }
     int acc = 0, pr = 0;
     const uint32_t s8 = (uint32_t)(32 * WPL * l);   // bit offset of the lane's first row
+    if constexpr (WPL == 8) {
+        // chunks l, l + 8, ... of eight rows
+#pragma unroll 1
+        for (int j = l; 8 * j < n; j += 8)
+            wide_chunk<GEN>(E, w1, w2, R1, R2, j, q, acc, pr);
+    } else
 #pragma unroll
-    for (int j = 0; j < WPL; ++j) {
+    for (int j = 0; j < NW; ++j) {
         // columns R1 and R2 of the changed rows are left out (the entry of a
         // double flip over two rows apart): their W reads as zero
         const uint32_t h1 = 8u * (uint32_t)R1 - s8 - 32u * j, h2 = 8u * (uint32_t)R2 - s8 - 32u * j;
@@ -643,9 +740,9 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
 __device__ __forceinline__ void best_keys(bool gen_obj, const Cand& q, bool act, int g, bool by_index, unsigned gm,
                                           uint32_t& A, uint32_t& B) {
     const int dc = (q.acc + 2048) >> 12, ds = q.acc - dc * 4096;
-    const uint32_t low = ((uint32_t)(dc + 256) << 5) | (uint32_t)g;
+    const uint32_t low = ((uint32_t)(dc + 512) << 5) | (uint32_t)g;
     if (!gen_obj) {
-        const uint32_t ka = by_index ? (uint32_t)g : ((uint32_t)(ds + 2048) << 14) | low;
+        const uint32_t ka = by_index ? (uint32_t)g : ((uint32_t)(ds + 2048) << 15) | low;
         A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
         B = A;
     } else {
@@ -865,6 +962,83 @@ __device__ __forceinline__ void commit(const Env& E, const Move& mv, int acc, in
     }
 }
 
+// The same above order 128: lane c rewrites chunk c of the two rows, then
+// lane o takes rows o, o + 32, ... of the columns.
+template <bool ONEZ>
+__device__ __forceinline__ void commit_wide(const Env& E, const Move& mv, int acc, int lane) {
+    const int n = E.n, m = ONEZ ? 1 : E.m, sparse = ONEZ ? 0 : E.sparse;
+    const uint32_t st = E.st, slot = E.slot, wbase = E.slot + Slot<8>::w, g = E.g, gst = E.gst;
+    const int R1 = (int)(mv.rc & 255u), R2 = (int)((mv.rc >> 8) & 255u);
+    const int C1 = (int)((mv.rc >> 16) & 255u), C2 = (int)(mv.rc >> 24);
+    const bool two = R2 != R1;
+    const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
+    auto half = [&](int row, int col) -> uint16_t* {
+        return reinterpret_cast<uint16_t*>(xw_smem + wide_at(g, gst, row, col >> 3)) + (col & 7);
+    };
+    uint32_t old1[8], old2[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int o = lane + 32 * k;
+        old1[k] = old2[k] = 0;
+        if (o < n) {
+            old1[k] = *half(R1, o);
+            old2[k] = *half(R2, o);
+        }
+    }
+    const bool mine = 8 * lane < n;
+    uint32_t g1[4], g2[4];
+    if (mine) {
+        const uint4 o1 = lds128(wide_at(g, gst, R1, lane)), o2 = lds128(wide_at(g, gst, R2, lane));
+        g1[0] = o1.x; g1[1] = o1.y; g1[2] = o1.z; g1[3] = o1.w;
+        g2[0] = o2.x; g2[1] = o2.y; g2[2] = o2.z; g2[3] = o2.w;
+        wide_rows(w1, w2, R1, R2, lane, (int)(int8_t)(mv.cf & 255u), (int)(int8_t)((mv.cf >> 8) & 255u),
+                  (int)(int8_t)((mv.cf >> 16) & 255u), (int)(int8_t)(mv.cf >> 24), (int)(int8_t)(mv.ax & 255u), g1, g2);
+    }
+    __syncwarp();
+    if (mine) {
+        *reinterpret_cast<uint4*>(xw_smem + wide_at(g, gst, R1, lane)) = make_uint4(g1[0], g1[1], g1[2], g1[3]);
+        if (two) *reinterpret_cast<uint4*>(xw_smem + wide_at(g, gst, R2, lane)) = make_uint4(g2[0], g2[1], g2[2], g2[3]);
+    }
+    __syncwarp();
+    int d1[8], d[8], S1 = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int o = lane + 32 * k;
+        d1[k] = d[k] = 0;
+        if (o < n) {
+            const uint32_t n1 = *half(R1, o), n2 = *half(R2, o);
+            *half(o, R1) = (uint16_t)n1;
+            if (o != R1) *half(o, R2) = (uint16_t)n2;
+            d1[k] = packed_abs((int)n1 - 32768) - packed_abs((int)old1[k] - 32768);
+            d[k] = d1[k] + (two ? packed_abs((int)n2 - 32768) - packed_abs((int)old2[k] - 32768) : 0);
+            S1 += d1[k];
+        }
+    }
+    S1 = __reduce_add_sync(FULL, S1);
+    const int dc = (acc + 2048) >> 12;
+    const int S = acc - dc * 4096 + dc * (1 << kConfShift);   // both rows, the pair entry once
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const int o = lane + 32 * k;
+        if (o < n) {
+            int* r = reinterpret_cast<int*>(xw_smem + slot + Slot<8>::res) + o;
+            *r += o == R1 ? S1 : o == R2 ? S - S1 + d1[k] : d[k];
+        }
+    }
+    if (lane < 4) {
+        const int cfc = (int)(int8_t)((mv.cf >> (8 * lane)) & 255u);
+        if (cfc != 0) {
+            const uint32_t a = ((lane & 1) ? w2 : w1) + (uint32_t)((lane & 2) ? R2 : R1);
+            xw_smem[a] = (uint8_t)(lds8(a) + (uint32_t)cfc);
+        }
+        if (lane < 2 && ((mv.ax >> (24 + lane)) & 1u)) {
+            const int lost = lane ? C2 : C1, got = lane ? C1 : C2;
+            const int p = (int)((mv.ax >> (8 + 8 * lane)) & 255u);
+            xw_smem[E.mino + (uint32_t)((lane ? R2 : R1) * m + p)] = (uint8_t)(sparse ? got : lost);
+        }
+    }
+}
+
 // tab[d-1] = ceil(exp(-d/T) * 2^32), computed with the same division and
 // exponential as metropolis_accept, so that for a 32-bit draw u
 //   u * 2^-32 < exp(-d/T)  <=>  u < tab[d-1]
@@ -896,12 +1070,55 @@ __device__ __forceinline__ uint64_t globaltimer() {
     return t;
 }
 
-// The replica's W as int8, column-major, into its record.
+// The replica's W as int8, column-major, into its record: a word (four rows
+// of a column) a lane.
 template <int WPL, int GW>
 __device__ __noinline__ void save_w(int8_t* dst, uint32_t wbase, uint32_t st, int n, int lane) {
+    const int wpc = (n + 3) >> 2;
+    const bool whole = (n & 3) == 0;   // every word of the record is aligned and full
+    int c = 0, q = lane;
 #pragma unroll 1
-    for (int c = 0; c < n; ++c)
-        for (int r = lane; r < n; r += GW) dst[(uint32_t)(c * n + r)] = (int8_t)((int)lds8(wbase + (uint32_t)c * st + (uint32_t)r) - 1);
+    for (;;) {
+        while (q >= wpc) {
+            q -= wpc;
+            ++c;
+        }
+        if (c >= n) break;
+        const uint32_t b = ((lds32(wbase + (uint32_t)c * st + 4u * (uint32_t)q) | 0x80808080u) - 0x01010101u) ^ 0x80808080u;
+        int8_t* d = dst + (uint32_t)(c * n + 4 * q);
+        if (whole) {
+            *reinterpret_cast<uint32_t*>(d) = b;
+        } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                if (4 * q + e < n) d[e] = (int8_t)(b >> (8 * e));
+        }
+        q += GW;
+    }
+}
+
+// The best W into the record: the journal's `jn` moves taken out of W,
+// written, and put back.
+template <int WPL, int GW>
+__device__ __forceinline__ void save_best(uint8_t* rec, const XwJob* J, const Env& E, int jn, int lane) {
+    const unsigned gm = group_mask<GW>();
+    const uint32_t wbase = E.slot + Slot<WPL>::w;
+    auto add = [&](int sign) {
+        for (int i = 0; i < jn; ++i) {
+            const uint2 mv = *reinterpret_cast<const uint2*>(xw_smem + E.slot + Slot<WPL>::jrn + 8u * (uint32_t)i);
+            const int cf = (int)(int8_t)((mv.y >> (8 * (lane & 3))) & 255u);
+            if (lane < 4 && cf != 0) {
+                const uint32_t a = wbase + ((lane & 1) ? mv.x >> 24 : (mv.x >> 16) & 255u) * E.st +
+                                   ((lane & 2) ? (mv.x >> 8) & 255u : mv.x & 255u);
+                xw_smem[a] = (uint8_t)((int)lds8(a) + sign * cf);
+            }
+            __syncwarp(gm);
+        }
+    };
+    add(-1);
+    save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_best), wbase, E.st, E.n, lane);
+    __syncwarp(gm);
+    add(1);
 }
 
 // The lane's context, from the job and the slot.
@@ -916,9 +1133,10 @@ __device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, 
     E.sparse = ONEZ ? 0 : J->sparse;
     E.full = !ONEZ && J->w == n;
     E.st = packed_stride(n, WPL);
+    E.gst = WPL == 8 ? wide_stride(n) : E.st;
     const uint32_t mat = xw_pad16((uint32_t)n * E.st);
     E.g = slot + Slot<WPL>::w + mat;
-    E.mino = E.g + mat;
+    E.mino = E.g + (WPL == 8 ? (uint32_t)n * E.gst : mat);
     E.ts = J->target_samples;
     E.bpc = 4 + (E.ts <= 4 ? 1 : 2);   // cached blocks per candidate
     E.cw = draws + (uint32_t)((lane / LPC) * E.bpc) * 16u;
@@ -931,39 +1149,17 @@ __device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, 
     }
 }
 
-// Loads replica `rid` into the slot: W and the minority lists; the masks,
-// the Gram matrix (by popcounts of support and sign masks) and the
-// residuals are rebuilt from W and checked against the header.  False when
-// the replica does not run (job done or solved, budget spent, or a failed
-// self-check, which flags the header).  The group's lanes call it.
-// `owner` false: a copy that writes nothing to the record; it also skips
-// the exits on the job's done and solved flags, which other kernels may set
-// while it loads (its owner decides whether the replica runs).
-template <int WPL, bool GEN, int GW, bool ONEZ>
-__device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane, uint64_t iters,
-                                             Env& E, bool owner) {
+// The slot's structures from the record's W: biased bytes, support masks,
+// minority lists (copied from the record once it holds them), the Gram
+// matrix by popcounts of support and sign masks, the packed residuals.
+// False when an entry is not ternary or a row's weight is not w.
+template <int WPL, int GW>
+__device__ __forceinline__ bool build_packed(const Env& E, const XwJob* J, const uint8_t* rec, uint32_t status0, int w,
+                                             int lane, int& score0, int& conf0, int& par0, long long& sq0) {
     constexpr int OPL = WPL;   // rows o, o + GW, ... of a lane: GW * OPL >= n
     const unsigned gm = group_mask<GW>();
-    uint8_t* rec = a.arena + a.rec_off[rid];
-    RepHeader* H = reinterpret_cast<RepHeader*>(rec);
-    XwJob* J = a.jobs + H->job;
-    if (owner && *(volatile int32_t*)&J->done) return false;
-    if (owner && a.stop_on_solve == 1 && *(volatile int32_t*)&J->solved) return false;
-    const int obj_kind = GEN ? H->obj_kind : 0;
-    if ((ONEZ && (J->m != 1 || J->sparse != 0)) || (!GEN && (H->obj_kind != 0 || J->move_set != 0))) {
-        // a launch of a specialised kernel met a replica it does not cover
-        if (lane == 0) H->err |= XW_ERR_KERNEL;
-        return false;
-    }
-    make_env<WPL, GW, ONEZ>(E, J, slot, slot + Slot<WPL>::draws, lane, obj_kind);
-    const int n = E.n, w = ONEZ ? n - 1 : J->w, m = E.m, sparse = E.sparse;
-    const uint64_t it = H->it;
-    if (J->budget_iters) {
-        if (it >= J->budget_iters) return false;
-        if (iters > J->budget_iters - it) iters = J->budget_iters - it;
-    }
-    const uint32_t status0 = H->status;
-    const uint32_t st = E.st, wbase = slot + Slot<WPL>::w;
+    const int n = E.n, m = E.m, sparse = E.sparse;
+    const uint32_t slot = E.slot, st = E.st, wbase = slot + Slot<WPL>::w;
 
     // W as biased bytes, the pad rows zero (biased 1); support and sign
     // masks of the lane's rows
@@ -1029,10 +1225,7 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
             }
         }
     }
-    if (__any_sync(gm, bad)) {
-        if (lane == 0 && owner) H->err |= XW_ERR_MINORITY;
-        return false;
-    }
+    if (__any_sync(gm, bad)) return false;
     __syncwarp(gm);
     int p_score = 0, p_conf = 0, p_par = 0;
     long long p_sq = 0;
@@ -1072,13 +1265,201 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
             p_conf += r_sum >> kConfShift;
         }
     }
-    const int score0 = __reduce_add_sync(gm, p_score) / 2;
-    const int conf0 = __reduce_add_sync(gm, p_conf) / 2;
+    score0 = __reduce_add_sync(gm, p_score) / 2;
+    conf0 = __reduce_add_sync(gm, p_conf) / 2;
 #pragma unroll
     for (int off = GW / 2; off > 0; off >>= 1) p_sq += __shfl_xor_sync(gm, p_sq, off, GW);
-    const long long sq0 = p_sq / 2;
-    const int par0 = __reduce_add_sync(gm, p_par) / 2;
+    sq0 = p_sq / 2;
+    par0 = __reduce_add_sync(gm, p_par) / 2;
     __syncwarp(gm);
+    return true;
+}
+
+// The same above order 128.  The masks of all rows (support and sign, 64
+// bytes a row) sit in the place of the last rows of G while the rows before
+// them are computed; those last rows (at most 32) are the transpose of what
+// is known by then and a block among themselves.
+__device__ __forceinline__ bool build_wide(const Env& E, const XwJob* J, const uint8_t* rec, uint32_t status0, int w,
+                                           int lane, int& score0, int& conf0, int& par0, long long& sq0) {
+    const int n = E.n, m = E.m, sparse = E.sparse;
+    const uint32_t slot = E.slot, st = E.st, wbase = slot + Slot<8>::w, g = E.g, gst = E.gst;
+    const int tail = (int)((64u * (uint32_t)n + gst - 1u) / gst), n0 = n - tail;
+    const uint32_t masks = g + (uint32_t)n0 * gst;   // row o: words 16 o + q support, + 8 sign
+    const int8_t* gw = reinterpret_cast<const int8_t*>(rec + J->off_w);
+    int bad = 0;
+#pragma unroll 1
+    for (int o = lane; o < (int)st; o += 32) {
+#pragma unroll 1
+        for (int q = 0; 32 * q < n; ++q) {
+            uint32_t sup = 0, neg = 0;
+            const int c1 = min(n, 32 * q + 32);
+#pragma unroll 8
+            for (int c = 32 * q; c < c1; ++c) {
+                const int v = o < n ? gw[(uint32_t)(c * n + o)] : 0;
+                if (v < -1 || v > 1) bad = 1;
+                if (v) sup |= 1u << (c & 31);
+                if (v < 0) neg |= 1u << (c & 31);
+                xw_smem[wbase + (uint32_t)c * st + (uint32_t)o] = (uint8_t)(v + 1);
+            }
+            if (o < n) {
+                reinterpret_cast<uint32_t*>(xw_smem + masks)[16 * o + q] = sup;
+                reinterpret_cast<uint32_t*>(xw_smem + masks)[16 * o + 8 + q] = neg;
+            }
+        }
+    }
+    if (m == 0 && lane == 0) xw_smem[E.mino] = 0;   // an empty list still reads as column 0
+    const int nq = (n + 31) >> 5;
+#pragma unroll 1
+    for (int o = lane; o < n; o += 32) {
+        int weight = 0, pos = 0;
+#pragma unroll 1
+        for (int q = 0; q < nq; ++q) {
+            const uint32_t sup = lds32(masks + 64u * (uint32_t)o + 4u * (uint32_t)q);
+            weight += __popc(sup);
+            if (m > 0 && !(status0 & XW_STATUS_INIT)) {
+                const int left = n - 32 * q;
+                uint32_t x = (sparse ? sup : ~sup) & (left >= 32 ? 0xffffffffu : (1u << left) - 1u);
+                while (x && pos < m) {
+                    xw_smem[E.mino + (uint32_t)(o * m + pos)] = (uint8_t)(32 * q + __ffs((int)x) - 1);
+                    x &= x - 1;
+                    ++pos;
+                }
+            }
+        }
+        if (weight != w) bad = 1;
+    }
+    if (m > 0 && (status0 & XW_STATUS_INIT)) {
+        const uint8_t* gm8 = rec + J->off_mino;
+        for (uint32_t i = lane; i < (uint32_t)(n * m); i += 32) xw_smem[E.mino + i] = gm8[i];
+    }
+    if (__any_sync(FULL, bad)) return false;
+    __syncwarp();
+    auto half = [&](int row, int col) -> uint16_t* {
+        return reinterpret_cast<uint16_t*>(xw_smem + wide_at(g, gst, row, col >> 3)) + (col & 7);
+    };
+    // the lane's row of the tail, before it is overwritten
+    uint32_t ts[8], tn[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        ts[q] = tn[q] = 0;
+        if (lane < tail && q < nq) {
+            ts[q] = lds32(masks + 64u * (uint32_t)(n0 + lane) + 4u * (uint32_t)q);
+            tn[q] = lds32(masks + 64u * (uint32_t)(n0 + lane) + 32u + 4u * (uint32_t)q);
+        }
+    }
+#pragma unroll 1
+    for (int o = lane; o < (int)st; o += 32) {
+        uint32_t sup[8], neg[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            sup[q] = neg[q] = 0;
+            if (o < n && q < nq) {
+                sup[q] = lds32(masks + 64u * (uint32_t)o + 4u * (uint32_t)q);
+                neg[q] = lds32(masks + 64u * (uint32_t)o + 32u + 4u * (uint32_t)q);
+            }
+        }
+#pragma unroll 2
+        for (int r = 0; r < n0; ++r) {
+            int dot = 0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4 rs = lds128(masks + 64u * (uint32_t)r + 16u * h), rn = lds128(masks + 64u * (uint32_t)r + 32u + 16u * h);
+                if (4 * h < nq) {
+                    const uint32_t b0 = sup[4 * h] & rs.x, b1 = sup[4 * h + 1] & rs.y, b2 = sup[4 * h + 2] & rs.z,
+                                   b3 = sup[4 * h + 3] & rs.w;
+                    dot += __popc(b0) + __popc(b1) + __popc(b2) + __popc(b3) -
+                           2 * (__popc(b0 & (neg[4 * h] ^ rn.x)) + __popc(b1 & (neg[4 * h + 1] ^ rn.y)) +
+                                __popc(b2 & (neg[4 * h + 2] ^ rn.z)) + __popc(b3 & (neg[4 * h + 3] ^ rn.w)));
+                }
+            }
+            *half(r, o) = (uint16_t)(32768 + (o == r || o >= n ? 0 : dot));
+        }
+    }
+    __syncwarp();
+    // the last rows: columns below n0 by symmetry, then the block of the tail
+#pragma unroll 1
+    for (int r = n0; r < n; ++r)
+        for (int o = lane; o < n0; o += 32) *half(r, o) = *half(o, r);
+#pragma unroll 1
+    for (int t = 0; t < tail; ++t) {
+        int dot = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t both = ts[q] & __shfl_sync(FULL, ts[q], t);
+            dot += __popc(both) - 2 * __popc(both & (tn[q] ^ __shfl_sync(FULL, tn[q], t)));
+        }
+        const int o = n0 + lane;
+        if (lane < tail) *half(n0 + t, o) = (uint16_t)(32768 + (lane == t ? 0 : dot));
+        // the row's pad
+        for (int c = n + lane; c < (int)st; c += 32) *half(n0 + t, c) = 32768;
+    }
+    __syncwarp();
+    int p_score = 0, p_conf = 0, p_par = 0;
+    long long p_sq = 0;
+#pragma unroll 1
+    for (int o = lane; o < n; o += 32) {
+        int r_sum = 0;
+#pragma unroll 4
+        for (int r = 0; r < n; ++r) {
+            const int v = (int)*half(r, o) - 32768;
+            r_sum += packed_abs(v);
+            p_sq += (long long)(v * v);
+            p_par += v & 1;
+        }
+        reinterpret_cast<int*>(xw_smem + slot + Slot<8>::res)[o] = r_sum;
+        p_score += r_sum & ((1 << kConfShift) - 1);
+        p_conf += r_sum >> kConfShift;
+    }
+    score0 = __reduce_add_sync(FULL, p_score) / 2;
+    conf0 = __reduce_add_sync(FULL, p_conf) / 2;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) p_sq += __shfl_xor_sync(FULL, p_sq, off);
+    sq0 = p_sq / 2;
+    par0 = __reduce_add_sync(FULL, p_par) / 2;
+    __syncwarp();
+    return true;
+}
+
+// Loads replica `rid` into the slot: W and the minority lists; the masks,
+// the Gram matrix (by popcounts of support and sign masks) and the
+// residuals are rebuilt from W and checked against the header.  False when
+// the replica does not run (job done or solved, budget spent, or a failed
+// self-check, which flags the header).  The group's lanes call it.
+// `owner` false: a copy that writes nothing to the record; it also skips
+// the exits on the job's done and solved flags, which other kernels may set
+// while it loads (its owner decides whether the replica runs).
+template <int WPL, bool GEN, int GW, bool ONEZ>
+__device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane, uint64_t iters,
+                                             Env& E, bool owner) {
+    const unsigned gm = group_mask<GW>();
+    uint8_t* rec = a.arena + a.rec_off[rid];
+    RepHeader* H = reinterpret_cast<RepHeader*>(rec);
+    XwJob* J = a.jobs + H->job;
+    if (owner && *(volatile int32_t*)&J->done) return false;
+    if (owner && a.stop_on_solve == 1 && *(volatile int32_t*)&J->solved) return false;
+    const int obj_kind = GEN ? H->obj_kind : 0;
+    if ((ONEZ && (J->m != 1 || J->sparse != 0)) || (!GEN && (H->obj_kind != 0 || J->move_set != 0))) {
+        // a launch of a specialised kernel met a replica it does not cover
+        if (lane == 0) H->err |= XW_ERR_KERNEL;
+        return false;
+    }
+    make_env<WPL, GW, ONEZ>(E, J, slot, slot + Slot<WPL>::draws, lane, obj_kind);
+    const int w = ONEZ ? E.n - 1 : J->w;
+    const uint64_t it = H->it;
+    if (J->budget_iters) {
+        if (it >= J->budget_iters) return false;
+        if (iters > J->budget_iters - it) iters = J->budget_iters - it;
+    }
+    const uint32_t status0 = H->status;
+    int score0, conf0, par0;
+    long long sq0;
+    bool ok;
+    if constexpr (WPL == 8) ok = build_wide(E, J, rec, status0, w, lane, score0, conf0, par0, sq0);
+    else ok = build_packed<WPL, GW>(E, J, rec, status0, w, lane, score0, conf0, par0, sq0);
+    if (!ok) {
+        if (lane == 0 && owner) H->err |= XW_ERR_MINORITY;
+        return false;
+    }
 
     const int64_t obj0 = obj_kind == 1 ? sq0 : obj_kind == 2 ? par0 : score0;
     const bool init = status0 & XW_STATUS_INIT;
@@ -1111,7 +1492,7 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
         c.mb = init ? -H->msi : 0;
         c.cb = init ? -H->cool_ctr : 0;
         c.k_end = (int32_t)(iters < 0x7ffffffeull ? iters : 0x7ffffffeull);
-        c.dirty = init ? 0 : 1;
+        c.jn = init ? -1 : 0;
         c.owner = owner ? 1 : 0;
         c.rid = rid;
         *con_of<WPL>(slot) = c;
@@ -1134,7 +1515,7 @@ __device__ __forceinline__ void store_replica(const AnnealArgs& a, const Env& E,
     RepHeader* H = reinterpret_cast<RepHeader*>(rec);
     const XwJob* J = a.jobs + H->job;
     const uint32_t wbase = E.slot + Slot<WPL>::w;
-    if (con->dirty) save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_best), wbase, E.st, E.n, lane);
+    if (con->jn >= 0) save_best<WPL, GW>(rec, J, E, con->jn, lane);
     save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_w), wbase, E.st, E.n, lane);
     uint8_t* gmo = rec + J->off_mino;
     for (uint32_t i = lane; i < (uint32_t)(E.n * E.m); i += GW) gmo[i] = xw_smem[E.mino + i];
@@ -1169,17 +1550,16 @@ __device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, c
     Con* con = con_of<WPL>(E.slot);
     const int dc = (acc + 2048) >> 12;
     int4 b = con->best, t = con->acc;
-    const bool dirty = con->dirty != 0;
+    const int jn = con->jn;
     b.x += acc - dc * 4096;
     b.y += dc;
     const bool improved = b.x < b.z || (b.x == b.z && b.y < b.w);
-    if (dirty && !improved && con->owner) {
+    if (jn == kJournal && !improved && con->owner) {
         uint8_t* rec = a.arena + a.rec_off[con->rid];
-        const XwJob* J = a.jobs + reinterpret_cast<RepHeader*>(rec)->job;
-        save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_best), E.slot + Slot<WPL>::w, E.st, E.n, lane);
-        __syncwarp(gm);
+        save_best<WPL, GW>(rec, a.jobs + reinterpret_cast<RepHeader*>(rec)->job, E, jn, lane);
     }
-    commit<WPL, GW, ONEZ>(E, mv, acc, lane);
+    if constexpr (WPL == 8) commit_wide<ONEZ>(E, mv, acc, lane);
+    else commit<WPL, GW, ONEZ>(E, mv, acc, lane);
     if (lane == 0) {
         const long long o = (long long)(((uint64_t)(uint32_t)t.y << 32) | (uint32_t)t.x) + prim;
         t.x = (int)(uint32_t)o;
@@ -1204,7 +1584,13 @@ __device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, c
             }
         }
         con->best = b;
-        con->dirty = improved ? 1 : 0;
+        if (improved) {
+            con->jn = 0;
+        } else if (jn >= 0) {
+            if (jn < kJournal)
+                *reinterpret_cast<uint2*>(xw_smem + E.slot + Slot<WPL>::jrn + 8u * (uint32_t)jn) = make_uint2(mv.rc, mv.cf);
+            con->jn = jn < kJournal ? jn + 1 : -1;
+        }
     }
     __syncwarp(gm);
     return improved;
