@@ -38,24 +38,89 @@ namespace xw {
 
 namespace {
 
-// The one-warp (or half-warp) replica loop.
+// Position of a replica's loop.
+struct Walk {
+    int k;               // calls made
+    int wpos;            // next iteration of the window of move-level draws
+    uint32_t wmask;      // bit j: iteration j of the window has several candidates
+    uint32_t multis;     // iterations of several candidates
+    uint32_t two_l;      // two-row candidates of this lane's group
+};
+
+// One step of a replica, at most to call k_lim: returns whether a move was
+// accepted; `improved`: it is the best yet.
 //
 // An iteration proposes one candidate or, with the job's greedy
-// probability, candidate_samples of them.  A step of this loop gives its
-// four candidate groups either the candidates of one iteration or, in a run
-// of one-candidate iterations, the next up to four iterations of the run:
+// probability, candidate_samples of them.  A step gives its four candidate
+// groups either the candidates of one iteration or, in a run of
+// one-candidate iterations, the next up to four iterations of the run:
 // their draws and the kind of each are known ahead (counter-based), and
 // while no move is accepted they see the same state.  The first accepted
 // one is committed; the iterations after it are proposed again.  The
 // trajectory is that of one iteration at a time.  (Acceptance is 11% on the
 // W(26,25) ladder: 0.85 steps an iteration.)
 template <int WPL, bool GEN, int GW, bool ONEZ>
-__device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane,
-                                            uint64_t iters) {
+__device__ __forceinline__ bool step(const AnnealArgs& a, const Env& E, Walk& w, int k_lim, int lane, bool& improved) {
     constexpr int LPC = GW / 4;
     constexpr int kWin = GW;   // iterations whose move-level draws are computed at once
     const unsigned gm = group_mask<GW>();
     const int wl0 = GW == 32 ? 0 : (int)(threadIdx.x & 16u);
+    const Con* con = con_of<WPL>(E.slot);
+    const int g = lane / LPC;
+    const uint32_t win = E.slot + Slot<WPL>::win;
+    if (w.wpos >= kWin) {
+        const uint4 b = draw_block(0u, con->it0 + (uint64_t)(w.k + lane), con->stream, con->k0, con->k1);
+        w.wmask = __ballot_sync(gm, (uint64_t)b.x < con->thr_greedy) >> wl0;
+        *reinterpret_cast<uint32_t*>(xw_smem + win + 4u * (uint32_t)lane) = b.y;
+        w.wpos = 0;
+        __syncwarp(gm);
+    }
+    const uint32_t rem = w.wmask >> w.wpos;
+    const bool multi = rem & 1u;
+    const uint64_t it = con->it0 + (uint64_t)w.k;
+    bool accept;
+    int used = 1, acc, prim;
+    Move mv;
+    w.multis += rem & 1u;
+    if (multi && con->cs > 4) {
+        const Winner c = choose_many<WPL, GEN, GW, ONEZ>(E, it, con->cs, lane);
+        mv = c.mv;
+        acc = c.acc;
+        prim = c.prim;
+        if (lane == 0) w.two_l += (uint32_t)c.two;
+        accept = accepts<WPL>(E.slot, prim, lds32(win + 4u * (uint32_t)w.wpos));
+    } else {
+        const int run = multi ? con->cs : min(min(__ffs((int)(rem | 16u)) - 1, kWin - w.wpos), k_lim - w.k);
+        const bool act = g < run;
+        fill_draws<GW>(E, con, it, 0, multi, lane);
+        __syncwarp(gm);
+        const Cand q = candidate<WPL, GEN, GW, ONEZ>(E, it, multi ? 0 : g, multi ? g : 0, act, lane);
+        const bool ok = accepts<WPL>(E.slot, q.prim, lds32(win + 4u * (uint32_t)(w.wpos + (multi ? 0 : g))));
+        const uint32_t oks = __ballot_sync(gm, act && ok) >> wl0;
+        // the best candidate, or the first accepted iteration of a run
+        uint32_t A, B;
+        best_keys(GEN && E.obj_kind != 0, q, act && (multi || ok), g, !multi, gm, A, B);
+        const int src = (int)(B & 3u) * LPC;
+        accept = (oks >> src) & 1u;   // (a run without one: group 3, whose bit is clear)
+        if (!multi) used = accept ? (int)(B & 3u) + 1 : run;
+        w.two_l += q.R2 != q.R1 && (multi ? act : g < used) ? 1u : 0u;
+        if (accept) {
+            mv = move_of(pack_move(q), wl0 + src, gm);
+            acc = __shfl_sync(gm, q.acc, wl0 + src);
+            prim = __shfl_sync(gm, q.prim, wl0 + src);
+        }
+    }
+    w.k += used;
+    w.wpos += used;
+    improved = accept && accept_move<WPL, GEN, GW, ONEZ>(a, E, mv, acc, prim, w.k, lane);
+    return accept;
+}
+
+// The one-warp (or half-warp) replica loop.
+template <int WPL, bool GEN, int GW, bool ONEZ>
+__device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, uint32_t slot, int lane,
+                                            uint64_t iters) {
+    constexpr int LPC = GW / 4;
     Env E;
     if (!load_replica<WPL, GEN, GW, ONEZ>(a, rid, slot, lane, iters, E, true)) return;
     auto job = [&]() -> XwJob* { return a.jobs + reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[rid])->job; };
@@ -69,14 +134,11 @@ __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, u
     };
     // the next k at which something besides moves happens
     auto event = [&](const Con* con, int k) -> int {
-        int e = max(next_event<WPL>(job(), con), k + 1);
+        int e = max(next_event(con), k + 1);
         if (a.stop_on_solve == 1) e = min(e, (k | 63) == k ? k + 64 : k | 63);
         return e;
     };
-    int k = 0;                       // calls made
-    uint32_t multis = 0, two_l = 0;  // iterations of several candidates; two-row candidates of this lane's group
-    uint32_t wmask = 0;              // bit j: iteration j of the window has several candidates
-    int wpos = kWin;
+    Walk w{0, GW, 0u, 0u, 0u};
     int k_evt = event(con_of<WPL>(slot), 0);
     bool live = !stops(con_of<WPL>(slot), 0);
 #pragma unroll 1
@@ -85,65 +147,20 @@ __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, u
         // across the loop they cost more in spilled registers
         asm volatile("" : "+r"(E.slot), "+r"(lane));
         const Con* con = con_of<WPL>(E.slot);
-        const int g = lane / LPC;
-        const uint32_t win = E.slot + Slot<WPL>::win;
-        if (wpos >= kWin) {
-            const uint4 b = draw_block(0u, con->it0 + (uint64_t)(k + lane), con->stream, con->k0, con->k1);
-            wmask = __ballot_sync(gm, (uint64_t)b.x < con->thr_greedy) >> wl0;
-            *reinterpret_cast<uint32_t*>(xw_smem + win + 4u * (uint32_t)lane) = b.y;
-            wpos = 0;
-            __syncwarp(gm);
-        }
-        const uint32_t rem = wmask >> wpos;
-        const bool multi = rem & 1u;
-        const uint64_t it = con->it0 + (uint64_t)k;
-        bool accept;
-        int used = 1, acc, prim;
-        Move mv;
-        multis += rem & 1u;
-        if (multi && con->cs > 4) {
-            const Winner w = choose_many<WPL, GEN, GW, ONEZ>(E, it, con->cs, lane);
-            mv = w.mv;
-            acc = w.acc;
-            prim = w.prim;
-            if (lane == 0) two_l += (uint32_t)w.two;
-            accept = accepts<WPL>(E.slot, prim, lds32(win + 4u * (uint32_t)wpos));
-        } else {
-            const int run = multi ? con->cs : min(min(__ffs((int)(rem | 16u)) - 1, kWin - wpos), k_evt - k);
-            const bool act = g < run;
-            fill_draws<GW>(E, con, it, 0, multi, lane);
-            __syncwarp(gm);
-            const Cand q = candidate<WPL, GEN, GW, ONEZ>(E, it, multi ? 0 : g, multi ? g : 0, act, lane);
-            const bool ok = accepts<WPL>(E.slot, q.prim, lds32(win + 4u * (uint32_t)(wpos + (multi ? 0 : g))));
-            const uint32_t oks = __ballot_sync(gm, act && ok) >> wl0;
-            // the best candidate, or the first accepted iteration of a run
-            uint32_t A, B;
-            best_keys(GEN && E.obj_kind != 0, q, act && (multi || ok), g, !multi, gm, A, B);
-            const int src = (int)(B & 3u) * LPC;
-            accept = (oks >> src) & 1u;   // (a run without one: group 3, whose bit is clear)
-            if (!multi) used = accept ? (int)(B & 3u) + 1 : run;
-            two_l += q.R2 != q.R1 && (multi ? act : g < used) ? 1u : 0u;
-            if (accept) {
-                mv = move_of(pack_move(q), wl0 + src, gm);
-                acc = __shfl_sync(gm, q.acc, wl0 + src);
-                prim = __shfl_sync(gm, q.prim, wl0 + src);
-            }
-        }
-        k += used;
-        wpos += used;
+        bool improved;
+        step<WPL, GEN, GW, ONEZ>(a, E, w, k_evt, lane, improved);
         // an improvement puts the reheat off (an event due now still comes)
-        if (accept && accept_move<WPL, GEN, GW, ONEZ>(a, E, mv, acc, prim, k, lane) && k < k_evt)
-            k_evt = a.stop_on_solve && con->best.z == 0 ? k : event(con, k);
-        if (k >= k_evt) {
-            temperature_step<WPL, GW>(a, E.slot, k, lane);
-            live = !stops(con, k);
-            k_evt = event(con, k);
+        if (improved && w.k < k_evt) k_evt = a.stop_on_solve && con->best.z == 0 ? w.k : event(con, w.k);
+        if (w.k >= k_evt) {
+            temperature_step<WPL, GW>(a, E.slot, w.k, lane);
+            live = !stops(con, w.k);
+            k_evt = event(con, w.k);
         }
     }
     const uint64_t evals =
-        (uint64_t)((uint32_t)k - multis) + (uint64_t)multis * (uint64_t)con_of<WPL>(E.slot)->cs;
-    const uint32_t evals2 = __reduce_add_sync(gm, (lane & (LPC - 1)) == 0 ? two_l : 0u);
-    store_replica<WPL, GW>(a, E, k, evals, evals2, lane);
+        (uint64_t)((uint32_t)w.k - w.multis) + (uint64_t)w.multis * (uint64_t)con_of<WPL>(E.slot)->cs;
+    const uint32_t evals2 = __reduce_add_sync(group_mask<GW>(), (lane & (LPC - 1)) == 0 ? w.two_l : 0u);
+    store_replica<WPL, GW>(a, E, w.k, evals, evals2, lane);
 }
 
 // Latency mode: one replica per CTA of K warps, speculating K iterations at
@@ -158,6 +175,15 @@ __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, u
 // move; a round advances by the run of rejections up to the next accept
 // (about 2-4 iterations at the acceptance rates of cooling runs) in about
 // the time of one iteration, so a lone search runs that much faster.
+
+//
+// Where moves are accepted every iteration or two a round advances no
+// further than one step of the one-warp loop and takes longer (2000
+// iterations of W(12,11) with its hottest replica accepting all: 3.15 ms in
+// the one-warp loop, 4.1 with 2 warps, 6.1 with 16, 8.2 with 64 on four SMs).
+// So warp 0 watches the advance: below kSoloAdvance iterations a round it
+// goes on alone, step by step, until accepts are rare enough again (in a
+// cluster every CTA's warp 0 makes the same steps on its copy).
 
 // Per-warp results and the round's control word, after the slot's own
 // (warp 0's) structures and the other warps' draw buffers.
@@ -218,6 +244,9 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
     bool ok = false;
     const int KT = K * CL;
     int k = 0, k_evt = 0, k_end = 0;
+    // a round's cost in steps of the one-warp loop, in tenths (measured)
+    const int cost10 = CL > 1 ? 26 : 12 + K / 2;
+    int rounds = 0, round_k = 0;   // rounds since the last look, and k then
     uint64_t evals = 0;
     uint32_t evals2 = 0;
     // warp 0 loads the replica; the round size goes to the others through
@@ -225,7 +254,7 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
     if (warp == 0) {
         ok = load_replica<WPL, GEN, 32, ONEZ>(a, rid, 0u, lane, a.iters, E, owner);
         if (ok) {
-            k_evt = max(next_event<WPL>(J, con), 1);
+            k_evt = max(next_event(con), 1);
             k_end = con->k_end;
         }
         if (lane == 0 && owner) {
@@ -322,12 +351,12 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
             auto after_call = [&]() {
                 if (k >= k_evt) {
                     temperature_step<WPL, 32>(a, 0u, k, lane);
-                    k_evt = max(next_event<WPL>(J, con), k + 1);
+                    k_evt = max(next_event(con), k + 1);
                 }
             };
             auto commit_of = [&](int q) {
                 if (accept_move<WPL, GEN, 32, ONEZ>(a, E, outs[q].mv, outs[q].dsc, outs[q].prim, k, lane) && k < k_evt)
-                    k_evt = max(next_event<WPL>(J, con), k + 1);
+                    k_evt = max(next_event(con), k + 1);
             };
             // lane l looks at iterations l and 32 + l (up to 64 iterations a
             // round, on a cluster of four)
@@ -369,6 +398,43 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
                 }
             }
             if (a.stop_on_solve && con->best.z == 0) stop = true;
+            // alone from here?  (a step of the one-warp loop makes 1.1
+            // iterations or more)
+            ++rounds;
+            bool solo = false;
+            if (rounds >= 8) {
+                solo = (k - round_k) * 100 < rounds * cost10 * 11;
+                rounds = 0;
+                round_k = k;
+            }
+            if (solo && !stop) {
+                Walk w{k, 32, 0u, 0u, 0u};
+                // the job's solved flag is looked at between rounds only
+                const int k_poll = a.stop_on_solve == 1 ? ((k | 63) == k ? k : k | 63) : k_end;
+                while (solo) {
+                    const int k1 = min(min(w.k + 64, k_poll), k_end);
+                    int steps = 0, accs = 0;
+                    while (w.k < k1) {
+                        bool improved;
+                        accs += step<WPL, GEN, 32, ONEZ>(a, E, w, min(k_evt, k1), lane, improved) ? 1 : 0;
+                        ++steps;
+                        if (improved && w.k < k_evt) k_evt = max(next_event(con), w.k + 1);
+                        if (w.k >= k_evt) {
+                            temperature_step<WPL, 32>(a, 0u, w.k, lane);
+                            k_evt = max(next_event(con), w.k + 1);
+                        }
+                        if (a.stop_on_solve && con->best.z == 0) {
+                            stop = true;
+                            break;
+                        }
+                    }
+                    solo = !stop && steps > 0 && w.k < k_poll && w.k < k_end && steps * 10 < accs * cost10;
+                }
+                evals += (uint64_t)((uint32_t)(w.k - k) - w.multis) + (uint64_t)w.multis * (uint64_t)con->cs;
+                evals2 += __reduce_add_sync(FULL, (lane & 7) == 0 ? w.two_l : 0u);
+                k = w.k;
+                round_k = k;
+            }
             if (lane == 0) {
                 ctl->k = k;
                 ctl->count = stop ? 0 : min(k_end - k, KT);
@@ -442,21 +508,21 @@ __global__ void __maxnreg__(anneal_maxnreg(OPL, GEN, GW)) anneal_kernel(AnnealAr
 
 // The latency mode: one CTA (CL = 1, a persistent loop over the launch's
 // replicas) or one cluster of CL CTAs (one replica per cluster) per replica.
-template <bool GEN, int CL>
+template <bool GEN, int CL, bool ONEZ>
 __global__ void __launch_bounds__(512, 1) anneal_spec_kernel(AnnealArgs a, int K) {
     __shared__ uint32_t s_item;
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     if constexpr (CL > 1) {
         const uint32_t item = blockIdx.x / CL;
-        if (item < a.n_items) run_replica_spec<1, GEN, CL, false>(a, a.items[item], warp, K, lane);
+        if (item < a.n_items) run_replica_spec<1, GEN, CL, ONEZ>(a, a.items[item], warp, K, lane);
     } else {
         for (;;) {
             if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1u);
             __syncthreads();
             const uint32_t item = s_item;
             if (item >= a.n_items) break;
-            run_replica_spec<1, GEN, 1, false>(a, a.items[item], warp, K, lane);
+            run_replica_spec<1, GEN, 1, ONEZ>(a, a.items[item], warp, K, lane);
             __syncthreads();
         }
     }
@@ -641,15 +707,20 @@ uint32_t anneal_spec_cta_bytes(uint32_t slot_bytes, int wpr, int ctas) {
     return spec_layout(slot_bytes, wpr / ctas, ctas).bytes;
 }
 
-const void* anneal_spec_kernel_fn(bool general, int ctas) {
+template <bool ONEZ>
+const void* spec_fn(bool general, int ctas) {
     if (ctas == 4)
-        return general ? reinterpret_cast<const void*>(&anneal_spec_kernel<true, 4>)
-                       : reinterpret_cast<const void*>(&anneal_spec_kernel<false, 4>);
+        return general ? reinterpret_cast<const void*>(&anneal_spec_kernel<true, 4, ONEZ>)
+                       : reinterpret_cast<const void*>(&anneal_spec_kernel<false, 4, ONEZ>);
     if (ctas == 2)
-        return general ? reinterpret_cast<const void*>(&anneal_spec_kernel<true, 2>)
-                       : reinterpret_cast<const void*>(&anneal_spec_kernel<false, 2>);
-    return general ? reinterpret_cast<const void*>(&anneal_spec_kernel<true, 1>)
-                   : reinterpret_cast<const void*>(&anneal_spec_kernel<false, 1>);
+        return general ? reinterpret_cast<const void*>(&anneal_spec_kernel<true, 2, ONEZ>)
+                       : reinterpret_cast<const void*>(&anneal_spec_kernel<false, 2, ONEZ>);
+    return general ? reinterpret_cast<const void*>(&anneal_spec_kernel<true, 1, ONEZ>)
+                   : reinterpret_cast<const void*>(&anneal_spec_kernel<false, 1, ONEZ>);
+}
+
+const void* anneal_spec_kernel_fn(bool general, int ctas, bool one_zero) {
+    return one_zero ? spec_fn<true>(general, ctas) : spec_fn<false>(general, ctas);
 }
 
 cudaError_t launch_anneal_spec(const AnnealArgs& args, bool general, int wpr, int ctas, int blocks,
@@ -660,7 +731,7 @@ cudaError_t launch_anneal_spec(const AnnealArgs& args, bool general, int wpr, in
     int k = wpr / CL;
     void* kargs[] = {const_cast<AnnealArgs*>(&args), &k};
     if (CL == 1)
-        return cudaLaunchKernel(anneal_spec_kernel_fn(general, 1), dim3(blocks), dim3(32 * k), kargs,
+        return cudaLaunchKernel(anneal_spec_kernel_fn(general, 1, args.one_zero != 0), dim3(blocks), dim3(32 * k), kargs,
                                 args.slot_bytes, stream);
     // one cluster of CL CTAs per replica
     cudaLaunchConfig_t cfg = {};
@@ -675,7 +746,7 @@ cudaError_t launch_anneal_spec(const AnnealArgs& args, bool general, int wpr, in
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelExC(&cfg, anneal_spec_kernel_fn(general, CL), kargs);
+    return cudaLaunchKernelExC(&cfg, anneal_spec_kernel_fn(general, CL, args.one_zero != 0), kargs);
 }
 
 cudaError_t launch_exchange(XwJob* jobs, int njobs, uint8_t* arena, const uint64_t* rec_off, const double* ladder,

@@ -825,7 +825,7 @@ bool Batch::configure_latency(size_t k, int wpr) {
         if (wpr % q == 0 && wpr / q >= 2 && wpr / q <= 16) cl = q;
     }
     if (cl == 0) return false;
-    const void* fn = anneal_spec_kernel_fn(c.general, cl);
+    const void* fn = anneal_spec_kernel_fn(c.general, cl, c.one_zero);
     raise_smem_limit(fn, params.device);
     const uint32_t bytes = anneal_spec_cta_bytes(c.slot_bytes, wpr, cl);
     int per_sm = 0;

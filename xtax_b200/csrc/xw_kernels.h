@@ -63,7 +63,7 @@ cudaError_t launch_anneal(const AnnealArgs& args, int opl, bool general, int war
 // one CTA, or a cluster of two or four (one replica per cluster, `blocks`
 // unused)
 uint32_t anneal_spec_cta_bytes(uint32_t slot_bytes, int wpr, int ctas);
-const void* anneal_spec_kernel_fn(bool general, int ctas);
+const void* anneal_spec_kernel_fn(bool general, int ctas, bool one_zero);
 cudaError_t launch_anneal_spec(const AnnealArgs& args, bool general, int wpr, int ctas, int blocks,
                                cudaStream_t stream);
 // Orders above XW_MAX_N (xw_anneal_large.cu), in one of three forms:

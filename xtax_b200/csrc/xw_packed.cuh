@@ -120,6 +120,7 @@ struct Con {
     int4 acc;            // objective total (64 bits), accepted moves, rows they changed
     double T;
     int32_t mb, cb;
+    int32_t mpc, stuck;  // calls per cooling step, calls without improvement before a reheat (tempering: never)
     int32_t k_end;       // iterations of this launch
     // moves accepted since the best W, all of them in the journal: the record
     // holds an older one.  -1: the record holds the best W.
@@ -1491,6 +1492,8 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
                           init ? (int)H->accepted_rows : 0);
         c.mb = init ? -H->msi : 0;
         c.cb = init ? -H->cool_ctr : 0;
+        c.mpc = J->tempering ? 0x7fffffff : J->moves_per_cool;
+        c.stuck = J->tempering ? 0x7fffffff : J->stuck_threshold;
         c.k_end = (int32_t)(iters < 0x7ffffffeull ? iters : 0x7ffffffeull);
         c.jn = init ? -1 : 0;
         c.owner = owner ? 1 : 0;
@@ -1599,14 +1602,9 @@ __device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, c
 // Calls that can be made after call k before the temperature changes or
 // the replica's calls end: the first k at which temperature_step has
 // something to do.
-template <int WPL>
-__device__ __forceinline__ int next_event(const XwJob* J, const Con* con) {
-    long long e = con->k_end;
-    if (!J->tempering) {
-        e = min(e, (long long)con->cb + J->moves_per_cool);
-        e = min(e, (long long)con->mb + J->stuck_threshold);
-    }
-    return (int)e;
+__device__ __forceinline__ int next_event(const Con* con) {
+    const long long e = min((long long)con->cb + con->mpc, (long long)con->mb + con->stuck);
+    return (int)min(e, (long long)con->k_end);
 }
 
 // Cooling and reheat after call k (xweigh_cuda.cu:1087-1129).
@@ -1614,11 +1612,10 @@ template <int WPL, int GW>
 __device__ __forceinline__ void temperature_step(const AnnealArgs& a, uint32_t slot, int k, int lane) {
     const unsigned gm = group_mask<GW>();
     Con* con = con_of<WPL>(slot);
+    const bool cool = (long long)k - con->cb >= con->mpc, heat = (long long)k - con->mb >= con->stuck;
+    if (!cool && !heat) return;
     const RepHeader* H = reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[con->rid]);
     const XwJob* J = a.jobs + H->job;
-    if (J->tempering) return;
-    const bool cool = (long long)k - con->cb >= J->moves_per_cool, heat = (long long)k - con->mb >= J->stuck_threshold;
-    if (!cool && !heat) return;
     const double T0 = con->T, t_min = J->t_min;
     double T = T0;
     if (cool) {
