@@ -88,6 +88,42 @@ def test_large_orders_match_oracle(form, n, w, R, iters, kw):
     run_and_replay(n, w, R, iters, kw, 5000 + n * 7 + w).close()
 
 
+@pytest.mark.parametrize("objective", [0, 1, 2])
+@pytest.mark.parametrize("n,same,iters", [(264, 200, 60), (264, 122, 400), (271, 123, 400), (280, 122, 400)])
+def test_gram_entries_around_the_byte_limit(n, same, iters, objective):
+    """The hybrid form's G in bytes holds entries up to 123: a start above it
+    (halfwords from the load on) and starts at it, which the walk leaves."""
+    rng = np.random.default_rng(n + same)
+    w = n - 1 if n % 2 == 0 else n
+    W = rng.choice(np.array([-1, 1], np.int8), size=(n, n))
+    if w < n:
+        W[np.arange(n), np.arange(n) // 2 * 2] = 0
+    for i in range(0, n - 1, 2):   # pairs of rows with a product of `same` or one more
+        W[i + 1] = W[i]
+        W[i + 1, rng.permutation(np.flatnonzero(W[i]))[:(w - same) // 2]] *= -1
+    start = np.ascontiguousarray(W.T)   # column-major
+    p = X.Params(stop_on_solve=0, t_init=1e6, t_min=1e5, moves_per_launch=iters // 2, candidate_samples=2,
+                 sign_fraction=0.6, objective=objective)
+    batch = X.Batch([{"n": n, "w": w, "seed": 5, "replicas": 1}], p, starts=start)
+    rep = O.Replica(oracle_job(n, w, 5, p), 0, start, batch.replica(0, 0)[0].reheat_temperature, 0)
+
+    def largest():
+        G = rep.get()[4].copy()
+        np.fill_diagonal(G, 0)
+        return np.abs(G).max()
+
+    assert (largest() > 123) == (same > 123)
+    seen = 0
+    for _ in range(20):
+        rep.run(iters // 20, stop_on_solve=False)
+        seen = max(seen, largest())
+    assert seen > 127   # no longer a byte
+    batch.run(iters)
+    batch.synchronize()
+    compare(batch, 0, 0, rep)
+    batch.close()
+
+
 @pytest.mark.parametrize("n,w,planes", [(276, 275, True), (448, 447, True), (449, 448, False), (1024, 1000, False)])
 def test_large_class_reports_its_form(monkeypatch, n, w, planes):
     """The bit-plane forms up to order 448 (the hybrid by default), the

@@ -105,7 +105,7 @@ __device__ __forceinline__ bool step(const AnnealArgs& a, const Env& E, Walk& w,
         if (!multi) used = accept ? (int)(B & 3u) + 1 : run;
         w.two_l += q.R2 != q.R1 && (multi ? act : g < used) ? 1u : 0u;
         if (accept) {
-            mv = move_of(pack_move(q), wl0 + src, gm);
+            mv = move_of(pack_move<WPL>(q), wl0 + src, gm);
             acc = __shfl_sync(gm, q.acc, wl0 + src);
             prim = __shfl_sync(gm, q.prim, wl0 + src);
         }
@@ -309,7 +309,7 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
                 uint32_t A, B = 0;
                 if (count > 1) best_keys(GEN && E.obj_kind != 0, q, act, c, false, FULL, A, B);
                 const int src = (int)(B & 3u) * 8;
-                o.mv = move_of(pack_move(q), src, FULL);
+                o.mv = move_of(pack_move<WPL>(q), src, FULL);
                 o.dsc = __shfl_sync(FULL, q.acc, src);
                 o.prim = __shfl_sync(FULL, q.prim, src);
                 o.evals2 = (uint32_t)__popc(__ballot_sync(FULL, act && q.R2 != q.R1 && (lane & 7) == 0));
@@ -472,6 +472,9 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
 #ifndef XW_ANNEAL_MAXNREG_WIDE
 #define XW_ANNEAL_MAXNREG_WIDE 208
 #endif
+#ifndef XW_ANNEAL_MAXNREG_HYBRID
+#define XW_ANNEAL_MAXNREG_HYBRID 168
+#endif
 constexpr int anneal_maxnreg(int opl, bool general, int gw) {
     return opl == 8 ? XW_ANNEAL_MAXNREG_WIDE
            : gw == 16 ? XW_ANNEAL_MAXNREG_PAIR
@@ -503,6 +506,34 @@ __global__ void __maxnreg__(anneal_maxnreg(OPL, GEN, GW)) anneal_kernel(AnnealAr
             run_replica<OPL, GEN, GW, ONEZ>(a, rid, slot, lane, hi - lo);
         }
         if (chunked) chunk_end(a.chunk_done + rid, c, ok, lane, gm);
+    }
+}
+
+// The hybrid form of the large-order kernel (orders up to 448, W in shared
+// memory, G in HBM): the same loop.
+template <bool GEN>
+__global__ void __maxnreg__(XW_ANNEAL_MAXNREG_HYBRID) anneal_hybrid_kernel(AnnealArgs a) {
+    for (uint32_t e = threadIdx.x; e < 256; e += blockDim.x) {
+        reinterpret_cast<uint2*>(xw_smem)[e] = nibble_entry(e);
+        reinterpret_cast<uint32_t*>(xw_smem + 2048)[e] = nibble_entry_bytes(e);
+    }
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const uint32_t slot = kNibbleTable + (threadIdx.x >> 5) * a.slot_bytes;
+    const uint64_t total = (uint64_t)a.n_items * a.chunks;
+    for (;;) {
+        uint32_t item = 0;
+        if (lane == 0) item = atomicAdd(a.counter, 1u);
+        item = __shfl_sync(FULL, item, 0);
+        if (item >= total) break;
+        const uint32_t c = a.chunks == 1 ? 0u : item / a.n_items;
+        const uint32_t rid = a.items[item - c * a.n_items];
+        const uint64_t lo = a.iters * c / a.chunks, hi = a.iters * (c + 1) / a.chunks;
+        RepHeader* H = reinterpret_cast<RepHeader*>(a.arena + a.rec_off[rid]);
+        const bool chunked = a.chunks > 1;
+        const bool ok = !chunked || chunk_begin(a.chunk_done + rid, c, a.chunk_wait_ns, &H->err, lane, FULL);
+        if (ok) run_replica<16, GEN, 32, false>(a, rid, slot, lane, hi - lo);
+        if (chunked) chunk_end(a.chunk_done + rid, c, ok, lane, FULL);
     }
 }
 
@@ -596,6 +627,7 @@ __global__ void collect_kernel(const XwJob* jobs, int njobs, const uint8_t* aren
     uint64_t fs_it = UINT64_MAX, fs_ns = 0;
     int fs = 0x7fffffff;
     uint32_t err = 0;
+#pragma unroll 2
     for (int r = lane; r < J.replicas; r += 32) {
         const RepHeader* H = reinterpret_cast<const RepHeader*>(arena + rec_off[J.rep_begin + r]);
         const int64_t s = H->best_score, c = H->best_conflicts;
@@ -643,7 +675,19 @@ __global__ void collect_kernel(const XwJob* jobs, int njobs, const uint8_t* aren
         const uint8_t* src = arena + rec_off[J.rep_begin + br] + J.off_best;
         int8_t* dst = best_out + best_out_off[warp];
         const int nn = J.n * J.n;
-        for (int i = lane; i < nn; i += 32) dst[i] = (int8_t)src[i];
+        int i = 0;
+        if (((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15u) == 0) {
+            const uint4* s16 = reinterpret_cast<const uint4*>(src);
+            for (int k = lane; k < nn / 16; k += 128) {
+                uint4 v[4];
+                for (int e = 0; e < 4; ++e)
+                    if (k + 32 * e < nn / 16) v[e] = s16[k + 32 * e];
+                for (int e = 0; e < 4; ++e)
+                    if (k + 32 * e < nn / 16) reinterpret_cast<uint4*>(dst)[k + 32 * e] = v[e];
+            }
+            i = nn & ~15;
+        }
+        for (i += lane; i < nn; i += 32) dst[i] = (int8_t)src[i];
     }
 }
 
@@ -689,6 +733,17 @@ const void* anneal_kernel_fn(int opl, bool general, int rpw, bool one_zero) {
     if (opl == 2) return reinterpret_cast<const void*>(&anneal_kernel<2, false, 32>);
     if (opl == 4) return reinterpret_cast<const void*>(&anneal_kernel<4, false, 32>);
     return reinterpret_cast<const void*>(&anneal_kernel<8, false, 32>);
+}
+
+uint32_t anneal_hybrid_slot_bytes(int n, int m) { return hybrid_slot_bytes(n, m); }
+
+uint64_t anneal_hybrid_arena_bytes(int n) { return hybrid_arena(n).bytes; }
+
+uint32_t anneal_hybrid_table_bytes() { return kNibbleTable; }
+
+const void* anneal_hybrid_kernel_fn(bool general) {
+    return general ? reinterpret_cast<const void*>(&anneal_hybrid_kernel<true>)
+                   : reinterpret_cast<const void*>(&anneal_hybrid_kernel<false>);
 }
 
 cudaError_t launch_anneal(const AnnealArgs& args, int opl, bool general, int warps_per_block, int blocks,

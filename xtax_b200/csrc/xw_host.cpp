@@ -730,19 +730,49 @@ uint32_t choose_chunks(uint32_t replicas, uint32_t slots) {
     return best;
 }
 
+// Warps per CTA of a large-order launch of `items` replicas (0: as many as
+// an SM can hold) and the CTAs an SM holds.  Forms 0 and 1: four.  The
+// hybrid form has its tables once per CTA and its Gram matrices in L2, where
+// fewer replicas at a time leave each a larger share: an SM's replicas are
+// split evenly over the fewest rounds, one CTA on an SM (1000 iterations of
+// W(276,275), ten warps fit: 2368 replicas, 16 to an SM, 15.4 ms on eight
+// warps and 17.4 on ten; 1480 replicas 11.2 and 10.3; 592 replicas 5.8 on
+// four, 6.9 on eight, 7.6 on ten, which fill only 60 SMs).
+static int large_shape(bool general, int form, uint32_t slot_bytes, int device, int sms, uint64_t items, int& per_sm) {
+    const void* fn = anneal_large_kernel_fn(general, form);
+    raise_smem_limit(fn, device);
+    auto resident = [&](int k) {
+        int b = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, fn, 32 * k, anneal_large_smem_bytes(form, k, slot_bytes)) !=
+            cudaSuccess) {
+            cudaGetLastError();
+            b = 0;
+        }
+        return b;
+    };
+    if (form != 2) {
+        per_sm = resident(4);
+        return 4;
+    }
+    int most = 12;   // warps: registers hold no more
+    while (most > 1 && resident(most) < 1) --most;
+    per_sm = resident(most);
+    if (items == 0 || per_sm < 1) return most;
+    const uint64_t each = (items + (uint64_t)sms - 1) / (uint64_t)sms;
+    const uint64_t rounds = (each + (uint64_t)most - 1) / (uint64_t)most;
+    per_sm = 1;
+    return (int)((each + rounds - 1) / rounds);
+}
+
 void Batch::configure_shape() {
     if (graph_exec) {
         cudaGraphExecDestroy(graph_exec);
         graph_exec = nullptr;
     }
     if (n_large) {
-        // four warps per CTA, as many CTAs as the SMs hold
-        const void* lfn = anneal_large_kernel_fn(general_large, large_form);
-        const size_t lsmem = (size_t)large_wpb * large_slot_bytes;
-        raise_smem_limit(lfn, params.device);
         int per_sm = 0;
-        check(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lfn, 32 * large_wpb, lsmem),
-              "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
+        large_wpb = large_shape(general_large, large_form, large_slot_bytes, params.device, props.multiProcessorCount,
+                                n_large, per_sm);
         if (per_sm < 1) throw std::length_error("CUDA large-order anneal kernel has zero occupancy");
         const int want = (int)((n_large + large_wpb - 1) / large_wpb);
         large_blocks = std::max(1, std::min(want, per_sm * props.multiProcessorCount));
@@ -1939,12 +1969,14 @@ int32_t xw_run(int32_t n, int32_t w, const xw_params* pin, const int8_t* start, 
         const uint32_t slot = large ? anneal_large_slot_bytes(n, m, form) : anneal_slot_bytes(n, m, anneal_opl(n, w));
         if (replicas == 0) {
             // one resident wave: warp slots per SM times SMs
-            const int wpb = large ? 4 : p.warps_per_block > 0 ? p.warps_per_block : 4;
-            int per_sm = 0;
-            const void* fn = large ? anneal_large_kernel_fn(needs_general_kernel(p), form)
-                                   : anneal_kernel_fn(anneal_opl(n, w), needs_general_kernel(p));
-            raise_smem_limit(fn, p.device);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * wpb, (size_t)wpb * slot);
+            int wpb = p.warps_per_block > 0 ? p.warps_per_block : 4, per_sm = 0;
+            if (large) {
+                wpb = large_shape(needs_general_kernel(p), form, slot, p.device, out->device.multiprocessors, 0, per_sm);
+            } else {
+                const void* fn = anneal_kernel_fn(anneal_opl(n, w), needs_general_kernel(p));
+                raise_smem_limit(fn, p.device);
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 32 * wpb, (size_t)wpb * slot);
+            }
             replicas = std::max(1, per_sm * wpb * out->device.multiprocessors);
         }
         if (p.tempering && replicas > XW_MAX_RUNGS) replicas = XW_MAX_RUNGS;

@@ -77,8 +77,16 @@ bool anneal_large_planes_fit(int n, int m);
 uint32_t anneal_large_slot_bytes(int n, int m, int form);
 uint64_t anneal_large_arena_bytes(int n, int form);
 const void* anneal_large_kernel_fn(bool general, int form);
+// dynamic shared memory of a CTA of `warps_per_block` warps
+size_t anneal_large_smem_bytes(int form, int warps_per_block, uint32_t slot_bytes);
 cudaError_t launch_anneal_large(const AnnealArgs& args, bool general, int form, int warps_per_block, int blocks,
                                 cudaStream_t stream);
+// Its form 2 runs the packed iteration of the smaller orders (xw_anneal.cu):
+// shared memory per warp, the CTA's table, arena bytes, the kernel.
+uint32_t anneal_hybrid_slot_bytes(int n, int m);
+uint32_t anneal_hybrid_table_bytes();
+uint64_t anneal_hybrid_arena_bytes(int n);
+const void* anneal_hybrid_kernel_fn(bool general);
 cudaError_t launch_exchange(XwJob* jobs, int njobs, uint8_t* arena, const uint64_t* rec_off,
                             const double* ladder, int stop_on_solve, cudaStream_t stream);
 

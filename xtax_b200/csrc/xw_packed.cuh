@@ -77,6 +77,7 @@ __device__ __forceinline__ uint64_t lds64(uint32_t a) { return *reinterpret_cast
 // mirrored column of a commit, one byte in each row, spreads over the banks.
 __host__ __device__ constexpr uint32_t packed_stride(int n, int wpl) {
     if (wpl == 8) return ((uint32_t)n + 7u) & ~7u;
+    if (wpl == 16) return 4u * (((uint32_t)n + 15u) >> 4);   // four nibble pairs to 16 rows
     const uint32_t q = 4u * (uint32_t)wpl;
     return ((((uint32_t)n + q - 1u) / q) | 1u) * q;
 }
@@ -129,6 +130,7 @@ struct Con {
     // identical copy in their own shared memory and write nothing)
     int32_t owner;
     uint32_t rid;
+    int32_t halves;      // hybrid form: G is in halfwords
 };
 
 // The slot: fixed regions first, so that their offsets are constants.
@@ -141,7 +143,7 @@ struct Slot {
     static constexpr uint32_t con = jrn + 8u * kJournal;
     static constexpr uint32_t res = con + 240u;               // packed residuals, 4 bytes a row
     static constexpr uint32_t mask = res + 128u * WPL;        // support masks, 4*WPL bytes a row
-    static constexpr uint32_t w = mask + (WPL == 8 ? 0u : 128u * WPL * WPL);
+    static constexpr uint32_t w = mask + (WPL >= 8 ? 0u : 128u * WPL * WPL);
 };
 
 static_assert(sizeof(Con) <= 240, "replica constants fit their region");
@@ -155,6 +157,48 @@ __host__ __device__ constexpr uint32_t packed_slot_bytes(int n, int m, int wpl) 
     return fixed + mat + gram + xw_pad16((uint32_t)(n * m) + 1u);
 }
 
+// The hybrid form of the large-order kernel (WPL 16, orders up to 448): W in
+// the slot as nibble pairs, a byte to four rows of a column (low nibble
+// support, high nibble sign), G in the replica's arena in HBM, rows of
+// 16-byte chunks; the minority lists (16 bits) in the slot when they take at
+// most kHybridMino bytes, else in the record.  G is kept as biased bytes
+// while its entries stay within kByteMax (a move changes one by at most 4;
+// entries of random rows have a standard deviation of sqrt(w)), and goes
+// over to biased halfwords for good when a row that is read holds a larger
+// one: half the bytes keep the Gram matrices of twice the replicas in L2.
+// Tables at the start of the CTA's shared memory turn a nibble pair into
+// four byte entries of W (one word) or four halfwords (two).
+constexpr int kHybridMaxOrder = 448;
+constexpr uint32_t kHybridMino = 8192;
+constexpr uint32_t kNibbleTable = 2048 + 1024;
+constexpr int kByteMax = 123;
+
+__host__ __device__ constexpr uint32_t hybrid_slot_bytes(int n, int m) {
+    const uint32_t mb = (uint32_t)n * (uint32_t)m * 2u;
+    return 512u + 4u * kThrTable + 8u * (uint32_t)kJournal + 240u + xw_pad16(4u * (uint32_t)n) +
+           xw_pad16((uint32_t)n * packed_stride(n, 16)) + (mb <= kHybridMino ? xw_pad16(mb + 2u) : 0u);
+}
+
+__host__ __device__ constexpr uint32_t hybrid_gram_stride(int n) { return (((uint32_t)n + 7u) >> 3) * 16u; }
+__host__ __device__ constexpr uint32_t hybrid_byte_stride(int n) { return ((uint32_t)n + 15u) & ~15u; }
+
+__host__ __device__ constexpr uint32_t hybrid_row_stride(int n) { return (((uint32_t)n + 63u) >> 6) * 32u; }
+
+// The arena of a replica in that form: packed residuals, the rows of W as
+// signed nibbles (used while G is built; then the first word says whether G
+// is in halfwords), G (room for halfwords).
+struct HybridArena {
+    uint64_t off_rows, off_g, bytes;
+};
+
+__host__ __device__ constexpr HybridArena hybrid_arena(int n) {
+    HybridArena A{};
+    A.off_rows = (4u * (uint64_t)n + 15u) & ~uint64_t(15);
+    A.off_g = A.off_rows + (uint64_t)n * hybrid_row_stride(n);
+    A.bytes = A.off_g + (uint64_t)n * hybrid_gram_stride(n);
+    return A;
+}
+
 // Loop-invariant context of a lane of a replica's group.
 struct Env {
     uint32_t slot;       // the replica's slot in xw_smem
@@ -163,10 +207,29 @@ struct Env {
     uint32_t g, mino;    // byte offsets of G and the minority lists
     uint32_t st;         // bytes from a column of W (and, up to order 128, a row of G) to the next
     uint32_t gst;        // the same of G above order 128
+    uint8_t* gp;         // hybrid form: G in the arena, the minority lists
+    uint16_t* mp;
     int n, m, sparse, full;   // full: w = n
     int ts, bpc, move_set, obj_kind;
     uint32_t dq[2];      // draw blocks this lane computes: candidate (or iteration) << 16 | 1 + block
 };
+
+// Entry (r, c) of W plus one.
+template <int WPL>
+__device__ __forceinline__ uint32_t w_at(uint32_t wbase, uint32_t st, int r, int c) {
+    if constexpr (WPL == 16) {
+        const uint32_t b = lds8(wbase + (uint32_t)c * st + ((uint32_t)r >> 2)) >> (r & 3);
+        return 1u + (b & 1u) - 2u * ((b >> 4) & 1u);
+    } else {
+        return lds8(wbase + (uint32_t)c * st + (uint32_t)r);
+    }
+}
+
+template <int WPL>
+__device__ __forceinline__ int mino_at(const Env& E, int i) {
+    if constexpr (WPL == 16) return E.mp[i];
+    else return (int)lds8(E.mino + (uint32_t)i);
+}
 
 template <int WPL>
 __device__ __forceinline__ Con* con_of(uint32_t slot) {
@@ -185,17 +248,23 @@ __device__ __forceinline__ int first_from(uint64_t m, int start) {
     return __ffsll((long long)(hi ? hi : m)) - 1;
 }
 
+// W's offset: a slot of the hybrid form has its residuals just before.
+template <int WPL>
+__device__ __forceinline__ uint32_t wbase_of(uint32_t slot, int n) {
+    return slot + (WPL == 16 ? Slot<WPL>::res + xw_pad16(4u * (uint32_t)n) : Slot<WPL>::w);
+}
+
 // First set bit at or after `start`, cyclically, of row `row`'s support
 // mask (COMPL: of its complement below n).
 template <int WPL, bool COMPL = false>
 __device__ __forceinline__ int mask_first(uint32_t slot, int row, int start, int n) {
     const uint32_t a = slot + Slot<WPL>::mask + (uint32_t)row * (4u * WPL);
-    if constexpr (WPL == 8) {
+    if constexpr (WPL >= 8) {
         // no masks: the columns in turn (at most n / w of them, or n / (n - w)
         // zeros, on average, and only the fuller kind is searched this way)
-        const uint32_t w = slot + Slot<WPL>::w + (uint32_t)row, st = packed_stride(n, 8);
+        const uint32_t w = wbase_of<WPL>(slot, n), st = packed_stride(n, WPL);
         int c = start;
-        while ((lds8(w + (uint32_t)c * st) == 1u) != COMPL) c = c + 1 == n ? 0 : c + 1;
+        while ((w_at<WPL>(w, st, row, c) == 1u) != COMPL) c = c + 1 == n ? 0 : c + 1;
         return c;
     } else if constexpr (WPL == 1) {
         uint32_t m = lds32(a);
@@ -241,13 +310,27 @@ __device__ __forceinline__ uint32_t slow_word(uint32_t slot, uint64_t it, uint32
 // b), propose_sign_flip (xweigh_cuda.cu:302-325): a minority pick for a
 // sparse row, else the first nonzero at or after a random column.
 template <int WPL, bool ONEZ>
-__device__ __forceinline__ int flip_col_exact(uint32_t slot, uint32_t mino, int n, int m, int sparse, uint32_t wd,
-                                              uint32_t dslot, uint64_t it, uint32_t stream, uint32_t k0, uint32_t k1,
-                                              int j, int row) {
+__device__ __forceinline__ int flip_col_exact(const Env& E, uint32_t wd, uint32_t dslot, uint64_t it, uint32_t stream,
+                                              uint32_t k0, uint32_t k1, int j, int row) {
+    const int n = E.n;
     if constexpr (ONEZ)
-        return after_zero((int)draw_index(wd, (uint32_t)n, dslot, it, stream, k0, k1, j), (int)lds8(mino + (uint32_t)row), n);
-    if (sparse && m > 0) return (int)lds8(mino + (uint32_t)(row * m) + draw_index(wd, (uint32_t)m, dslot, it, stream, k0, k1, j));
-    return mask_first<WPL>(slot, row, (int)draw_index(wd, (uint32_t)n, dslot, it, stream, k0, k1, j), n);
+        return after_zero((int)draw_index(wd, (uint32_t)n, dslot, it, stream, k0, k1, j), mino_at<WPL>(E, row), n);
+    if (E.sparse && E.m > 0)
+        return mino_at<WPL>(E, row * E.m + (int)draw_index(wd, (uint32_t)E.m, dslot, it, stream, k0, k1, j));
+    return mask_first<WPL>(E.slot, row, (int)draw_index(wd, (uint32_t)n, dslot, it, stream, k0, k1, j), n);
+}
+
+// The row of a group's largest tournament key; `mine`: the row behind the
+// lane's own (a key has room for its low eight bits, distinct by sample).
+template <int WPL, int LPC>
+__device__ __forceinline__ int best_row(uint32_t key, uint32_t mine, unsigned gm) {
+    uint32_t top = key;
+#pragma unroll
+    for (int d = 1; d < LPC; d <<= 1) top = max(top, __shfl_xor_sync(gm, top, d));
+    if constexpr (WPL < 16) return (int)(top & 255u);
+    const int wl = (int)(threadIdx.x & 31u), base = wl & ~(LPC - 1);
+    const uint32_t at = (__ballot_sync(gm, key == top) >> base) & ((1u << LPC) - 1u);
+    return (int)__shfl_sync(gm, mine, base + __ffs((int)at) - 1);
 }
 
 // Hot-row tournament of candidate `c` (hot_row, xweigh_cuda.cu:291-300),
@@ -258,18 +341,20 @@ __device__ __forceinline__ int tournament(uint32_t slot, uint32_t cw, int n, int
                                           unsigned gm) {
     constexpr int LPC = GW / 4;
     const Con* con = con_of<WPL>(slot);
-    uint32_t key = 0;
+    uint32_t key = 0, mine = 0;
 #pragma unroll 1
     for (int s = l; s < ts; s += LPC) {
         const uint32_t ds = cand_slot(c, 4 + (s >> 2));
         const uint32_t wd = s < 8 ? lds32(cw + 64u + 4u * (uint32_t)s)
                                   : slow_word(ds, it, con->stream, con->k0, con->k1, s & 3);
         const uint32_t r = draw_index(wd, (uint32_t)n, ds, it, con->stream, con->k0, con->k1, s & 3);
-        key = max(key, (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - s) << 8) | r);
+        const uint32_t k = (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - s) << 8) | (r & 255u);
+        if (k > key) {
+            key = k;
+            mine = r;
+        }
     }
-#pragma unroll
-    for (int d = 1; d < LPC; d <<= 1) key = max(key, __shfl_xor_sync(gm, key, d));
-    return (int)(key & 255u);
+    return best_row<WPL, LPC>(key, mine, gm);
 }
 
 // The whole proposal of candidate `c` with exact index draws and every
@@ -282,13 +367,13 @@ __device__ __forceinline__ int tournament(uint32_t slot, uint32_t cw, int n, int
 // blocks.  `need`: this lane's group wants a proposal (the other lanes take
 // part in the collectives only); `from`: the first attempt to try (1 when
 // attempt 0 is known to fail).  Returns
-// {R1 | R2<<8 | C1<<16 | C2<<24, kind | p1<<8 | p2<<16 | s1<<24 | s2<<25}.
+// {R1 | R2<<16, C1 | C2<<16, p1 | p2<<16, kind | s1<<2 | s2<<3}.
 template <int WPL, int GW, bool ONEZ>
-__device__ __forceinline__ uint2 propose_exact(const Env& E, bool need, int from, int hot, int c, uint64_t it, int l) {
+__device__ __forceinline__ uint4 propose_exact(const Env& E, bool need, int from, int hot, int c, uint64_t it, int l) {
     constexpr int LPC = GW / 4;
     const unsigned gm = group_mask<GW>();
     const int wl = threadIdx.x & 31, base = wl - l;
-    const uint32_t slot = E.slot, cw = E.cw, mino = E.mino, st = E.st;
+    const uint32_t slot = E.slot, cw = E.cw, st = E.st, wbase = wbase_of<WPL>(E.slot, E.n);
     const int n = E.n, m = ONEZ ? 1 : E.m, sparse = ONEZ ? 0 : E.sparse;
     const Con* con = con_of<WPL>(slot);
     const uint32_t k0 = con->k0, k1 = con->k1, stream = con->stream;
@@ -296,7 +381,7 @@ __device__ __forceinline__ uint2 propose_exact(const Env& E, bool need, int from
         return (int)draw_index(wd, count, cand_slot(c, b), it, stream, k0, k1, j);
     };
     auto fcol = [&](uint32_t wd, int b, int j, int row) -> int {
-        return flip_col_exact<WPL, ONEZ>(slot, mino, n, m, sparse, wd, cand_slot(c, b), it, stream, k0, k1, j, row);
+        return flip_col_exact<WPL, ONEZ>(E, wd, cand_slot(c, b), it, stream, k0, k1, j, row);
     };
     int row = 0, r2 = 0, c1 = 0, c2 = 0, p1 = 0, p2 = 0, kind = -1;
     bool s1 = false, s2 = false, dbl = false, flip = false;
@@ -353,7 +438,7 @@ __device__ __forceinline__ uint2 propose_exact(const Env& E, bool need, int from
 #pragma unroll 1
         for (int a0 = __any_sync(gm, pend && dbl) ? 0 : from; a0 < 24; a0 += AT) {
             const int a = a0 + (l & (AT - 1)), b = a == 0 ? 1 : 36 + 2 * (a - 1), o = a == 0 ? 1 : 0;
-            int rr = 0, x1 = 0;
+            int rr = 0, x1 = 0, pp = 0;
             uint4 d = make_uint4(0, 0, 0, 0);
             bool ok = false;
             if (pend && a < 24) {
@@ -366,27 +451,28 @@ __device__ __forceinline__ uint2 propose_exact(const Env& E, bool need, int from
                     rr = ix(d.x, (uint32_t)(n - 1), b, o);
                     if (rr >= row) ++rr;
                     const int q = ix(d.y, (uint32_t)m, b, o + 1), qq = ix(d.z, (uint32_t)m, b, o + 2);
-                    const int q1 = (int)lds8(mino + (uint32_t)(row * m + q)), q2 = (int)lds8(mino + (uint32_t)(rr * m + qq));
+                    const int q1 = mino_at<WPL>(E, row * m + q), q2 = mino_at<WPL>(E, rr * m + qq);
                     // entries (row, C2) and (rr, C1) are zeros, (row, C1) and
                     // (rr, C2) nonzeros: one pair by the choice of q1, q2
-                    const uint32_t e1 = lds8(slot + Slot<WPL>::w + (uint32_t)q2 * st + (uint32_t)row);
-                    const uint32_t e2 = lds8(slot + Slot<WPL>::w + (uint32_t)q1 * st + (uint32_t)rr);
+                    const uint32_t e1 = w_at<WPL>(wbase, st, row, q2), e2 = w_at<WPL>(wbase, st, rr, q1);
                     ok = sparse ? e1 == 1u && e2 == 1u : e1 != 1u && e2 != 1u;
-                    x1 = (sparse ? q1 : q2) | ((sparse ? q2 : q1) << 8) | (q << 16) | (qq << 24);
+                    x1 = (sparse ? q1 : q2) | ((sparse ? q2 : q1) << 16);
+                    pp = q | (qq << 16);
                 }
             }
             const unsigned hit = (__ballot_sync(gm, ok) >> base) & ((1u << LPC) - 1u);
             const int src = hit ? base + __ffs((int)hit) - 1 : wl;
             rr = __shfl_sync(gm, rr, src);
             x1 = __shfl_sync(gm, x1, src);
+            pp = __shfl_sync(gm, pp, src);
             const uint32_t sw1 = __shfl_sync(gm, d.w, src), sw2 = __shfl_sync(gm, d.x, hit ? src + AT : wl);
             if (pend && hit) {
                 kind = 1;
                 r2 = rr;
-                c1 = x1 & 255;
-                c2 = (x1 >> 8) & 255;
-                p1 = (x1 >> 16) & 255;
-                p2 = (int)((uint32_t)x1 >> 24);
+                c1 = x1 & 0xffff;
+                c2 = x1 >> 16;
+                p1 = pp & 0xffff;
+                p2 = pp >> 16;
                 s1 = (uint64_t)sw1 < con->thr_swsign;
                 s2 = (uint64_t)sw2 < con->thr_swsign;
                 pend = false;
@@ -399,16 +485,17 @@ __device__ __forceinline__ uint2 propose_exact(const Env& E, bool need, int from
         r2 = row;
         c1 = c2 = fcol(lds32(cw + 40u), 2, 2, row);
     }
-    return make_uint2((uint32_t)row | ((uint32_t)r2 << 8) | ((uint32_t)c1 << 16) | ((uint32_t)c2 << 24),
-                      (uint32_t)(kind & 3) | ((uint32_t)p1 << 8) | ((uint32_t)p2 << 16) | (s1 ? 1u << 24 : 0u) |
-                          (s2 ? 1u << 25 : 0u));
+    return make_uint4((uint32_t)row | ((uint32_t)r2 << 16), (uint32_t)c1 | ((uint32_t)c2 << 16),
+                      (uint32_t)p1 | ((uint32_t)p2 << 16),
+                      (uint32_t)(kind & 3) | (s1 ? 4u : 0u) | (s2 ? 8u : 0u));
 }
 
 // A move in three words:
 //   rc  R1 | R2<<8 | C1<<16 | C2<<24 (R2 = R1: one row)
 //   cf  the coefficients a1, b1 (row R1, columns C1, C2), a2, b2 (row R2)
 //   ax  change of G[R1][R2] | p1<<8 | p2<<16 | support change<<24 (bit 0 R1,
-//       bit 1 R2), p1, p2 the changed entries of the minority lists
+//       bit 1 R2), p1, p2 the changed entries of the minority lists; bits
+//       26..29 the ninth bits of R1, R2, C1, C2
 struct Move {
     uint32_t rc, cf, ax;
 };
@@ -421,13 +508,21 @@ struct Cand {
     int acc, prim;
 };
 
+template <int WPL>
 __device__ __forceinline__ Move pack_move(const Cand& q) {
     Move mv;
-    mv.rc = (uint32_t)q.R1 | ((uint32_t)q.R2 << 8) | ((uint32_t)q.C1 << 16) | ((uint32_t)q.C2 << 24);
     mv.cf = (uint32_t)(q.a1 & 255) | ((uint32_t)(q.b1 & 255) << 8) | ((uint32_t)(q.a2 & 255) << 16) |
             ((uint32_t)q.b2 << 24);
     mv.ax = (uint32_t)(q.pk & 255) | ((uint32_t)q.p1 << 8) | ((uint32_t)q.p2 << 16) |
             (q.kind == 1 ? 3u << 24 : q.kind == 3 ? 1u << 24 : 0u);
+    if constexpr (WPL == 16) {
+        mv.rc = (uint32_t)(q.R1 & 255) | ((uint32_t)(q.R2 & 255) << 8) | ((uint32_t)(q.C1 & 255) << 16) |
+                ((uint32_t)q.C2 << 24);
+        mv.ax |= ((uint32_t)(q.R1 >> 8) << 26) | ((uint32_t)(q.R2 >> 8) << 27) | ((uint32_t)(q.C1 >> 8) << 28) |
+                 ((uint32_t)(q.C2 >> 8) << 29);
+    } else {
+        mv.rc = (uint32_t)q.R1 | ((uint32_t)q.R2 << 8) | ((uint32_t)q.C1 << 16) | ((uint32_t)q.C2 << 24);
+    }
     return mv;
 }
 
@@ -491,30 +586,206 @@ __device__ __forceinline__ uint32_t abs_halves(uint32_t v) {
     return (t ^ m) + (m & 0x00010001u);
 }
 
+// The sums of eight entries of two changed rows: score + 4096 x conflicts,
+// and the change of the squared or parity objective.
 template <bool GEN>
-__device__ __forceinline__ void wide_chunk(const Env& E, uint32_t w1, uint32_t w2, int R1, int R2, int j,
-                                           const Cand& q, int& acc, int& pr) {
-    const uint4 o1 = lds128(wide_at(E.g, E.gst, R1, j)), o2 = lds128(wide_at(E.g, E.gst, R2, j));
-    uint32_t g1[4] = {o1.x, o1.y, o1.z, o1.w}, g2[4] = {o2.x, o2.y, o2.z, o2.w};
-    wide_rows(w1, w2, R1, R2, j, q.a1, q.b1, q.a2, q.b2, q.pk, g1, g2);
-    const uint32_t old1[4] = {o1.x, o1.y, o1.z, o1.w}, old2[4] = {o2.x, o2.y, o2.z, o2.w};
+__device__ __forceinline__ void wide_sums(int obj_kind, const uint32_t (&g1)[4], const uint32_t (&g2)[4],
+                                          const uint32_t (&old1)[4], const uint32_t (&old2)[4], int& acc, int& pr) {
 #pragma unroll
     for (int h = 0; h < 4; ++h) {
-        const uint32_t v = abs_halves(g1[h]) + abs_halves(g2[h]);   // at most 512 a half
-        const uint32_t z = (((abs_halves(g1[h]) + 0x7fff7fffu) & 0x80008000u) >> 15) +
-                           (((abs_halves(g2[h]) + 0x7fff7fffu) & 0x80008000u) >> 15);
-        acc = __dp2a_lo((int)v, 0x0101, acc);
-        acc = __dp2a_lo((int)(z << 12), 0x0101, acc);               // 4096 a conflict
+        const uint32_t v1 = abs_halves(g1[h]), v2 = abs_halves(g2[h]);
+        const uint32_t z = (((v1 + 0x7fff7fffu) & 0x80008000u) >> 15) + (((v2 + 0x7fff7fffu) & 0x80008000u) >> 15);
+        acc = __dp2a_lo((int)(v1 + v2), 0x0101, acc);   // at most 896 a half
+        acc = __dp2a_lo((int)(z << 12), 0x0101, acc);   // 4096 a conflict
         if (GEN) {
-            if (E.obj_kind == 1) {
+            if (obj_kind == 1) {
                 auto sq = [](uint32_t a) -> int {
                     const int lo = (int)(a & 0xffffu) - 32768, hi = (int)(a >> 16) - 32768;
                     return lo * lo + hi * hi;
                 };
                 pr += sq(g1[h]) + sq(g2[h]) - sq(old1[h]) - sq(old2[h]);
-            } else if (E.obj_kind == 2) {
+            } else if (obj_kind == 2) {
                 pr += __popc((g1[h] & 0x00010001u) | ((g2[h] & 0x00010001u) << 1)) -
                       __popc((old1[h] & 0x00010001u) | ((old2[h] & 0x00010001u) << 1));
+            }
+        }
+    }
+}
+
+template <bool GEN>
+__device__ __forceinline__ void wide_chunk(const Env& E, uint32_t w1, uint32_t w2, int R1, int R2, int j,
+                                           const Cand& q, int& acc, int& pr) {
+    const uint4 o1 = lds128(wide_at(E.g, E.gst, R1, j)), o2 = lds128(wide_at(E.g, E.gst, R2, j));
+    const uint32_t old1[4] = {o1.x, o1.y, o1.z, o1.w}, old2[4] = {o2.x, o2.y, o2.z, o2.w};
+    uint32_t g1[4] = {o1.x, o1.y, o1.z, o1.w}, g2[4] = {o2.x, o2.y, o2.z, o2.w};
+    wide_rows(w1, w2, R1, R2, j, q.a1, q.b1, q.a2, q.b2, q.pk, g1, g2);
+    wide_sums<GEN>(E.obj_kind, g1, g2, old1, old2, acc, pr);
+}
+
+// Hybrid form: new halfwords of chunk j of the changed rows, as wide_rows;
+// entries R1 and R2 are left out of both columns.  `sym`: the change of
+// G[R1][R2] goes into row R2's entry too (a commit writes both).
+__device__ __forceinline__ void hybrid_chunk(uint32_t w1, uint32_t w2, int R1, int R2, int j, int a1, int b1, int a2,
+                                             int b2, int pk, bool sym, uint32_t (&g1)[4], uint32_t (&g2)[4]) {
+    auto bits = [&](int R) -> uint32_t { return (R >> 3) == j ? 0x11u << ((R & 3) + 2 * (R & 4)) : 0u; };
+    const uint32_t keep = ~(bits(R1) | bits(R2));
+    const uint32_t x = *reinterpret_cast<const uint16_t*>(xw_smem + w1 + 2u * (uint32_t)j) & keep;
+    const uint32_t y = *reinterpret_cast<const uint16_t*>(xw_smem + w2 + 2u * (uint32_t)j) & keep;
+    const uint2 xa = *reinterpret_cast<const uint2*>(xw_smem + 8u * (x & 255u)),
+                xb = *reinterpret_cast<const uint2*>(xw_smem + 8u * (x >> 8));
+    const uint2 ya = *reinterpret_cast<const uint2*>(xw_smem + 8u * (y & 255u)),
+                yb = *reinterpret_cast<const uint2*>(xw_smem + 8u * (y >> 8));
+    const uint32_t X[4] = {xa.x, xa.y, xb.x, xb.y}, Y[4] = {ya.x, ya.y, yb.x, yb.y};
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const uint32_t o = 128u * (uint32_t)j + 32u * h;
+        g1[h] += (uint32_t)a1 * X[h] + (uint32_t)b1 * Y[h] + shl_clamp((uint32_t)pk, 16u * (uint32_t)R2 - o);
+        g2[h] += (uint32_t)a2 * X[h] + (uint32_t)b2 * Y[h] + (sym ? shl_clamp((uint32_t)pk, 16u * (uint32_t)R1 - o) : 0u);
+    }
+}
+
+// Entry `e` of the tables of nibble pairs: four entries of W (low nibble
+// support, high nibble sign) as the sum of w_i 256^i, or of w_i 65536^i of
+// each two.
+__device__ __forceinline__ uint32_t nibble_entry_bytes(uint32_t e) {
+    uint32_t x = 0;
+    for (int i = 3; i >= 0; --i) x = x * 256u + ((e >> i) & 1u) - 2u * ((e >> (4 + i)) & 1u);
+    return x;
+}
+
+__device__ __forceinline__ uint2 nibble_entry(uint32_t e) {
+    auto w = [&](int i) -> int { return (int)((e >> i) & 1u) - 2 * (int)((e >> (4 + i)) & 1u); };
+    return make_uint2((uint32_t)w(0) + ((uint32_t)w(1) << 16), (uint32_t)w(2) + ((uint32_t)w(3) << 16));
+}
+
+// The same from a G in bytes: new bytes of the 16 entries of chunk j.
+__device__ __forceinline__ void hybrid_chunk_bytes(uint32_t w1, uint32_t w2, int R1, int R2, int j, int a1, int b1,
+                                                   int a2, int b2, int pk, bool sym, uint32_t (&g1)[4],
+                                                   uint32_t (&g2)[4]) {
+    auto bits = [&](int R) -> uint32_t { return (R >> 4) == j ? 0x11u << ((R & 3) + 2 * (R & 12)) : 0u; };
+    const uint32_t keep = ~(bits(R1) | bits(R2));
+    const uint32_t x = lds32(w1 + 4u * (uint32_t)j) & keep, y = lds32(w2 + 4u * (uint32_t)j) & keep;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+        const uint32_t X = lds32(2048u + 4u * ((x >> (8 * h)) & 255u)), Y = lds32(2048u + 4u * ((y >> (8 * h)) & 255u));
+        const uint32_t o = 128u * (uint32_t)j + 32u * h;
+        g1[h] += (uint32_t)a1 * X + (uint32_t)b1 * Y + shl_clamp((uint32_t)pk, 8u * (uint32_t)R2 - o);
+        g2[h] += (uint32_t)a2 * X + (uint32_t)b2 * Y + (sym ? shl_clamp((uint32_t)pk, 8u * (uint32_t)R1 - o) : 0u);
+    }
+}
+
+// The lane's 16-byte chunks l, l + 8, ... of a candidate from a G in bytes.
+// `over`: a row read holds an entry above kByteMax (the sums are then void).
+template <bool GEN>
+__device__ __forceinline__ void hybrid_rows_bytes(const Env& E, uint32_t w1, uint32_t w2, int R1, int R2, int l,
+                                                  const Cand& q, int& acc, int& pr, bool& over) {
+    constexpr int kFlight = 4;   // chunks of both rows in flight (all of them: n <= 512)
+    const int nch = (E.n + 15) >> 4;
+    const uint32_t bst = hybrid_byte_stride(E.n);
+    const uint8_t* p1 = E.gp + (size_t)R1 * bst;
+    const uint8_t* p2 = E.gp + (size_t)R2 * bst;
+    const bool two = R2 != R1;
+    uint4 o1[kFlight], o2[kFlight];
+#pragma unroll
+    for (int k = 0; k < kFlight; ++k) {
+        const int j = l + 8 * k;
+        o1[k] = make_uint4(0x80808080u, 0x80808080u, 0x80808080u, 0x80808080u);
+        if (j < nch) o1[k] = __ldcg(reinterpret_cast<const uint4*>(p1) + j);
+        o2[k] = o1[k];
+        if (two && j < nch) o2[k] = __ldcg(reinterpret_cast<const uint4*>(p2) + j);
+    }
+    uint32_t big = 0, ac = (uint32_t)acc;
+#pragma unroll
+    for (int k = 0; k < kFlight; ++k) {
+        const int j = l + 8 * k;
+        if (j < nch) {
+            const uint32_t old1[4] = {o1[k].x, o1[k].y, o1[k].z, o1[k].w};
+            const uint32_t old2[4] = {o2[k].x, o2[k].y, o2[k].z, o2[k].w};
+            uint32_t g1[4] = {o1[k].x, o1[k].y, o1[k].z, o1[k].w}, g2[4] = {o2[k].x, o2[k].y, o2[k].z, o2[k].w};
+            hybrid_chunk_bytes(w1, w2, R1, R2, j, q.a1, q.b1, q.a2, q.b2, q.pk, false, g1, g2);
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                const uint32_t m1 = __vabsdiffu4(old1[h], 0x80808080u), m2 = __vabsdiffu4(old2[h], 0x80808080u);
+                big |= (m1 + (uint32_t)(127 - kByteMax) * 0x01010101u) | (m2 + (uint32_t)(127 - kByteMax) * 0x01010101u);
+                const uint32_t v1 = __vabsdiffu4(g1[h], 0x80808080u), v2 = __vabsdiffu4(g2[h], 0x80808080u);
+                const uint32_t z1 = (v1 + 0x7f7f7f7fu) & 0x80808080u, z2 = (v2 + 0x7f7f7f7fu) & 0x80808080u;
+                ac = __dp4a(v1, 0x01010101u, ac);
+                ac = __dp4a(v2, 0x01010101u, ac);
+                ac = __dp4a(z1, 0x20202020u, ac);   // 128 * 32: 4096 a conflict
+                ac = __dp4a(z2, 0x20202020u, ac);
+                if (GEN) {
+                    if (E.obj_kind == 1) {
+                        const int d1 = (int)(g1[h] ^ 0x80808080u), d2 = (int)(g2[h] ^ 0x80808080u);
+                        const int e1 = (int)(old1[h] ^ 0x80808080u), e2 = (int)(old2[h] ^ 0x80808080u);
+                        pr += __dp4a(d1, d1, 0) + __dp4a(d2, d2, 0) - __dp4a(e1, e1, 0) - __dp4a(e2, e2, 0);
+                    } else if (E.obj_kind == 2) {
+                        pr += __popc((g1[h] & 0x01010101u) | ((g2[h] & 0x01010101u) << 1)) -
+                              __popc((old1[h] & 0x01010101u) | ((old2[h] & 0x01010101u) << 1));
+                    }
+                }
+            }
+        }
+    }
+    acc = (int)ac;
+    over = (big & 0x80808080u) != 0u;
+}
+
+// G from bytes to halfwords, in place: rows from the last, each read whole
+// before its (longer, later) place is written.
+__device__ __noinline__ void widen_gram(uint8_t* gp, int n, int lane) {
+    const uint32_t bst = hybrid_byte_stride(n), hst = hybrid_gram_stride(n);
+#pragma unroll 1
+    for (int r = n - 1; r >= 0; --r) {
+        uint32_t w[4];   // words lane, lane + 32, ... of the row
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = (uint32_t)(lane + 32 * k);
+            w[k] = 4u * i < bst ? __ldcg(reinterpret_cast<const uint32_t*>(gp + (size_t)r * bst) + i) : 0x80808080u;
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const uint32_t i = (uint32_t)(lane + 32 * k);
+            if (8u * i < hst) {
+                const uint32_t lo = __byte_perm(w[k], 0u, 0x4140u) + 0x7f807f80u, hi = __byte_perm(w[k], 0u, 0x4342u) + 0x7f807f80u;
+                *reinterpret_cast<uint2*>(gp + (size_t)r * hst + 8u * i) = make_uint2(lo, hi);
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The lane's chunks l, l + 8, ... of a candidate in the hybrid form: the
+// Gram rows come from HBM or L2, kFlight chunks of both rows in flight
+// before the first is used (all of them up to order 320).
+template <bool GEN>
+__device__ __forceinline__ void hybrid_rows(const Env& E, uint32_t w1, uint32_t w2, int R1, int R2, int l,
+                                            const Cand& q, int& acc, int& pr) {
+    constexpr int kFlight = 5;
+    const int nch = (E.n + 7) >> 3;
+    const uint8_t* p1 = E.gp + (size_t)R1 * E.gst;
+    const uint8_t* p2 = E.gp + (size_t)R2 * E.gst;
+    const bool two = R2 != R1;
+#pragma unroll 1
+    for (int j0 = l; j0 < nch; j0 += 8 * kFlight) {
+        uint4 o1[kFlight], o2[kFlight];
+#pragma unroll
+        for (int k = 0; k < kFlight; ++k) {
+            const int j = j0 + 8 * k;
+            o1[k] = make_uint4(0, 0, 0, 0);
+            if (j < nch) o1[k] = __ldcg(reinterpret_cast<const uint4*>(p1) + j);
+            o2[k] = o1[k];
+            if (two && j < nch) o2[k] = __ldcg(reinterpret_cast<const uint4*>(p2) + j);
+        }
+#pragma unroll
+        for (int k = 0; k < kFlight; ++k) {
+            const int j = j0 + 8 * k;
+            if (j < nch) {
+                const uint32_t old1[4] = {o1[k].x, o1[k].y, o1[k].z, o1[k].w};
+                const uint32_t old2[4] = {o2[k].x, o2[k].y, o2[k].z, o2[k].w};
+                uint32_t g1[4] = {o1[k].x, o1[k].y, o1[k].z, o1[k].w}, g2[4] = {o2[k].x, o2[k].y, o2[k].z, o2[k].w};
+                hybrid_chunk(w1, w2, R1, R2, j, q.a1, q.b1, q.a2, q.b2, q.pk, false, g1, g2);
+                wide_sums<GEN>(E.obj_kind, g1, g2, old1, old2, acc, pr);
             }
         }
     }
@@ -529,7 +800,7 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     constexpr int LPC = GW / 4;
     const unsigned gm = group_mask<GW>();
     const int n = E.n, m = ONEZ ? 1 : E.m, sparse = ONEZ ? 0 : E.sparse;
-    const uint32_t st = E.st, slot = E.slot, wbase = E.slot + Slot<WPL>::w, cw = E.cw;
+    const uint32_t st = E.st, slot = E.slot, wbase = wbase_of<WPL>(E.slot, E.n), cw = E.cw;
     const Con* con = con_of<WPL>(slot);
     const int l = lane & (LPC - 1);
     Cand q;
@@ -544,11 +815,9 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     int hot;
     if (GW == 32 && E.ts <= 8) {
         const uint32_t r = (uint32_t)ix(lds32(cw + 64u + 4u * (uint32_t)l), (uint32_t)n);
-        uint32_t key = (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - l) << 8) | r;
+        uint32_t key = (lds32(slot + Slot<WPL>::res + 4u * r) << 14) | ((uint32_t)(63 - l) << 8) | (r & 255u);
         if (l >= E.ts) key = 0;
-#pragma unroll
-        for (int d = 1; d < LPC; d <<= 1) key = max(key, __shfl_xor_sync(gm, key, d));
-        hot = (int)(key & 255u);
+        hot = best_row<WPL, LPC>(key, r, gm);
     } else {
         hot = tournament<WPL, GW>(slot, cw, n, E.ts, c, it + (uint64_t)d_it, l, gm);
     }
@@ -571,7 +840,7 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     bool bad;
     if constexpr (ONEZ) {
         // the row's only zero is its minority entry
-        const int z1 = (int)lds8(E.mino + (uint32_t)R1), z2 = (int)lds8(E.mino + (uint32_t)R2);
+        const int z1 = mino_at<WPL>(E, R1), z2 = mino_at<WPL>(E, R2);
         const int f1 = after_zero(ix(dbl ? b2.w : b1.x, (uint32_t)n), z1, n), f2 = after_zero(ix(b3.z, (uint32_t)n), z2, n);
         const bool sw = !dbl && !flip;
         C1 = sw ? z2 : f1;
@@ -580,15 +849,14 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     } else {
         auto fcol = [&](uint32_t wd, int row) -> int {
             const int i = ix(wd, (uint32_t)(sparse ? m : n));
-            return sparse ? (int)lds8(E.mino + (uint32_t)(row * m + i)) : mask_first<WPL>(slot, row, i, n);
+            return sparse ? mino_at<WPL>(E, row * m + i) : mask_first<WPL>(slot, row, i, n);
         };
         const int f1 = fcol(dbl ? b2.w : b1.x, R1);
         const int f2 = fcol(b3.z, R2);
         p1 = ix(b1.z, (uint32_t)m);
         p2 = ix(b1.w, (uint32_t)m);
-        const int q1 = (int)lds8(E.mino + (uint32_t)(R1 * m + p1)), q2 = (int)lds8(E.mino + (uint32_t)(R2 * m + p2));
-        const uint32_t e1 = lds8(wbase + (uint32_t)q2 * st + (uint32_t)R1);
-        const uint32_t e2 = lds8(wbase + (uint32_t)q1 * st + (uint32_t)R2);
+        const int q1 = mino_at<WPL>(E, R1 * m + p1), q2 = mino_at<WPL>(E, R2 * m + p2);
+        const uint32_t e1 = w_at<WPL>(wbase, st, R1, q2), e2 = w_at<WPL>(wbase, st, R2, q1);
         const bool illegal = sparse ? e1 != 1u || e2 != 1u : e1 == 1u || e2 == 1u;
         const bool sw = !dbl && !flip;
         C1 = sw ? (sparse ? q1 : q2) : f1;
@@ -608,18 +876,18 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
         const bool need = (__ballot_sync(gm, act && (bad || edge)) >> ((threadIdx.x & 31u) - (uint32_t)l)) & ((1u << LPC) - 1u);
         const bool exact = __any_sync(gm, edge);
         if (exact) hot = tournament<WPL, GW>(slot, cw, n, E.ts, c, it + (uint64_t)d_it, l, gm);
-        const uint2 x = propose_exact<WPL, GW, ONEZ>(E, need, exact ? 0 : 1, hot, c, it + (uint64_t)d_it, l);
+        const uint4 x = propose_exact<WPL, GW, ONEZ>(E, need, exact ? 0 : 1, hot, c, it + (uint64_t)d_it, l);
         if (need) {
-            R1 = (int)(x.x & 255u);
+            R1 = (int)(x.x & 0xffffu);
             if (kind != 3) {
-                R2 = (int)((x.x >> 8) & 255u);
-                C1 = (int)((x.x >> 16) & 255u);
-                C2 = (int)(x.x >> 24);
-                kind = (int)(x.y & 3u);
-                p1 = (int)((x.y >> 8) & 255u);
-                p2 = (int)((x.y >> 16) & 255u);
-                s1 = (x.y >> 24) & 1u;
-                s2 = (x.y >> 25) & 1u;
+                R2 = (int)(x.x >> 16);
+                C1 = (int)(x.y & 0xffffu);
+                C2 = (int)(x.y >> 16);
+                p1 = (int)(x.z & 0xffffu);
+                p2 = (int)(x.z >> 16);
+                kind = (int)(x.w & 3u);
+                s1 = (x.w >> 2) & 1u;
+                s2 = (x.w >> 3) & 1u;
             }
         }
     }
@@ -630,7 +898,7 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
                                         sparse ? 1 : 2);
         const int start = (int)draw_index(sparse ? b1.z : b1.y, (uint32_t)n, dsl, it + (uint64_t)d_it, con->stream, con->k0, con->k1,
                                           sparse ? 2 : 1);
-        const int z = (int)lds8(E.mino + (uint32_t)(R1 * m + pos));
+        const int z = mino_at<WPL>(E, R1 * m + pos);
         p1 = pos;
         R2 = R1;
         if constexpr (ONEZ) {
@@ -645,9 +913,9 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
 
     // E: coefficients, then the new values of the lane's rows
     const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
-    const bool lact = WPL == 8 || 4 * WPL * l < n;               // the lane holds rows below n
+    const bool lact = WPL >= 8 || 4 * WPL * l < n;               // the lane holds rows below n
     const uint32_t loff = lact ? (uint32_t)(4 * WPL * l) : 0u;   // their byte offset
-    constexpr int NW = WPL == 8 ? 1 : WPL;
+    constexpr int NW = WPL >= 8 ? 1 : WPL;
     uint32_t x[NW], y[NW], g1[NW], g2[NW];
     if constexpr (WPL < 8) {
         load_words<WPL>(w1 + loff, x);
@@ -655,9 +923,9 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
         load_words<WPL>(E.g + (uint32_t)R1 * st + loff, g1);
         load_words<WPL>(E.g + (uint32_t)R2 * st + loff, g2);
     }
-    const uint32_t rs = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R1) +
-                        lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R2);
-    const int e11 = (int)lds8(w1 + (uint32_t)R1) - 1, e22 = (int)lds8(w2 + (uint32_t)R2) - 1;
+    const uint32_t rs1 = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R1);
+    const uint32_t rs2 = lds32(slot + Slot<WPL>::res + 4u * (uint32_t)R2);
+    const int e11 = (int)w_at<WPL>(wbase, st, R1, C1) - 1, e22 = (int)w_at<WPL>(wbase, st, R2, C2) - 1;
     const bool two = R2 != R1, sw = kind == 1, pair = kind == 2 && two;
     const int m11 = sw || (GEN && kind == 3) ? -e11 : -2 * e11, m22 = sw ? -e22 : -2 * e22;
     q.a1 = m11;
@@ -667,7 +935,7 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     if (GEN && kind == 3) q.b1 = s1 ? 1 : -1;
     {
         // double flip over two rows (xweigh_cuda.cu:564-583): G[R1][R2]
-        const int e21 = (int)lds8(w1 + (uint32_t)R2) - 1, e12 = (int)lds8(w2 + (uint32_t)R1) - 1;
+        const int e21 = (int)w_at<WPL>(wbase, st, R2, C1) - 1, e12 = (int)w_at<WPL>(wbase, st, R1, C2) - 1;
         const int pk = m11 * e21 + m22 * (e12 + (C1 == C2 ? m11 : 0));
         q.pk = pair ? pk : 0;
     }
@@ -678,6 +946,21 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
 #pragma unroll 1
         for (int j = l; 8 * j < n; j += 8)
             wide_chunk<GEN>(E, w1, w2, R1, R2, j, q, acc, pr);
+    } else if constexpr (WPL == 16) {
+        bool halves = con->halves != 0;
+        if (!halves) {
+            bool over = false;
+            if (act) hybrid_rows_bytes<GEN>(E, w1, w2, R1, R2, l, q, acc, pr, over);
+            if (__any_sync(FULL, over)) {
+                widen_gram(E.gp, n, lane);
+                if (lane == 0) con_of<WPL>(slot)->halves = 1;
+                __syncwarp();
+                halves = true;
+                acc = 0;
+                pr = 0;
+            }
+        }
+        if (halves && act) hybrid_rows<GEN>(E, w1, w2, R1, R2, l, q, acc, pr);
     } else
 #pragma unroll
     for (int j = 0; j < NW; ++j) {
@@ -713,8 +996,16 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
         acc = 0;
         pr = 0;
     }
-    // less the rows' old sums (their conflicts weigh 4096 here, 2^18 in rs)
-    if (l == 0) acc -= (int)rs - (int)(rs >> kConfShift) * ((1 << kConfShift) - 4096);
+    // less the rows' old sums (their conflicts weigh 4096 here, 2^18 there)
+    if (l == 0) {
+        if constexpr (WPL == 16) {   // (two rows' sums do not fit 18 bits)
+            acc -= (int)rs1 - (int)(rs1 >> kConfShift) * ((1 << kConfShift) - 4096);
+            acc -= (int)rs2 - (int)(rs2 >> kConfShift) * ((1 << kConfShift) - 4096);
+        } else {
+            const uint32_t rs = rs1 + rs2;
+            acc -= (int)rs - (int)(rs >> kConfShift) * ((1 << kConfShift) - 4096);
+        }
+    }
 #pragma unroll
     for (int d = 1; d < LPC; d <<= 1) acc += __shfl_xor_sync(gm, acc, d);
     if (GEN && E.obj_kind != 0) {
@@ -741,13 +1032,13 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
 __device__ __forceinline__ void best_keys(bool gen_obj, const Cand& q, bool act, int g, bool by_index, unsigned gm,
                                           uint32_t& A, uint32_t& B) {
     const int dc = (q.acc + 2048) >> 12, ds = q.acc - dc * 4096;
-    const uint32_t low = ((uint32_t)(dc + 512) << 5) | (uint32_t)g;
+    const uint32_t low = ((uint32_t)(ds + 2048) << 16) | ((uint32_t)(dc + 1024) << 5) | (uint32_t)g;
     if (!gen_obj) {
-        const uint32_t ka = by_index ? (uint32_t)g : ((uint32_t)(ds + 2048) << 15) | low;
+        const uint32_t ka = by_index ? (uint32_t)g : low;
         A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
         B = A;
     } else {
-        const uint32_t ka = by_index ? (uint32_t)g : ((uint32_t)(q.prim + (1 << 19)) << 12) | (uint32_t)(ds + 2048);
+        const uint32_t ka = by_index ? (uint32_t)g : (uint32_t)(q.prim + (1 << 22));
         A = __reduce_min_sync(gm, act ? ka : 0xffffffffu);
         B = __reduce_min_sync(gm, act && ka == A ? low : 0xffffffffu);
     }
@@ -833,7 +1124,7 @@ __device__ __forceinline__ Winner choose_many(const Env E, uint64_t it, int coun
             bestA = ka;
             bestB = kb;
             const int src = wl0 + (int)(B & 3u) * LPC;
-            w.mv = move_of(pack_move(q), src, gm);
+            w.mv = move_of(pack_move<WPL>(q), src, gm);
             w.acc = __shfl_sync(gm, q.acc, src);
             w.prim = __shfl_sync(gm, q.prim, src);
         }
@@ -1040,6 +1331,116 @@ __device__ __forceinline__ void commit_wide(const Env& E, const Move& mv, int ac
     }
 }
 
+// Adds `d` to entry (r, c) of a nibble-pair W.
+__device__ __forceinline__ void nibble_add(uint32_t wbase, uint32_t st, int r, int c, int d) {
+    const uint32_t a = wbase + (uint32_t)c * st + ((uint32_t)r >> 2), b = lds8(a);
+    const int i = r & 3, w = (int)((b >> i) & 1u) - 2 * (int)((b >> (4 + i)) & 1u) + d;
+    const uint32_t v = (w != 0 ? 1u : 0u) | (w < 0 ? 16u : 0u);
+    xw_smem[a] = (uint8_t)((b & ~(0x11u << i)) | (v << i));
+}
+
+// Commit in the hybrid form: lane c rewrites chunks c, c + 32 of the two
+// rows and the entries of columns R1 and R2 in the rows of those chunks.
+__device__ __forceinline__ void commit_hybrid(const Env& E, const Move& mv, int acc, int lane) {
+    const int n = E.n, m = E.m, nch = (n + 7) >> 3;
+    const uint32_t st = E.st, slot = E.slot, wbase = wbase_of<16>(slot, n);
+    const int R1 = (int)((mv.rc & 255u) | ((mv.ax >> 18) & 256u)), R2 = (int)(((mv.rc >> 8) & 255u) | ((mv.ax >> 19) & 256u));
+    const int C1 = (int)(((mv.rc >> 16) & 255u) | ((mv.ax >> 20) & 256u)), C2 = (int)((mv.rc >> 24) | ((mv.ax >> 21) & 256u));
+    const bool two = R2 != R1;
+    const int a1 = (int)(int8_t)(mv.cf & 255u), b1 = (int)(int8_t)((mv.cf >> 8) & 255u);
+    const int a2 = (int)(int8_t)((mv.cf >> 16) & 255u), b2 = (int)(int8_t)(mv.cf >> 24);
+    const int pk = (int)(int8_t)(mv.ax & 255u);
+    int S1 = 0, dpair = 0;
+    const bool halves = con_of<16>(slot)->halves != 0;
+    if (!halves && lane < (n + 15) >> 4) {
+        // bytes: at most 28 chunks of 16 entries
+        const uint32_t bst = hybrid_byte_stride(n);
+        uint4* q1 = reinterpret_cast<uint4*>(E.gp + (size_t)R1 * bst) + lane;
+        uint4* q2 = reinterpret_cast<uint4*>(E.gp + (size_t)R2 * bst) + lane;
+        const uint4 o1 = __ldcg(q1), o2 = two ? __ldcg(q2) : o1;
+        const uint32_t old1[4] = {o1.x, o1.y, o1.z, o1.w}, old2[4] = {o2.x, o2.y, o2.z, o2.w};
+        uint32_t g1[4] = {o1.x, o1.y, o1.z, o1.w}, g2[4] = {o2.x, o2.y, o2.z, o2.w};
+        hybrid_chunk_bytes(wbase + (uint32_t)C1 * st, wbase + (uint32_t)C2 * st, R1, R2, lane, a1, b1, a2, b2, pk, true,
+                           g1, g2);
+        *q1 = make_uint4(g1[0], g1[1], g1[2], g1[3]);
+        if (two) *q2 = make_uint4(g2[0], g2[1], g2[2], g2[3]);
+        int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res) + 16 * lane;
+        const int wt1 = 0x0000ff01, wt = two ? (int)0xff01ff01u : wt1;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            const int o = 16 * lane + i, sh = 8 * (i & 3);
+            if (o < n) {
+                const uint32_t n1 = (g1[i >> 2] >> sh) & 255u, n2 = (g2[i >> 2] >> sh) & 255u;
+                const uint32_t v = __vabsdiffu4(n1 | (((old1[i >> 2] >> sh) & 255u) << 8) | (n2 << 16) |
+                                                    (((old2[i >> 2] >> sh) & 255u) << 24),
+                                                0x80808080u);
+                const uint32_t z = ((v + 0x7f7f7f7fu) & 0x80808080u) >> 7;
+                const int d1 = __dp4a((int)v, wt1, 0) + (__dp4a((int)z, wt1, 0) << kConfShift);
+                S1 += d1;
+                if (o == R2) dpair = d1;
+                if (o != R1 && o != R2) {
+                    uint8_t* row = E.gp + (size_t)o * bst;
+                    row[R1] = (uint8_t)n1;
+                    if (two) row[R2] = (uint8_t)n2;
+                    res[i] += __dp4a((int)v, wt, 0) + (__dp4a((int)z, wt, 0) << kConfShift);
+                }
+            }
+        }
+    }
+#pragma unroll 1
+    for (int j = halves ? lane : nch; j < nch; j += 32) {
+        uint4* q1 = reinterpret_cast<uint4*>(E.gp + (size_t)R1 * E.gst) + j;
+        uint4* q2 = reinterpret_cast<uint4*>(E.gp + (size_t)R2 * E.gst) + j;
+        const uint4 o1 = __ldcg(q1), o2 = two ? __ldcg(q2) : o1;
+        const uint32_t old1[4] = {o1.x, o1.y, o1.z, o1.w}, old2[4] = {o2.x, o2.y, o2.z, o2.w};
+        uint32_t g1[4] = {o1.x, o1.y, o1.z, o1.w}, g2[4] = {o2.x, o2.y, o2.z, o2.w};
+        hybrid_chunk(wbase + (uint32_t)C1 * st, wbase + (uint32_t)C2 * st, R1, R2, j, a1, b1, a2, b2, pk, true, g1, g2);
+        *q1 = make_uint4(g1[0], g1[1], g1[2], g1[3]);
+        if (two) *q2 = make_uint4(g2[0], g2[1], g2[2], g2[3]);
+        int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res) + 8 * j;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int o = 8 * j + i, sh = 16 * (i & 1);
+            const uint32_t n1 = (g1[i >> 1] >> sh) & 0xffffu, n2 = (g2[i >> 1] >> sh) & 0xffffu;
+            const int d1 = packed_abs((int)n1 - 32768) - packed_abs((int)((old1[i >> 1] >> sh) & 0xffffu) - 32768);
+            const int d2 = packed_abs((int)n2 - 32768) - packed_abs((int)((old2[i >> 1] >> sh) & 0xffffu) - 32768);
+            if (o < n) {
+                S1 += d1;
+                if (o == R2) dpair = d1;
+                // rows R1 and R2 themselves are written by chunks only: a
+                // lane may still have to read its chunk of them
+                if (o != R1 && o != R2) {
+                    uint16_t* row = reinterpret_cast<uint16_t*>(E.gp + (size_t)o * E.gst);
+                    row[R1] = (uint16_t)n1;
+                    if (two) row[R2] = (uint16_t)n2;
+                    res[i] += two ? d1 + d2 : d1;
+                }
+            }
+        }
+    }
+    S1 = __reduce_add_sync(FULL, S1);
+    const int dc = (acc + 2048) >> 12;
+    const int S = acc - dc * 4096 + dc * (1 << kConfShift);   // both rows, the pair entry once
+    int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res);
+    if ((halves ? (R2 >> 3) & 31 : R2 >> 4) == lane && two) res[R2] += S - S1 + dpair;
+    if (lane == 0) res[R1] += S1;
+    // (every lane has read W's columns; two entries may share a byte)
+    __syncwarp();
+    if (lane == 0) {
+        if (a1) nibble_add(wbase, st, R1, C1, a1);
+        if (a2) nibble_add(wbase, st, R2, C1, a2);
+    }
+    if (lane == (C1 == C2 ? 0 : 1)) {
+        if (b1) nibble_add(wbase, st, R1, C2, b1);
+        if (b2) nibble_add(wbase, st, R2, C2, b2);
+    }
+    if (lane < 2 && ((mv.ax >> (24 + lane)) & 1u)) {
+        const int lost = lane ? C2 : C1, got = lane ? C1 : C2;
+        const int p = (int)((mv.ax >> (8 + 8 * lane)) & 255u);
+        E.mp[(lane ? R2 : R1) * m + p] = (uint16_t)(E.sparse ? got : lost);
+    }
+}
+
 // tab[d-1] = ceil(exp(-d/T) * 2^32), computed with the same division and
 // exponential as metropolis_accept, so that for a 32-bit draw u
 //   u * 2^-32 < exp(-d/T)  <=>  u < tab[d-1]
@@ -1077,6 +1478,26 @@ template <int WPL, int GW>
 __device__ __noinline__ void save_w(int8_t* dst, uint32_t wbase, uint32_t st, int n, int lane) {
     const int wpc = (n + 3) >> 2;
     const bool whole = (n & 3) == 0;   // every word of the record is aligned and full
+    if constexpr (WPL == 16) {
+#pragma unroll 1
+        for (int j = lane; j < wpc; j += 32) {
+#pragma unroll 4
+            for (int k = 0; k < n; ++k) {
+                // bit i of a nibble to byte i
+                const uint32_t x = lds8(wbase + (uint32_t)k * st + (uint32_t)j);
+                const uint32_t v = (((x & 15u) * 0x00204081u) & 0x01010101u) + (((x >> 4) * 0x00204081u) & 0x01010101u) * 0xfeu;
+                int8_t* d = dst + (uint32_t)(k * n + 4 * j);
+                if (whole) {
+                    *reinterpret_cast<uint32_t*>(d) = v;
+                } else {
+#pragma unroll
+                    for (int e = 0; e < 4; ++e)
+                        if (4 * j + e < n) d[e] = (int8_t)(v >> (8 * e));
+                }
+            }
+        }
+        return;
+    }
     int c = 0, q = lane;
 #pragma unroll 1
     for (;;) {
@@ -1103,15 +1524,32 @@ __device__ __noinline__ void save_w(int8_t* dst, uint32_t wbase, uint32_t st, in
 template <int WPL, int GW>
 __device__ __forceinline__ void save_best(uint8_t* rec, const XwJob* J, const Env& E, int jn, int lane) {
     const unsigned gm = group_mask<GW>();
-    const uint32_t wbase = E.slot + Slot<WPL>::w;
+    const uint32_t wbase = wbase_of<WPL>(E.slot, E.n);
     auto add = [&](int sign) {
-        for (int i = 0; i < jn; ++i) {
+        // (out newest first, so that every entry stays ternary on the way)
+        for (int k = 0; k < jn; ++k) {
+            const int i = sign < 0 ? jn - 1 - k : k;
             const uint2 mv = *reinterpret_cast<const uint2*>(xw_smem + E.slot + Slot<WPL>::jrn + 8u * (uint32_t)i);
-            const int cf = (int)(int8_t)((mv.y >> (8 * (lane & 3))) & 255u);
-            if (lane < 4 && cf != 0) {
-                const uint32_t a = wbase + ((lane & 1) ? mv.x >> 24 : (mv.x >> 16) & 255u) * E.st +
-                                   ((lane & 2) ? (mv.x >> 8) & 255u : mv.x & 255u);
-                xw_smem[a] = (uint8_t)((int)lds8(a) + sign * cf);
+            // entry e: row R1 or R2 (bit 1), column C1 or C2 (bit 0)
+            auto entry = [&](int e, int& r, int& c) -> int {
+                r = (int)(((mv.x >> ((e & 2) ? 8 : 0)) & 255u) | (((mv.y >> ((e & 2) ? 17 : 16)) & 1u) << 8));
+                c = (int)(((mv.x >> ((e & 1) ? 24 : 16)) & 255u) | (((mv.y >> ((e & 1) ? 19 : 18)) & 1u) << 8));
+                return sign * ((int)(mv.y << (28 - 4 * e)) >> 28);
+            };
+            int r, c;
+            if constexpr (WPL == 16) {
+                if (lane == 0) {   // (two entries may share a byte)
+                    for (int e = 0; e < 4; ++e) {
+                        const int d = entry(e, r, c);
+                        if (d) nibble_add(wbase, E.st, r, c, d);
+                    }
+                }
+            } else {
+                const int d = entry(lane & 3, r, c);
+                if (lane < 4 && d != 0) {
+                    const uint32_t a = wbase + (uint32_t)c * E.st + (uint32_t)r;
+                    xw_smem[a] = (uint8_t)((int)lds8(a) + d);
+                }
             }
             __syncwarp(gm);
         }
@@ -1134,10 +1572,12 @@ __device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, 
     E.sparse = ONEZ ? 0 : J->sparse;
     E.full = !ONEZ && J->w == n;
     E.st = packed_stride(n, WPL);
-    E.gst = WPL == 8 ? wide_stride(n) : E.st;
+    E.gst = WPL == 16 ? hybrid_gram_stride(n) : WPL == 8 ? wide_stride(n) : E.st;
     const uint32_t mat = xw_pad16((uint32_t)n * E.st);
-    E.g = slot + Slot<WPL>::w + mat;
-    E.mino = E.g + (WPL == 8 ? (uint32_t)n * E.gst : mat);
+    E.g = wbase_of<WPL>(slot, n) + mat;
+    E.mino = WPL == 16 ? E.g : E.g + (WPL == 8 ? (uint32_t)n * E.gst : mat);
+    E.gp = nullptr;
+    E.mp = nullptr;
     E.ts = J->target_samples;
     E.bpc = 4 + (E.ts <= 4 ? 1 : 2);   // cached blocks per candidate
     E.cw = draws + (uint32_t)((lane / LPC) * E.bpc) * 16u;
@@ -1421,6 +1861,201 @@ __device__ __forceinline__ bool build_wide(const Env& E, const XwJob* J, const u
     return true;
 }
 
+__device__ __forceinline__ void mma_s8(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                       uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// G of the hybrid form, and the packed residuals, from the rows of W as
+// signed nibbles: mma.m16n8k32 on bytes, 16 rows against 8 at a time.  A
+// nibble in the upper half of a byte is 16 w, so that the products carry a
+// factor of 256 and no sign has to be extended; lane t of a quad holds
+// columns 64 Q + 16 t .. + 15 of its row in both operands, an order of the
+// contraction index that leaves the sums alone.  (By popcounts of row masks
+// the same took 18 POPC an entry: 3.9 of 4.9 ms that 2368 replicas of
+// W(276,275) took to load, 10 warps on an SM.)  Byte form: true when an
+// entry exceeds kByteMax.
+__device__ __forceinline__ bool hybrid_gram(bool halves, uint8_t* gp, const uint8_t* rows, int* res, int n, int lane,
+                                            int& p_score, int& p_conf, int& p_par, long long& p_sq) {
+    constexpr int kMaxK = kHybridMaxOrder / 64;
+    const int g = lane >> 2, t = lane & 3, nk = (n + 63) >> 6;
+    const uint32_t rst = hybrid_row_stride(n), gst = halves ? hybrid_gram_stride(n) : hybrid_byte_stride(n);
+    const int nc = halves ? (n + 7) >> 3 : (int)(gst >> 3);
+    bool over = false;
+    auto load = [&](int row, uint2 (&x)[kMaxK]) {
+        const uint2* p = reinterpret_cast<const uint2*>(rows + (uint32_t)row * rst) + t;
+#pragma unroll
+        for (int Q = 0; Q < kMaxK; ++Q) {
+            x[Q] = make_uint2(0u, 0u);
+            if (Q < nk && row < n) x[Q] = __ldcg(p + 4 * Q);
+        }
+    };
+    auto lo = [](uint32_t x) -> uint32_t { return (x << 4) & 0xf0f0f0f0u; };
+    auto hi = [](uint32_t x) -> uint32_t { return x & 0xf0f0f0f0u; };
+#pragma unroll 1
+    for (int rb = 0; rb < n; rb += 16) {
+        uint2 a0[kMaxK], a1[kMaxK], b[kMaxK], nx[kMaxK];
+        load(rb + g, a0);
+        load(rb + 8 + g, a1);
+        load(g, nx);
+        int sum[2] = {0, 0};
+#pragma unroll 1
+        for (int cb = 0; cb < nc; ++cb) {
+#pragma unroll
+            for (int Q = 0; Q < kMaxK; ++Q) b[Q] = nx[Q];
+            if (cb + 1 < nc) load(8 * (cb + 1) + g, nx);
+            int c[4] = {0, 0, 0, 0};
+#pragma unroll
+            for (int Q = 0; Q < kMaxK; ++Q) {
+                if (Q < nk) {
+                    mma_s8(c, lo(a0[Q].x), lo(a1[Q].x), hi(a0[Q].x), hi(a1[Q].x), lo(b[Q].x), hi(b[Q].x));
+                    mma_s8(c, lo(a0[Q].y), lo(a1[Q].y), hi(a0[Q].y), hi(a1[Q].y), lo(b[Q].y), hi(b[Q].y));
+                }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = rb + 8 * h + g, o = 8 * cb + 2 * t;
+                const int d0 = r == o ? 0 : c[2 * h] >> 8, d1 = r == o + 1 ? 0 : c[2 * h + 1] >> 8;
+                over = over || iabs(d0) > kByteMax || iabs(d1) > kByteMax;
+                sum[h] += packed_abs(d0) + packed_abs(d1);
+                p_sq += (long long)(d0 * d0 + d1 * d1);
+                p_par += (d0 & 1) + (d1 & 1);
+                if (r < n) {
+                    if (halves) *reinterpret_cast<uint32_t*>(gp + (uint32_t)r * gst + 2u * (uint32_t)o) =
+                        (uint32_t)(32768 + d0) | ((uint32_t)(32768 + d1) << 16);
+                    else *reinterpret_cast<uint16_t*>(gp + (uint32_t)r * gst + (uint32_t)o) =
+                        (uint16_t)((uint32_t)((128 + d0) & 255) | ((uint32_t)((128 + d1) & 255) << 8));
+                }
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            sum[h] += __shfl_xor_sync(FULL, sum[h], 1);
+            sum[h] += __shfl_xor_sync(FULL, sum[h], 2);
+            const int r = rb + 8 * h + g;
+            if (t == 0 && r < n) {
+                res[r] = sum[h];
+                p_score += sum[h] & ((1 << kConfShift) - 1);
+                p_conf += sum[h] >> kConfShift;
+            }
+        }
+    }
+    return __any_sync(FULL, !halves && over);
+}
+
+// Hybrid form: W as nibble pairs and the minority lists into the slot; G
+// and the residuals from the arena when it holds them (XW_STATUS_GRAM: the
+// totals are then the residuals' and the header's), else G built into it.
+__device__ __forceinline__ bool build_hybrid(const Env& E, const XwJob* J, const uint8_t* rec, uint8_t* arena,
+                                             uint32_t status0, int w, int lane, int& score0, int& conf0, int& par0,
+                                             long long& sq0, bool& halves) {
+    const int n = E.n, m = E.m, sparse = E.sparse;
+    const uint32_t slot = E.slot, st = E.st, wbase = wbase_of<16>(slot, n);
+    const int8_t* gw = reinterpret_cast<const int8_t*>(rec + J->off_w);
+    int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res);
+    const bool cached = status0 & XW_STATUS_GRAM;
+    int bad = 0;
+    if (n > kHybridMaxOrder) return false;
+    const bool whole = (n & 3) == 0;   // every word of the record is aligned and full
+#pragma unroll 1
+    for (int q = lane; q < (int)st; q += 32) {
+        const bool word = whole && 4 * q < n;
+#pragma unroll 1
+        for (int c0 = 0; c0 < n; c0 += 4) {
+            uint32_t v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int8_t* g = gw + (uint32_t)((c0 + k) * n + 4 * q);
+                if (word && c0 + k < n) {
+                    v[k] = *reinterpret_cast<const uint32_t*>(g);
+                } else if (c0 + k < n) {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        if (4 * q + i < n) v[k] |= (uint32_t)(uint8_t)g[i] << (8 * i);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (__vabs4(v[k]) & 0xfefefefeu) bad = 1;
+                // bits 0, 8, 16, 24 to bits 24..27
+                const uint32_t sup = ((v[k] & 0x01010101u) * 0x01020408u) >> 24,
+                               neg = (((v[k] >> 7) & 0x01010101u) * 0x01020408u) >> 24;
+                if (c0 + k < n) xw_smem[wbase + (uint32_t)(c0 + k) * st + (uint32_t)q] = (uint8_t)((sup & 15u) | ((neg & 15u) << 4));
+            }
+        }
+    }
+    const uint16_t* gmo = reinterpret_cast<const uint16_t*>(rec + J->off_mino);
+    if (m == 0 && lane == 0 && (uint32_t)(2 * n * m) <= kHybridMino) E.mp[0] = 0;   // an empty list reads as column 0
+    if (m > 0 && (status0 & XW_STATUS_INIT) && E.mp != gmo)
+        for (int i = lane; i < n * m; i += 32) E.mp[i] = gmo[i];
+    __syncwarp();
+    int p_score = 0, p_conf = 0, p_par = 0;
+    long long p_sq = 0;
+    halves = false;
+    if (cached) {
+        halves = *reinterpret_cast<const uint32_t*>(arena + hybrid_arena(n).off_rows) != 0;
+        const int* ares = reinterpret_cast<const int*>(arena);
+        for (int o = lane; o < n; o += 32) {
+            const int r = ares[o];
+            res[o] = r;
+            p_score += r & ((1 << kConfShift) - 1);
+            p_conf += r >> kConfShift;
+        }
+    } else {
+        uint8_t* rows = arena + hybrid_arena(n).off_rows;
+        const uint32_t rst = hybrid_row_stride(n);
+#pragma unroll 1
+        for (int o = lane; o < n; o += 32) {
+            int weight = 0, pos = 0;
+#pragma unroll 1
+            for (uint32_t q = 0; 16u * q < rst; ++q) {
+                uint32_t sup = 0, w4[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    const int c = 32 * (int)q + i;
+                    if (c < n) {
+                        const uint32_t v = w_at<16>(wbase, st, o, c) - 1u;
+                        sup |= (v & 1u) << i;
+                        w4[i >> 3] |= (v & 15u) << (4 * (i & 7));
+                    }
+                }
+                *reinterpret_cast<uint4*>(rows + (uint32_t)o * rst + 16u * q) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+                weight += __popc(sup);
+                const int left = n - 32 * (int)q;
+                if (m > 0 && !(status0 & XW_STATUS_INIT) && left > 0) {
+                    uint32_t x = (sparse ? sup : ~sup) & (left >= 32 ? 0xffffffffu : (1u << left) - 1u);
+                    while (x && pos < m) {
+                        E.mp[o * m + pos] = (uint16_t)(32 * q + __ffs((int)x) - 1);
+                        x &= x - 1;
+                        ++pos;
+                    }
+                }
+            }
+            if (weight != w) bad = 1;
+        }
+        if (__any_sync(FULL, bad)) return false;
+        __syncwarp();
+#pragma unroll 1
+        while (hybrid_gram(halves, E.gp, rows, res, n, lane, p_score, p_conf, p_par, p_sq)) {
+            halves = true;
+            p_score = p_conf = p_par = 0;
+            p_sq = 0;
+            __syncwarp();
+        }
+    }
+    if (__any_sync(FULL, bad)) return false;
+    score0 = __reduce_add_sync(FULL, p_score) / 2;
+    conf0 = __reduce_add_sync(FULL, p_conf) / 2;
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) p_sq += __shfl_xor_sync(FULL, p_sq, off);
+    sq0 = p_sq / 2;
+    par0 = __reduce_add_sync(FULL, p_par) / 2;
+    __syncwarp();
+    return true;
+}
+
 // Loads replica `rid` into the slot: W and the minority lists; the masks,
 // the Gram matrix (by popcounts of support and sign masks) and the
 // residuals are rebuilt from W and checked against the header.  False when
@@ -1455,14 +2090,22 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
     int score0, conf0, par0;
     long long sq0;
     bool ok;
-    if constexpr (WPL == 8) ok = build_wide(E, J, rec, status0, w, lane, score0, conf0, par0, sq0);
+    bool halves = false, cached = false;   // hybrid form: G is in halfwords; the arena holds this W's G and residuals
+    if constexpr (WPL == 16) {
+        uint8_t* arena = a.gram + a.gram_off[rid];
+        E.gp = arena + hybrid_arena(E.n).off_g;
+        E.mp = (uint32_t)(2 * E.n * E.m) <= kHybridMino ? reinterpret_cast<uint16_t*>(xw_smem + E.mino)
+                                                        : reinterpret_cast<uint16_t*>(rec + J->off_mino);
+        cached = status0 & XW_STATUS_GRAM;
+        ok = build_hybrid(E, J, rec, arena, status0, w, lane, score0, conf0, par0, sq0, halves);
+    } else if constexpr (WPL == 8) ok = build_wide(E, J, rec, status0, w, lane, score0, conf0, par0, sq0);
     else ok = build_packed<WPL, GW>(E, J, rec, status0, w, lane, score0, conf0, par0, sq0);
     if (!ok) {
         if (lane == 0 && owner) H->err |= XW_ERR_MINORITY;
         return false;
     }
 
-    const int64_t obj0 = obj_kind == 1 ? sq0 : obj_kind == 2 ? par0 : score0;
+    const int64_t obj0 = cached && obj_kind != 0 ? H->obj_total : obj_kind == 1 ? sq0 : obj_kind == 2 ? par0 : score0;
     const bool init = status0 & XW_STATUS_INIT;
     if (init && (H->score != score0 || H->conflicts != conf0 || H->obj_total != obj0)) {
         if (lane == 0 && owner) H->err |= XW_ERR_SCORE;
@@ -1497,6 +2140,7 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
         c.k_end = (int32_t)(iters < 0x7ffffffeull ? iters : 0x7ffffffeull);
         c.jn = init ? -1 : 0;
         c.owner = owner ? 1 : 0;
+        c.halves = halves ? 1 : 0;
         c.rid = rid;
         *con_of<WPL>(slot) = c;
     }
@@ -1517,11 +2161,21 @@ __device__ __forceinline__ void store_replica(const AnnealArgs& a, const Env& E,
     uint8_t* rec = a.arena + a.rec_off[con->rid];
     RepHeader* H = reinterpret_cast<RepHeader*>(rec);
     const XwJob* J = a.jobs + H->job;
-    const uint32_t wbase = E.slot + Slot<WPL>::w;
+    const uint32_t wbase = wbase_of<WPL>(E.slot, E.n);
     if (con->jn >= 0) save_best<WPL, GW>(rec, J, E, con->jn, lane);
     save_w<WPL, GW>(reinterpret_cast<int8_t*>(rec + J->off_w), wbase, E.st, E.n, lane);
-    uint8_t* gmo = rec + J->off_mino;
-    for (uint32_t i = lane; i < (uint32_t)(E.n * E.m); i += GW) gmo[i] = xw_smem[E.mino + i];
+    if constexpr (WPL == 16) {
+        uint16_t* gmo = reinterpret_cast<uint16_t*>(rec + J->off_mino);
+        if (gmo != E.mp)
+            for (int i = lane; i < E.n * E.m; i += GW) gmo[i] = E.mp[i];
+        int* res = reinterpret_cast<int*>(a.gram + a.gram_off[con->rid]);
+        if (lane == 0)
+            *reinterpret_cast<uint32_t*>(a.gram + a.gram_off[con->rid] + hybrid_arena(E.n).off_rows) = con->halves ? 1u : 0u;
+        for (int o = lane; o < E.n; o += GW) res[o] = reinterpret_cast<const int*>(xw_smem + E.slot + Slot<WPL>::res)[o];
+    } else {
+        uint8_t* gmo = rec + J->off_mino;
+        for (uint32_t i = lane; i < (uint32_t)(E.n * E.m); i += GW) gmo[i] = xw_smem[E.mino + i];
+    }
     if (lane == 0) {
         const bool init = H->status & XW_STATUS_INIT;
         H->it = con->it0 + (uint64_t)k;
@@ -1538,7 +2192,7 @@ __device__ __forceinline__ void store_replica(const AnnealArgs& a, const Env& E,
         H->temperature = con->T;
         H->msi = k - con->mb;
         H->cool_ctr = J->tempering ? -con->cb : k - con->cb;   // tempering leaves it alone
-        H->status = H->status | XW_STATUS_INIT | (con->best.z == 0 ? XW_STATUS_SOLVED : 0u);
+        H->status = H->status | XW_STATUS_INIT | (WPL == 16 ? XW_STATUS_GRAM : 0u) | (con->best.z == 0 ? XW_STATUS_SOLVED : 0u);
     }
     __syncwarp(gm);
 }
@@ -1561,14 +2215,15 @@ __device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, c
         uint8_t* rec = a.arena + a.rec_off[con->rid];
         save_best<WPL, GW>(rec, a.jobs + reinterpret_cast<RepHeader*>(rec)->job, E, jn, lane);
     }
-    if constexpr (WPL == 8) commit_wide<ONEZ>(E, mv, acc, lane);
+    if constexpr (WPL == 16) commit_hybrid(E, mv, acc, lane);
+    else if constexpr (WPL == 8) commit_wide<ONEZ>(E, mv, acc, lane);
     else commit<WPL, GW, ONEZ>(E, mv, acc, lane);
     if (lane == 0) {
         const long long o = (long long)(((uint64_t)(uint32_t)t.y << 32) | (uint32_t)t.x) + prim;
         t.x = (int)(uint32_t)o;
         t.y = (int)(o >> 32);
         t.z += 1;
-        t.w += (mv.rc & 255u) != ((mv.rc >> 8) & 255u) ? 2 : 1;
+        t.w += (mv.rc & 255u) != ((mv.rc >> 8) & 255u) || ((mv.ax >> 26) & 1u) != ((mv.ax >> 27) & 1u) ? 2 : 1;
         con->acc = t;
         if (improved) {
             b.z = b.x;
@@ -1591,7 +2246,9 @@ __device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, c
             con->jn = 0;
         } else if (jn >= 0) {
             if (jn < kJournal)
-                *reinterpret_cast<uint2*>(xw_smem + E.slot + Slot<WPL>::jrn + 8u * (uint32_t)jn) = make_uint2(mv.rc, mv.cf);
+                *reinterpret_cast<uint2*>(xw_smem + E.slot + Slot<WPL>::jrn + 8u * (uint32_t)jn) =
+                    make_uint2(mv.rc, (mv.cf & 15u) | ((mv.cf >> 4) & 0xf0u) | ((mv.cf >> 8) & 0xf00u) |
+                                          ((mv.cf >> 12) & 0xf000u) | (((mv.ax >> 26) & 15u) << 16));
             con->jn = jn < kJournal ? jn + 1 : -1;
         }
     }
