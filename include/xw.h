@@ -336,9 +336,10 @@ int32_t xw_batch_solve(const xw_job_spec* jobs, int32_t njobs, const xw_params* 
  * (xweigh_anneal.hpp:429-453, 239-264).  stats receives 4 int32 per matrix:
  * L1 score sum_{i<j}|G_ij|, conflicts #{i<j: G_ij != 0}, squared score
  * sum_{i<j} G_ij^2, and 1 when G = wI exactly (else 0).  gram (nullable)
- * receives each G as n*n row-major int32.  n a multiple of 32 runs on the
- * tensor cores (tcgen05 kind::i8, int32 accumulation, exact since
- * |G_ij| <= n); other n <= 128 on a SIMT kernel.  Host buffers. */
+ * receives each G as n*n row-major int32.  Runs on the tensor cores
+ * (tcgen05 kind::i8, int32 accumulation, exact since |G_ij| <= n); tiny
+ * orders (n <= 8, and n <= 12 below 4000 matrices) on a SIMT kernel, whose
+ * launch is cheaper.  Host buffers. */
 int32_t xw_rescore(const int8_t* W_rowmajor, int64_t count, int32_t n, int32_t w, int32_t* stats,
                    int32_t* gram);
 /* Same on device buffers, enqueued on `stream` (cudaStream_t); simt != 0

@@ -1232,8 +1232,7 @@ __device__ void run_large(const AnnealArgs& a, uint32_t rid, uint8_t* slot, int 
 
 // CTAs of four warps per SM the register budget is sized for: the
 // stored-Gram form hides HBM latency with warps; the bit-plane form holds
-// two CTAs (its slots fill shared memory) and spends the registers on its
-// per-lane Gram rows
+// two CTAs (its slots fill shared memory)
 #ifndef XW_LARGE_MIN_BLOCKS
 #define XW_LARGE_MIN_BLOCKS 4
 #endif

@@ -1,6 +1,6 @@
 // xw_packed.cuh -- one annealing iteration on packed rows, for orders up to
-// 256: the device code shared by the one-warp replica loop and the latency
-// mode of xw_anneal.cu.
+// 448: the device code shared by the one-warp replica loop, the latency mode
+// and the large orders' kernel of xw_anneal.cu.
 //
 // W and its Gram matrix sit in the replica's shared-memory slot as biased
 // bytes, four rows of a column of W (or four entries of a row of G) to a
@@ -1352,37 +1352,56 @@ __device__ __forceinline__ void commit_hybrid(const Env& E, const Move& mv, int 
     const int pk = (int)(int8_t)(mv.ax & 255u);
     int S1 = 0, dpair = 0;
     const bool halves = con_of<16>(slot)->halves != 0;
-    if (!halves && lane < (n + 15) >> 4) {
-        // bytes: at most 28 chunks of 16 entries
+    if (!halves) {
+        // bytes: words lane, lane + 32, ... of both rows, one ahead (a loop
+        // of four rows against one pass over sixteen a lane, which left 14
+        // lanes of W(276,275) idle and fetched four times the code: 2368
+        // replicas 15.3 -> 14.2 ms, 148 replicas 5.1 -> 4.8, 2368 of
+        // W(400,200) 41.6 -> 36.9; the same loop for the evaluation's reads,
+        // which then wait for each other: 14.7, 5.4 and 40.7)
         const uint32_t bst = hybrid_byte_stride(n);
-        uint4* q1 = reinterpret_cast<uint4*>(E.gp + (size_t)R1 * bst) + lane;
-        uint4* q2 = reinterpret_cast<uint4*>(E.gp + (size_t)R2 * bst) + lane;
-        const uint4 o1 = __ldcg(q1), o2 = two ? __ldcg(q2) : o1;
-        const uint32_t old1[4] = {o1.x, o1.y, o1.z, o1.w}, old2[4] = {o2.x, o2.y, o2.z, o2.w};
-        uint32_t g1[4] = {o1.x, o1.y, o1.z, o1.w}, g2[4] = {o2.x, o2.y, o2.z, o2.w};
-        hybrid_chunk_bytes(wbase + (uint32_t)C1 * st, wbase + (uint32_t)C2 * st, R1, R2, lane, a1, b1, a2, b2, pk, true,
-                           g1, g2);
-        *q1 = make_uint4(g1[0], g1[1], g1[2], g1[3]);
-        if (two) *q2 = make_uint4(g2[0], g2[1], g2[2], g2[3]);
-        int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res) + 16 * lane;
-        const int wt1 = 0x0000ff01, wt = two ? (int)0xff01ff01u : wt1;
+        uint32_t* q1 = reinterpret_cast<uint32_t*>(E.gp + (size_t)R1 * bst);
+        uint32_t* q2 = reinterpret_cast<uint32_t*>(E.gp + (size_t)R2 * bst);
+        const uint32_t w1 = wbase + (uint32_t)C1 * st, w2 = wbase + (uint32_t)C2 * st;
+        const int nwd = (n + 3) >> 2, wt1 = 0x0000ff01, wt = two ? (int)0xff01ff01u : wt1;
+        uint32_t next1 = 0, next2 = 0;
+        if (lane < nwd) {
+            next1 = __ldcg(q1 + lane);
+            next2 = __ldcg(q2 + lane);
+        }
+#pragma unroll 1
+        for (int j = lane; j < nwd; j += 32) {
+            const uint32_t old1 = next1, old2 = next2;
+            if (j + 32 < nwd) {
+                next1 = __ldcg(q1 + j + 32);
+                next2 = __ldcg(q2 + j + 32);
+            }
+            const uint32_t keep = ~((R1 >> 2) == j ? 0x11u << (R1 & 3) : 0u) & ~((R2 >> 2) == j ? 0x11u << (R2 & 3) : 0u);
+            const uint32_t X = lds32(2048u + 4u * (lds8(w1 + (uint32_t)j) & keep)),
+                           Y = lds32(2048u + 4u * (lds8(w2 + (uint32_t)j) & keep));
+            const uint32_t o32 = 32u * (uint32_t)j;
+            const uint32_t g1 = old1 + (uint32_t)a1 * X + (uint32_t)b1 * Y + shl_clamp((uint32_t)pk, 8u * (uint32_t)R2 - o32);
+            const uint32_t g2 = old2 + (uint32_t)a2 * X + (uint32_t)b2 * Y + shl_clamp((uint32_t)pk, 8u * (uint32_t)R1 - o32);
+            q1[j] = g1;
+            if (two) q2[j] = g2;
+            int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res) + 4 * j;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const int o = 16 * lane + i, sh = 8 * (i & 3);
-            if (o < n) {
-                const uint32_t n1 = (g1[i >> 2] >> sh) & 255u, n2 = (g2[i >> 2] >> sh) & 255u;
-                const uint32_t v = __vabsdiffu4(n1 | (((old1[i >> 2] >> sh) & 255u) << 8) | (n2 << 16) |
-                                                    (((old2[i >> 2] >> sh) & 255u) << 24),
-                                                0x80808080u);
-                const uint32_t z = ((v + 0x7f7f7f7fu) & 0x80808080u) >> 7;
-                const int d1 = __dp4a((int)v, wt1, 0) + (__dp4a((int)z, wt1, 0) << kConfShift);
-                S1 += d1;
-                if (o == R2) dpair = d1;
-                if (o != R1 && o != R2) {
-                    uint8_t* row = E.gp + (size_t)o * bst;
-                    row[R1] = (uint8_t)n1;
-                    if (two) row[R2] = (uint8_t)n2;
-                    res[i] += __dp4a((int)v, wt, 0) + (__dp4a((int)z, wt, 0) << kConfShift);
+            for (int i = 0; i < 4; ++i) {
+                const int o = 4 * j + i, sh = 8 * i;
+                if (o < n) {
+                    const uint32_t n1 = (g1 >> sh) & 255u, n2 = (g2 >> sh) & 255u;
+                    const uint32_t v = __vabsdiffu4(n1 | (((old1 >> sh) & 255u) << 8) | (n2 << 16) | (((old2 >> sh) & 255u) << 24),
+                                                    0x80808080u);
+                    const uint32_t z = ((v + 0x7f7f7f7fu) & 0x80808080u) >> 7;
+                    const int d1 = __dp4a((int)v, wt1, 0) + (__dp4a((int)z, wt1, 0) << kConfShift);
+                    S1 += d1;
+                    if (o == R2) dpair = d1;
+                    if (o != R1 && o != R2) {
+                        uint8_t* row = E.gp + (size_t)o * bst;
+                        row[R1] = (uint8_t)n1;
+                        if (two) row[R2] = (uint8_t)n2;
+                        res[i] += __dp4a((int)v, wt, 0) + (__dp4a((int)z, wt, 0) << kConfShift);
+                    }
                 }
             }
         }
@@ -1422,7 +1441,7 @@ __device__ __forceinline__ void commit_hybrid(const Env& E, const Move& mv, int 
     const int dc = (acc + 2048) >> 12;
     const int S = acc - dc * 4096 + dc * (1 << kConfShift);   // both rows, the pair entry once
     int* res = reinterpret_cast<int*>(xw_smem + slot + Slot<16>::res);
-    if ((halves ? (R2 >> 3) & 31 : R2 >> 4) == lane && two) res[R2] += S - S1 + dpair;
+    if ((halves ? (R2 >> 3) & 31 : (R2 >> 2) & 31) == lane && two) res[R2] += S - S1 + dpair;
     if (lane == 0) res[R1] += S1;
     // (every lane has read W's columns; two entries may share a byte)
     __syncwarp();

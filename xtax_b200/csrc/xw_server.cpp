@@ -783,8 +783,9 @@ void Server::start() {
     for (bool general : {false, true}) raise_smem_limit(anneal_kernel_fn(1, general, 1, true), cfg.device);
     if (cfg.max_active_replicas <= 0) {
         // eight waves of the resident warps at the order-32 slot: enough work
-        // per round to keep every SM busy through the round's tails (the C5
-        // stream, 400 requests: 0.567 G moves/s at four waves and 1000
+        // per round to keep every SM busy through the round's tails (a
+        // Poisson stream of 400 mixed requests, with a kernel of 0.9 G moves/s
+        // on W(26,25): 0.567 G moves/s at four waves and 1000
         // iterations per round, 0.612 G at eight and 2000, with p50/p99
         // time-to-exact 1.16 s / 23.3 s against 1.44 s / 25.2 s; a stream the
         // device keeps up with: p50 0.096 s against 0.099 s)
