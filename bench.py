@@ -206,7 +206,7 @@ def make_params():
                     squared_objective_fraction=0.0, parity_objective_fraction=0.0, stop_on_solve=0)
 
 
-def algorithmic_smem_bytes(cand_evals, two_row_evals, accepted_rows, n=N_ORDER, g=4):
+def algorithmic_smem_bytes(cand_evals, two_row_evals, accepted_rows, n=N_ORDER, g=1):
     """Shared-memory bytes the moves need at minimum, from the move
     statistics the kernel counts: each evaluated candidate reads, per row it
     changes (one, or two for the counted two-row candidates), (n-1) Gram
@@ -577,7 +577,7 @@ def large_bench(X, iters, ref_seconds):
                 "launch_class": cls,
                 "kernel": "anneal_large_kernel, " + {1: "Gram matrix in HBM",
                                                      2: "bit planes in shared memory, Gram entries recomputed",
-                                                     3: "bit planes in shared memory, Gram matrix in HBM"}[cls["large"]]}
+                                                     3: "W in shared memory, Gram matrix in HBM"}[cls["large"]]}
 
     out = {"workload": f"W({LARGE_N},{LARGE_W}) x {LARGE_R} replicas, cooling from T 6 (t_min 0.1), L1 objective, "
                        f"the reference's moves, {iters} iterations per replica",
