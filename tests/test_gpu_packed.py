@@ -7,6 +7,8 @@ tournament counts that take several passes, coins of probability 0 and 1,
 runs of one-candidate iterations of every length, temperatures above the
 32-bit threshold table, and index draws in Lemire's rejection zone.
 """
+import struct
+
 import pytest
 
 import oracle_lib as O
@@ -89,3 +91,72 @@ def test_an_index_draw_in_the_rejection_zone():
 @pytest.mark.parametrize("n,w", [(13, 12), (26, 24), (32, 31)])
 def test_latency_mode_at_odd_counts(n, w):
     replay(n, w, 2, 500, 60 + n, warps_per_replica=6, candidate_samples=6, t_init=0.7, t_min=0.1, moves_per_cool=23)
+
+
+def set_stagnation(path, value):
+    """Sets the moves since the last improvement of every replica of a
+    snapshot file (the header's field at byte 64 of its record)."""
+    d = bytearray(open(path, "rb").read())
+    job, header, params, jobs = struct.unpack_from("<4I", d, 8)
+    replicas, arena, rungs = struct.unpack_from("<3Q", d, 24)
+    assert header == 128
+    off = 48 + params + job * jobs
+    records = struct.unpack_from(f"<{replicas}Q", d, off)
+    base = off + 8 * (replicas + rungs + jobs)
+    assert len(d) == base + arena
+    for r in records:
+        struct.pack_into("<i", d, base + r + 64, value)
+    open(path, "wb").write(bytes(d))
+
+
+@pytest.mark.parametrize("n,w,R,kw", [(12, 11, 4, dict(warps_per_replica=1)), (13, 6, 4, dict(warps_per_replica=1)),
+                                      (14, 13, 5, dict(warps_per_replica=1, replicas_per_warp=2)),
+                                      (12, 11, 4, dict(warps_per_replica=8)), (24, 23, 4, dict(warps_per_replica=32)),
+                                      (16, 4, 4, dict(warps_per_replica=64, objective=1)), (40, 20, 4, {}), (100, 99, 4, {}),
+                                      (150, 149, 4, {}), (260, 259, 4, {}),
+                                      (12, 11, 1, dict(warps_per_replica=1, t_min=1e3, reheat=3.0)),
+                                      (12, 11, 1, dict(warps_per_replica=16, t_min=1e3, reheat=3.0)),
+                                      (260, 130, 1, dict(t_min=1e3, reheat=3.0))], ids=str)
+def test_a_tempering_replica_is_never_reheated(n, w, R, kw, tmp_path):
+    # replicas whose count of moves without improvement passes 2^31 - 1 early
+    # in the second half of the run: the upper rungs of a hot ladder, which a
+    # reheat (factor 1e-6) would freeze, or a ladder of one, whose temperature
+    # no exchange sets again
+    p = X.Params(**{**dict(stop_on_solve=0, tempering=1, exchange_interval=300, t_min=50.0, t_init=1e4, reheat=1e-6, greedy_fraction=0.0,
+                           squared_objective_fraction=0.0, parity_objective_fraction=0.0), **kw})
+    seed, top = 600 + n, 2 ** 31 - 1 - 5
+    jobs = [{"n": n, "w": w, "seed": seed, "replicas": R}]
+    first = X.Batch(jobs, p)
+    first.run(300)
+    first.synchronize()
+    path = str(tmp_path / "population")
+    first.save(path)
+    first.close()
+    set_stagnation(path, top)
+    batch = X.Batch.load(path, jobs)
+    batch.run(300)
+    batch.synchronize()
+    ratio = (p.t_init / p.t_min) ** (1.0 / max(R - 1, 1))
+    ladder = [p.t_min]
+    while len(ladder) < R:
+        ladder.append(ladder[-1] * ratio)
+    job = oracle_job(n, w, seed, p)
+    reps = [O.Replica(job, r, start_of(n, w, seed, r, p), ladder[r], r) for r in range(R)]
+    for k in range(2):
+        for rep in reps:
+            rep.run(300, stop_on_solve=False)
+        if R > 1:
+            O.exchange(job, reps, ladder, k)
+    for r, rep in enumerate(reps):
+        st, W, B, M = batch.replica(0, r)
+        s, oW, oB, oM, _, _ = rep.get()
+        assert (st.error, st.iterations, st.moves, st.candidate_evaluations) == (0, s.it, s.moves, s.cand_evals), r
+        assert (st.score, st.conflicts, st.best_score, st.best_conflicts) == (s.score, s.conflicts, s.best_score,
+                                                                              s.best_conflicts), r
+        assert (st.temperature, st.rung, st.objective_total) == (s.temperature, s.rung, s.obj_total), r
+        assert (W == oW).all() and (B == oB).all() and (M == oM).all(), r
+        # counted from the last improvement, or on from the snapshot's count,
+        # which wraps
+        assert st.moves_since_improvement == (s.msi if s.msi < 300 else top + 300 - 2 ** 32), r
+        assert st.cooling_counter == s.cool_ctr, r
+    batch.close()

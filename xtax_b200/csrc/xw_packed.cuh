@@ -121,7 +121,8 @@ struct Con {
     int4 acc;            // objective total (64 bits), accepted moves, rows they changed
     double T;
     int32_t mb, cb;
-    int32_t mpc, stuck;  // calls per cooling step, calls without improvement before a reheat (tempering: never)
+    int32_t mpc, stuck;  // calls per cooling step, calls without improvement before a reheat
+    int32_t fixed;       // tempering: the temperature is the rung's, which only an exchange changes
     int32_t k_end;       // iterations of this launch
     // moves accepted since the best W, all of them in the journal: the record
     // holds an older one.  -1: the record holds the best W.
@@ -2152,10 +2153,13 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
         c.best = make_int4(score0, conf0, init ? H->best_score : score0, init ? H->best_conflicts : conf0);
         c.acc = make_int4((int)(uint32_t)obj0, (int)(obj0 >> 32), init ? (int)H->accepted : 0,
                           init ? (int)H->accepted_rows : 0);
-        c.mb = init ? -H->msi : 0;
+        // (a tempering replica's count of calls without improvement goes on
+        // for as long as it runs, and wraps)
+        c.mb = init ? (int32_t)(0u - (uint32_t)H->msi) : 0;
         c.cb = init ? -H->cool_ctr : 0;
-        c.mpc = J->tempering ? 0x7fffffff : J->moves_per_cool;
-        c.stuck = J->tempering ? 0x7fffffff : J->stuck_threshold;
+        c.mpc = J->moves_per_cool;
+        c.stuck = J->stuck_threshold;
+        c.fixed = J->tempering;
         c.k_end = (int32_t)(iters < 0x7ffffffeull ? iters : 0x7ffffffeull);
         c.jn = init ? -1 : 0;
         c.owner = owner ? 1 : 0;
@@ -2209,7 +2213,7 @@ __device__ __forceinline__ void store_replica(const AnnealArgs& a, const Env& E,
         H->best_conflicts = con->best.w;
         H->obj_total = (int64_t)(((uint64_t)(uint32_t)con->acc.y << 32) | (uint32_t)con->acc.x);
         H->temperature = con->T;
-        H->msi = k - con->mb;
+        H->msi = (int32_t)((uint32_t)k - (uint32_t)con->mb);
         H->cool_ctr = J->tempering ? -con->cb : k - con->cb;   // tempering leaves it alone
         H->status = H->status | XW_STATUS_INIT | (WPL == 16 ? XW_STATUS_GRAM : 0u) | (con->best.z == 0 ? XW_STATUS_SOLVED : 0u);
     }
@@ -2279,15 +2283,18 @@ __device__ __forceinline__ bool accept_move(const AnnealArgs& a, const Env& E, c
 // the replica's calls end: the first k at which temperature_step has
 // something to do.
 __device__ __forceinline__ int next_event(const Con* con) {
+    if (con->fixed) return con->k_end;
     const long long e = min((long long)con->cb + con->mpc, (long long)con->mb + con->stuck);
     return (int)min(e, (long long)con->k_end);
 }
 
-// Cooling and reheat after call k (xweigh_cuda.cu:1087-1129).
+// Cooling and reheat after call k (xweigh_cuda.cu:1087-1129); neither under
+// tempering.
 template <int WPL, int GW>
 __device__ __forceinline__ void temperature_step(const AnnealArgs& a, uint32_t slot, int k, int lane) {
     const unsigned gm = group_mask<GW>();
     Con* con = con_of<WPL>(slot);
+    if (con->fixed) return;
     const bool cool = (long long)k - con->cb >= con->mpc, heat = (long long)k - con->mb >= con->stuck;
     if (!cool && !heat) return;
     const RepHeader* H = reinterpret_cast<const RepHeader*>(a.arena + a.rec_off[con->rid]);
