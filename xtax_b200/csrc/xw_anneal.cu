@@ -69,7 +69,7 @@ __device__ __forceinline__ bool step(const AnnealArgs& a, const Env& E, Walk& w,
     const int g = lane / LPC;
     const uint32_t win = E.slot + Slot<WPL>::win;
     if (w.wpos >= kWin) {
-        const uint4 b = draw_block(0u, con->it0 + (uint64_t)(w.k + lane), con->stream, con->k0, con->k1);
+        const uint4 b = draw_block(0u, con->it0 + (uint64_t)w.k + (uint64_t)lane, con->stream, con->k0, con->k1);
         w.wmask = __ballot_sync(gm, (uint64_t)b.x < con->thr_greedy) >> wl0;
         *reinterpret_cast<uint32_t*>(xw_smem + win + 4u * (uint32_t)lane) = b.y;
         w.wpos = 0;
@@ -134,8 +134,8 @@ __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, u
     };
     // the next k at which something besides moves happens
     auto event = [&](const Con* con, int k) -> int {
-        int e = max(next_event(con), k + 1);
-        if (a.stop_on_solve == 1) e = min(e, (k | 63) == k ? k + 64 : k | 63);
+        int e = xw_event_after(next_event(con), k);
+        if (a.stop_on_solve == 1) e = min(e, xw_event_after(0, k) | 63);   // calls 63, 127, ...
         return e;
     };
     Walk w{0, GW, 0u, 0u, 0u};
@@ -254,7 +254,7 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
     if (warp == 0) {
         ok = load_replica<WPL, GEN, 32, ONEZ>(a, rid, 0u, lane, a.iters, E, owner);
         if (ok) {
-            k_evt = max(next_event(con), 1);
+            k_evt = xw_event_after(next_event(con), 0);
             k_end = con->k_end;
         }
         if (lane == 0 && owner) {
@@ -351,12 +351,12 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
             auto after_call = [&]() {
                 if (k >= k_evt) {
                     temperature_step<WPL, 32>(a, 0u, k, lane);
-                    k_evt = max(next_event(con), k + 1);
+                    k_evt = xw_event_after(next_event(con), k);
                 }
             };
             auto commit_of = [&](int q) {
                 if (accept_move<WPL, GEN, 32, ONEZ>(a, E, outs[q].mv, outs[q].dsc, outs[q].prim, k, lane) && k < k_evt)
-                    k_evt = max(next_event(con), k + 1);
+                    k_evt = xw_event_after(next_event(con), k);
             };
             // lane l looks at iterations l and 32 + l (up to 64 iterations a
             // round, on a cluster of four)
@@ -412,16 +412,16 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
                 // the job's solved flag is looked at between rounds only
                 const int k_poll = a.stop_on_solve == 1 ? ((k | 63) == k ? k : k | 63) : k_end;
                 while (solo) {
-                    const int k1 = min(min(w.k + 64, k_poll), k_end);
+                    const int k1 = min(xw_calls_to(w.k, 64, k_end), k_poll);
                     int steps = 0, accs = 0;
                     while (w.k < k1) {
                         bool improved;
                         accs += step<WPL, GEN, 32, ONEZ>(a, E, w, min(k_evt, k1), lane, improved) ? 1 : 0;
                         ++steps;
-                        if (improved && w.k < k_evt) k_evt = max(next_event(con), w.k + 1);
+                        if (improved && w.k < k_evt) k_evt = xw_event_after(next_event(con), w.k);
                         if (w.k >= k_evt) {
                             temperature_step<WPL, 32>(a, 0u, w.k, lane);
-                            k_evt = max(next_event(con), w.k + 1);
+                            k_evt = xw_event_after(next_event(con), w.k);
                         }
                         if (a.stop_on_solve && con->best.z == 0) {
                             stop = true;

@@ -101,3 +101,26 @@ static_assert(sizeof(RepHeader) == 128, "replica header is 128 bytes");
 #endif
 
 static inline XW_HD XW_CONSTEXPR uint32_t xw_pad16(uint32_t v) { return (v + 15u) & ~15u; }
+
+// ---- counting the calls of a launch -----------------------------------
+// A replica counts the calls it makes in a launch in 32 bits: rounds are at
+// most 2^31 - 1 iterations long (moves_per_launch, exchange_interval and a
+// server's quantum are int32), so every count is exact and none of these
+// leaves the range.
+
+// Calls of a launch of `iters` iterations.
+static inline XW_HD int32_t xw_launch_calls(uint64_t iters) {
+    return iters < 0x7fffffffull ? (int32_t)iters : 0x7fffffff;
+}
+
+// The first call after call k to look for more than moves, `event` or the
+// next one if that is past.
+static inline XW_HD int32_t xw_event_after(int32_t event, int32_t k) {
+    const int32_t next = k < 0x7fffffff ? k + 1 : k;
+    return event > next ? event : next;
+}
+
+// At most `most` calls from call k in a launch of k_end calls: the last.
+static inline XW_HD int32_t xw_calls_to(int32_t k, int32_t most, int32_t k_end) {
+    return k_end - k < most ? k_end : k + most;
+}

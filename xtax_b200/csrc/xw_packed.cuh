@@ -2160,7 +2160,7 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
         c.mpc = J->moves_per_cool;
         c.stuck = J->stuck_threshold;
         c.fixed = J->tempering;
-        c.k_end = (int32_t)(iters < 0x7ffffffeull ? iters : 0x7ffffffeull);
+        c.k_end = xw_launch_calls(iters);
         c.jn = init ? -1 : 0;
         c.owner = owner ? 1 : 0;
         c.halves = halves ? 1 : 0;
