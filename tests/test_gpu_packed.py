@@ -160,3 +160,16 @@ def test_a_tempering_replica_is_never_reheated(n, w, R, kw, tmp_path):
         assert st.moves_since_improvement == (s.msi if s.msi < 300 else top + 300 - 2 ** 32), r
         assert st.cooling_counter == s.cool_ctr, r
     batch.close()
+
+
+@pytest.mark.parametrize("n,w,kw", [(12, 11, dict(warps_per_replica=1)), (12, 4, dict(warps_per_replica=1, replicas_per_warp=2)),
+                                    (20, 13, dict(warps_per_replica=8)), (40, 20, {}), (100, 99, {}), (150, 20, {}),
+                                    (260, 259, {})], ids=str)
+def test_a_certain_sign_flip_is_never_a_row_swap(n, w, kw):
+    # iteration 78 of replica 0 at this seed draws 2^32 - 1 for the flip's
+    # coin (by exhaustive search), which lies below the threshold 2^32 of
+    # probability 1
+    seed = 4352672
+    assert O.philox([1, 78, 0, 0], X.philox_key(seed))[3] == 2 ** 32 - 1
+    replay(n, w, 1, 120, seed, move_set=1, start_kind=1, sign_fraction=1.0, greedy_fraction=0.0, objective=0,
+           t_init=1e9, t_min=1e9, **kw)

@@ -210,7 +210,8 @@ struct Env {
     uint32_t gst;        // the same of G above order 128
     uint8_t* gp;         // hybrid form: G in the arena, the minority lists
     uint16_t* mp;
-    int n, m, sparse, full;   // full: w = n
+    int n, m, sparse;
+    int flips;           // every move but the double flips is a sign flip: w = n, or a coin of 2^32
     int ts, bpc, move_set, obj_kind;
     uint32_t dq[2];      // draw blocks this lane computes: candidate (or iteration) << 16 | 1 + block
 };
@@ -390,7 +391,7 @@ __device__ __forceinline__ uint4 propose_exact(const Env& E, bool need, int from
         const uint4 b0 = lds128(cw);
         row = (uint64_t)b0.x < con->thr_target ? hot : ix(b0.y, (uint32_t)n, 0, 1);
         dbl = (uint64_t)b0.z < con->thr_dbl;
-        flip = (!ONEZ && E.full) || (uint64_t)b0.w < con->thr_sign;
+        flip = (!ONEZ && E.flips) || (uint64_t)b0.w < con->thr_sign;
     }
     // double flip (xweigh_cuda.cu:389-421): attempt 0 from block 3, attempt
     // a > 0 from block 19 + a, 16 in all
@@ -829,8 +830,11 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
     const int rdraw = ix(b0.y, (uint32_t)n);
     int R1 = b0.x < coins.x ? hot : rdraw;
     const bool dbl = b0.z < coins.y;
+    // (the coin's 32 bits leave out the largest draw of a certain flip: the
+    // exact proposal sees to it, and a row swap, which has none, must not
+    // begin)
     bool flip = b0.w < coins.z;
-    if (!ONEZ) flip = flip || E.full;
+    if (!ONEZ || GEN) flip = flip || E.flips;
     flip = flip && !dbl;
     const bool rowswap = GEN && E.move_set == 1 && !flip && !dbl;
     const uint4 b1 = lds128(cw + 16), b2 = lds128(cw + 32), b3 = lds128(cw + 48);
@@ -1590,7 +1594,7 @@ __device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, 
     E.n = n;
     E.m = ONEZ ? 1 : J->m;
     E.sparse = ONEZ ? 0 : J->sparse;
-    E.full = !ONEZ && J->w == n;
+    E.flips = (!ONEZ && J->w == n) || (J->thr_sign >> 32) != 0;
     E.st = packed_stride(n, WPL);
     E.gst = WPL == 16 ? hybrid_gram_stride(n) : WPL == 8 ? wide_stride(n) : E.st;
     const uint32_t mat = xw_pad16((uint32_t)n * E.st);
