@@ -169,3 +169,24 @@ def test_rescore_of_entries_that_do_not_fit_a_byte(n, top):
                      np.zeros(count, dtype=np.int64)], 1)
     assert want.max() < 2 ** 30   # twice the squared score is summed in 32 bits
     assert (X.rescore(W, n, n // 2) == want).all()
+
+
+@pytest.mark.parametrize("n", [128, 216, 256])
+def test_rescore_of_equal_full_rows(n):
+    # every Gram entry is +-n: the largest squared score of ternary
+    # matrices, twice which passes 2^31 from n = 216 on
+    W = np.ones((3, n, n), dtype=np.int8)
+    W[1, ::2] = -1
+    want = [n * (n - 1) // 2 * n, n * (n - 1) // 2, n * (n - 1) // 2 * n * n, 0]
+    assert want[2] < 2 ** 31
+    stats, G = X.rescore(W, n, n, gram=True)
+    assert (np.abs(G) == n).all()
+    assert stats.tolist() == [want] * 3
+    assert X.rescore(W, n, n).tolist() == [want] * 3
+    torch = pytest.importorskip("torch")
+    import ctypes as C
+    d, out = torch.from_numpy(W).cuda(), torch.zeros((3, 4), dtype=torch.int32, device="cuda")
+    assert X.lib().xw_rescore_device(C.c_void_p(d.data_ptr()), 3, n, n, C.c_void_p(out.data_ptr()), None, 1,
+                                     None) == X.XW_OK
+    torch.cuda.synchronize()
+    assert out.tolist() == [want] * 3

@@ -362,9 +362,11 @@ __device__ __forceinline__ bool tile_rows(const RescoreParams& p, uint32_t tacc,
     return ok;
 }
 
-// symmetric G: the off-diagonal sums count each pair twice
+// symmetric G: the off-diagonal sums count each pair twice.  The doubled
+// squared sum of a ternary matrix is at most 256 * 255 * 256^2 < 2^32 (2^31 is
+// passed from order 216 on): its 32 bits are unsigned.
 __device__ __forceinline__ int4 matrix_stats(int abs_sum, int nz_sum, int sq_sum, int diag_ok) {
-    return make_int4(abs_sum / 2, nz_sum / 2, sq_sum / 2, (nz_sum == 0 && diag_ok) ? 1 : 0);
+    return make_int4(abs_sum / 2, nz_sum / 2, (int)((uint32_t)sq_sum / 2u), (nz_sum == 0 && diag_ok) ? 1 : 0);
 }
 
 // Rows 0..nv-1 of matrices mat0 .. mat0 + nmat - 1, columns [k0, k0 + 128),
@@ -791,7 +793,7 @@ __global__ void rescore_simt_kernel(const int8_t* W, int count, int n, int w, in
     s_nz = __reduce_add_sync(0xffffffffu, s_nz);
     s_sq = __reduce_add_sync(0xffffffffu, s_sq);
     diag_ok = (int)__reduce_and_sync(0xffffffffu, (unsigned)diag_ok);
-    if (lane == 0) stats[warp] = make_int4(s_abs / 2, s_nz / 2, s_sq / 2, (s_nz == 0 && diag_ok) ? 1 : 0);
+    if (lane == 0) stats[warp] = matrix_stats(s_abs, s_nz, s_sq, diag_ok);
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
