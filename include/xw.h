@@ -338,8 +338,9 @@ int32_t xw_batch_solve(const xw_job_spec* jobs, int32_t njobs, const xw_params* 
  * sum_{i<j} G_ij^2, and 1 when G = wI exactly (else 0).  gram (nullable)
  * receives each G as n*n row-major int32.  Runs on the tensor cores
  * (tcgen05 kind::i8, int32 accumulation, exact since |G_ij| <= n); tiny
- * orders (n <= 8, and n <= 12 below 4000 matrices) on a SIMT kernel, whose
- * launch is cheaper.  Host buffers. */
+ * orders (n <= 8, n = 9 below 8000 matrices and n <= 12 below 4000) on a SIMT
+ * kernel, whose launch is cheaper.  The sums are exact for ternary matrices.
+ * Host buffers. */
 int32_t xw_rescore(const int8_t* W_rowmajor, int64_t count, int32_t n, int32_t w, int32_t* stats,
                    int32_t* gram);
 /* Same on device buffers, enqueued on `stream` (cudaStream_t); simt != 0

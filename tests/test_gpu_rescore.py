@@ -190,3 +190,14 @@ def test_rescore_of_equal_full_rows(n):
                                      None) == X.XW_OK
     torch.cuda.synchronize()
     assert out.tolist() == [want] * 3
+
+
+@pytest.mark.parametrize("n,count", [(9, 3999), (9, 7999), (9, 8000), (10, 3999), (10, 4000), (12, 4000)])
+def test_rescore_on_both_sides_of_the_tiny_orders_line(n, count):
+    W = random_fixed_degree(40, n, n - 1, seed=n).repeat((count + 39) // 40, axis=0)[:count]
+    W[count - 1] = np.eye(n, dtype=np.int8)
+    ref = np.matmul(W.astype(np.int64), W.astype(np.int64).transpose(0, 2, 1))
+    off = ref * (1 - np.eye(n, dtype=np.int64))
+    want = np.stack([np.abs(off).sum((1, 2)) // 2, (off != 0).sum((1, 2)) // 2, (off * off).sum((1, 2)) // 2,
+                     (ref == np.eye(n, dtype=np.int64)).all((1, 2))], 1)
+    assert (X.rescore(W, n, 1) == want).all()

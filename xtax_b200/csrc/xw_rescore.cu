@@ -849,11 +849,12 @@ int32_t rescore_device(const int8_t* W, int64_t count, int n, int w, int32_t* st
     // to 128, and addresses, are padded by the packing warps; orders above by
     // rescore_big_kernel.  Tiny orders stay on the SIMT kernel, whose launch
     // is cheaper than a tile of mostly padding (us a call, SIMT / packed:
-    // n = 8, 1000 matrices 5.0 / 8.5, 20000 16.7 / 18.7; n = 12, 1000
+    // n = 8, 1000 matrices 5.0 / 8.5, 20000 16.7 / 18.7; n = 9, 4000 matrices
+    // 6.3 / 7.6, 8000 9.4 / 9.5; n = 10, 4000 matrices 7.7 / 7.6; n = 12, 1000
     // matrices 6.5 / 8.5, 4000 10.6 / 10.5; n = 16, 1000 matrices 8.5 / 8.5;
     // n = 26, one matrix 15.4 / 6.7; n = 100, one matrix 646 / 10.6, 8192
-    // matrices 7850 / 78).
-    const bool tc = !force_simt && !(n <= 8 || (n <= 12 && count < 4000));
+    // matrices 7850 / 68).
+    const bool tc = !force_simt && !(n <= 8 || (n <= 12 && count < (n == 9 ? 8000 : 4000)));
     const bool pack = n % 32 != 0 || ((uintptr_t)W % 16) != 0;
     if (!tc) {
         const int blocks = (int)((count * 32 + 255) / 256);
