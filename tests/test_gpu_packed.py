@@ -173,3 +173,10 @@ def test_a_certain_sign_flip_is_never_a_row_swap(n, w, kw):
     assert O.philox([1, 78, 0, 0], X.philox_key(seed))[3] == 2 ** 32 - 1
     replay(n, w, 1, 120, seed, move_set=1, start_kind=1, sign_fraction=1.0, greedy_fraction=0.0, objective=0,
            t_init=1e9, t_min=1e9, **kw)
+
+
+@pytest.mark.parametrize("ts,target", [(9, 0.0), (9, 0.05), (64, 0.0), (64, 0.05), (64, 1.0)])
+@pytest.mark.parametrize("n,w,kw", [(12, 11, dict(replicas_per_warp=2)), (14, 5, dict(warps_per_replica=8)), (26, 25, {}),
+                                    (40, 20, {}), (100, 99, {}), (140, 70, {})], ids=str)
+def test_long_tournaments_that_few_candidates_need(n, w, kw, ts, target):
+    replay(n, w, 2, 250 if n < 100 else 60, 8 * n + ts, target_samples=ts, target_fraction=target, **kw)
