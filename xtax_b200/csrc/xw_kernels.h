@@ -51,6 +51,7 @@ int anneal_opl(int n, int w);
 // `one_zero`: the instantiation for launches whose replicas all have one zero
 // per row (AnnealArgs::one_zero); it applies to opl 1, rpw 1 only.
 const void* anneal_kernel_fn(int opl, bool general, int rpw = 1, bool one_zero = false);
+const void* anneal_wide_kernel_fn(int opl, bool general);   // its opl 2, 4 and 8 (xw_anneal_wide.cu)
 cudaError_t launch_anneal(const AnnealArgs& args, int opl, bool general, int warps_per_block, int blocks,
                           cudaStream_t stream, int rpw = 1);
 // Latency mode (orders up to 32): one replica per CTA of K warps (2..16),
@@ -64,6 +65,8 @@ cudaError_t launch_anneal(const AnnealArgs& args, int opl, bool general, int war
 // unused)
 uint32_t anneal_spec_cta_bytes(uint32_t slot_bytes, int wpr, int ctas);
 const void* anneal_spec_kernel_fn(bool general, int ctas, bool one_zero);
+const void* anneal_spec_lean_fn(int ctas, bool one_zero);      // its two modules
+const void* anneal_spec_general_fn(int ctas, bool one_zero);
 cudaError_t launch_anneal_spec(const AnnealArgs& args, bool general, int wpr, int ctas, int blocks,
                                cudaStream_t stream);
 // Orders above XW_MAX_N (xw_anneal_large.cu), in one of three forms:
@@ -81,7 +84,7 @@ const void* anneal_large_kernel_fn(bool general, int form);
 size_t anneal_large_smem_bytes(int form, int warps_per_block, uint32_t slot_bytes);
 cudaError_t launch_anneal_large(const AnnealArgs& args, bool general, int form, int warps_per_block, int blocks,
                                 cudaStream_t stream);
-// Its form 2 runs the packed iteration of the smaller orders (xw_anneal.cu):
+// Its form 2 runs the packed iteration of the smaller orders (xw_anneal_wide.cu):
 // shared memory per warp, the CTA's table, arena bytes, the kernel.
 uint32_t anneal_hybrid_slot_bytes(int n, int m);
 uint32_t anneal_hybrid_table_bytes();
