@@ -580,6 +580,13 @@ int32_t xw_cpu_run(int32_t n, int32_t w, const xw_cpu_params* p, const int8_t* s
  * keeping all scratch state in a static device array of
  * XW_NOALLOC_SCRATCH_BYTES (4 MiB) that every GPU loading this library holds
  * until exit; a request that needs more is rejected with XW_ERR_CAPACITY.
+ * So is one whose p->warps_per_block (0: four) plain replicas exceed a
+ * block's shared memory (227 KB), a plain replica of W(n,w) having
+ * n*n + 4n(n|1) + 20n + n*min(w, n-w) + 1184 bytes up to order 128, above it
+ * n*n + 2n(n|1) + 36n + n*min(w, n-w) + 1184: the batch engine packs its
+ * replicas tighter, but the orders this entry takes are part of its
+ * interface.  W(n,n-1) at four warps: orders up to 104 and 129..131; at two,
+ * up to 189; at one, every order.
  * Inputs and outputs are the caller's device buffers:
  *   starts  replicas*n*n int8, column-major start states
  *   best    replicas*n*n int8, each replica's best state

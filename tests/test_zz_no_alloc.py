@@ -130,3 +130,23 @@ def test_noalloc_call_leaves_a_larger_batch_launchable():
     plain = run(False)
     assert all(e == 0 for _, _, e in plain)
     assert run(True) == plain
+
+
+@pytest.mark.parametrize("n,wpb,accepted", [(104, 0, True), (105, 0, False), (128, 0, False), (128, 2, True), (129, 0, True),
+                                            (131, 4, True), (132, 4, False), (189, 2, True), (190, 2, False),
+                                            (256, 1, True)])
+def test_noalloc_takes_the_orders_its_interface_states(n, wpb, accepted):
+    torch = pytest.importorskip("torch")
+    dev = torch.device("cuda:0")
+    p = X.Params(seed=5, t_init=2.0, stop_on_solve=0, warps_per_block=wpb)
+    st = torch.from_numpy(X.random_start(n, n - 1, 3)).to(dev)
+    best = torch.zeros(n * n, dtype=torch.int8, device=dev)
+    stats = torch.zeros(4, dtype=torch.int64, device=dev)
+    rc = X.lib().xw_anneal_noalloc(n, n - 1, C.byref(p.to_c()), 1, 2, C.c_void_p(st.data_ptr()),
+                                   C.c_void_p(best.data_ptr()), C.c_void_p(stats.data_ptr()), None)
+    torch.cuda.synchronize()
+    assert rc == (X.XW_OK if accepted else X.XW_ERR_CAPACITY)
+    if accepted:
+        assert int(stats[3]) == 2
+    else:
+        assert f"at {wpb or 4} warps per block is beyond this entry's limit" in X.lib().xw_last_error().decode()

@@ -213,15 +213,22 @@ extern "C" int32_t xw_anneal_noalloc(int32_t n, int32_t w, const xw_params* p, i
     // limit a batch or server launch of a larger order relies on
     int optin = 0;
     e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    // the calls this entry refuses are fixed by the size of a plain slot, up
-    // to order 128 W, a 32-bit Gram matrix with a padded row, row masks and
-    // buffers, whatever the kernel's own (smaller) slots take
+    // which orders this entry takes at a number of warps per block is fixed by
+    // its interface (include/xw.h), in terms of a plain replica: up to order
+    // 128 W, a 32-bit Gram matrix with a padded row, row masks and buffers.
+    // The kernel's own slots are smaller
     const uint32_t N = (uint32_t)n;
     const uint32_t plain = n > 128 ? slot
                                    : xw_pad16(N * N) + xw_pad16(4u * N * (N | 1u)) + xw_pad16(4u * N) +
                                          xw_pad16(N * (uint32_t)m) + 16u * N + 1184u;
-    if (e == cudaSuccess && (size_t)wpb * plain > (size_t)optin)
-        return nfail(XW_ERR_CAPACITY, "xw_anneal_noalloc: the replicas' shared memory exceeds the device's limit");
+    if (e == cudaSuccess && (size_t)wpb * plain > (size_t)optin) {
+        char msg[256];
+        std::snprintf(msg, sizeof msg,
+                      "xw_anneal_noalloc: W(%d,%d) at %d warps per block is beyond this entry's limit: %d plain replicas "
+                      "(%u bytes each) in a block's %d bytes of shared memory",
+                      n, w, wpb, optin / (int)plain, plain, optin);
+        return nfail(XW_ERR_CAPACITY, msg);
+    }
     cudaFuncAttributes attr{};
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&attr, fn);
     if (e == cudaSuccess)
