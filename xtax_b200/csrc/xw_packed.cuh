@@ -211,7 +211,9 @@ struct Env {
     uint8_t* gp;         // hybrid form: G in the arena, the minority lists
     uint16_t* mp;
     int n, m, sparse;
-    int flips;           // every move but the double flips is a sign flip: w = n, or a coin of 2^32
+    // every move but the double flips is a sign flip: w = n, or (kernels with
+    // row swaps) a coin of 2^32
+    int flips;
     int ts, bpc, move_set, obj_kind;
     uint32_t dq[2];      // draw blocks this lane computes: candidate (or iteration) << 16 | 1 + block
 };
@@ -825,9 +827,9 @@ __device__ __forceinline__ Cand candidate(const Env& E, uint64_t it, int d_it, i
         // tournament when no candidate takes its row.  1028 replicas of
         // W(23,22), 64 samples, a target fraction of 0, 400 iterations: 0.74 ms
         // against 1.56, and 0.92 in a kernel of one row a lane.  Orders above
-        // 256 always run it: the test costs every move of theirs 0.6%)
+        // 128 always run it: the test costs every move of theirs 0.6-1%)
         hot = 0;
-        if (WPL == 16 || E.ts <= 8 || __any_sync(gm, act && lds32(cw) < con->coins.x))
+        if (WPL >= 8 || E.ts <= 8 || __any_sync(gm, act && lds32(cw) < con->coins.x))
             hot = tournament<WPL, GW>(slot, cw, n, E.ts, c, it + (uint64_t)d_it, l, gm);
     }
 
@@ -1592,7 +1594,7 @@ __device__ __forceinline__ void save_best(uint8_t* rec, const XwJob* J, const En
 }
 
 // The lane's context, from the job and the slot.
-template <int WPL, int GW, bool ONEZ>
+template <int WPL, bool GEN, int GW, bool ONEZ>
 __device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, uint32_t draws, int lane, int obj_kind) {
     constexpr int LPC = GW / 4;
     const int n = J->n;
@@ -1601,7 +1603,7 @@ __device__ __forceinline__ void make_env(Env& E, const XwJob* J, uint32_t slot, 
     E.n = n;
     E.m = ONEZ ? 1 : J->m;
     E.sparse = ONEZ ? 0 : J->sparse;
-    E.flips = (!ONEZ && J->w == n) || (J->thr_sign >> 32) != 0;
+    E.flips = (!ONEZ && J->w == n ? 1 : 0) | (GEN ? (int)(J->thr_sign >> 32) : 0);
     E.st = packed_stride(n, WPL);
     E.gst = WPL == 16 ? hybrid_gram_stride(n) : WPL == 8 ? wide_stride(n) : E.st;
     const uint32_t mat = xw_pad16((uint32_t)n * E.st);
@@ -2110,7 +2112,7 @@ __device__ __forceinline__ bool load_replica(const AnnealArgs& a, uint32_t rid, 
         if (lane == 0) H->err |= XW_ERR_KERNEL;
         return false;
     }
-    make_env<WPL, GW, ONEZ>(E, J, slot, slot + Slot<WPL>::draws, lane, obj_kind);
+    make_env<WPL, GEN, GW, ONEZ>(E, J, slot, slot + Slot<WPL>::draws, lane, obj_kind);
     const int w = ONEZ ? E.n - 1 : J->w;
     const uint64_t it = H->it;
     if (J->budget_iters) {

@@ -126,7 +126,7 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
     // every warp: the replica's structures (read-only until warp 0 commits)
     // and its own draw buffer
     if (warp != 0)
-        make_env<WPL, 32, ONEZ>(E, J, 0u, L.off_extra + (uint32_t)(warp - 1) * 512u, lane, GEN ? H->obj_kind : 0);
+        make_env<WPL, GEN, 32, ONEZ>(E, J, 0u, L.off_extra + (uint32_t)(warp - 1) * 512u, lane, GEN ? H->obj_kind : 0);
 
     const int g = rank * K + warp;   // this warp's iteration within the round
 #pragma unroll 1
