@@ -53,7 +53,9 @@ extern "C" {
  * the same order, followed by the extensions of this implementation. */
 typedef struct xw_params {
     int32_t device;
-    int32_t replicas;             /* 0 = occupancy-based */
+    int32_t replicas;             /* 0 = one resident wave of the kernel: a count that depends on the
+                                     device and on this library's kernels, and with it the
+                                     run of a given seed */
     int32_t moves_per_launch;     /* iterations per replica between host checks */
     uint64_t seed;                /* 0 = random_device */
     double max_seconds;

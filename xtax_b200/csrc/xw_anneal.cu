@@ -1,10 +1,11 @@
-// xw_anneal.cu -- the population annealing kernel for weighing matrices.
+// xw_anneal.cu -- the population annealing kernel for weighing matrices: its
+// instantiations for orders up to 32, and its launches.
 //
 // One warp (or a half-warp) owns one replica at a time, its state in the
 // warp's shared-memory slot; the whole iteration is warp-synchronous: no
-// __syncthreads, no block-wide reductions.  The iteration itself is in
-// xw_packed.cuh: rows of W and G packed into words, bytes of G up to order
-// 128, halfwords above.
+// __syncthreads, no block-wide reductions.  The replica loop is in
+// xw_replica.cuh, the iteration itself in xw_packed.cuh: rows of W and G
+// packed into words, bytes of G up to order 128, halfwords above.
 //
 // Per iteration (the semantics of the reference kernel anneal_kernel,
 // src/xweigh_cuda.cu:988-1130, with cuRAND replaced by counter-based Philox):

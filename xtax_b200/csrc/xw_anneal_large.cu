@@ -20,7 +20,7 @@
 //
 // For orders up to 448 W can instead sit in the warp's slot.  Two forms do
 // that: the hybrid (the default there; anneal_hybrid_kernel in
-// xw_anneal.cu, the packed iteration of the smaller orders with G in the
+// xw_anneal_wide.cu, the packed iteration of the smaller orders with G in the
 // arena); and the bit-plane form here, W as support and sign bit planes and
 // no G: each Gram entry is recomputed by popcounts, so a move makes no HBM
 // traffic.  Its arena keeps residuals, planes and the best state's planes
@@ -64,7 +64,7 @@ struct LView {
 
 // The large orders' forms: the Gram matrix and masks in HBM; bit planes in
 // shared memory with every Gram entry recomputed; and W in shared memory
-// with the Gram matrix in HBM (another kernel, xw_anneal.cu).
+// with the Gram matrix in HBM (another kernel, xw_anneal_wide.cu).
 enum LargeForm : int { kFormGram = 0, kFormPlanes = 1, kFormHybrid = 2 };
 
 // Shared memory per warp.  Every replica: residuals (int32 x n), the
@@ -206,7 +206,7 @@ __device__ __noinline__ int l_cyclic_first(const LView* v, int row, int start, b
 //   x = valid | kind<<1 | r1<<3 | r2<<13 | (W[r1][c1]+1)<<23 | (W[r2][c2]+1)<<25
 //   y = c1 | c2<<10 | (v1+1)<<20 | (v2+1)<<22
 //   z = p1 | p2<<10
-// kinds as in xw_anneal.cu: 0 sign flip, 1 support switch, 2 double flip,
+// kinds as in xw_packed.cuh: 0 sign flip, 1 support switch, 2 double flip,
 // 3 within-row swap.  The proposer, which runs in parallel across the
 // candidates, carries the two current entries, so that decoding a move in
 // the serial evaluation and commit needs no dependent load from HBM.
@@ -348,7 +348,7 @@ __device__ __noinline__ LMove l_propose(const LView* v, uint64_t it, int c, bool
     return col < 0 ? none() : lpack(0, row, 0, col, 0, 0, 0, 0, 0, l_at(v, row, col), 0);
 }
 
-// A decoded move as at most two row updates (see xw_anneal.cu)
+// A decoded move as at most two row updates
 struct LUpdate {
     int R1, X1, Y1, A1, B1;
     int R2, X2, Y2, A2, B2;
@@ -756,7 +756,7 @@ __device__ void p_store_w(int8_t* dst, const ulonglong2* P, int n, int lane) {
     }
 }
 
-// tab[d-1] = ceil(exp(-d/T) * 2^32) (see build_thresholds, xw_anneal.cu)
+// tab[d-1] = ceil(exp(-d/T) * 2^32) (see build_thresholds, xw_packed.cuh)
 __device__ __noinline__ void l_thresholds(uint64_t* tab, double T, int lane) {
     const double t = T > 1.0e-12 ? T : 1.0e-12;
     for (uint32_t d = lane + 1; d <= kThrTable; d += 32) {
@@ -1242,7 +1242,7 @@ __global__ void __launch_bounds__(128, FORM != kFormGram ? 2 : XW_LARGE_MIN_BLOC
     const int lane = threadIdx.x & 31;
     const int warp = threadIdx.x >> 5;
     uint8_t* slot = smem + (size_t)warp * a.slot_bytes;
-    // work items as in anneal_kernel (xw_anneal.cu): whole replicas, or
+    // work items as in anneal_kernel (xw_replica.cuh): whole replicas, or
     // chunks of their iterations in chunk-major order
     const uint64_t total = (uint64_t)a.n_items * a.chunks;
     for (;;) {

@@ -173,10 +173,7 @@ __device__ __forceinline__ void release_chunk(uint32_t* flag, uint32_t value, in
 // One chunk of a chunked launch: chunk_begin waits for the replica's
 // previous chunk and says whether this one runs (false: flag the replica,
 // skip); chunk_end publishes this chunk's count, poisoned when it did not
-// run.  Every lane of the replica's lane group `gm` calls both.  (The chunk
-// body is called between them by the kernel itself: wrapping it in a lambda
-// raised the lean kernel's spills from 40 to 412 bytes a thread and made the
-// W(26,25) tempering batch 9% slower on B200.)
+// run.  Every lane of the replica's lane group `gm` calls both.
 __device__ __forceinline__ bool chunk_begin(const uint32_t* done, uint32_t c, uint64_t limit_ns, uint32_t* err,
                                             int lane, unsigned gm) {
     bool ok = true;

@@ -9,13 +9,15 @@
 //
 // each section padded to 16 bytes.  The Gram matrix, the row residuals and
 // the row support masks are not stored: the kernel rebuilds them in shared
-// memory from W when it loads a replica (O(n^3/32) per lane, negligible next
-// to the thousands of moves per launch) and checks the rebuilt score against
-// the tracked one.
+// memory from W when it loads a replica (popcounts of support and sign masks,
+// n^3/32 words over the warp's lanes, negligible next to the thousands of
+// moves per launch) and checks the rebuilt score against the tracked one.
 //
 // Orders above XW_MAX_N keep 16-bit minority lists (n*m u16) and a Gram
-// arena beside the records (int16 G, support and sign masks per replica)
-// that persists between launches; see xw_anneal_large.cu.
+// arena beside the records that persists between launches: in the default
+// form up to order 448 the packed residuals, rows of W as signed nibbles and G
+// in bytes or halfwords (HybridArena, xw_packed.cuh); in the others int16 G
+// with support and sign masks, or bit planes (xw_anneal_large.cu).
 #pragma once
 
 #include <stdint.h>
@@ -28,8 +30,7 @@
 
 #define XW_STATUS_INIT 1u      // record holds incremental state (score etc.)
 #define XW_STATUS_SOLVED 2u    // best score reached 0
-#define XW_STATUS_GRAM 4u      // large orders: the arena holds this W's Gram and masks (or, in
-                               // bit-plane mode, its planes and residuals)
+#define XW_STATUS_GRAM 4u      // large orders: the arena holds what its form keeps of this W
 #define XW_ERR_SCORE 1u        // rebuilt score differs from the tracked one
 #define XW_ERR_MINORITY 2u     // W row weights disagree with the minority lists
 #define XW_ERR_KERNEL 4u       // a lean launch met a replica that needs the general kernel

@@ -1,6 +1,7 @@
 // xw_packed.cuh -- one annealing iteration on packed rows, for orders up to
-// 448: the device code shared by the one-warp replica loop, the latency mode
-// and the large orders' kernel of xw_anneal.cu.
+// 448: the device code shared by the one-warp replica loop (xw_replica.cuh),
+// the latency mode (xw_spec.cuh) and the large orders' kernel
+// (xw_anneal_wide.cu).
 //
 // W and its Gram matrix sit in the replica's shared-memory slot as biased
 // bytes, four rows of a column of W (or four entries of a row of G) to a
@@ -25,16 +26,17 @@
 // over candidates with one row per lane.
 //
 // What bounds it: instruction issue of dependent integer chains (W(26,25)
-// ladder, 10^4 iterations of 4096 replicas: issue slots 71% used, ALU pipe
-// 61%, 375 warp instructions an iteration, 19.5 ms).  Measured on B200
-// against a loop over candidates with one row per lane and a 32-bit Gram
-// matrix (843 instructions, 44.7 ms): packed rows alone 30.5 ms; runs of
-// one-candidate iterations side by side and the constants and the state of
-// accepted moves in shared memory instead of registers 26.9; no calls in
-// the loop (a call keeps what lives across it in few registers: 80 bytes of
-// spills a thread) and round keys from shared memory 19.5.  W(100,50), 592
-// replicas of 1000 iterations: 13.5 -> 5.1 ms (bytes let six warps share an
-// SM instead of three; the lanes try a switch's attempts side by side).
+// ladder, 4096 replicas: issue slots 62% used, ALU pipe 55%, 395 warp
+// instructions an iteration with load and store, 19.2 ms per 10^4 of them).
+// Measured on B200 against a loop over candidates with one row per lane and
+// a 32-bit Gram matrix (838 instructions, 44.7 ms): packed rows alone 30.5
+// ms; runs of one-candidate iterations side by side and the constants and
+// the state of accepted moves in shared memory instead of registers 26.9; no
+// calls in the loop (a call keeps what lives across it in few registers: 80
+// bytes of spills a thread) and round keys from shared memory 19.2.
+// W(100,50), 592 replicas of 1000 iterations: 13.6 -> 5.1 ms (bytes let six
+// warps share an SM instead of three; the lanes try a switch's attempts side
+// by side), 3.7 with the journal of moves since the best W.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -173,6 +175,11 @@ constexpr int kHybridMaxOrder = 448;
 constexpr uint32_t kHybridMino = 8192;
 constexpr uint32_t kNibbleTable = 2048 + 1024;
 constexpr int kByteMax = 123;
+
+// A candidate's two deltas travel in one word, score change + 4096 x conflict
+// change: a move changes at most 2n entries of G by at most 2 each (or n by
+// 4), so the score change of any order here stays below 2048.
+static_assert(4 * kHybridMaxOrder < 2048, "score changes fit half of 4096");
 
 __host__ __device__ constexpr uint32_t hybrid_slot_bytes(int n, int m) {
     const uint32_t mb = (uint32_t)n * (uint32_t)m * 2u;

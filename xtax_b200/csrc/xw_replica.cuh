@@ -149,7 +149,7 @@ __device__ __forceinline__ void run_replica(const AnnealArgs& a, uint32_t rid, u
 // Register budget per thread; it sets how many replica warps an SM holds.
 // An SM's registers are split between its four schedulers (16384 each): 80
 // registers per thread give 6 warps per scheduler, 96 give 5, 112 and 128
-// give 4.  The one-row kernels take the smallest budget without spills:
+// give 4.  The one-row kernels take the smallest budget next to free of spills:
 // measured on B200 (W(26,25) ladder, 4096 replicas, 10^4 iterations) 19.5
 // ms at 96 registers, 20.8 at 112, 21.7 at 80 (180 bytes of spills a
 // thread), 24.1 at 72; the general kernel (W(24,23), 2368 replicas, 4096

@@ -23,15 +23,16 @@ namespace {
 // move; a round advances by the run of rejections up to the next accept
 // (about 2-4 iterations at the acceptance rates of cooling runs) in about
 // the time of one iteration, so a lone search runs that much faster.
-
 //
 // Where moves are accepted every iteration or two a round advances no
 // further than one step of the one-warp loop and takes longer (2000
 // iterations of W(12,11) with its hottest replica accepting all: 3.15 ms in
 // the one-warp loop, 4.1 with 2 warps, 6.1 with 16, 8.2 with 64 on four SMs).
-// So warp 0 watches the advance: below kSoloAdvance iterations a round it
-// goes on alone, step by step, until accepts are rare enough again (in a
-// cluster every CTA's warp 0 makes the same steps on its copy).
+// So warp 0 watches the advance: while a round advances by less than it costs
+// in steps of the one-warp loop (cost10 below, tenths of a step, measured on
+// W(12,11): 2.6 on a cluster, 1.2 + K / 20 on one CTA) it goes on alone, step
+// by step, until accepts are rare enough again (in a cluster every CTA's warp 0
+// makes the same steps on its copy).
 
 // Per-warp results and the round's control word, after the slot's own
 // (warp 0's) structures and the other warps' draw buffers.
