@@ -276,3 +276,26 @@ def test_restarts_at_a_large_order_with_weight_near_half_stay_quick():
     t = [float(line.split("seconds=")[1].split()[0]) for line in restarts]
     assert max(b - a for a, b in zip(t, t[1:])) < 2.0
     assert X.score(512, 256, r.best.entries)[0] == r.best.score
+
+
+@pytest.mark.parametrize("small,n,w", [(False, 257, 256), (False, 258, 5), (False, 259, 130), (False, 260, 259), (False, 271, 271),
+                                       (False, 320, 319), (False, 447, 446), (False, 448, 4), (True, 5, 4), (True, 6, 3),
+                                       (True, 16, 15), (True, 17, 4), (True, 64, 63), (True, 65, 2), (True, 130, 129)])
+def test_rounds_of_a_few_iterations(large_from, small, n, w):
+    """W and G pass from launch to launch through the arena: many launches of
+    two iterations, at orders of every remainder by a word, from the start
+    again after a reset."""
+    if small:
+        large_from(1)
+    p = X.Params(stop_on_solve=0, t_init=3.0, moves_per_launch=2, moves_per_cool=3)
+    batch = X.Batch([{"n": n, "w": w, "seed": 70 + n, "replicas": 2}], p)
+    temps = [batch.replica(0, r)[0].reheat_temperature for r in range(2)]
+    for iters in (21, 14):
+        batch.reset()
+        batch.run(iters)
+        batch.synchronize()
+        for r in range(2):
+            rep = O.Replica(oracle_job(n, w, 70 + n, p), r, start_of(n, w, 70 + n, r, p), temps[r], r)
+            rep.run(iters, stop_on_solve=False)
+            compare(batch, 0, r, rep)
+    batch.close()

@@ -193,8 +193,9 @@ __host__ __device__ constexpr uint32_t hybrid_byte_stride(int n) { return ((uint
 __host__ __device__ constexpr uint32_t hybrid_row_stride(int n) { return (((uint32_t)n + 63u) >> 6) * 32u; }
 
 // The arena of a replica in that form: packed residuals, the rows of W as
-// signed nibbles (used while G is built; then the first word says whether G
-// is in halfwords), G (room for halfwords).
+// signed nibbles (used while G is built; in their place then a word that says
+// whether G is in halfwords and, 16 bytes on, the slot's W for the next
+// launch), G (room for halfwords).
 struct HybridArena {
     uint64_t off_rows, off_g, bytes;
 };
@@ -206,6 +207,16 @@ __host__ __device__ constexpr HybridArena hybrid_arena(int n) {
     A.bytes = A.off_g + (uint64_t)n * hybrid_gram_stride(n);
     return A;
 }
+
+// bytes of the slot's W; it fits the place of the rows
+__host__ __device__ constexpr uint32_t hybrid_w_bytes(int n) { return xw_pad16((uint32_t)n * packed_stride(n, 16)); }
+
+constexpr bool hybrid_w_fits() {
+    for (int n = 1; n <= kHybridMaxOrder; ++n)
+        if (16u + hybrid_w_bytes(n) > (uint32_t)n * hybrid_row_stride(n)) return false;
+    return true;
+}
+static_assert(hybrid_w_fits(), "the slot's W fits the arena's rows");
 
 // Loop-invariant context of a lane of a replica's group.
 struct Env {
@@ -1519,22 +1530,40 @@ __device__ __noinline__ void save_w(int8_t* dst, uint32_t wbase, uint32_t st, in
     const int wpc = (n + 3) >> 2;
     const bool whole = (n & 3) == 0;   // every word of the record is aligned and full
     if constexpr (WPL == 16) {
+        // four entries of column k from nibble pair j: bit i of a nibble to byte i
+        auto entries = [&](int k, int j) -> uint32_t {
+            const uint32_t x = lds8(wbase + (uint32_t)k * st + (uint32_t)j);
+            return (((x & 15u) * 0x00204081u) & 0x01010101u) + (((x >> 4) * 0x00204081u) & 0x01010101u) * 0xfeu;
+        };
+        // the pairs that are whole, a lane each, by the widest store that n aligns
+        auto columns = [&](auto store) {
 #pragma unroll 1
-        for (int j = lane; j < wpc; j += 32) {
+            for (int j = lane; j < (n >> 2); j += 32) {
+                int8_t* d = dst + 4 * j;
 #pragma unroll 4
-            for (int k = 0; k < n; ++k) {
-                // bit i of a nibble to byte i
-                const uint32_t x = lds8(wbase + (uint32_t)k * st + (uint32_t)j);
-                const uint32_t v = (((x & 15u) * 0x00204081u) & 0x01010101u) + (((x >> 4) * 0x00204081u) & 0x01010101u) * 0xfeu;
-                int8_t* d = dst + (uint32_t)(k * n + 4 * j);
-                if (whole) {
-                    *reinterpret_cast<uint32_t*>(d) = v;
-                } else {
-#pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (4 * j + e < n) d[e] = (int8_t)(v >> (8 * e));
-                }
+                for (int k = 0; k < n; ++k, d += n) store(d, entries(k, j));
             }
+        };
+        if (whole) {
+            columns([](int8_t* d, uint32_t v) { *reinterpret_cast<uint32_t*>(d) = v; });
+            return;
+        }
+        if ((n & 1) == 0) {
+            columns([](int8_t* d, uint32_t v) {
+                reinterpret_cast<uint16_t*>(d)[0] = (uint16_t)v;
+                reinterpret_cast<uint16_t*>(d)[1] = (uint16_t)(v >> 16);
+            });
+        } else {
+            columns([](int8_t* d, uint32_t v) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) d[e] = (int8_t)(v >> (8 * e));
+            });
+        }
+        // the last rows, a column a lane
+#pragma unroll 1
+        for (int k = lane; k < n; k += 32) {
+            const uint32_t v = entries(k, n >> 2);
+            for (int e = 0; e < (n & 3); ++e) dst[(uint32_t)(k * n + (n & ~3) + e)] = (int8_t)(v >> (8 * e));
         }
         return;
     }
@@ -1998,9 +2027,18 @@ __device__ __forceinline__ bool build_hybrid(const Env& E, const XwJob* J, const
     const bool cached = status0 & XW_STATUS_GRAM;
     int bad = 0;
     if (n > kHybridMaxOrder) return false;
+    if (cached) {
+        // the slot's W as the last launch left it (made from the record's bytes
+        // again, and stored with a test on each byte, a launch of one iteration
+        // of W(276,275) took 178 us and one of W(286,265) 379; 36 and 51 so)
+        const uint4* src = reinterpret_cast<const uint4*>(arena + hybrid_arena(n).off_rows + 16u);
+        const int chunks = (int)(hybrid_w_bytes(n) / 16u);
+#pragma unroll 8
+        for (int i = lane; i < chunks; i += 32) reinterpret_cast<uint4*>(xw_smem + wbase)[i] = __ldcg(src + i);
+    }
     const bool whole = (n & 3) == 0;   // every word of the record is aligned and full
 #pragma unroll 1
-    for (int q = lane; q < (int)st; q += 32) {
+    for (int q = cached ? (int)st : lane; q < (int)st; q += 32) {
         const bool word = whole && 4 * q < n;
 #pragma unroll 1
         for (int c0 = 0; c0 < n; c0 += 4) {
@@ -2215,6 +2253,9 @@ __device__ __forceinline__ void store_replica(const AnnealArgs& a, const Env& E,
         if (lane == 0)
             *reinterpret_cast<uint32_t*>(a.gram + a.gram_off[con->rid] + hybrid_arena(E.n).off_rows) = con->halves ? 1u : 0u;
         for (int o = lane; o < E.n; o += GW) res[o] = reinterpret_cast<const int*>(xw_smem + E.slot + Slot<WPL>::res)[o];
+        uint4* keep = reinterpret_cast<uint4*>(a.gram + a.gram_off[con->rid] + hybrid_arena(E.n).off_rows + 16u);
+        for (int i = lane; i < (int)(hybrid_w_bytes(E.n) / 16u); i += GW)
+            keep[i] = *reinterpret_cast<const uint4*>(xw_smem + wbase + 16u * (uint32_t)i);
     } else {
         uint8_t* gmo = rec + J->off_mino;
         for (uint32_t i = lane; i < (uint32_t)(E.n * E.m); i += GW) gmo[i] = xw_smem[E.mino + i];
