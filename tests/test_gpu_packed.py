@@ -180,3 +180,14 @@ def test_a_certain_sign_flip_is_never_a_row_swap(n, w, kw):
                                     (40, 20, {}), (100, 99, {}), (140, 70, {})], ids=str)
 def test_long_tournaments_that_few_candidates_need(n, w, kw, ts, target):
     replay(n, w, 2, 250 if n < 100 else 60, 8 * n + ts, target_samples=ts, target_fraction=target, **kw)
+
+
+@pytest.mark.parametrize("wpr", [6, 16, 32, 64])
+@pytest.mark.parametrize("mpc,stuck,launch", [(m, 10 ** 6, 64) for m in (1, 6, 16, 64)] +
+                         [(500, 12, 50), (500, 64, 100), (7, 13, 6), (500, 50000, 1)])
+def test_latency_mode_with_steps_at_the_ends_of_rounds(wpr, mpc, stuck, launch):
+    # a cold replica, whose rounds are mostly rejections: cooling steps,
+    # reheats and launch ends that fall on a round's last call, before it and
+    # after it
+    replay(12, 11, 2, 400, 9, warps_per_replica=wpr, t_init=0.4, t_min=0.2, cooling=0.99, reheat=1.5, moves_per_cool=mpc,
+           stuck_threshold=stuck, moves_per_launch=launch)

@@ -187,9 +187,9 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
         if (warp == 0) {
             // Iterations in order until the first accepted move.  Fast path:
             // the rejected calls before it change only counters unless one
-            // of them reaches a cooling or reheat step, so when none can,
-            // they are counted in bulk and only the accepted move is
-            // committed.  Otherwise the ordered walk.
+            // of them reaches a cooling or reheat step before the span's last
+            // call, so when none can, they are counted in bulk and only the
+            // accepted move is committed.  Otherwise the ordered walk.
             // The job's solved flag: read here on one CTA, as the owner read
             // it this round on a cluster.
             auto solved = [&]() -> bool {
@@ -214,8 +214,9 @@ __device__ void run_replica_spec(const AnnealArgs& a, uint32_t rid, int warp, in
                                    ((uint64_t)__ballot_sync(FULL, l1 && outs[l1 ? 32 + lane : 0].acc != 0) << 32);
             const int ja = acc_m ? __ffsll((long long)acc_m) - 1 : -1;
             const int jend = ja >= 0 ? ja + 1 : cnt;
-            const int rejects = ja >= 0 ? jend - 1 : jend;
-            bool fast = rejects < k_evt - k;
+            // (a step due at the span's last call, as the launch's end often
+            // is, comes after it)
+            bool fast = jend <= k_evt - k;
             // a check of the job's solved flag (every 64th iteration) that
             // falls in the span and finds it set: take the span in order
             if (fast && a.stop_on_solve == 1 && (k | 63) < k + jend && solved()) fast = false;
