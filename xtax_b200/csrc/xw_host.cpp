@@ -156,7 +156,7 @@ int large_min_order() {
 
 // The large orders' form where W fits a warp's slot (n <= 448): by default
 // 2, W in shared memory with the Gram matrix in HBM (W(276,275) x 2368 on
-// B200: 210 M moves/s against 69 M for form 0 and 60 M for form 1);
+// B200: 218 M moves/s against 69 M for form 0 and 60 M for form 1);
 // XW_LARGE_PLANES=0 the Gram matrix and masks in HBM (the form of larger
 // orders), 1 bit planes with every Gram entry recomputed (no Gram matrix: a
 // quarter of the device memory per replica at n = 276, and no HBM traffic per
